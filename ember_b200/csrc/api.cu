@@ -68,7 +68,7 @@ int ember_attention_fwd(const void *q, const void *k, const void *v, void *out, 
     a.scale = scale; a.causal = causal ? 1 : 0; a.dtype = dtype;
     cudaStream_t s = pick_stream(stream, st);
     if (sm100_fwd_supported(a)) return sm100_attention_fwd(a, st, s);
-    return simt_attention_fwd(a, s);
+    return simt_attention_fwd(a, st, s);
 }
 
 int ember_attention_bwd(const void *q, const void *k, const void *v, const void *out, const float *lse,
@@ -100,7 +100,7 @@ int ember_attention_bwd(const void *q, const void *k, const void *v, const void 
         float *acc = det ? nullptr : (float *)((char *)workspace + delta_bytes(batch_heads, lq));
         return sm100_attention_bwd(a, (float *)workspace, acc, det, st, s);
     }
-    return simt_attention_bwd(a, (float *)workspace, s);
+    return simt_attention_bwd(a, (float *)workspace, st, s);
 }
 
 int ember_set_deterministic(int on)

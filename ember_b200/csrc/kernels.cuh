@@ -20,8 +20,8 @@ struct AttnArgs {
 };
 
 // CUDA-core kernels (attn_simt.cu): float32 math, f32 or bf16 storage, d <= 128.
-int simt_attention_fwd(const AttnArgs &a, cudaStream_t s);
-int simt_attention_bwd(const AttnArgs &a, float *delta, cudaStream_t s);
+int simt_attention_fwd(const AttnArgs &a, DeviceState *st, cudaStream_t s);
+int simt_attention_bwd(const AttnArgs &a, float *delta, DeviceState *st, cudaStream_t s);
 int launch_delta(const AttnArgs &a, float *delta, cudaStream_t s);
 
 // tcgen05 kernels (attn_fwd_sm100.cu / attn_bwd_sm100.cu): bf16 storage, d in {64, 128}.
