@@ -99,6 +99,9 @@ int column_sums(const MatView &a, void *out, int dtype, cudaStream_t s);  // out
 // tcgen05 kernel (gemm_sm100.cu): bf16 storage; see sm100_gemm_supported for the shapes it takes.
 bool sm100_gemm_supported(const GemmArgs &g);
 int sm100_gemm(const GemmArgs &g, DeviceState *st, cudaStream_t s);
+// tcgen05 kernel for at most 128 rows (gemm_skinny_sm100.cu): a decode step's projections.
+bool sm100_skinny_gemm_supported(const GemmArgs &g);
+int sm100_skinny_gemm(const GemmArgs &g, DeviceState *st, cudaStream_t s);
 int make_tensor_map_bf16_view(CUtensorMap *map, const MatView &v, uint32_t box_cols, uint32_t box_rows);
 
 }  // namespace ember

@@ -45,6 +45,7 @@ MatView view(const void *p, long long rows, int cols, int heads, const LinearSha
 
 int run(const GemmArgs &g, DeviceState *st, cudaStream_t s)
 {
+    if (sm100_skinny_gemm_supported(g)) return sm100_skinny_gemm(g, st, s);
     if (sm100_gemm_supported(g)) return sm100_gemm(g, st, s);
     return simt_gemm(g, s);
 }
@@ -129,7 +130,7 @@ const char *ember_linear_kernel_name(int product, long long m, int n, int k, int
         g.a = view(p, m, k, x_heads, sh); g.b = view(p, k, n, 0, sh); g.c = view(p, m, n, y_heads, sh);
         g.m = m; g.n = n; g.k = k;
     }
-    return sm100_gemm_supported(g) ? "sm100_tcgen05" : "simt_f32";
+    return sm100_skinny_gemm_supported(g) || sm100_gemm_supported(g) ? "sm100_tcgen05" : "simt_f32";
 }
 
 }  // extern "C"

@@ -1,0 +1,48 @@
+"""Linear layers with few rows, few columns or a short contraction (decode steps, classifier heads),
+against the CPU oracle: edges of the tiles, contractions that do not fill the splits, one row, one
+column, head-major operands of sequences of length 1.
+
+Tolerances: float32 results are sums of up to k products of order one in another order than the
+oracle's double accumulation: sqrt(k) * 2^-24 of the terms, held to 1e-5 of the largest result.
+bfloat16: half a unit in the last place of the result (2^-9) plus the same sum's rounding."""
+import numpy as np
+import pytest
+
+import ember_b200 as em
+from conftest import bf16_round, seeded
+from oracle import cpu_oracle
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [(1, 8, 8), (1, 136, 64), (8, 6144, 256), (16, 128, 2048), (17, 520, 72), (33, 72, 1000), (64, 64, 64), (65, 200, 136),
+          (100, 384, 200), (128, 2056, 328), (129, 40, 24), (256, 10, 784), (300, 1, 50), (7, 33, 5), (40, 1000, 10), (513, 17, 640),
+          (200, 200, 200)]
+
+
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+@pytest.mark.parametrize("m,n,k", SHAPES)
+def test_forward_and_backward(m, n, k, dtype):
+    rnd = bf16_round if dtype == "bfloat16" else (lambda a: a)
+    x, w, b, g = rnd(seeded((m, k), 1)), rnd(seeded((k, n), 2)), rnd(seeded((n,), 3)), rnd(seeded((m, n), 4))
+    tx, tw, tb, tg = (em.Tensor(a, dtype) for a in (x, w, b, g))
+    got = (em.linear_forward(tx, tw, tb), *em.linear_backward(tx, tw, tg))
+    ref = (cpu_oracle.linear_fwd(x, w, b), *cpu_oracle.linear_bwd(x, w, g))
+    tol = 2.0 ** -8 if dtype == "bfloat16" else 1e-5
+    for name, a, r in zip(("y", "grad_x", "grad_w", "grad_b"), got, ref):
+        assert np.abs(a.to_np() - r).max() <= tol * np.abs(r).max(), name
+
+
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+@pytest.mark.parametrize("batch,heads,dim", [(1, 2, 64), (9, 3, 64), (32, 4, 128)])
+def test_head_major_rows_of_single_positions(batch, heads, dim, dtype):
+    rnd = bf16_round if dtype == "bfloat16" else (lambda a: a)
+    e = heads * dim
+    x, w, b = rnd(seeded((batch, 1, e), 1)), rnd(seeded((e, 3 * e), 2)), rnd(seeded((3 * e,), 3))
+    o, wo = rnd(seeded((batch, heads, 1, dim), 4)), rnd(seeded((e, e), 5))
+    tol = 2.0 ** -8 if dtype == "bfloat16" else 1e-5
+    y = em.linear_forward(em.Tensor(x, dtype), em.Tensor(w, dtype), em.Tensor(b, dtype), y_heads=heads).to_np()
+    r = cpu_oracle.linear_fwd(x.reshape(batch, e), w, b).reshape(batch, 1, 3, heads, dim).transpose(2, 0, 3, 1, 4)
+    assert y.shape == r.shape and np.abs(y - r).max() <= tol * np.abs(r).max()
+    y = em.linear_forward(em.Tensor(o, dtype), em.Tensor(wo, dtype), None, x_heads=heads).to_np()
+    r = cpu_oracle.linear_fwd(o.reshape(batch, e), wo, None).reshape(batch, 1, e)
+    assert np.abs(y - r).max() <= tol * np.abs(r).max()
