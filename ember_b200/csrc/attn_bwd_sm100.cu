@@ -1388,7 +1388,8 @@ int launch_fused(const AttnArgs &a, float *delta, float *dq_acc, DeviceState *st
     p.scale_log2 = a.scale * LOG2E_B;
     p.status = st->status;
     auto k1 = sm100_bwd_fused_kernel<HD>;
-    EMBER_CUDA_TRY(cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
+    static SmemOptIn opt_in1;
+    EMBER_CUDA_TRY(opt_in1(k1, C::SMEM_BYTES));
     const size_t touched = ((size_t)a.lq + a.lk) * HD * 2 * 4 + (size_t)a.lq * HD * 4;  // + the float32 dQ accumulator
     p.order = make_work_order(a.bh, (a.lk + 127) / 128, st->sm_count, touched, a.causal != 0);
     cudaLaunchAttribute pdl[1];
@@ -1435,8 +1436,10 @@ int launch(const AttnArgs &a, float *delta, DeviceState *st, cudaStream_t s)
     p.status = st->status;
     auto k1 = sm100_bwd_dkdv_kernel<HD>;
     auto k2 = sm100_bwd_dq_kernel<HD>;
-    EMBER_CUDA_TRY(cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
-    EMBER_CUDA_TRY(cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
+    static SmemOptIn opt_in1;
+    EMBER_CUDA_TRY(opt_in1(k1, C::SMEM_BYTES));
+    static SmemOptIn opt_in2;
+    EMBER_CUDA_TRY(opt_in2(k2, C::SMEM_BYTES));
     const size_t touched = ((size_t)a.lq + a.lk) * HD * 2 * 4;  // Q, dO, dQ, K, V, dK, dV and the row vectors
     p.order = make_work_order(a.bh, (a.lk + 127) / 128, st->sm_count, touched, a.causal != 0);
     k1<<<dim3((unsigned)(p.order.units * p.order.blocks)), BWD_THREADS, C::SMEM_BYTES, s>>>(tq, tk, tv, tdo, p);

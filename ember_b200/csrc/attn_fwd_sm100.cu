@@ -617,7 +617,8 @@ int launch_pair(const AttnArgs &a, DeviceState *st, cudaStream_t s)
     p.lens_div = 1;
     p.seq_lens = nullptr;
     auto kern = sm100_fwd_kernel<HD, EMU, true>;
-    EMBER_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
+    static SmemOptIn opt_in;
+    EMBER_CUDA_TRY(opt_in(kern, C::SMEM_BYTES));
     // a work item is a 512-row block of one unit, taken by one pair of CTAs
     p.order = make_work_order(a.bh, (a.lq + 511) / 512, st->sm_count / 2, ((size_t)a.lq + a.lk) * HD * 2 * 2, a.causal != 0);
     cudaLaunchConfig_t cfg = {};
@@ -694,7 +695,8 @@ int launch(const AttnArgs &a, DeviceState *st, cudaStream_t s)
     p.lens_div = 1;
     p.seq_lens = nullptr;
     auto kern = sm100_fwd_kernel<HD, EMU, false>;
-    EMBER_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
+    static SmemOptIn opt_in;
+    EMBER_CUDA_TRY(opt_in(kern, C::SMEM_BYTES));
     p.order = make_work_order(a.bh, (a.lq + p.block_rows - 1) / p.block_rows, st->sm_count, ((size_t)a.lq + a.lk) * HD * 2 * 2,  // Q, O, K, V
                               a.causal != 0);
     dim3 grid((unsigned)(p.order.units * p.order.blocks));
@@ -760,7 +762,8 @@ int launch_cache_decode(const CacheDecodeArgs &a, DeviceState *st, cudaStream_t 
     p.seq_lens = a.seq_lens;
     p.order = make_work_order(units * a.splits, 1, st->sm_count, 1, false);
     auto kern = sm100_fwd_kernel<HD, 1, false>;
-    EMBER_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
+    static SmemOptIn opt_in;
+    EMBER_CUDA_TRY(opt_in(kern, C::SMEM_BYTES));
     kern<<<(unsigned)(units * a.splits), FWD_THREADS, C::SMEM_BYTES, s>>>(tq, tk, tv, p);
     EMBER_CUDA_TRY(cudaGetLastError());
     if (split) {

@@ -467,7 +467,8 @@ int launch_fwd(const AttnArgs &a, cudaStream_t s)
     constexpr int BM = 8 * R;
     const size_t smem = (size_t)(BM + 2 * TN) * DPAD * 4 + BM * TN * 4;
     auto kern = simt_fwd_kernel<T, FAST, DPAD, R>;
-    EMBER_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    static SmemOptIn opt_in;
+    EMBER_CUDA_TRY(opt_in(kern, smem));
     SimtFwd p = {a.q, a.k, a.v, a.out, a.lse, a.bh, a.lq, a.lk, a.d, a.causal, (a.lq + BM - 1) / BM, a.scale * LOG2E_S};
     const long long grid = (long long)p.bh * p.blocks;
     if (grid > 0x7fffffffLL) return too_many_blocks();
@@ -482,7 +483,8 @@ int launch_bwd(const AttnArgs &a, const float *delta, cudaStream_t s)
     constexpr int BM = 8 * R;
     const size_t smem = (size_t)(2 * BM + 2 * TN) * DPAD * 4 + BM * TN * 4 + 512;
     auto kern = simt_bwd_kernel<T, FAST, DPAD, R>;
-    EMBER_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    static SmemOptIn opt_in;
+    EMBER_CUDA_TRY(opt_in(kern, smem));
     SimtBwd p = {a.q, a.k, a.v, a.dout, a.lse, delta, a.dq, a.dk, a.dv, a.bh, a.lq, a.lk, a.d, a.causal,
                  (a.lk + BM - 1) / BM, (a.lq + BM - 1) / BM, a.scale};
     const long long grid = (long long)p.bh * ((long long)p.kblocks + p.qblocks);

@@ -7,6 +7,8 @@
 #include <stdint.h>
 #include <stdio.h>
 
+#include <atomic>
+
 #include "../../include/ember_b200.h"
 
 namespace ember {
@@ -35,6 +37,25 @@ DeviceState *device_state();
 
 void set_error(const char *fmt, ...);
 int cuda_fail(cudaError_t e, const char *what);
+
+// Raises a kernel's dynamic shared-memory limit once per device instead of on every launch (the call
+// takes about as long as a quarter of a launch). One static SmemOptIn per kernel, at the launch site;
+// setting the same value twice from two threads is harmless.
+struct SmemOptIn {
+    std::atomic<unsigned long long> devices{0};  // bit d: done on device d
+    template <typename K>
+    cudaError_t operator()(K *kern, size_t bytes)
+    {
+        int dev = 0;
+        cudaError_t e = cudaGetDevice(&dev);
+        if (e != cudaSuccess) return e;
+        const unsigned long long bit = 1ull << (dev & 63);
+        if (devices.load(std::memory_order_acquire) & bit) return cudaSuccess;
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        if (e == cudaSuccess) devices.fetch_or(bit, std::memory_order_release);
+        return e;
+    }
+};
 
 inline cudaStream_t pick_stream(void *stream, DeviceState *st)
 {

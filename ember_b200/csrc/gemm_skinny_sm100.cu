@@ -206,7 +206,8 @@ int launch_mp(const GemmArgs &g, DeviceState *st, cudaStream_t s)
     while (splits < MAX_SPLIT && tiles * splits * 2 <= 2 * sms && kblocks >= splits * 4) splits *= 2;
     SkinnyParams p = {(int)g.m, g.n, g.k, splits, g.c, (const __nv_bfloat16 *)g.bias, st->status};
     auto kern = skinny_gemm_kernel<MP, TRANS_W>;
-    EMBER_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
+    static SmemOptIn opt_in;
+    EMBER_CUDA_TRY(opt_in(kern, C::SMEM_BYTES));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(tiles * splits));
     cfg.blockDim = dim3(THREADS);

@@ -344,7 +344,8 @@ int launch(const GemmArgs &g, DeviceState *st, cudaStream_t s)
     p.bias = (const __nv_bfloat16 *)g.bias;
     p.status = st->status;
     auto kern = sm100_gemm_kernel<MODE>;
-    EMBER_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+    static SmemOptIn opt_in;
+    EMBER_CUDA_TRY(opt_in(kern, SMEM_BYTES));
     const long long tiles = (long long)p.tiles_m * p.tiles_n;
     const int sms = st->sm_count > 0 ? st->sm_count : 148;
     const int pairs = (int)(tiles < sms / 2 ? tiles : sms / 2);

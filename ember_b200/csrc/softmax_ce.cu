@@ -403,7 +403,8 @@ int launch_rows(const T *x, const T *target, T *y, float *row_loss, long long ro
 #define EMBER_LAUNCH_ROWS(W, VEC)                                                                               \
     do {                                                                                                        \
         auto kern = row_softmax_kernel<T, W, MODE, VEC>;                                                        \
-        EMBER_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));     \
+        static SmemOptIn opt_in; /* the size varies with the row: the largest any row needs */                   \
+        EMBER_CUDA_TRY(opt_in(kern, 128 + CACHE_BYTES));                                                        \
         kern<<<grid, block, smem, s>>>(x, target, y, row_loss, rows, cols, cache_elems);                         \
     } while (0)
     if (width == 32) {

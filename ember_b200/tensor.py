@@ -21,8 +21,11 @@ import numpy as np
 from . import _core
 
 _DT = {"float32": _core.F32, "bfloat16": _core.BF16}
+_new = object.__new__
 
 
+# Shape products use math.prod throughout: np.prod converts the tuple to an array first and takes 4 us, as
+# long as launching a kernel; a step of a decode loop makes a dozen such products.
 class Tensor:
     """A contiguous device tensor of float32 or bfloat16 elements."""
 
@@ -36,14 +39,13 @@ class Tensor:
 
     @classmethod
     def _from_core(cls, core, shape, dtype: str) -> "Tensor":
-        t = cls.__new__(cls)
+        t = _new(cls)
         t.shape, t.dtype, t._core = tuple(shape), dtype, core
         return t
 
     @classmethod
     def empty(cls, shape, dtype: str = "float32") -> "Tensor":
-        n = int(np.prod(shape, dtype=np.int64)) if len(shape) else 1
-        return cls._from_core(_core._Tensor(n, _DT[dtype]), shape, dtype)
+        return cls._from_core(_core._Tensor(math.prod(map(int, shape)), _DT[dtype]), shape, dtype)
 
     @classmethod
     def from_np(cls, arr, dtype: str = "float32") -> "Tensor":
@@ -51,7 +53,7 @@ class Tensor:
 
     @property
     def size(self) -> int:
-        return int(np.prod(self.shape, dtype=np.int64)) if len(self.shape) else 1
+        return math.prod(map(int, self.shape))
 
     @property
     def ptr(self) -> int:
@@ -61,8 +63,7 @@ class Tensor:
     def view(self, offset: int, shape) -> "Tensor":
         """A tensor of the given shape over this tensor's elements from ``offset`` on (no copy; the
         view keeps the memory alive)."""
-        n = int(np.prod(shape, dtype=np.int64)) if len(shape) else 1
-        return Tensor._from_core(self._core._view(int(offset), n), shape, self.dtype)
+        return Tensor._from_core(self._core._view(int(offset), math.prod(map(int, shape))), shape, self.dtype)
 
     def to_bf16(self) -> "Tensor":
         return Tensor._from_core(_core._convert(self._core, _core.BF16), self.shape, "bfloat16")
@@ -94,7 +95,7 @@ def _check_qkv(q, k, v, fn):
         raise TypeError(f"{fn}: q, k and v must share a dtype, got {q.dtype}, {k.dtype}, {v.dtype}")
     lead = q.shape[:-2]
     heads = lead[-1] if lead else 1
-    batch = int(np.prod(lead[:-1], dtype=np.int64)) if len(lead) > 1 else 1
+    batch = math.prod(lead[:-1])
     return batch, heads, q.shape[-2], k.shape[-2], q.shape[-1]
 
 
