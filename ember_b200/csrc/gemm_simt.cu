@@ -4,6 +4,7 @@
 // kernel does not take. Also the column sums that give the bias gradient.
 #include "common.cuh"
 #include "kernels.cuh"
+#include "ptx.cuh"
 
 namespace ember {
 
@@ -14,54 +15,215 @@ __device__ __forceinline__ float ld(const __nv_bfloat16 *p, size_t i) { return _
 __device__ __forceinline__ void st(float *p, size_t i, float v) { p[i] = v; }
 __device__ __forceinline__ void st(__nv_bfloat16 *p, size_t i, float v) { p[i] = __float2bfloat16_rn(v); }
 
-constexpr int TS = 64, TK = 16;  // 64 x 64 output tile, K in steps of 16; 16 x 16 threads, 4 x 4 results each
+// Matrix products on the FMA pipe. A block owns a TM x TN tile of the result and walks the contraction in
+// slabs of KG * KD; its 256 threads are KG groups, each of which multiplies its own KD rows of every slab
+// over the whole tile, 8 x 8 results per thread: 2 + 2 shared-memory loads of 16 bytes for 32 packed FMAs.
+//   128 x 128, KG = 1   enough tiles to fill the SMs
+//    64 x  64, KG = 4
+//    32 x  32, KG = 16  small results: one slab is 128 deep (32 for the shortest contractions), so a contraction of 784 is 7 rounds of loads
+//                       instead of the 49 of a 64 x 64 tile with 16-deep steps
+// and when even the 32 x 32 tiles leave SMs idle, a cluster of up to 8 blocks splits the contraction and adds
+// the partial tiles in rank order through distributed shared memory. The partial sums of the groups are added
+// in a fixed order too, so results repeat bit for bit.
+// Slabs lie k-major in shared memory; the next one is loaded into registers while this one is multiplied.
+using ptx::f32x2;
 
-template <typename T, int MODE>
-__global__ void __launch_bounds__(256) simt_gemm_kernel(MatView a, MatView b, MatView c, const T *bias, long long m, int n,
-                                                        int k)
-{
-    __shared__ float as[TK][TS + 1], bs[TK][TS + 1];
-    const T *ap = (const T *)a.ptr, *bp = (const T *)b.ptr;
-    const long long m0 = (long long)blockIdx.y * TS;
-    const int n0 = blockIdx.x * TS;
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-    float acc[4][4] = {};
-    for (int k0 = 0; k0 < k; k0 += TK) {
-        for (int e = threadIdx.x; e < TS * TK; e += 256) {
-            const int kk = e % TK, ii = e / TK;
-            const long long gi = m0 + ii;
-            const int gk = k0 + kk, gj = n0 + ii;
-            float av = 0.f, bv = 0.f;
-            if (gi < m && gk < k) av = (MODE == GEMM_TN) ? ld(ap, view_offset(a, gk, (int)gi)) : ld(ap, view_offset(a, gi, gk));
-            if (gj < n && gk < k) bv = (MODE == GEMM_NT) ? ld(bp, view_offset(b, gj, gk)) : ld(bp, view_offset(b, gk, gj));
-            as[kk][ii] = av;
-            bs[kk][ii] = bv;
+template <int TM_, int TN_, int KD_>
+struct Tile {
+    static constexpr int TM = TM_, TN = TN_, KD = KD_;
+    static constexpr int GT = (TM / 8) * (TN / 8), KG = 256 / GT, SLAB = KG * KD;  // threads per group, groups, slab depth
+    static constexpr int PA = TM + 4, PB = TN + 4;                                   // padded rows of the slabs
+    static constexpr int UA = TM * SLAB / 4 / 256, UB = TN * SLAB / 4 / 256;          // 4-element loads per thread and slab
+    static constexpr int SLAB_FLOATS = SLAB * (PA + PB);
+    static constexpr int PITCH = TN + 4, PART = TM * PITCH;                           // a group's partial tile
+    static constexpr int FLOATS = KG > 1 && KG * PART > SLAB_FLOATS ? KG * PART : SLAB_FLOATS;
+    static_assert(UA >= 1 && UB >= 1 && GT * KG == 256, "");
+};
+
+// One 4-element load of an operand. KC: the contraction runs along memory (rows of the view are tile rows);
+// otherwise the tile's rows do. FAST: float32, 16-byte pieces that lie inside a row or head and are aligned.
+template <typename T, bool KC, bool FAST, int EXT>
+struct Operand {
+    static __device__ __forceinline__ void coords(int u, int &mn, int &kk)
+    {
+        if constexpr (KC) {
+            mn = u % EXT;
+            kk = u / EXT * 4;
+        } else {
+            mn = u % (EXT / 4) * 4;
+            kk = u / (EXT / 4);
         }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < TK; kk++) {
-            float ar[4], br[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                ar[i] = as[kk][ty * 4 + i];
-                br[i] = bs[kk][tx * 4 + i];
-            }
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-#pragma unroll
-                for (int j = 0; j < 4; j++) acc[i][j] = fmaf(ar[i], br[j], acc[i][j]);
-        }
-        __syncthreads();
     }
+    static __device__ __forceinline__ float4 load(const MatView &v, long long mn, int kk, long long mn_end, int k_end)
+    {
+        const T *p = (const T *)v.ptr;
+        const long long row = KC ? mn : kk, row_end = KC ? mn_end : k_end;
+        const long long col = KC ? kk : mn, col_end = KC ? k_end : mn_end;
+        float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (row >= row_end) return r;
+        if constexpr (FAST) {
+            if (col < col_end) r = *reinterpret_cast<const float4 *>(p + view_offset(v, row, (int)col));
+        } else {
+            if (col < col_end) r.x = ld(p, view_offset(v, row, (int)col));
+            if (col + 1 < col_end) r.y = ld(p, view_offset(v, row, (int)col + 1));
+            if (col + 2 < col_end) r.z = ld(p, view_offset(v, row, (int)col + 2));
+            if (col + 3 < col_end) r.w = ld(p, view_offset(v, row, (int)col + 3));
+        }
+        return r;
+    }
+    static __device__ __forceinline__ void store(float *slab, int pitch, int mn, int kk, const float4 &r)
+    {
+        if constexpr (KC) {
+            slab[kk * pitch + mn] = r.x;
+            slab[(kk + 1) * pitch + mn] = r.y;
+            slab[(kk + 2) * pitch + mn] = r.z;
+            slab[(kk + 3) * pitch + mn] = r.w;
+        } else {
+            *reinterpret_cast<float4 *>(slab + kk * pitch + mn) = r;
+        }
+    }
+};
+
+__device__ __forceinline__ float4 ld_cluster4(uint32_t addr)
+{
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+    return v;
+}
+
+template <typename T, int MODE, bool FA, bool FB, typename C>
+__global__ void __launch_bounds__(256, 2) simt_gemm_kernel(const MatView a, const MatView b, const MatView c, const T *bias,
+                                                        const long long m, const int n, const int k, const int tiles_n,
+                                                        const int splits)
+{
+    using OA = Operand<T, MODE != GEMM_TN, FA, C::TM>;
+    using OB = Operand<T, MODE == GEMM_NT, FB, C::TN>;
+    extern __shared__ __align__(16) float sm[];
+    float *as = sm, *bs = sm + C::SLAB * C::PA;
+    const int rank = splits > 1 ? (int)ptx::cluster_ctarank() : 0;
+    const int tile = blockIdx.x / splits;
+    const long long m0 = (long long)(tile / tiles_n) * C::TM;
+    const int n0 = (tile % tiles_n) * C::TN;
+    const int slabs = (k + C::SLAB - 1) / C::SLAB;
+    const int s0 = (int)((long long)slabs * rank / splits), s1 = (int)((long long)slabs * (rank + 1) / splits);
+    const int group = threadIdx.x / C::GT, t = threadIdx.x % C::GT;
+    const int tx = t % (C::TN / 8), ty = t / (C::TN / 8);
+
+    f32x2 acc[8][4];
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc[i][j] = 0;
+    float4 ra[C::UA], rb[C::UB];
+    auto fetch = [&](int slab) {
+        const int k0 = slab * C::SLAB;
+#pragma unroll
+        for (int i = 0; i < C::UA; i++) {
+            int mn, kk;
+            OA::coords(threadIdx.x + i * 256, mn, kk);
+            ra[i] = OA::load(a, m0 + mn, k0 + kk, m, k);
+        }
+#pragma unroll
+        for (int i = 0; i < C::UB; i++) {
+            int mn, kk;
+            OB::coords(threadIdx.x + i * 256, mn, kk);
+            rb[i] = OB::load(b, n0 + mn, k0 + kk, n, k);
+        }
+    };
+    if (s0 < s1) fetch(s0);
+    for (int slab = s0; slab < s1; slab++) {
+        if (slab != s0) __syncthreads();
+#pragma unroll
+        for (int i = 0; i < C::UA; i++) {
+            int mn, kk;
+            OA::coords(threadIdx.x + i * 256, mn, kk);
+            OA::store(as, C::PA, mn, kk, ra[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < C::UB; i++) {
+            int mn, kk;
+            OB::coords(threadIdx.x + i * 256, mn, kk);
+            OB::store(bs, C::PB, mn, kk, rb[i]);
+        }
+        __syncthreads();
+        if (slab + 1 < s1) fetch(slab + 1);
+        const float *ga = as + group * C::KD * C::PA + ty * 4, *gb = bs + group * C::KD * C::PB + tx * 4;
+#pragma unroll
+        for (int kk = 0; kk < C::KD; kk++) {
+            // rows ty*4 + {0..3} and TM/2 + the same, columns likewise: 16-byte loads, no bank conflicts
+            const float4 a0 = *reinterpret_cast<const float4 *>(ga + kk * C::PA), a1 = *reinterpret_cast<const float4 *>(ga + kk * C::PA + C::TM / 2);
+            const ulonglong2 b0 = *reinterpret_cast<const ulonglong2 *>(gb + kk * C::PB), b1 = *reinterpret_cast<const ulonglong2 *>(gb + kk * C::PB + C::TN / 2);
+            const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+            const f32x2 bv[4] = {b0.x, b0.y, b1.x, b1.y};
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const f32x2 aa = ptx::pack2(av[i], av[i]);
+#pragma unroll
+                for (int j = 0; j < 4; j++) acc[i][j] = ptx::fma2(aa, bv[j], acc[i][j]);
+            }
+        }
+    }
+    auto row_of = [&](int i) { return (i / 4) * (C::TM / 2) + ty * 4 + i % 4; };
+    auto col_of = [&](int j) { return (j / 2) * (C::TN / 2) + tx * 4 + (j % 2) * 2; };
+
     T *cp = (T *)c.ptr;
+    if constexpr (C::KG == 1) {
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const long long gi = m0 + ty * 4 + i;
-        if (gi >= m) continue;
+        for (int i = 0; i < 8; i++) {
+            const long long gi = m0 + row_of(i);
+            if (gi >= m) continue;
+            const size_t row_off = view_offset(c, gi, 0);  // rows and columns of a view address independently
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int gj = n0 + tx * 4 + j;
-            if (gj < n) st(cp, view_offset(c, gi, gj), acc[i][j] + (bias ? ld(bias, (size_t)gj) : 0.f));
+            for (int j = 0; j < 4; j++) {
+                float v[2];
+                ptx::unpack2(acc[i][j], v[0], v[1]);
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const int gj = n0 + col_of(j) + h;
+                    if (gj < n) st(cp, row_off + view_offset(c, 0, gj), v[h] + (bias ? ld(bias, (size_t)gj) : 0.f));
+                }
+            }
+        }
+    } else {
+        // Every group leaves its partial tile in shared memory; then all 256 threads add them, group 0 first.
+        __syncthreads();
+        float *mine = sm + group * C::PART;
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) *reinterpret_cast<f32x2 *>(mine + row_of(i) * C::PITCH + col_of(j)) = acc[i][j];
+        __syncthreads();
+        auto store4 = [&](int e, const float4 &s) {
+            const long long gi = m0 + e / (C::TN / 4);
+            const int gj = n0 + e % (C::TN / 4) * 4;
+            if (gi >= m) return;
+            const size_t row_off = view_offset(c, gi, 0);
+            const float v[4] = {s.x, s.y, s.z, s.w};
+#pragma unroll
+            for (int h = 0; h < 4; h++)
+                if (gj + h < n) st(cp, row_off + view_offset(c, 0, gj + h), v[h] + (bias ? ld(bias, (size_t)(gj + h)) : 0.f));
+        };
+        auto add4 = [](float4 &s, const float4 &v) {
+            s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+        };
+        for (int e = threadIdx.x; e < C::TM * C::TN / 4; e += 256) {
+            float *p = sm + e / (C::TN / 4) * C::PITCH + e % (C::TN / 4) * 4;
+            float4 s = *reinterpret_cast<const float4 *>(p);
+#pragma unroll
+            for (int g = 1; g < C::KG; g++) add4(s, *reinterpret_cast<const float4 *>(p + g * C::PART));
+            if (splits == 1) store4(e, s);
+            else *reinterpret_cast<float4 *>(p) = s;  // only this thread reads this place of group 0's tile
+        }
+        if (splits > 1) {
+            // ---- the cluster's tiles, rank 0 first; every block adds its share of the elements
+            ptx::cluster_sync_all();
+            for (int e = rank * 256 + threadIdx.x; e < C::TM * C::TN / 4; e += splits * 256) {
+                const uint32_t at = ptx::smem_u32(sm + e / (C::TN / 4) * C::PITCH + e % (C::TN / 4) * 4);
+                float4 s = ld_cluster4(ptx::map_to_cta(at, 0));
+                for (int r = 1; r < splits; r++) add4(s, ld_cluster4(ptx::map_to_cta(at, (uint32_t)r)));
+                store4(e, s);
+            }
+            ptx::cluster_sync_all();  // nobody reads this block's shared memory any more
         }
     }
 }
@@ -124,29 +286,78 @@ __global__ void __launch_bounds__(256) column_sum_kernel(MatView a, T *out)
     if (lane == 0) st(out, (size_t)col, s);
 }
 
-template <typename T>
-int launch_gemm(const GemmArgs &g, cudaStream_t s)
+template <typename T, int MODE, bool FA, bool FB, typename C>
+int launch_tile(const GemmArgs &g, int splits, cudaStream_t s)
 {
-    dim3 grid((g.n + TS - 1) / TS, (unsigned)((g.m + TS - 1) / TS));
-    if (g.mode == GEMM_NN)
-        simt_gemm_kernel<T, GEMM_NN><<<grid, 256, 0, s>>>(g.a, g.b, g.c, (const T *)g.bias, g.m, g.n, g.k);
-    else if (g.mode == GEMM_NT)
-        simt_gemm_kernel<T, GEMM_NT><<<grid, 256, 0, s>>>(g.a, g.b, g.c, (const T *)g.bias, g.m, g.n, g.k);
-    else
-        simt_gemm_kernel<T, GEMM_TN><<<grid, 256, 0, s>>>(g.a, g.b, g.c, (const T *)g.bias, g.m, g.n, g.k);
-    EMBER_CUDA_TRY(cudaGetLastError());
+    const long long tiles_m = (g.m + C::TM - 1) / C::TM, tiles_n = (g.n + C::TN - 1) / C::TN;
+    if (tiles_m * tiles_n * splits > 0x7fffffffLL) {
+        set_error("linear: %lld x %d results are too many for the CUDA-core kernel", g.m, g.n);
+        return EMBER_ERR_UNSUPPORTED;
+    }
+    auto kern = simt_gemm_kernel<T, MODE, FA, FB, C>;
+    static SmemOptIn opt_in;
+    EMBER_CUDA_TRY(opt_in(kern, C::FLOATS * sizeof(float)));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(tiles_m * tiles_n * splits));
+    cfg.blockDim = dim3(256);
+    cfg.dynamicSmemBytes = C::FLOATS * sizeof(float);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = splits;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = splits > 1 ? 1 : 0;
+    EMBER_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, g.a, g.b, g.c, (const T *)g.bias, g.m, g.n, g.k, (int)tiles_n, splits));
     return EMBER_OK;
+}
+
+template <typename T, int MODE, bool FA, bool FB>
+int launch_mode(const GemmArgs &g, int sms, cudaStream_t s)
+{
+    auto tiles = [&](int t) { return (g.m + t - 1) / t * (long long)((g.n + t - 1) / t); };
+    // The largest tile that still gives (nearly) every SM one block.
+    if (tiles(128) >= sms) return launch_tile<T, MODE, FA, FB, Tile<128, 128, 16>>(g, 1, s);
+    if (4 * tiles(64) >= 3LL * sms) return launch_tile<T, MODE, FA, FB, Tile<64, 64, 8>>(g, 1, s);
+    if (g.k <= 64) return launch_tile<T, MODE, FA, FB, Tile<32, 32, 2>>(g, 1, s);  // a slab of 128 would be mostly padding
+    // 32 x 32, and the contraction over a cluster while that still leaves every block a slab
+    int splits = 1;
+    while (splits < 8 && tiles(32) * splits * 2 <= 2LL * sms && g.k > 128LL * splits) splits *= 2;
+    return launch_tile<T, MODE, FA, FB, Tile<32, 32, 8>>(g, splits, s);
+}
+
+bool view_fast(const MatView &v)  // 4-element float pieces stay inside a row or head, 16-byte aligned
+{
+    return ((uintptr_t)v.ptr & 15) == 0 && (v.heads ? v.dim % 4 == 0 : v.cols % 4 == 0);
+}
+
+template <typename T, int MODE>
+int launch_views(const GemmArgs &g, int sms, cudaStream_t s)
+{
+    if constexpr (sizeof(T) == 4) {
+        const bool fa = view_fast(g.a), fb = view_fast(g.b);
+        if (fa && fb) return launch_mode<T, MODE, true, true>(g, sms, s);
+        if (fa) return launch_mode<T, MODE, true, false>(g, sms, s);
+        if (fb) return launch_mode<T, MODE, false, true>(g, sms, s);
+    }
+    return launch_mode<T, MODE, false, false>(g, sms, s);
+}
+
+template <typename T>
+int launch_gemm(const GemmArgs &g, int sms, cudaStream_t s)
+{
+    if (g.mode == GEMM_NN) return launch_views<T, GEMM_NN>(g, sms, s);
+    if (g.mode == GEMM_NT) return launch_views<T, GEMM_NT>(g, sms, s);
+    return launch_views<T, GEMM_TN>(g, sms, s);
 }
 
 }  // namespace
 
-int simt_gemm(const GemmArgs &g, cudaStream_t s)
+int simt_gemm(const GemmArgs &g, DeviceState *st, cudaStream_t s)
 {
-    if ((g.m + TS - 1) / TS > 65535) {
-        set_error("linear: more than %d rows are not supported by the CUDA-core kernel", 65535 * TS);
-        return EMBER_ERR_UNSUPPORTED;
-    }
-    return g.dtype == EMBER_BF16 ? launch_gemm<__nv_bfloat16>(g, s) : launch_gemm<float>(g, s);
+    const int sms = st->sm_count > 0 ? st->sm_count : 148;
+    return g.dtype == EMBER_BF16 ? launch_gemm<__nv_bfloat16>(g, sms, s) : launch_gemm<float>(g, sms, s);
 }
 
 // Column sums of a large bf16 matrix in two passes, both coalesced: the rows are cut into chunks; a block

@@ -94,7 +94,7 @@ struct GemmArgs {
 };
 
 // CUDA-core kernels (gemm_simt.cu): float32 math, any shape and view.
-int simt_gemm(const GemmArgs &g, cudaStream_t s);
+int simt_gemm(const GemmArgs &g, DeviceState *st, cudaStream_t s);
 int column_sums(const MatView &a, void *out, int dtype, cudaStream_t s);  // out[j] = sum over rows of a(:, j)
 // tcgen05 kernel (gemm_sm100.cu): bf16 storage; see sm100_gemm_supported for the shapes it takes.
 bool sm100_gemm_supported(const GemmArgs &g);

@@ -47,7 +47,7 @@ int run(const GemmArgs &g, DeviceState *st, cudaStream_t s)
 {
     if (sm100_skinny_gemm_supported(g)) return sm100_skinny_gemm(g, st, s);
     if (sm100_gemm_supported(g)) return sm100_gemm(g, st, s);
-    return simt_gemm(g, s);
+    return simt_gemm(g, st, s);
 }
 
 }  // namespace
