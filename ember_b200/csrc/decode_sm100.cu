@@ -1,0 +1,499 @@
+// Decode over a contiguous bf16 key/value cache on the tensor cores (HBM-bound): one query row per
+// (batch, query head), G = q_heads / kv_heads query heads read the same K/V head.
+//
+// The bound is reading the cache once, so the kernel is a stream: one CTA per SM, each with an equal
+// share of ALL key tiles of the step (the (unit, 128-key tile) pairs of every batch entry and K/V head laid
+// end to end and cut into equal slices), TMA producers running 3 K and 3 V tiles (192 KB) ahead, across the
+// boundaries between units. A slice begins and ends inside a unit as a rule; those two segments leave
+// float32 partials (output, maximum, sum) that a small second kernel merges, the units between them are
+// finished by the CTA itself. Equal slices have no last wave: cutting every unit into splits of 512 keys
+// left 1.7 waves of CTAs at 128 units x 4001 keys.
+//
+// The products are formed with the KEYS as the rows of the MMA, so that almost nothing is padding:
+//   S^T (128 keys x 16)  = K (128 x D) Q^T      query heads are the 16 columns (N), zero-filled past G
+//   O^T (D x 16)        += V^T (D x 128) P^T    V is the MN-major A operand straight from its TMA tile
+// One thread owns one key: G scores to scale, exponentiate and write as bf16 into a 4 KB B operand. With
+// the query heads as the 128 rows instead, every tile cost a full 128 x 128 softmax for G useful rows,
+// 2850 clocks, about what the tile takes to arrive from HBM (5.5 TB/s); here it takes about 600.
+// A tile's maximum is taken over its 128 threads (shuffles, shared memory, one named barrier); the running
+// reference moves, and O is rescaled in tensor memory, only when it grew by more than 2^8.
+//
+// Warps 0-3: softmax and results. Warp 4: tensor memory, MMA issue. Warp 5: TMA.
+#include <math.h>
+
+#include "common.cuh"
+#include "kernels.cuh"
+#include "ptx.cuh"
+
+namespace ember {
+
+namespace {
+
+using namespace ptx;
+
+constexpr int THREADS = 192, NG = 16;  // NG: columns of the transposed products
+constexpr float LOG2E_D = 1.4426950408889634f, LN2_D = 0.6931471805599453f, RESCALE_D = 8.f;
+
+template <int HD>
+struct Cfg {
+    static constexpr int NSUB = HD / 64, SUB = 128 * 128, TILE = NSUB * SUB;
+    static constexpr int ST = HD == 128 ? 3 : 6;  // stages of K and of V
+    static constexpr int Q_BYTES = NSUB * NG * 128, P_BYTES = 2 * NG * 128;
+    static constexpr int OFF_K = 0, OFF_V = OFF_K + ST * TILE, OFF_Q = OFF_V + ST * TILE, OFF_P = OFF_Q + 2 * Q_BYTES;
+    static constexpr int OFF_RED = OFF_P + 2 * P_BYTES;  // [2][4 warps][16] maxima (and sums)
+    static constexpr int OFF_BAR = OFF_RED + 2 * 4 * NG * 4;
+    static constexpr int B_KFULL = 0, B_KEMPTY = B_KFULL + ST, B_VFULL = B_KEMPTY + ST, B_VEMPTY = B_VFULL + ST,
+                         B_QFULL = B_VEMPTY + ST, B_QEMPTY = B_QFULL + 2, B_S = B_QEMPTY + 2, B_R = B_S + 2, B_P = B_R + 2,
+                         B_O = B_P + 2, NUM_BARS = B_O + 2;
+    static constexpr int USED = OFF_BAR + 8 * NUM_BARS + 16, SMEM = USED + 1024;
+    static constexpr int TMEM_S = 0, TMEM_O = 32, TMEM_COLS = 64;
+};
+
+enum { WD_KEMPTY = 401, WD_VEMPTY, WD_QEMPTY, WD_K, WD_V, WD_Q, WD_R, WD_P, WD_S, WD_O };
+
+struct DecParams {
+    __nv_bfloat16 *out;
+    float *lse, *part_o, *part_ml;
+    const int *seq_lens;
+    int units, kv_heads, rows;  // rows: query heads per unit
+    int lk, tiles;              // tiles: 128-key tiles per unit
+    float scale_log2;
+    DeviceStatus *status;
+};
+
+// Slice of CTA i of n: tiles [first, first + count) of the units * tiles laid end to end.
+__host__ __device__ inline long long slice_begin(long long total, int i, int n) { return total * i / n; }
+
+// The tiles of a slice in order, those past a sequence's length left out.
+struct TileIter {
+    long long t, end;
+    int unit, kt, last, len;  // tile kt of [kt, last) of this unit's segment; len: valid keys of the unit
+    bool first;               // first tile of a segment
+
+    __device__ __forceinline__ bool seek(const DecParams &p)  // to the next tile that has keys, starting a segment
+    {
+        while (t < end) {
+            unit = (int)(t / p.tiles);
+            kt = (int)(t - (long long)unit * p.tiles);
+            len = p.seq_lens ? max(0, min(p.lk, p.seq_lens[unit / p.kv_heads])) : p.lk;
+            const long long unit_end = (long long)(unit + 1) * p.tiles;
+            last = kt + (int)(min(end, unit_end) - t);
+            last = min(last, (len + 127) / 128);
+            first = true;
+            if (kt < last) return true;
+            t = unit_end;
+        }
+        return false;
+    }
+    __device__ __forceinline__ bool start(const DecParams &p, long long b, long long e)
+    {
+        t = b;
+        end = e;
+        return seek(p);
+    }
+    __device__ __forceinline__ bool next(const DecParams &p)
+    {
+        if (kt + 1 < last) {
+            kt++;
+            first = false;
+            return true;
+        }
+        t = (long long)(unit + 1) * p.tiles;
+        return seek(p);
+    }
+};
+
+template <int HD, int G>
+__global__ void __launch_bounds__(THREADS, 1) decode_sm100_kernel(const __grid_constant__ CUtensorMap tm_q,
+                                                                  const __grid_constant__ CUtensorMap tm_k,
+                                                                  const __grid_constant__ CUtensorMap tm_v, const DecParams p)
+{
+    using C = Cfg<HD>;
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    uint8_t *smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
+    const uint32_t bar0 = smem_base + C::OFF_BAR;
+    auto BAR = [&](int i) { return bar0 + 8u * (uint32_t)i; };
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem_gen + C::OFF_BAR + 8 * C::NUM_BARS);
+    volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+
+    if (threadIdx.x == 0) {
+        *abort_flag = 0;
+        for (int i = 0; i < C::NUM_BARS; i++) mbar_init(BAR(i), (i >= C::B_R && i < C::B_O) ? 4 : 1);  // R and P: one arrival per softmax warp
+        fence_mbar_init();
+    }
+    if (warp == 4) {
+        tmem_alloc(smem_u32(tmem_slot), C::TMEM_COLS);
+        tmem_relinquish();
+    }
+    if (warp == 5 && lane == 0) {
+        prefetch_tensormap(&tm_q);
+        prefetch_tensormap(&tm_k);
+        prefetch_tensormap(&tm_v);
+    }
+    // rows of P past the query heads stay zero
+    for (int i = threadIdx.x; i < 2 * C::P_BYTES / 16; i += THREADS)
+        *reinterpret_cast<uint4 *>(smem_gen + C::OFF_P + i * 16) = make_uint4(0, 0, 0, 0);
+    fence_proxy_async();
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+    pdl_launch_dependents();
+    pdl_wait();  // the cache's new rows may come from the kernel before this one
+
+    const long long total = (long long)p.units * p.tiles;
+    const long long t0 = slice_begin(total, blockIdx.x, gridDim.x), t1 = slice_begin(total, blockIdx.x + 1, gridDim.x);
+
+    if (warp == 5) {
+        if (lane == 0) {
+            // ------------------------------------------------------------ TMA producer
+            TileIter ti;
+            int it = 0, seg = 0;
+            bool ok = true;
+            for (bool more = ti.start(p, t0, t1); more && ok; more = ti.next(p), it++) {
+                const int s = it % C::ST, par = ((it / C::ST) & 1) ^ 1;
+                if (ti.first) {
+                    const int qs = seg & 1;
+                    if (!(ok = mbar_wait(BAR(C::B_QEMPTY + qs), ((seg >> 1) & 1) ^ 1, abort_flag, p.status, WD_QEMPTY))) break;
+                    mbar_arrive_expect_tx(BAR(C::B_QFULL + qs), C::Q_BYTES);
+                    for (int sub = 0; sub < C::NSUB; sub++)
+                        tma_load_3d(smem_base + C::OFF_Q + qs * C::Q_BYTES + sub * NG * 128, &tm_q, BAR(C::B_QFULL + qs), sub * 64, 0, ti.unit);
+                    seg++;
+                }
+                if (!(ok = mbar_wait(BAR(C::B_KEMPTY + s), par, abort_flag, p.status, WD_KEMPTY))) break;
+                mbar_arrive_expect_tx(BAR(C::B_KFULL + s), C::TILE);
+                for (int sub = 0; sub < C::NSUB; sub++)
+                    tma_load_3d(smem_base + C::OFF_K + s * C::TILE + sub * C::SUB, &tm_k, BAR(C::B_KFULL + s), sub * 64, ti.kt * 128, ti.unit);
+                if (!(ok = mbar_wait(BAR(C::B_VEMPTY + s), par, abort_flag, p.status, WD_VEMPTY))) break;
+                mbar_arrive_expect_tx(BAR(C::B_VFULL + s), C::TILE);
+                for (int sub = 0; sub < C::NSUB; sub++)
+                    tma_load_3d(smem_base + C::OFF_V + s * C::TILE + sub * C::SUB, &tm_v, BAR(C::B_VFULL + s), sub * 64, ti.kt * 128, ti.unit);
+            }
+            // A CTA that gave up stays until its copies have landed: every full barrier whose phase is open
+            // is polled, bounded, for the last copies that were issued (it counts whole iterations, so
+            // one more K tile may be in flight).
+            const long long c0 = clock64();
+            for (int j = max(0, it - C::ST); j < it + (ok ? 0 : 1); j++)
+                for (int b = C::B_KFULL; b <= C::B_VFULL; b += C::B_VFULL - C::B_KFULL)
+                    while (!mbar_try_wait(BAR(b + j % C::ST), (j / C::ST) & 1) && clock64() - c0 < kWaitLimitCycles && (ok || clock64() - c0 < 1000000)) {}
+        }
+    } else if (warp == 4) {
+        // ---------------------------------------------------------------- MMA issue
+        constexpr uint32_t IDESC_S = idesc_bf16_f32(128, NG, 0, 0), IDESC_O = idesc_bf16_f32(128, NG, 1, 0);
+        TileIter ahead, cur;
+        bool ok = true;
+        int its = 0, seg = 0, it = 0;  // next score tile, its segment, current PV tile
+        auto issue_s = [&]() {         // scores of tile `ahead`
+            const int s = its % C::ST, b = its & 1;
+            if (ahead.first) {
+                ok = ok && mbar_wait(BAR(C::B_QFULL + (seg & 1)), (seg >> 1) & 1, abort_flag, p.status, WD_Q);
+                seg++;
+            }
+            ok = ok && mbar_wait(BAR(C::B_KFULL + s), (its / C::ST) & 1, abort_flag, p.status, WD_K);
+            if (its >= 2) ok = ok && mbar_wait(BAR(C::B_R + b), ((its >> 1) - 1) & 1, abort_flag, p.status, WD_R);
+            tc_fence_after();
+            const uint32_t k_lo = desc_lo(smem_base + C::OFF_K + s * C::TILE, 16);
+            const uint32_t q_lo = desc_lo(smem_base + C::OFF_Q + ((seg - 1) & 1) * C::Q_BYTES, 16);
+#pragma unroll
+            for (int ks = 0; ks < HD / 16; ks++)
+                mma_ss_lo(tmem + C::TMEM_S + b * NG, k_lo + (((ks / 4) * C::SUB + (ks % 4) * 32) >> 4),
+                          q_lo + (((ks / 4) * NG * 128 + (ks % 4) * 32) >> 4), IDESC_S, ks > 0);
+            tc_commit_elect(BAR(C::B_S + b));
+            tc_commit_elect(BAR(C::B_KEMPTY + s));
+            if (ahead.kt + 1 >= ahead.last) tc_commit_elect(BAR(C::B_QEMPTY + ((seg - 1) & 1)));
+            its++;
+        };
+        bool more_s = ahead.start(p, t0, t1);
+        if (more_s) {
+            issue_s();
+            more_s = ahead.next(p);
+        }
+        for (bool more = cur.start(p, t0, t1); more && ok; more = cur.next(p), it++) {
+            if (more_s) {
+                issue_s();
+                more_s = ahead.next(p);
+            }
+            const int s = it % C::ST, b = it & 1;
+            ok = ok && mbar_wait(BAR(C::B_VFULL + s), (it / C::ST) & 1, abort_flag, p.status, WD_V);
+            if (p.seq_lens && cur.kt * 128 + 128 > cur.len) {
+                // TMA zero-fills rows past the MAP's end only; between a sequence's own length and there
+                // the cache may hold anything, and 0 * Inf would poison the product: zero those rows here
+                uint8_t *vt = smem_gen + C::OFF_V + s * C::TILE;
+                const int r0 = cur.len - cur.kt * 128;
+                for (int i = lane; i < (128 - r0) * C::NSUB * 8; i += 32) {
+                    const int rr = r0 + i / (C::NSUB * 8), sub = (i / 8) % C::NSUB, ch = i % 8;
+                    *reinterpret_cast<uint4 *>(vt + sub * C::SUB + rr * 128 + ch * 16) = make_uint4(0, 0, 0, 0);
+                }
+                fence_proxy_async();
+                __syncwarp();
+            }
+            ok = ok && mbar_wait(BAR(C::B_P + b), (it >> 1) & 1, abort_flag, p.status, WD_P);
+            tc_fence_after();
+            // HD = 64: the 64 columns of V stand in for rows 64-127 of the MMA a second time; nobody reads those
+            const uint32_t v_lo = desc_lo(smem_base + C::OFF_V + s * C::TILE, HD == 128 ? C::SUB : 0);
+            const uint32_t p_lo = desc_lo(smem_base + C::OFF_P + b * C::P_BYTES, 16);
+#pragma unroll
+            for (int ks = 0; ks < 8; ks++)
+                mma_ss_lo(tmem + C::TMEM_O, v_lo + ks * (2048 >> 4), p_lo + (((ks / 4) * NG * 128 + (ks % 4) * 32) >> 4), IDESC_O,
+                          (!cur.first || ks > 0) ? 1u : 0u);
+            tc_commit_elect(BAR(C::B_VEMPTY + s));
+            tc_commit_elect(BAR(C::B_O + b));
+        }
+    } else {
+        // ---------------------------------------------------------------- softmax: one thread per key
+        const uint32_t lane_sel = (uint32_t)(warp * 32) << 16;
+        float *red = reinterpret_cast<float *>(smem_gen + C::OFF_RED);
+        const int tid = threadIdx.x;
+        TileIter ti;
+        int it = 0;
+        bool ok = true;
+        float m[G], l[G];
+        // slot of a partial segment: a CTA has at most two, the one its slice begins in and the one it ends in
+        auto finish = [&](int unit, int kt0, int kt1, bool empty) {
+            uint32_t o[NG];
+            if (!empty) {
+                ok = ok && mbar_wait(BAR(C::B_O + ((it - 1) & 1)), ((it - 1) >> 1) & 1, abort_flag, p.status, WD_O);
+                tc_fence_after();
+                tmem_ld_32x32b_x16(tmem + lane_sel + C::TMEM_O, o);
+                tmem_wait_ld();
+                tc_fence_before();
+            }
+            // sums over the 128 keys' threads
+            named_bar_sync(1, 128);
+            float lt[G];
+#pragma unroll
+            for (int g = 0; g < G; g++) {
+                float v = empty ? 0.f : l[g];
+#pragma unroll
+                for (int t = 16; t > 0; t >>= 1) v += __shfl_xor_sync(0xffffffffu, v, t);
+                if (lane == 0) red[warp * NG + g] = v;
+            }
+            named_bar_sync(1, 128);
+#pragma unroll
+            for (int g = 0; g < G; g++) lt[g] = (red[g] + red[NG + g]) + (red[2 * NG + g] + red[3 * NG + g]);
+            named_bar_sync(1, 128);  // red is written again by the next tile
+            const bool whole = kt0 == 0 && kt1 == p.tiles;
+            const int slot = 2 * blockIdx.x + (slice_begin((long long)p.units * p.tiles, blockIdx.x, gridDim.x) >= (long long)unit * p.tiles ? 0 : 1);
+#pragma unroll
+            for (int g = 0; g < G; g++) {
+                if (g >= p.rows || !ok) continue;
+                const float ov = empty ? 0.f : __uint_as_float(o[g]);
+                if (whole) {
+                    const size_t row = (size_t)unit * p.rows + g;
+                    if (tid < HD) p.out[row * HD + tid] = __float2bfloat16_rn(empty ? 0.f : ov * (1.f / lt[g]));
+                    if (tid == 0 && p.lse) p.lse[row] = empty ? -INFINITY : (m[g] + log2f(lt[g])) * LN2_D;
+                } else {
+                    const size_t row = (size_t)slot * p.rows + g;
+                    if (tid < HD) p.part_o[row * HD + tid] = ov;
+                    if (tid == 0) {
+                        p.part_ml[row * 2] = empty ? -INFINITY : m[g];
+                        p.part_ml[row * 2 + 1] = lt[g];
+                    }
+                }
+            }
+        };
+        // Walks every unit of the slice (also those without keys here, which leave an empty result).
+        // A thread that gave up on a wait carries on, so that all 128 still meet at the named barriers.
+        for (long long t = t0; t < t1;) {
+            const int unit = (int)(t / p.tiles), kt0 = (int)(t - (long long)unit * p.tiles);
+            const long long unit_end = (long long)(unit + 1) * p.tiles;
+            const int kt1 = kt0 + (int)(min(t1, unit_end) - t);
+            const bool some = ti.start(p, t, min(t1, unit_end));
+            if (!some) {
+                finish(unit, kt0, kt1, true);
+                t = min(t1, unit_end);
+                continue;
+            }
+            for (bool more = some; more; more = ti.next(p), it++) {
+                const int b = it & 1;
+                ok = ok && mbar_wait(BAR(C::B_S + b), (it >> 1) & 1, abort_flag, p.status, WD_S);
+                tc_fence_after();
+                uint32_t u[NG];
+                tmem_ld_32x32b_x16(tmem + lane_sel + C::TMEM_S + b * NG, u);
+                tmem_wait_ld();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(BAR(C::B_R + b));
+                const bool valid = ti.kt * 128 + tid < ti.len;
+                float x[G], mt[G];
+#pragma unroll
+                for (int g = 0; g < G; g++) {
+                    x[g] = valid ? __uint_as_float(u[g]) * p.scale_log2 : -INFINITY;
+                    float v = x[g];
+#pragma unroll
+                    for (int t2 = 16; t2 > 0; t2 >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, t2));
+                    if (lane == 0) red[(b * 4 + warp) * NG + g] = v;
+                }
+                named_bar_sync(1, 128);
+                bool grow = false;
+#pragma unroll
+                for (int g = 0; g < G; g++) {
+                    const float *r = red + b * 4 * NG + g;
+                    mt[g] = fmaxf(fmaxf(r[0], r[NG]), fmaxf(r[2 * NG], r[3 * NG]));  // finite: the tile has a key
+                    if (ti.first) {
+                        m[g] = mt[g];
+                        l[g] = 0.f;
+                    }
+                    grow = grow || mt[g] - m[g] > RESCALE_D;  // the same in all 128 threads
+                }
+                if (grow) {
+                    float alpha[G];
+#pragma unroll
+                    for (int g = 0; g < G; g++) {
+                        const float mn = fmaxf(m[g], mt[g]);
+                        alpha[g] = ex2(m[g] - mn);
+                        m[g] = mn;
+                        l[g] *= alpha[g];
+                    }
+                    ok = ok && mbar_wait(BAR(C::B_O + ((it - 1) & 1)), ((it - 1) >> 1) & 1, abort_flag, p.status, WD_O);
+                    tc_fence_after();
+                    uint32_t o[NG];
+                    tmem_ld_32x32b_x16(tmem + lane_sel + C::TMEM_O, o);
+                    tmem_wait_ld();
+#pragma unroll
+                    for (int g = 0; g < G; g++) o[g] = __float_as_uint(__uint_as_float(o[g]) * alpha[g]);
+                    tmem_st_32x32b_x16(tmem + lane_sel + C::TMEM_O, o);
+                    tmem_wait_st();
+                    tc_fence_before();
+                }
+                if (it >= 2) ok = ok && mbar_wait(BAR(C::B_O + b), ((it >> 1) - 1) & 1, abort_flag, p.status, WD_O);  // P(it-2) has been read
+                uint8_t *pb = smem_gen + C::OFF_P + b * C::P_BYTES + (tid / 64) * (NG * 128) + (tid % 8) * 2;
+#pragma unroll
+                for (int g = 0; g < G; g++) {
+                    const float pr = ex2(x[g] - m[g]);
+                    l[g] += pr;
+                    *reinterpret_cast<__nv_bfloat16 *>(pb + g * 128 + ((((tid % 64) / 8) ^ (g & 7)) << 4)) = __float2bfloat16_rn(pr);
+                }
+                fence_proxy_async();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(BAR(C::B_P + b));
+            }
+            finish(unit, kt0, kt1, false);
+            t = min(t1, unit_end);
+        }
+    }
+    __syncwarp();
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 4) tmem_dealloc(tmem, C::TMEM_COLS);
+}
+
+// Merges the partial segments of the units that several CTAs share: one block per (unit, query head).
+__global__ void __launch_bounds__(128) decode_merge_kernel(const float *__restrict__ part_o, const float *__restrict__ part_ml,
+                                                           __nv_bfloat16 *__restrict__ out, float *__restrict__ lse, int rows,
+                                                           int tiles, int units, int ncta, int d)
+{
+    const int unit = blockIdx.x / rows, g = blockIdx.x - unit * rows;
+    const long long total = (long long)units * tiles, begin = (long long)unit * tiles, end = begin + tiles;
+    // the CTA whose slice holds tile `begin`
+    int first = (int)(begin * ncta / total);
+    while (slice_begin(total, first + 1, ncta) <= begin) first++;
+    while (slice_begin(total, first, ncta) > begin) first--;
+    pdl_wait();
+    if (slice_begin(total, first + 1, ncta) >= end) return;  // one CTA had all of it and wrote the result
+    float mx = -INFINITY;
+    for (int i = first; i < ncta && slice_begin(total, i, ncta) < end; i++) {
+        const size_t row = (size_t)(2 * i + (slice_begin(total, i, ncta) >= begin ? 0 : 1)) * rows + g;
+        mx = fmaxf(mx, part_ml[row * 2]);
+    }
+    float l = 0.f, acc = 0.f;
+    for (int i = first; i < ncta && slice_begin(total, i, ncta) < end; i++) {
+        const size_t row = (size_t)(2 * i + (slice_begin(total, i, ncta) >= begin ? 0 : 1)) * rows + g;
+        const float mi = part_ml[row * 2];
+        if (mi == -INFINITY) continue;
+        const float w = exp2f(mi - mx);
+        l += part_ml[row * 2 + 1] * w;
+        if ((int)threadIdx.x < d) acc += part_o[row * d + threadIdx.x] * w;
+    }
+    const size_t r = (size_t)unit * rows + g;
+    if ((int)threadIdx.x < d) out[r * d + threadIdx.x] = __float2bfloat16_rn(l > 0.f ? acc * (1.f / l) : 0.f);
+    if (threadIdx.x == 0 && lse) lse[r] = l > 0.f ? (mx + log2f(l)) * LN2_D : -INFINITY;
+}
+
+int slices(const CacheDecodeArgs &a, int sms)
+{
+    const long long total = (long long)a.batch * a.kv_heads * ((a.lk + 127) / 128);
+    return (int)(total < sms ? total : sms);
+}
+
+template <int HD, int G>
+int launch(const CacheDecodeArgs &a, DeviceState *st, cudaStream_t s)
+{
+    using C = Cfg<HD>;
+    const int units = a.batch * a.kv_heads, rows = a.q_heads / a.kv_heads;
+    const int ncta = slices(a, st->sm_count > 0 ? st->sm_count : 148);
+    CUtensorMap tq, tk, tv;
+    int rc;
+    if ((rc = make_tensor_map_bf16_3d(&tq, a.q, HD, rows, units, 64, NG)) != EMBER_OK) return rc;
+    if ((rc = make_tensor_map_bf16_3d(&tk, a.k_cache, HD, a.lk, units, 64, 128, a.capacity)) != EMBER_OK) return rc;
+    if ((rc = make_tensor_map_bf16_3d(&tv, a.v_cache, HD, a.lk, units, 64, 128, a.capacity)) != EMBER_OK) return rc;
+    DecParams p;
+    p.out = (__nv_bfloat16 *)a.out;
+    p.lse = a.lse;
+    p.part_o = (float *)a.workspace;
+    p.part_ml = p.part_o + (size_t)2 * ncta * rows * HD;
+    p.seq_lens = a.seq_lens;
+    p.units = units;
+    p.kv_heads = a.kv_heads;
+    p.rows = rows;
+    p.lk = a.lk;
+    p.tiles = (a.lk + 127) / 128;
+    p.scale_log2 = a.scale * LOG2E_D;
+    p.status = st->status;
+    auto kern = decode_sm100_kernel<HD, G>;
+    static SmemOptIn opt_in;
+    EMBER_CUDA_TRY(opt_in(kern, C::SMEM));
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)ncta);
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = C::SMEM;
+    cfg.stream = s;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    EMBER_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, tq, tk, tv, p));
+    // a unit is shared whenever a slice begins inside it
+    const long long total = (long long)units * p.tiles;
+    if (ncta > 1 && !(total % ncta == 0 && (total / ncta) % p.tiles == 0)) {
+        cfg.gridDim = dim3((unsigned)(units * rows));
+        cfg.blockDim = dim3(128);
+        cfg.dynamicSmemBytes = 0;
+        EMBER_CUDA_TRY(cudaLaunchKernelEx(&cfg, decode_merge_kernel, (const float *)p.part_o, (const float *)p.part_ml, p.out, p.lse,
+                                          rows, p.tiles, units, ncta, HD));
+    }
+    return EMBER_OK;
+}
+
+template <int HD>
+int dispatch(const CacheDecodeArgs &a, DeviceState *st, cudaStream_t s)
+{
+    const int rows = a.q_heads / a.kv_heads;
+    if (rows == 1) return launch<HD, 1>(a, st, s);
+    if (rows == 2) return launch<HD, 2>(a, st, s);
+    if (rows <= 4) return launch<HD, 4>(a, st, s);
+    if (rows <= 8) return launch<HD, 8>(a, st, s);
+    return launch<HD, 16>(a, st, s);
+}
+
+}  // namespace
+
+bool sm100_decode_supported(const CacheDecodeArgs &a)
+{
+    if (a.dtype != EMBER_BF16 || (a.d != 64 && a.d != 128)) return false;
+    if (a.q_heads % a.kv_heads != 0 || a.q_heads / a.kv_heads > NG || !isfinite(a.scale)) return false;
+    const uintptr_t bits = (uintptr_t)a.q | (uintptr_t)a.k_cache | (uintptr_t)a.v_cache;
+    return (bits & 15) == 0;
+}
+
+size_t sm100_decode_workspace_bytes(int rows, int d, int sms) { return (size_t)2 * sms * rows * (d + 2) * sizeof(float); }
+
+int sm100_decode(const CacheDecodeArgs &a, DeviceState *st, cudaStream_t s)
+{
+    return a.d == 128 ? dispatch<128>(a, st, s) : dispatch<64>(a, st, s);
+}
+
+}  // namespace ember

@@ -51,6 +51,12 @@ bool sm100_cache_decode_supported(const CacheDecodeArgs &a);
 size_t sm100_cache_decode_workspace_bytes(int units, int rows, int d, int splits);
 int sm100_cache_decode(const CacheDecodeArgs &a, DeviceState *st, cudaStream_t s);
 
+// Decode over a contiguous bf16 cache with up to 16 query heads per K/V head (decode_sm100.cu); splits,
+// chunk are not used.
+bool sm100_decode_supported(const CacheDecodeArgs &a);
+size_t sm100_decode_workspace_bytes(int rows, int d, int sms);
+int sm100_decode(const CacheDecodeArgs &a, DeviceState *st, cudaStream_t s);
+
 // Split-KV decode (attn_decode.cu): lq == 1, bf16 or f32 storage, d <= 256 and d % 8 == 0.
 int decode_pick_splits(int bh, int lk, int d, int dtype, int sm_count);
 size_t decode_workspace_bytes(int bh, int d, int splits);

@@ -10,15 +10,13 @@
 //   queries / outputs  (batch, q_heads, d), q_heads = group * kv_heads; query head h reads K/V head
 //                      h / group
 //
-// Two decode paths. With bf16 storage, head dimension 64 or 128, a contiguous cache and several
-// query heads per K/V head, the step runs on the tensor cores: the forward kernel of
-// attn_fwd_sm100.cu takes the group's query heads as the rows of one (zero-padded) 128-row tile, one
-// CTA per (batch, kv_head, split) streams its keys by TMA, and a small kernel merges the splits'
-// normalised partial outputs by their log-sum-exps. On CUDA cores the same step is bound by
-// arithmetic as soon as four query heads share a key row (1.85 TB/s of cache traffic measured for
-// groups of 4, no faster than reading the cache once per query head).
-// Everything else (one query head per K/V head, float32, a page table, other head dimensions)
-// runs the CUDA-core kernel below,
+// Three decode paths. With bf16 storage, head dimension 64 or 128, a contiguous cache and up to 16
+// query heads per K/V head, the step runs on the tensor cores with the keys as the MMA's rows
+// (decode_sm100.cu). With more query heads per K/V head they fill a tile of the forward kernel of
+// attn_fwd_sm100.cu, one CTA per (batch, kv_head, split), and a small kernel merges the splits. On CUDA
+// cores a step is bound by arithmetic as soon as four query heads share a key row (1.85 TB/s of cache
+// traffic measured for groups of 4, no faster than reading the cache once per query head).
+// Everything else (float32, a page table, other head dimensions) runs the CUDA-core kernel below,
 // the split-KV kernel of attn_decode.cu with one change that matters for
 // bandwidth: a CTA owns one (batch, kv_head, split) and ALL `group` query heads that share it, so a
 // K or V row is loaded from HBM once and used by every query head of the group (the cache is the
@@ -30,6 +28,7 @@
 
 #include "common.cuh"
 #include "kernels.cuh"
+#include "ptx.cuh"
 
 namespace ember {
 
@@ -296,6 +295,7 @@ __global__ void __launch_bounds__(256) kv_append_kernel(uint4 *__restrict__ kc, 
                                                         const CacheGeom g, int batch, int n_new, int pos, int vec_per_row,
                                                         int elems_per_vec, DeviceStatus *status)
 {
+    ptx::pdl_launch_dependents();  // the decode kernel behind it may set itself up meanwhile
     const size_t total = (size_t)batch * g.kv_heads * n_new * vec_per_row;
     const int limit = g.block_table ? (g.max_blocks << g.page_shift) : g.capacity;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
@@ -494,7 +494,9 @@ size_t ember_attention_decode_cache_workspace_bytes(int batch, int q_heads, int 
     int tsplits, tchunk;
     tensor_core_split(batch * kv_heads, lk, st ? st->sm_count : 148, num_splits, tsplits, tchunk);
     const size_t tneed = sm100_cache_decode_workspace_bytes(batch * kv_heads, q_heads / kv_heads, d, tsplits);
-    return tneed > need ? tneed : need;
+    if (tneed > need) need = tneed;
+    const size_t dneed = sm100_decode_workspace_bytes(q_heads / kv_heads, d, st && st->sm_count > 0 ? st->sm_count : 148);
+    return dneed > need ? dneed : need;
 }
 
 int ember_attention_decode_cache(const void *q, const void *k_cache, const void *v_cache, void *out, float *lse, int batch,
@@ -513,13 +515,17 @@ int ember_attention_decode_cache(const void *q, const void *k_cache, const void 
     DeviceState *st = device_state();
     if (!st) return EMBER_ERR_CUDA;
     cudaStream_t s = pick_stream(stream, st);
-    if (!block_table && q_heads / kv_heads > 1) {
-        // Grouped-query heads over a contiguous bf16 cache: tensor cores (the CUDA-core kernel below
-        // is arithmetic-bound once several query heads share a key row).
+    if (!block_table) {
         CacheDecodeArgs t;
         t.q = q; t.k_cache = k_cache; t.v_cache = v_cache; t.out = out; t.lse = lse;
         t.batch = batch; t.q_heads = q_heads; t.kv_heads = kv_heads; t.lk = lk; t.capacity = capacity; t.d = d;
         t.dtype = dtype; t.scale = scale; t.seq_lens = seq_lens;
+        // (a caller that sized its workspace for one split and passes none gets the kernels below)
+        if (sm100_decode_supported(t) && workspace && ((uintptr_t)workspace & 255) == 0 &&
+            workspace_bytes >= sm100_decode_workspace_bytes(q_heads / kv_heads, d, st->sm_count > 0 ? st->sm_count : 148)) {
+            t.workspace = workspace;
+            return sm100_decode(t, st, s);
+        }
         if (sm100_cache_decode_supported(t)) {
             tensor_core_split(batch * kv_heads, lk, st->sm_count, num_splits, t.splits, t.chunk);
             const size_t tneed = sm100_cache_decode_workspace_bytes(batch * kv_heads, q_heads / kv_heads, d, t.splits);

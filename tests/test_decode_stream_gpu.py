@@ -1,0 +1,81 @@
+"""Decode over a bf16 cache where the step's key tiles are cut into equal slices over the SMs: lengths
+round the 128-key tiles, slices that begin and end inside units, fewer tiles than SMs, groups that fill
+the tile's 16 columns partly, and sequences of different lengths, against the CPU oracle.
+
+Tolerance: 2^-8 relative to the largest result for the bf16 rounding of the probabilities and the
+output (each half a unit of 2^-8), 2e-3 absolute on the log-sum-exp (float32 sums of exact products)."""
+import ctypes
+import math
+
+import numpy as np
+import pytest
+
+import ember_b200 as em
+from conftest import bf16_round, seeded
+from ember_b200 import _lib
+from oracle import cpu_oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def _reference(q, k, v, lens):
+    B, Hq, D = q.shape
+    group = Hq // k.shape[1]
+    out, lse = np.zeros_like(q), np.full((B, Hq), -np.inf, np.float32)
+    for b in range(B):
+        for h in range(Hq if lens[b] > 0 else 0):
+            n = lens[b]
+            o, l = cpu_oracle.attention_fwd(q[b, h][None], k[b, h // group, :n], v[b, h // group, :n], None, False)
+            out[b, h], lse[b, h] = o[0], l[0]
+    return out, lse
+
+
+def _check(o, l, q, k, v, lens):
+    ro, rl = _reference(q, k, v, lens)
+    full = np.isfinite(rl)
+    assert np.abs(o - ro).max() <= 2.0 ** -7 * np.abs(ro).max()
+    assert np.array_equal(np.isfinite(l), full) and np.abs(l[full] - rl[full]).max() <= 2e-3
+    where = ctypes.c_int(0)
+    _lib.check(_lib.lib().ember_check_device_status(None, ctypes.byref(where)))
+
+
+@pytest.mark.parametrize("batch,kv_heads,group,lk,dim", [
+    (1, 1, 1, 1, 64), (1, 1, 8, 127, 128), (2, 1, 2, 128, 64), (1, 2, 4, 129, 128), (3, 5, 1, 1000, 128), (2, 3, 3, 511, 64),
+    (37, 4, 4, 130, 64), (30, 5, 1, 257, 128), (4, 2, 16, 700, 64), (1, 149, 1, 128, 64), (1, 1, 1, 20000, 128), (5, 31, 8, 385, 128),
+])
+def test_slices(batch, kv_heads, group, lk, dim):
+    q = bf16_round(seeded((batch, kv_heads * group, dim), 1, 2.0))
+    k, v = (bf16_round(seeded((batch, kv_heads, lk, dim), s, 0.7)) for s in (2, 3))
+    cache = em.KVCache(batch, kv_heads, lk + 3, dim, "bfloat16")
+    cache.append(em.Tensor(k, "bfloat16"), em.Tensor(v, "bfloat16"))
+    o, l = cache.decode(em.Tensor(q, "bfloat16"))
+    _check(o.to_np(), l.to_np(), q, k, v, [lk] * batch)
+
+
+@pytest.mark.parametrize("kv_heads,group,dim", [(1, 1, 64), (3, 4, 128), (2, 8, 64)])
+def test_lengths_and_rising_maxima(kv_heads, group, dim):
+    """Sequences of unequal lengths (one empty); scores that grow along the keys by far more than the
+    rescaling threshold; cache rows past a length are NaN and must not reach the result."""
+    torch = pytest.importorskip("torch")
+    lens = [0, 1, 64, 128, 129, 400, 700]
+    batch, cap = len(lens), 700
+    q = bf16_round(seeded((batch, kv_heads * group, dim), 1))
+    ramp = np.linspace(0.1, 6.0, cap, dtype=np.float32)[:, None]
+    k = bf16_round(seeded((batch, kv_heads, cap, dim), 2) * ramp)
+    v = bf16_round(seeded((batch, kv_heads, cap, dim), 3))
+    kd, vd = k.copy(), v.copy()
+    for b, n in enumerate(lens):
+        kd[b, :, n:], vd[b, :, n:] = np.nan, np.nan
+    L = _lib.lib()
+    dev = lambda a: torch.from_numpy(a).cuda().to(torch.bfloat16)  # noqa: E731
+    tq, tk, tv = dev(q), dev(kd), dev(vd)
+    tl = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    o, l = torch.empty_like(tq), torch.empty(batch, kv_heads * group, device="cuda")
+    n = L.ember_attention_decode_cache_workspace_bytes(batch, kv_heads * group, kv_heads, cap, dim, 0)
+    ws = torch.empty(n, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    _lib.check(L.ember_attention_decode_cache(tq.data_ptr(), tk.data_ptr(), tv.data_ptr(), o.data_ptr(), l.data_ptr(), batch,
+                                              kv_heads * group, kv_heads, cap, cap, dim, 1.0 / math.sqrt(dim), _lib.EMBER_BF16,
+                                              tl.data_ptr(), None, 0, 0, 0, ws.data_ptr(), n, None))
+    torch.cuda.synchronize()
+    _check(o.float().cpu().numpy(), l.cpu().numpy(), q, k, v, lens)
