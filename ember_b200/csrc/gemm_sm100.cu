@@ -49,14 +49,18 @@ constexpr int GROUP_M = 16;                           // tiles that share B colu
 enum { B_FULL = 0, B_EMPTY = B_FULL + STAGES, B_ACCFULL = B_EMPTY + STAGES, B_ACCEMPTY = B_ACCFULL + 2, NUM_BARS = B_ACCEMPTY + 2 };
 enum { WG_EMPTY = 201, WG_FULL, WG_ACCEMPTY, WG_ACCFULL, WG_SMEM };
 
+// seq: rows from one batch entry to the next in the TILE's row space, see GemmParams::seq_pad
 struct ViewGeom {
     int heads, seq, dim;
 };
 
 struct GemmParams {
-    long long m;
-    int n, k;
+    int n, kblocks;
     int tiles_m, tiles_n;
+    // The result's rows: `batch` entries of `seq` rows, walked in blocks of 128 rows that never cross an
+    // entry, i.e. in a row space where an entry takes seq_pad rows. One entry of all m rows unless an operand
+    // or the result lies head-major with a seq that is no multiple of the boxes.
+    int batch, seq, seq_pad;
     ViewGeom a, b;
     MatView c;
     const __nv_bfloat16 *bias;
@@ -66,8 +70,8 @@ struct GemmParams {
 // TMA coordinates of a 64-column box of a view, walked along the contraction index. The producer
 // computes coordinates on the critical path of every stage, so the divisions that split a row into
 // (batch, position) and a column into (part, head, element) are done once per tile and the walk
-// itself only adds and carries (all steps are 64; seq and dim are multiples of 64 for head-major
-// views the kernel accepts).
+// itself only adds and carries (all steps are 64; the padded seq is a multiple of 64, dim too unless
+// there is a single head: a row-major matrix walked by batch entries).
 struct BoxWalker {
     int c0, c1, c2, c3, c4;  // column | element, row | position, head, batch, part
     int heads, seq, dim;
@@ -142,7 +146,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
 
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const int num_tiles = p.tiles_m * p.tiles_n;  // tiles of 2*BM x BN, one per CTA pair at a time
-    const int kblocks = (p.k + BK - 1) / BK;
+    const int kblocks = p.kblocks;
     const uint32_t rank = cluster_ctarank();      // 0 issues the MMAs
     const int pair = blockIdx.x / 2, npairs = gridDim.x / 2;
 
@@ -254,7 +258,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
             int tm, tn;
             tile_coords(p, tile, tm, tn);
             const int buf = tcount & 1;
-            const long long m0 = (long long)tm * 2 * BM + (long long)rank * BM;
+            const int m0 = (tm * 2 + (int)rank) * BM, entry = m0 / p.seq_pad, l0 = m0 - entry * p.seq_pad;
+            const int rows_valid = entry < p.batch ? min(BM, p.seq - l0) : 0;  // may be <= 0: padding alone
             const int n0 = tn * BN;
             named_bar_sync(1, 128);  // the previous tile's bias has been read by every thread
             for (int j = r; j < BN; j += 128)
@@ -291,20 +296,18 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                 __syncwarp();
                 // Each warp copies its own 32 rows: two rows of 16 chunks per instruction. The destination
                 // of a chunk is found without divisions in the loop: this thread's column is fixed, and
-                // the 128 rows of a CTA's tile are consecutive in memory rows (row-major: `cols` apart;
-                // head-major: the tile lies inside one batch entry because seq is a multiple of 128, so
-                // consecutive rows are `dim` apart).
+                // the 128 rows of a CTA's tile lie inside one batch entry and therefore at one distance
+                // from each other (row-major: `cols` apart; head-major: `dim`).
                 const int chunk = lane % 16;
                 const int col = n0 + half * 128 + chunk * 8;
                 const size_t row_stride = p.c.heads == 0 ? (size_t)p.c.cols : (size_t)p.c.dim;
-                const size_t base = (m0 < p.m && col < p.n) ? view_offset(p.c, m0, col) : 0;
+                const size_t base = (rows_valid > 0 && col < p.n) ? view_offset(p.c, (long long)entry * p.seq + l0, col) : 0;
 #pragma unroll 4
                 for (int it2 = 0; it2 < 16; it2++) {
                     const int rr = warp * 32 + it2 * 2 + lane / 16;
                     const int sw = (chunk & ~7) | ((chunk ^ rr) & 7);
                     const uint4 wv = *reinterpret_cast<const uint4 *>(stage + rr * 256 + sw * 16);
-                    const long long grow = m0 + rr;
-                    if (ok && grow < p.m && col < p.n) *reinterpret_cast<uint4 *>(cptr + base + (size_t)rr * row_stride) = wv;
+                    if (ok && rr < rows_valid && col < p.n) *reinterpret_cast<uint4 *>(cptr + base + (size_t)rr * row_stride) = wv;
                 }
                 __syncwarp();
             }
@@ -317,29 +320,71 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     if (warp == 4) tmem_dealloc_pair(tmem, 512);
 }
 
-bool view_ok(const MatView &v, int row_box)
+// The batch entries the rows of a product are walked by. A head-major view whose seq is a multiple of the
+// boxes' rows can be tiled as if its rows were consecutive; otherwise tiles (NN, NT: rows of A and C) or
+// contraction steps (TN: rows of A and B) stop at the end of each entry, the copy engine fills the rest
+// of the box with zeros, and what is computed for them is not stored. A row-major view on the same row
+// axis is then described as one head of `cols` columns, so that its boxes end there too (with rows of the
+// next entry in their place, an infinity among those would meet the other operand's zeros).
+struct RowPlan {
+    bool by_entry;
+    int batch, seq, seq_pad;
+};
+
+RowPlan row_plan(const GemmArgs &g)
+{
+    const MatView *axis[2] = {&g.a, g.mode == GEMM_TN ? &g.b : &g.c};
+    const long long rows = g.mode == GEMM_TN ? g.k : g.m;
+    const int box = g.mode == GEMM_TN ? BK : BM;
+    for (const MatView *v : axis)
+        if (v->heads > 0 && v->seq % box != 0) return {true, (int)(rows / v->seq), v->seq, (v->seq + box - 1) / box * box};
+    return {false, 1, (int)rows, (int)((rows + 2 * BM - 1) / (2 * BM) * (2 * BM))};
+}
+
+bool view_ok(const MatView &v)
 {
     if (((uintptr_t)v.ptr & 15) != 0) return false;
     if (v.heads == 0) return v.cols % 8 == 0;
-    // head-major: a box of 64 columns must stay inside one head and a box of rows inside one batch entry
-    return v.dim % 64 == 0 && v.seq % row_box == 0 && v.rows % v.seq == 0 && v.cols % (v.heads * v.dim) == 0;
+    // head-major: a box of 64 columns must stay inside one head
+    return v.dim % 64 == 0 && v.rows % v.seq == 0 && v.cols % (v.heads * v.dim) == 0;
 }
 
 template <int MODE>
 int launch(const GemmArgs &g, DeviceState *st, cudaStream_t s)
 {
+    const RowPlan rows = row_plan(g);
+    MatView va = g.a, vb = g.b;
+    ViewGeom ga = {va.heads, va.seq, va.dim}, gb = {vb.heads, vb.seq, vb.dim};
+    auto by_entry = [&](MatView &v, ViewGeom &geom) {
+        if (v.heads == 0) { v.heads = 1; v.seq = rows.seq; v.dim = v.cols; }
+        geom = {v.heads, rows.seq_pad, v.dim};
+    };
+    if (rows.by_entry) {
+        by_entry(va, ga);
+        if (MODE == GEMM_TN) by_entry(vb, gb);
+    }
     CUtensorMap ta, tb;
     int rc;
-    if ((rc = make_tensor_map_bf16_view(&ta, g.a, 64, MODE == GEMM_TN ? 64 : BM)) != EMBER_OK) return rc;
-    if ((rc = make_tensor_map_bf16_view(&tb, g.b, 64, MODE == GEMM_NT ? BNH : 64)) != EMBER_OK) return rc;
+    if ((rc = make_tensor_map_bf16_view(&ta, va, 64, MODE == GEMM_TN ? 64 : BM)) != EMBER_OK) return rc;
+    if ((rc = make_tensor_map_bf16_view(&tb, vb, 64, MODE == GEMM_NT ? BNH : 64)) != EMBER_OK) return rc;
     GemmParams p;
-    p.m = g.m;
     p.n = g.n;
-    p.k = g.k;
-    p.tiles_m = (int)((g.m + 2 * BM - 1) / (2 * BM));
+    if (MODE == GEMM_TN) {  // the result's rows are columns of A: one entry
+        p.tiles_m = (int)((g.m + 2 * BM - 1) / (2 * BM));
+        p.kblocks = rows.by_entry ? rows.batch * (rows.seq_pad / BK) : (g.k + BK - 1) / BK;
+        p.batch = 1;
+        p.seq = (int)g.m;
+        p.seq_pad = p.tiles_m * 2 * BM;
+    } else {
+        p.batch = rows.batch;
+        p.seq = rows.seq;
+        p.seq_pad = rows.seq_pad;
+        p.tiles_m = (int)(((long long)p.batch * p.seq_pad + 2 * BM - 1) / (2 * BM));
+        p.kblocks = (g.k + BK - 1) / BK;
+    }
     p.tiles_n = (g.n + BN - 1) / BN;
-    p.a = {g.a.heads, g.a.seq, g.a.dim};
-    p.b = {g.b.heads, g.b.seq, g.b.dim};
+    p.a = ga;
+    p.b = gb;
     p.c = g.c;
     p.bias = (const __nv_bfloat16 *)g.bias;
     p.status = st->status;
@@ -372,10 +417,21 @@ bool sm100_gemm_supported(const GemmArgs &g)
     if (g.dtype != EMBER_BF16 || g.m <= 0 || g.n <= 0 || g.k <= 0) return false;
     if (g.m > 0x7fffff00LL || g.a.rows > 0x7fffff00LL || g.b.rows > 0x7fffff00LL) return false;  // 32-bit box coordinates
     if ((g.m + 2 * BM - 1) / (2 * BM) * (long long)((g.n + BN - 1) / BN) > 0x7fffffffLL) return false;
-    if (g.n % 8 != 0 || ((uintptr_t)g.c.ptr & 15) != 0) return false;       // 16-byte output chunks
-    if (g.c.heads > 0 && (g.c.dim % 8 != 0 || g.c.seq % BM != 0)) return false;  // a CTA's 128 result rows lie in one batch entry
-    const int a_rows = g.mode == GEMM_TN ? 64 : BM, b_rows = g.mode == GEMM_NT ? BNH : 64;
-    return view_ok(g.a, a_rows) && view_ok(g.b, b_rows);
+    if (g.n % 8 != 0 || ((uintptr_t)g.c.ptr & 15) != 0) return false;  // 16-byte output chunks
+    if (g.c.heads > 0 && g.c.dim % 8 != 0) return false;
+    if (!view_ok(g.a) || !view_ok(g.b)) return false;
+    if (g.mode != GEMM_TN && g.b.heads != 0) return false;  // no caller has a head-major weight
+    const RowPlan rows = row_plan(g);
+    if (!rows.by_entry) return true;
+    // Every head-major view on the row axis has the same entries. Padding an entry to whole boxes pays
+    // while the tensor core still beats the CUDA cores on the valid rows: they run at 20 to 25 TFLOP/s, this
+    // kernel at 600 and more, so from one row in sixteen.
+    for (const MatView *v : {&g.a, g.mode == GEMM_TN ? &g.b : &g.c})
+        if (v->heads > 0 && v->seq != rows.seq) return false;
+    const long long padded = (long long)rows.batch * rows.seq_pad;
+    const long long total = g.mode == GEMM_TN ? g.k : g.m;
+    if ((long long)rows.batch * rows.seq != total || rows.seq * 16LL < rows.seq_pad) return false;
+    return padded <= 0x7fffff00LL && (g.mode == GEMM_TN || (padded + 2 * BM - 1) / (2 * BM) * (long long)((g.n + BN - 1) / BN) <= 0x7fffffffLL);
 }
 
 int sm100_gemm(const GemmArgs &g, DeviceState *st, cudaStream_t s)
