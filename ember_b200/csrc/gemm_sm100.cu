@@ -63,6 +63,7 @@ struct GemmParams {
     int batch, seq, seq_pad;
     ViewGeom a, b;
     MatView c;
+    int c_vec;  // rows of c are 16-byte aligned: 16-byte stores
     const __nv_bfloat16 *bias;
     DeviceStatus *status;
 };
@@ -298,6 +299,26 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                 // of a chunk is found without divisions in the loop: this thread's column is fixed, and
                 // the 128 rows of a CTA's tile lie inside one batch entry and therefore at one distance
                 // from each other (row-major: `cols` apart; head-major: `dim`).
+                if (!p.c_vec) {
+                    // Rows at any alignment (row-major, columns no multiple of 8): one element per lane,
+                    // 64 contiguous bytes per store instruction.
+                    if (rows_valid > 0) {
+                        __nv_bfloat16 *crow = cptr + ((size_t)l0 + warp * 32) * p.c.cols + n0 + half * 128;
+                        const int rows_here = min(32, rows_valid - warp * 32), cols_here = min(128, p.n - n0 - half * 128);
+#pragma unroll 4
+                        for (int rr = 0; rr < rows_here; rr++) {
+                            const int tr = warp * 32 + rr;
+#pragma unroll
+                            for (int i = 0; i < 4; i++) {
+                                const int e = i * 32 + lane, chunk = e / 8, sw = (chunk & ~7) | ((chunk ^ tr) & 7);
+                                const __nv_bfloat16 v = *reinterpret_cast<const __nv_bfloat16 *>(stage + tr * 256 + sw * 16 + (e % 8) * 2);
+                                if (ok && e < cols_here) crow[(size_t)rr * p.c.cols + e] = v;
+                            }
+                        }
+                    }
+                    __syncwarp();
+                    continue;
+                }
                 const int chunk = lane % 16;
                 const int col = n0 + half * 128 + chunk * 8;
                 const size_t row_stride = p.c.heads == 0 ? (size_t)p.c.cols : (size_t)p.c.dim;
@@ -340,6 +361,8 @@ RowPlan row_plan(const GemmArgs &g)
         if (v->heads > 0 && v->seq % box != 0) return {true, (int)(rows / v->seq), v->seq, (v->seq + box - 1) / box * box};
     return {false, 1, (int)rows, (int)((rows + 2 * BM - 1) / (2 * BM) * (2 * BM))};
 }
+
+bool c_rows_aligned(const GemmArgs &g) { return g.n % 8 == 0 && ((uintptr_t)g.c.ptr & 15) == 0; }
 
 bool view_ok(const MatView &v)
 {
@@ -386,6 +409,7 @@ int launch(const GemmArgs &g, DeviceState *st, cudaStream_t s)
     p.a = ga;
     p.b = gb;
     p.c = g.c;
+    p.c_vec = c_rows_aligned(g);
     p.bias = (const __nv_bfloat16 *)g.bias;
     p.status = st->status;
     auto kern = sm100_gemm_kernel<MODE>;
@@ -417,12 +441,12 @@ bool sm100_gemm_supported(const GemmArgs &g)
     if (g.dtype != EMBER_BF16 || g.m <= 0 || g.n <= 0 || g.k <= 0) return false;
     if (g.m > 0x7fffff00LL || g.a.rows > 0x7fffff00LL || g.b.rows > 0x7fffff00LL) return false;  // 32-bit box coordinates
     if ((g.m + 2 * BM - 1) / (2 * BM) * (long long)((g.n + BN - 1) / BN) > 0x7fffffffLL) return false;
-    if (g.n % 8 != 0 || ((uintptr_t)g.c.ptr & 15) != 0) return false;  // 16-byte output chunks
-    if (g.c.heads > 0 && g.c.dim % 8 != 0) return false;
+    if (g.c.heads > 0 && (g.c.dim % 8 != 0 || !c_rows_aligned(g))) return false;  // 16-byte output chunks
     if (!view_ok(g.a) || !view_ok(g.b)) return false;
     if (g.mode != GEMM_TN && g.b.heads != 0) return false;  // no caller has a head-major weight
     const RowPlan rows = row_plan(g);
     if (!rows.by_entry) return true;
+    if (g.mode != GEMM_TN && !c_rows_aligned(g)) return false;  // element stores know one batch entry only
     // Every head-major view on the row axis has the same entries. Padding an entry to whole boxes pays
     // while the tensor core still beats the CUDA cores on the valid rows: they run at 20 to 25 TFLOP/s, this
     // kernel at 600 and more, so from one row in sixteen.
@@ -432,6 +456,52 @@ bool sm100_gemm_supported(const GemmArgs &g)
     const long long total = g.mode == GEMM_TN ? g.k : g.m;
     if ((long long)rows.batch * rows.seq != total || rows.seq * 16LL < rows.seq_pad) return false;
     return padded <= 0x7fffff00LL && (g.mode == GEMM_TN || (padded + 2 * BM - 1) / (2 * BM) * (long long)((g.n + BN - 1) / BN) <= 0x7fffffffLL);
+}
+
+// dst (rows x 8*chunks) = src (rows x cols) with zeros past the last column. The source has rows at any
+// alignment: a lane makes 16 bytes of a row from 4 words, or from 3 words and the halves at the two ends.
+// A block takes 8 rows x 256 chunks, a warp one row, so that short and long rows both spread over the SMs.
+__global__ void __launch_bounds__(256) pack_rows_kernel(const unsigned short *__restrict__ src, uint4 *__restrict__ dst, long long rows,
+                                                        int cols, int chunks)
+{
+    const long long row = (long long)blockIdx.x * 8 + threadIdx.x / 32;
+    if (row >= rows) return;
+    const int end = min(chunks, ((int)blockIdx.y + 1) * 256);
+    const unsigned short *r = src + (size_t)row * cols;
+    const bool odd = ((uintptr_t)r & 2) != 0;  // rows are 2-byte aligned
+#pragma unroll 4
+    for (int c = blockIdx.y * 256 + threadIdx.x % 32; c < end; c += 32) {
+        uint32_t w[4];
+        const unsigned short *e = r + (size_t)c * 8;
+        if (c * 8 + 8 > cols) {
+            unsigned short h[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) h[i] = c * 8 + i < cols ? e[i] : (unsigned short)0;
+#pragma unroll
+            for (int i = 0; i < 4; i++) w[i] = (uint32_t)h[2 * i] | (uint32_t)h[2 * i + 1] << 16;
+        } else if (odd) {
+            const uint32_t *m = reinterpret_cast<const uint32_t *>(e + 1);
+            const uint32_t first = e[0], a = m[0], b = m[1], d = m[2], last = e[7];
+            w[0] = first | a << 16;
+            w[1] = a >> 16 | b << 16;
+            w[2] = b >> 16 | d << 16;
+            w[3] = d >> 16 | last << 16;
+        } else {
+            const uint32_t *m = reinterpret_cast<const uint32_t *>(e);
+#pragma unroll
+            for (int i = 0; i < 4; i++) w[i] = m[i];
+        }
+        dst[(size_t)row * chunks + c] = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+}
+
+int pack_rows(const MatView &v, void *dst, cudaStream_t s)
+{
+    const int chunks = (v.cols + 7) / 8;
+    const dim3 grid((unsigned)((v.rows + 7) / 8), (unsigned)((chunks + 255) / 256));
+    pack_rows_kernel<<<grid, 256, 0, s>>>((const unsigned short *)v.ptr, (uint4 *)dst, v.rows, v.cols, chunks);
+    EMBER_CUDA_TRY(cudaGetLastError());
+    return EMBER_OK;
 }
 
 int sm100_gemm(const GemmArgs &g, DeviceState *st, cudaStream_t s)

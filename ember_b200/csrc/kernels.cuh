@@ -105,6 +105,8 @@ int column_sums(const MatView &a, void *out, int dtype, cudaStream_t s);  // out
 // tcgen05 kernel (gemm_sm100.cu): bf16 storage; see sm100_gemm_supported for the shapes it takes.
 bool sm100_gemm_supported(const GemmArgs &g);
 int sm100_gemm(const GemmArgs &g, DeviceState *st, cudaStream_t s);
+// dst (bf16, 16-byte aligned, rows of v.cols rounded up to 8) = v (row-major, any alignment), zeros past v.cols
+int pack_rows(const MatView &v, void *dst, cudaStream_t s);
 // tcgen05 kernel for at most 128 rows (gemm_skinny_sm100.cu): a decode step's projections.
 bool sm100_skinny_gemm_supported(const GemmArgs &g);
 int sm100_skinny_gemm(const GemmArgs &g, DeviceState *st, cudaStream_t s);

@@ -43,8 +43,72 @@ MatView view(const void *p, long long rows, int cols, int heads, const LinearSha
     return v;
 }
 
-int run(const GemmArgs &g, DeviceState *st, cudaStream_t s)
+// Copies of operands whose rows are no multiple of 16 bytes (a vocabulary of 50257 columns, say), padded with
+// zeros to rows that the copy engine can fetch. They live for one entry point's call, so that the two
+// gradients of a backward call share the copy of dy, and are freed in stream order.
+struct PackedOperands {
+    cudaStream_t stream;
+    int count = 0;
+    MatView from[4], to[4];  // x, dy and w are all there are
+
+    explicit PackedOperands(cudaStream_t s) : stream(s) {}
+    PackedOperands(const PackedOperands &) = delete;
+    PackedOperands &operator=(const PackedOperands &) = delete;
+    ~PackedOperands()
+    {
+        for (int i = 0; i < count; i++) cudaFreeAsync(const_cast<void *>(to[i].ptr), stream);
+    }
+    int get(MatView &v)
+    {
+        for (int i = 0; i < count; i++)
+            if (from[i].ptr == v.ptr && from[i].rows == v.rows && from[i].cols == v.cols) {
+                v = to[i];
+                return EMBER_OK;
+            }
+        MatView t = v;
+        t.cols = (v.cols + 7) / 8 * 8;
+        void *buf = nullptr;
+        EMBER_CUDA_TRY(cudaMallocAsync(&buf, (size_t)t.rows * t.cols * 2, stream));
+        t.ptr = buf;
+        from[count] = v;
+        to[count++] = t;
+        const int rc = pack_rows(v, buf, stream);
+        v = t;
+        return rc;
+    }
+};
+
+bool needs_packing(const MatView &v) { return v.heads == 0 && (v.cols % 8 != 0 || ((uintptr_t)v.ptr & 15) != 0); }
+
+// Whether a product that the tensor-core kernels refuse for its operands' rows is to run on copies of them.
+// A copy costs a launch or two and the CUDA-core kernel is quick on small products. Forward / both gradients, us,
+// CUDA cores -> copies: 2.7e7 flop a product (256 x 101 x 512) 14 / 33 -> 21 / 39, 6.7e7 (256 x 513 x 256)
+// 19 / 45 -> 19 / 43, 1.1e8 (512 x 101 x 1024) 29 / 50 -> 23 / 40, 2.1e9 (1024 x 1001 x 1024) 160 / 268 -> 25 / 50,
+// 1.2e10 (2000 x 3001 x 1024) 566 / 1372 -> 35 / 71.
+constexpr double kPackFlops = 8e7;
+
+bool worth_packing(const GemmArgs &g)
 {
+    if (g.dtype != EMBER_BF16 || (!needs_packing(g.a) && !needs_packing(g.b))) return false;
+    if (2.0 * (double)g.m * g.n * g.k < kPackFlops) return false;
+    if (g.a.rows > 0x7fffff00LL || g.b.rows > 0x7fffff00LL) return false;
+    GemmArgs t = g;
+    for (MatView *v : {&t.a, &t.b})
+        if (needs_packing(*v)) {
+            if (v->cols > 0x7ffffff0) return false;
+            v->cols = (v->cols + 7) / 8 * 8;
+            v->ptr = (const void *)(uintptr_t)256;
+        }
+    return sm100_skinny_gemm_supported(t) || sm100_gemm_supported(t);
+}
+
+int run(GemmArgs g, DeviceState *st, cudaStream_t s, PackedOperands &packed)
+{
+    if (worth_packing(g)) {
+        int rc;
+        if (needs_packing(g.a) && (rc = packed.get(g.a)) != EMBER_OK) return rc;
+        if (needs_packing(g.b) && (rc = packed.get(g.b)) != EMBER_OK) return rc;
+    }
     if (sm100_skinny_gemm_supported(g)) return sm100_skinny_gemm(g, st, s);
     if (sm100_gemm_supported(g)) return sm100_gemm(g, st, s);
     return simt_gemm(g, st, s);
@@ -70,7 +134,8 @@ int ember_linear_fwd(const void *x, const void *w, const void *bias, void *y, lo
     g.c = view(y, m, n, y_heads, sh);
     g.bias = bias;
     g.m = m; g.n = n; g.k = k; g.dtype = dtype;
-    return run(g, st, pick_stream(stream, st));
+    PackedOperands packed(pick_stream(stream, st));
+    return run(g, st, packed.stream, packed);
 }
 
 int ember_linear_bwd(const void *x, const void *w, const void *dy, void *dx, void *dw, void *db, long long m, int n,
@@ -85,6 +150,7 @@ int ember_linear_bwd(const void *x, const void *w, const void *dy, void *dx, voi
     DeviceState *st = device_state();
     if (!st) return EMBER_ERR_CUDA;
     cudaStream_t s = pick_stream(stream, st);
+    PackedOperands packed(s);
     const MatView vx = view(x, m, k, x_heads, sh), vdy = view(dy, m, n, y_heads, sh);
     if (dw) {  // grad_w (k x n) = x^T dy
         GemmArgs g;
@@ -93,7 +159,7 @@ int ember_linear_bwd(const void *x, const void *w, const void *dy, void *dx, voi
         g.b = vdy;
         g.c = view(dw, k, n, 0, sh);
         g.m = k; g.n = n; g.k = (int)m; g.dtype = dtype;
-        if ((rc = run(g, st, s)) != EMBER_OK) return rc;
+        if ((rc = run(g, st, s, packed)) != EMBER_OK) return rc;
     }
     if (db && (rc = column_sums(vdy, db, dtype, s)) != EMBER_OK) return rc;  // grad_b = sum(dy, axis 0)
     if (dx) {  // grad_x (m x k) = dy w^T
@@ -103,7 +169,7 @@ int ember_linear_bwd(const void *x, const void *w, const void *dy, void *dx, voi
         g.b = view(w, k, n, 0, sh);
         g.c = view(dx, m, k, x_heads, sh);
         g.m = m; g.n = k; g.k = n; g.dtype = dtype;
-        if ((rc = run(g, st, s)) != EMBER_OK) return rc;
+        if ((rc = run(g, st, s, packed)) != EMBER_OK) return rc;
     }
     return EMBER_OK;
 }
@@ -130,7 +196,7 @@ const char *ember_linear_kernel_name(int product, long long m, int n, int k, int
         g.a = view(p, m, k, x_heads, sh); g.b = view(p, k, n, 0, sh); g.c = view(p, m, n, y_heads, sh);
         g.m = m; g.n = n; g.k = k;
     }
-    return sm100_skinny_gemm_supported(g) || sm100_gemm_supported(g) ? "sm100_tcgen05" : "simt_f32";
+    return worth_packing(g) || sm100_skinny_gemm_supported(g) || sm100_gemm_supported(g) ? "sm100_tcgen05" : "simt_f32";
 }
 
 }  // extern "C"

@@ -1,0 +1,62 @@
+"""Linear layers whose rows are no multiple of 16 bytes (odd vocabularies, odd feature counts, operands at odd
+offsets): products large enough run on the tensor-core kernels with padded copies of the operands. Against the
+CPU oracle; results in a canary-filled buffer, so that a store past a row's or the matrix's end shows.
+
+Tolerance: bfloat16 results, half a unit in the last place (2^-9 of the value) plus the float32 sum's rounding."""
+import numpy as np
+import pytest
+
+import ember_b200 as em
+from conftest import bf16_round, seeded
+from ember_b200 import _lib
+from oracle import cpu_oracle
+
+pytestmark = pytest.mark.gpu
+TOL = 2.0 ** -8
+
+
+def close(got, ref, name):
+    assert got.shape == ref.shape and np.abs(got - ref).max() <= TOL * np.abs(ref).max(), name
+
+
+# one column past and short of a tile, less than 8 columns past it, odd features, few rows, one extent odd at a time
+@pytest.mark.parametrize("m,n,k", [(512, 513, 512), (300, 1023, 520), (200, 1025, 1000), (260, 2001, 261), (1000, 300, 777),
+                                   (129, 4999, 344), (100, 2047, 1024), (16, 8190, 1024), (2000, 101, 1024), (515, 768, 515)])
+def test_odd_extents(m, n, k):
+    for product in range(3):
+        assert _lib.lib().ember_linear_kernel_name(product, m, n, k, _lib.EMBER_BF16, 0, 0, 0, 0) == b"sm100_tcgen05"
+    x, w, b, g = (bf16_round(seeded(s, i)) for i, s in enumerate(((m, k), (k, n), (n,), (m, n)), 1))
+    tx, tw, tb, tg = (em.Tensor(a, "bfloat16") for a in (x, w, b, g))
+    close(em.linear_forward(tx, tw, tb).to_np(), cpu_oracle.linear_fwd(x, w, b), "y")
+    for got, ref, name in zip(em.linear_backward(tx, tw, tg), cpu_oracle.linear_bwd(x, w, g), ("grad_x", "grad_w", "grad_b")):
+        close(got.to_np(), ref, name)
+
+
+@pytest.mark.parametrize("m,n,k,offset", [(300, 1001, 512, 0), (300, 1000, 512, 3), (130, 1999, 600, 4)])
+def test_stores_stay_inside_and_bases_at_any_offset(m, n, k, offset):
+    x, w, b = (bf16_round(seeded(s, i)) for i, s in enumerate(((m, k), (k, n), (n,)), 1))
+    lead, canary = 8 + offset, 7.0
+
+    def placed(a):
+        flat = np.full(a.size + 2 * lead, canary, np.float32)
+        flat[lead:lead + a.size] = a.ravel()
+        t = em.Tensor(flat, "bfloat16")
+        return t, t.view(lead, a.shape)
+
+    (_, vx), (_, vw), (_, vb) = placed(x), placed(w), placed(b)
+    ty, vy = placed(np.zeros((m, n), np.float32))
+    L = _lib.lib()
+    _lib.check(L.ember_linear_fwd(vx.ptr, vw.ptr, vb.ptr, vy.ptr, m, n, k, _lib.EMBER_BF16, 0, 0, 0, 0, None))
+    flat = ty.to_np()
+    assert (flat[:lead] == canary).all() and (flat[lead + m * n:] == canary).all()
+    close(flat[lead:lead + m * n].reshape(m, n), cpu_oracle.linear_fwd(x, w, b), "y")
+
+
+def test_non_finite_values_stay_where_they_belong():
+    m, n, k = 300, 1001, 515
+    x, w = (bf16_round(np.abs(seeded(s, i)) + 0.5) for i, s in enumerate(((m, k), (k, n)), 1))
+    x[7, k - 1], w[k - 1, n - 1] = np.inf, np.inf
+    y = em.linear_forward(em.Tensor(x, "bfloat16"), em.Tensor(w, "bfloat16"), None).to_np()
+    want = np.zeros((m, n), bool)
+    want[7], want[:, n - 1] = True, True
+    assert np.array_equal(np.isinf(y), want) and not np.isnan(y).any()
