@@ -156,13 +156,16 @@ __device__ __forceinline__ void f_tma_3d(uint32_t dst, const CUtensorMap *m, uin
     if constexpr (PAIR) tma_load_3d_pair(dst, m, bar, c0, c1, c2); else tma_load_3d(dst, m, bar, c0, c1, c2);
 }
 
-template <int HD, int EMU, bool PAIR>
+// PART: head dimensions below HD. The tiles in shared memory keep HD columns (zeros past d), but the score
+// products stop after the last 16 columns that hold anything and the PV products are that many columns wide.
+template <int HD, int EMU, bool PAIR, bool PART = false>
 __global__ void __launch_bounds__(FWD_THREADS, 1)
     sm100_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                      const __grid_constant__ CUtensorMap tm_v, const FwdParams p)
 {
     using C = FwdCfg<HD, PAIR>;
     static_assert(!PAIR || HD == 128, "the pair form halves V along its 128 columns");
+    static_assert(!PAIR || !PART, "pairs take whole tiles");
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t *smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -315,7 +318,8 @@ __global__ void __launch_bounds__(FWD_THREADS, 1)
             // ------------------------------------------------------------ MMA issue for tile t (of both CTAs of a pair)
             const int t = warp - 8;
             constexpr uint32_t IDESC_S = idesc_bf16_f32(PAIR ? 256 : 128, 128, 0, 0);
-            constexpr uint32_t IDESC_O = idesc_bf16_f32(PAIR ? 256 : 128, HD, 0, 1);
+            const int ksteps = PART ? (p.d + 15) / 16 : HD / 16;
+            const uint32_t IDESC_O = idesc_bf16_f32(PAIR ? 256 : 128, ksteps * 16, 0, 1);
             const int nt = n_t[t], no = n_t[1 - t];  // key tiles of this tile / of the other tile
             const uint32_t q_lo = desc_lo(smem_base + C::OFF_Q + t * C::TILE_BYTES, 16);
             bool ok = mbar_wait(BAR(B_Q), 0, abort_flag, p.status, W_MMA_Q);
@@ -339,7 +343,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 1)
                 for (int ks = 0; ks < HD / 16; ks++) {
                     const uint32_t o16 = ((ks / 4) * C::SUB_BYTES + (ks % 4) * 32) >> 4;
                     const uint32_t k16 = ((ks / 4) * C::K_SUB_BYTES + (ks % 4) * 32) >> 4;
-                    f_mma_ss<PAIR>(tmem + C::TMEM_S, q_lo + o16, k_lo + k16, IDESC_S, ks > 0);
+                    if (!PART || ks < ksteps) f_mma_ss<PAIR>(tmem + C::TMEM_S, q_lo + o16, k_lo + k16, IDESC_S, ks > 0);
                 }
                 f_commit<PAIR>(BAR(B_S + t));
             };
@@ -670,8 +674,8 @@ static int fwd_block_rows(const AttnArgs &a, DeviceState *st)
     return 256;
 }
 
-template <int HD, int EMU>
-int launch(const AttnArgs &a, DeviceState *st, cudaStream_t s)
+template <int HD, int EMU, bool PART>
+int launch_form(const AttnArgs &a, DeviceState *st, cudaStream_t s)
 {
     using C = FwdCfg<HD>;
     CUtensorMap tq, tk, tv;
@@ -694,7 +698,7 @@ int launch(const AttnArgs &a, DeviceState *st, cudaStream_t s)
     p.chunk = a.lk;
     p.lens_div = 1;
     p.seq_lens = nullptr;
-    auto kern = sm100_fwd_kernel<HD, EMU, false>;
+    auto kern = sm100_fwd_kernel<HD, EMU, false, PART>;
     static SmemOptIn opt_in;
     EMBER_CUDA_TRY(opt_in(kern, C::SMEM_BYTES));
     p.order = make_work_order(a.bh, (a.lq + p.block_rows - 1) / p.block_rows, st->sm_count, ((size_t)a.lq + a.lk) * HD * 2 * 2,  // Q, O, K, V
@@ -703,6 +707,12 @@ int launch(const AttnArgs &a, DeviceState *st, cudaStream_t s)
     kern<<<grid, FWD_THREADS, C::SMEM_BYTES, s>>>(tq, tk, tv, p);
     EMBER_CUDA_TRY(cudaGetLastError());
     return EMBER_OK;
+}
+
+template <int HD, int EMU>
+int launch(const AttnArgs &a, DeviceState *st, cudaStream_t s)
+{
+    return a.d <= HD - 16 ? launch_form<HD, EMU, true>(a, st, s) : launch_form<HD, EMU, false>(a, st, s);
 }
 
 // Merges the normalised partial outputs of the splits of one (unit, query row):
