@@ -219,10 +219,42 @@ __global__ void __launch_bounds__(W < 256 ? 256 : W) row_softmax_kernel(const T 
 // W = 256: 64 KB) this replaces the shared-memory cache of row_softmax_kernel: there a thread has four
 // loads in flight during the first pass only, and nothing while it reduces and writes, which left the
 // kernels latency-bound at 0.5-0.75 of the copy bandwidth. Two blocks per SM (128 registers per thread)
-// so that one block's loads run under the other's arithmetic. 16-byte aligned rows only. MAXV: pieces
+// so that one block's loads run under the other's arithmetic. MAXV: pieces
 // per thread (a power of two up to 16, the smallest that covers the row: loops over pieces that do not
 // exist would still cost their issue slots).
-template <typename T, int W, int MODE, int MAXV>
+// EDGE: rows of any length. The pieces are those of the whole tensor's 16-byte grid that the row touches; its
+// first and last piece may hold elements of the neighbours, which become -inf as soon as they are loaded
+// (no weight in the maximum or the sum), take no part in the loss and are not stored. Element by element, as
+// such rows were read before, 2000 x 3001 bf16 cross-entropy took 35 us (22 now, cold caches).
+template <typename T>
+__device__ __forceinline__ void clear_outside(uint4 &u, int e0, int cols)  // element i of the piece is element e0 + i of the row
+{
+    uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        if constexpr (sizeof(T) == 4) {
+            if (e0 + i < 0 || e0 + i >= cols) w[i] = 0xff800000u;
+        } else {
+            if (e0 + 2 * i < 0 || e0 + 2 * i >= cols) w[i] = (w[i] & 0xffff0000u) | 0xff80u;
+            if (e0 + 2 * i + 1 < 0 || e0 + 2 * i + 1 >= cols) w[i] = (w[i] & 0xffffu) | 0xff800000u;
+        }
+    }
+    u = make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// Piece `g` of a tensor of `total` elements; the last one may reach past the end and is then put together.
+template <typename T>
+__device__ __forceinline__ uint4 load_piece(const T *base, size_t g, size_t total)
+{
+    constexpr int NV = Vec16<T>::NV;
+    if ((g + 1) * NV <= total) return reinterpret_cast<const uint4 *>(base)[g];
+    float v[NV];
+#pragma unroll
+    for (int i = 0; i < NV; i++) v[i] = g * NV + i < total ? ldf(base + g * NV + i) : 0.f;
+    return Vec16<T>::pack(v);
+}
+
+template <typename T, int W, int MODE, int MAXV, bool EDGE>
 __global__ void __launch_bounds__(256, 2) row_softmax_regs_kernel(const T *__restrict__ x, const T *__restrict__ target,
                                                                    T *__restrict__ y, float *__restrict__ row_loss,
                                                                    long long rows, int cols)
@@ -231,16 +263,22 @@ __global__ void __launch_bounds__(256, 2) row_softmax_regs_kernel(const T *__res
     constexpr int GROUPS = 256 / W, NV = Vec16<T>::NV;
     constexpr float kLog2e = 1.4426950408889634f;
     const int group = threadIdx.x / W, t = threadIdx.x % W;
-    const int nvec = cols / NV;
     for (long long row0 = (long long)blockIdx.x * GROUPS; row0 < rows; row0 += (long long)gridDim.x * GROUPS) {
         const long long row = row0 + group;
         const bool active = row < rows;  // W == 256: always true; W == 32: the whole warp agrees
-        const uint4 *xv = reinterpret_cast<const uint4 *>(x + (size_t)(active ? row : 0) * cols);
+        const size_t first = (size_t)(active ? row : 0) * cols, g0 = first / NV, total = (size_t)rows * cols;
+        const int lead = EDGE ? (int)(first - g0 * NV) : 0;  // elements of the row before in the first piece
+        const int nvec = EDGE ? (lead + cols + NV - 1) / NV : cols / NV;
+        const uint4 *xv = reinterpret_cast<const uint4 *>(x) + g0;
+        auto whole = [&](int j) { return !EDGE || (j * NV >= lead && (j + 1) * NV <= lead + cols); };
         uint4 raw[MAXV];
 #pragma unroll
         for (int i = 0; i < MAXV; i++) {
             const int j = t + i * W;
-            if (active && j < nvec) raw[i] = xv[j];
+            if (active && j < nvec) {
+                raw[i] = EDGE ? load_piece(x, g0 + j, total) : xv[j];
+                if (!whole(j)) clear_outside<T>(raw[i], j * NV - lead, cols);
+            }
         }
         // ---- maximum
         float m = -INFINITY;
@@ -272,8 +310,9 @@ __global__ void __launch_bounds__(256, 2) row_softmax_regs_kernel(const T *__res
         const float mlg2 = (m + lg) * kLog2e;  // exp(x - m - lg) = exp2(x * log2(e) - mlg2)
         float loss = 0.f;
         if (active) {
-            uint4 *yv = reinterpret_cast<uint4 *>(y + (size_t)row * cols);
-            const uint4 *tv4 = MODE == MODE_CROSS_ENTROPY ? reinterpret_cast<const uint4 *>(target + (size_t)row * cols) : nullptr;
+            uint4 *yv = reinterpret_cast<uint4 *>(y) + g0;
+            const uint4 *tv4 = MODE == MODE_CROSS_ENTROPY ? reinterpret_cast<const uint4 *>(target) + g0 : nullptr;
+            auto load_target = [&](int j) { return EDGE ? load_piece(target, g0 + j, total) : tv4[j]; };
             // cross-entropy: the targets are fetched four pieces at a time (the registers hold the row),
             // one group ahead of the group being computed
             constexpr int TB = MAXV < 4 ? MAXV : 4;
@@ -281,7 +320,7 @@ __global__ void __launch_bounds__(256, 2) row_softmax_regs_kernel(const T *__res
             if (MODE == MODE_CROSS_ENTROPY) {
 #pragma unroll
                 for (int i = 0; i < TB; i++)
-                    if (t + i * W < nvec) tnext[i] = tv4[t + i * W];
+                    if (t + i * W < nvec) tnext[i] = load_target(t + i * W);
             }
 #pragma unroll
             for (int i0 = 0; i0 < MAXV; i0 += TB) {
@@ -292,7 +331,7 @@ __global__ void __launch_bounds__(256, 2) row_softmax_regs_kernel(const T *__res
                     if (i0 + TB < MAXV) {
 #pragma unroll
                         for (int i = 0; i < TB; i++)
-                            if (t + (i0 + TB + i) * W < nvec) tnext[i] = tv4[t + (i0 + TB + i) * W];
+                            if (t + (i0 + TB + i) * W < nvec) tnext[i] = load_target(t + (i0 + TB + i) * W);
                     }
                 }
 #pragma unroll
@@ -309,10 +348,19 @@ __global__ void __launch_bounds__(256, 2) row_softmax_regs_kernel(const T *__res
                             } else {
                                 const float lp = (v[k] - m) - lg;
                                 o[k] = MODE == MODE_LOG_SOFTMAX ? lp : fast_exp2(fmaf(v[k], kLog2e, -mlg2));
-                                if (MODE == MODE_CROSS_ENTROPY) loss = fmaf(tv[k], lp, loss);
+                                if (MODE == MODE_CROSS_ENTROPY && (whole(j) || (j * NV + k >= lead && j * NV + k < lead + cols)))
+                                    loss = fmaf(tv[k], lp, loss);
                             }
                         }
-                        yv[j] = Vec16<T>::pack(o);
+                        if (whole(j)) {
+                            yv[j] = Vec16<T>::pack(o);
+                        } else {
+#pragma unroll
+                            for (int k = 0; k < NV; k++) {
+                                const int e = j * NV + k - lead;
+                                if (e >= 0 && e < cols) stf(y + first + e, o[k]);
+                            }
+                        }
                     }
                 }
             }
@@ -348,6 +396,10 @@ __global__ void __launch_bounds__(BLOCK) ce_backward_kernel(const T *__restrict_
         const uint4 *pv = reinterpret_cast<const uint4 *>(probs), *tv = reinterpret_cast<const uint4 *>(target);
         uint4 *gv = reinterpret_cast<uint4 *>(grad);
         const size_t nvec = total / NV;
+        if (blockIdx.x == 0 && threadIdx.x < total - nvec * NV) {  // what is left of the last piece
+            const size_t i = nvec * NV + threadIdx.x;
+            stf(grad + i, (ldf(probs + i) - ldf(target + i)) * inv_n);
+        }
         for (size_t i = (size_t)blockIdx.x * BLOCK + threadIdx.x; i < nvec; i += (size_t)gridDim.x * BLOCK) {
             float p[NV], t[NV], g[NV];
             Vec16<T>::unpack(pv[i], p);
@@ -369,16 +421,24 @@ int launch_rows(const T *x, const T *target, T *y, float *row_loss, long long ro
                 cudaStream_t s)
 {
     constexpr int NV = Vec16<T>::NV;
-    const bool vec = cols % NV == 0 && aligned16(x) && aligned16(y) && (MODE != MODE_CROSS_ENTROPY || aligned16(target));
+    const bool bases = aligned16(x) && aligned16(y) && (MODE != MODE_CROSS_ENTROPY || aligned16(target));
+    const bool vec = cols % NV == 0 && bases;
     const size_t row_bytes = (size_t)cols * sizeof(T);
     const int width = row_bytes <= WARP_ROW_MAX_BYTES ? 32 : (row_bytes <= BLOCK_ROW_MAX_BYTES ? 256 : 1024);
-    if (vec && width <= 256) {  // the row fits the registers of the threads that own it
-        const int groups_r = 256 / width;
+    // 16-byte pieces that a row touches (without vec: at most, wherever it starts)
+    const long long touched = vec ? cols / NV : ((long long)cols + 2 * NV - 2) / NV;
+    const int width_r = touched <= 16 * 32 ? 32 : 256;
+    if (bases && touched <= 16 * 256 && (vec || cols >= 2 * NV)) {  // the row fits the registers of the threads that own it
+        const int groups_r = 256 / width_r;
         const long long need_r = (rows + groups_r - 1) / groups_r;
         const long long cap_r = (long long)(sm_count > 0 ? sm_count : 148) * 16;
         const int grid_r = (int)(need_r < cap_r ? need_r : cap_r);
-        const int pieces = (cols / NV + width - 1) / width;  // per thread, at most 16 here
-#define EMBER_LAUNCH_REGS(W, NP) row_softmax_regs_kernel<T, W, MODE, NP><<<grid_r, 256, 0, s>>>(x, target, y, row_loss, rows, cols)
+        const int pieces = (int)((touched + width_r - 1) / width_r);  // per thread, at most 16 here
+#define EMBER_LAUNCH_REGS(W, NP)                                                                                                  \
+    do {                                                                                                                          \
+        if (vec) row_softmax_regs_kernel<T, W, MODE, NP, false><<<grid_r, 256, 0, s>>>(x, target, y, row_loss, rows, cols);       \
+        else row_softmax_regs_kernel<T, W, MODE, NP, true><<<grid_r, 256, 0, s>>>(x, target, y, row_loss, rows, cols);            \
+    } while (0)
 #define EMBER_LAUNCH_REGS_W(W)                    \
     do {                                          \
         if (pieces <= 1) EMBER_LAUNCH_REGS(W, 1); \
@@ -387,7 +447,7 @@ int launch_rows(const T *x, const T *target, T *y, float *row_loss, long long ro
         else if (pieces <= 8) EMBER_LAUNCH_REGS(W, 8); \
         else EMBER_LAUNCH_REGS(W, 16);            \
     } while (0)
-        if (width == 32) EMBER_LAUNCH_REGS_W(32); else EMBER_LAUNCH_REGS_W(256);
+        if (width_r == 32) EMBER_LAUNCH_REGS_W(32); else EMBER_LAUNCH_REGS_W(256);
 #undef EMBER_LAUNCH_REGS_W
 #undef EMBER_LAUNCH_REGS
         EMBER_CUDA_TRY(cudaGetLastError());
@@ -497,7 +557,7 @@ int ember_cross_entropy_bwd(const void *probs, const void *target, void *grad, l
     cudaStream_t s = pick_stream(stream, st);
     const size_t total = (size_t)rows * cols;
     const size_t nv = dtype == EMBER_BF16 ? 8 : 4;
-    const bool vec = total % nv == 0 && aligned16(probs) && aligned16(target) && aligned16(grad);
+    const bool vec = aligned16(probs) && aligned16(target) && aligned16(grad);
     const size_t per_block = (size_t)BLOCK * (vec ? nv : 1);
     const size_t want = (total + per_block - 1) / per_block;
     const size_t cap = (size_t)(st->sm_count > 0 ? st->sm_count : 148) * 32;

@@ -1,0 +1,68 @@
+"""Softmax, log-softmax and cross-entropy over rows that start and end inside a 16-byte piece: every alignment
+of a row occurs, rows share their first and last pieces with their neighbours, and the last row's last piece
+reaches past the tensor. Sizes where a row's pieces fill a thread's registers (16 per thread: 512 pieces for a
+warp, 4096 for a block) and one more. Against float64, in buffers with a guard value around the results.
+
+float32: exponentials by ex2.approx (2 ulp of values up to 1) and sums of cols terms: 1e-5. bfloat16: half a
+unit in the last place of the result (2^-9 of the value) besides."""
+import numpy as np
+import pytest
+
+from conftest import bf16_round, seeded
+from ember_b200 import _lib
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+COLS = [16, 33, 63, 129, 1001, 2043, 4089, 4090, 16381, 32753, 32761]
+
+
+@pytest.mark.parametrize("bf16", [False, True])
+@pytest.mark.parametrize("cols", COLS)
+@pytest.mark.parametrize("rows", [1, 9])
+def test_against_float64(rows, cols, bf16):
+    L = _lib.lib()
+    dt, td = (_lib.EMBER_BF16, torch.bfloat16) if bf16 else (_lib.EMBER_F32, torch.float32)
+    x = seeded((rows, cols), 1, 3.0)
+    x = bf16_round(x) if bf16 else x
+    x[0, cols // 3] = -np.inf
+    t = np.zeros((rows, cols), np.float32)
+    t[np.arange(rows), (np.arange(rows) * 7 + cols - 1) % cols] = 1.0
+    z = x.astype(np.float64) - x.max(1, keepdims=True).astype(np.float64)
+    p = np.exp(z) / np.exp(z).sum(1, keepdims=True)
+    tx, tt = torch.from_numpy(x).to("cuda", td), torch.from_numpy(t).to("cuda", td)
+
+    def result():  # the result between two guards of 8 elements
+        buf = torch.full((rows * cols + 16,), 9.0, device="cuda", dtype=td)
+        torch.cuda.synchronize()  # the library works on a stream of its own
+        return buf, buf.data_ptr() + 8 * buf.element_size()
+
+    def check(buf, ref, scale=1.0):
+        torch.cuda.synchronize()
+        b = buf.float().cpu().numpy()
+        assert (b[:8] == 9).all() and (b[-8:] == 9).all()
+        got, ref = b[8:-8].reshape(rows, cols), ref.astype(np.float32)
+        ok = np.isfinite(ref)
+        bound = 1e-5 * (scale + np.abs(ref[ok])) + (2.0 ** -8 * np.abs(ref[ok]) if bf16 else 0)
+        assert (np.abs(got[ok] - ref[ok]) <= bound).all() and np.array_equal(got[~ok], ref[~ok])
+
+    for log in (0, 1):
+        buf, ptr = result()
+        _lib.check(L.ember_softmax_fwd(tx.data_ptr(), ptr, rows, cols, dt, log, None))
+        with np.errstate(divide="ignore"):
+            check(buf, z - np.log(np.exp(z).sum(1, keepdims=True)) if log else p)
+    x[0, cols // 3] = 0.0  # the loss is not defined with an infinite logit
+    tx = torch.from_numpy(x).to("cuda", td)
+    z = x.astype(np.float64) - x.max(1, keepdims=True).astype(np.float64)
+    lse = np.log(np.exp(z).sum(1, keepdims=True))
+    loss = torch.zeros(1, device="cuda")
+    ws = torch.empty(L.ember_cross_entropy_workspace_bytes(rows), device="cuda", dtype=torch.uint8)
+    buf, ptr = result()
+    _lib.check(L.ember_cross_entropy_fwd(tx.data_ptr(), tt.data_ptr(), ptr, loss.data_ptr(), rows, cols, dt, ws.data_ptr(), ws.numel(), None))
+    check(buf, np.exp(z - lse))
+    exact = -((z - lse) * t).sum() / rows
+    assert abs(float(loss[0]) - exact) <= 1e-5 * max(1, abs(exact))
+    probs = buf[8:-8].clone()
+    grad, gptr = result()
+    _lib.check(L.ember_cross_entropy_bwd(probs.data_ptr(), tt.data_ptr(), gptr, rows, cols, dt, None))
+    check(grad, (probs.float().cpu().numpy().reshape(rows, cols).astype(np.float64) - t) / rows, 1 / rows)
