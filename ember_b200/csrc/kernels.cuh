@@ -101,7 +101,8 @@ struct GemmArgs {
 
 // CUDA-core kernels (gemm_simt.cu): float32 math, any shape and view.
 int simt_gemm(const GemmArgs &g, DeviceState *st, cudaStream_t s);
-int column_sums(const MatView &a, void *out, int dtype, cudaStream_t s);  // out[j] = sum over rows of a(:, j)
+// column_sums.cu: out[j] = sum over rows of a(:, j), any shape and view
+int column_sums(const MatView &a, void *out, int dtype, DeviceState *st, cudaStream_t s);
 // tcgen05 kernel (gemm_sm100.cu): bf16 storage; see sm100_gemm_supported for the shapes it takes.
 bool sm100_gemm_supported(const GemmArgs &g);
 int sm100_gemm(const GemmArgs &g, DeviceState *st, cudaStream_t s);

@@ -161,7 +161,7 @@ int ember_linear_bwd(const void *x, const void *w, const void *dy, void *dx, voi
         g.m = k; g.n = n; g.k = (int)m; g.dtype = dtype;
         if ((rc = run(g, st, s, packed)) != EMBER_OK) return rc;
     }
-    if (db && (rc = column_sums(vdy, db, dtype, s)) != EMBER_OK) return rc;  // grad_b = sum(dy, axis 0)
+    if (db && (rc = column_sums(vdy, db, dtype, st, s)) != EMBER_OK) return rc;  // grad_b = sum(dy, axis 0)
     if (dx) {  // grad_x (m x k) = dy w^T
         GemmArgs g;
         g.mode = GEMM_NT;

@@ -1,0 +1,36 @@
+"""Bias gradients (column sums) over the forms the kernel takes: whole 16-byte pieces and single elements, one
+row, fewer rows than a block has, rows that do not divide among a cluster's blocks, one column, head-major
+sequences of length 1, shorter and longer than a block's step.
+
+Float32 sums of m values of order one: within m * 2^-24 of the sum of magnitudes; bfloat16 results another 2^-9."""
+import numpy as np
+import pytest
+
+import ember_b200 as em
+from conftest import bf16_round, seeded
+
+pytestmark = pytest.mark.gpu
+
+
+def check(got, rows, dtype):
+    exact, size = rows.astype(np.float64).sum(0), np.abs(rows).astype(np.float64).sum(0)
+    bound = rows.shape[0] * 2.0 ** -24 * size + (2.0 ** -8 * np.abs(exact) if dtype == "bfloat16" else 0) + 1e-30
+    assert (np.abs(got - exact) <= bound).all()
+
+
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+@pytest.mark.parametrize("m,n", [(1, 8), (1, 1), (31, 64), (33, 72), (64, 3), (255, 130), (1000, 2048), (4099, 77), (5000, 136), (2048, 4608)])
+def test_row_major(m, n, dtype):
+    g = (bf16_round if dtype == "bfloat16" else np.float32)(seeded((m, n), 1))
+    x, w = em.Tensor(np.ones((m, 8), np.float32), dtype), em.Tensor(np.ones((8, n), np.float32), dtype)
+    check(em.linear_backward(x, w, em.Tensor(g, dtype))[2].to_np(), g, dtype)
+
+
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+@pytest.mark.parametrize("batch,seq,heads,dim", [(300, 1, 2, 64), (50, 7, 3, 16), (9, 33, 2, 64), (2, 1000, 1, 128), (3, 129, 2, 5)])
+def test_head_major(batch, seq, heads, dim, dtype):
+    g = (bf16_round if dtype == "bfloat16" else np.float32)(seeded((3, batch, heads, seq, dim), 1))
+    e = heads * dim
+    x, w = em.Tensor(np.ones((batch, seq, e), np.float32), dtype), em.Tensor(np.ones((e, 3 * e), np.float32), dtype)
+    rows = g.transpose(1, 3, 0, 2, 4).reshape(batch * seq, 3 * e)
+    check(em.linear_backward(x, w, em.Tensor(g, dtype), y_heads=heads)[2].to_np(), rows, dtype)
