@@ -34,17 +34,23 @@ namespace {
 
 using namespace ptx;
 
-constexpr int BM = 128, BN = 256, BK = 64, STAGES = 6;  // BM: rows per CTA; a pair covers 2 * BM
-constexpr int BNH = BN / 2;                             // B columns held by one CTA of a pair
-constexpr int A_BYTES = BM * BK * 2, B_BYTES = BNH * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
-constexpr int SUB_BYTES = 64 * 128;                   // 64 rows x 128 bytes
-constexpr int OFF_OUT = STAGES * STAGE_BYTES;         // 128 rows x 128 columns of bf16 for the epilogue
-constexpr int OFF_BIAS = OFF_OUT + BM * 128 * 2;      // 256 floats
-constexpr int OFF_BAR = OFF_BIAS + BN * 4;
-constexpr int USED_BYTES = OFF_BAR + 128;
-constexpr int SMEM_BYTES = 232448;                    // the whole opt-in limit; the base is checked in the kernel
+constexpr int BM = 128, BK = 64, STAGES = 6;  // BM: rows per CTA; a pair covers 2 * BM
+constexpr int A_BYTES = BM * BK * 2;
+constexpr int SUB_BYTES = 64 * 128;           // 64 rows x 128 bytes
 constexpr int GEMM_THREADS = 192;
-constexpr int GROUP_M = 16;                           // tiles that share B columns run together
+constexpr int GROUP_M = 16;                   // tiles that share B columns run together
+
+// BN: columns of a pair's tile, 256, or 128 for results of few tiles: see launch.
+template <int BN>
+struct GemmCfg {
+    static constexpr int BNH = BN / 2;                     // B columns held by one CTA of a pair
+    static constexpr int STAGE_BYTES = A_BYTES + BNH * BK * 2;
+    static constexpr int OFF_OUT = STAGES * STAGE_BYTES;   // 128 rows x 128 columns of bf16 for the epilogue
+    static constexpr int OFF_BIAS = OFF_OUT + BM * 128 * 2;  // BN floats
+    static constexpr int OFF_BAR = OFF_BIAS + BN * 4;
+    static constexpr int USED_BYTES = OFF_BAR + 128;
+    static constexpr int SMEM_BYTES = BN == 256 ? 232448 : USED_BYTES + 1024;  // 256: the whole opt-in limit; the base is checked in the kernel
+};
 
 enum { B_FULL = 0, B_EMPTY = B_FULL + STAGES, B_ACCFULL = B_EMPTY + STAGES, B_ACCEMPTY = B_ACCFULL + 2, NUM_BARS = B_ACCEMPTY + 2 };
 enum { WG_EMPTY = 201, WG_FULL, WG_ACCEMPTY, WG_ACCFULL, WG_SMEM };
@@ -119,11 +125,14 @@ __device__ __forceinline__ void tile_coords(const GemmParams &p, int tile, int &
     tm = g * GROUP_M + (rem - tn * rows_here);
 }
 
-template <int MODE>
+template <int MODE, int BN>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
     sm100_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
                       const GemmParams p)
 {
+    using C = GemmCfg<BN>;
+    constexpr int BNH = C::BNH, STAGE_BYTES = C::STAGE_BYTES, OFF_OUT = C::OFF_OUT, OFF_BIAS = C::OFF_BIAS, OFF_BAR = C::OFF_BAR,
+                  USED_BYTES = C::USED_BYTES;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t *smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -270,13 +279,13 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
             tc_fence_after();
             const uint32_t tacc = tmem + lane_sel + buf * BN;
 #pragma unroll 1
-            for (int half = 0; half < 2; half++) {
+            for (int half = 0; half < BN / 128; half++) {
 #pragma unroll
                 for (int ch = 0; ch < 4; ch++) {
                     uint32_t u[32];
                     tmem_ld_32x32b_x32(tacc + half * 128 + ch * 32, u);
                     tmem_wait_ld();
-                    if (half == 1 && ch == 3) {  // the accumulator is in registers: the next tile may use it
+                    if (half == BN / 128 - 1 && ch == 3) {  // the accumulator is in registers: the next tile may use it
                         tc_fence_before();
                         __syncwarp();
                         if (lane == 0) mbar_arrive_cluster(accempty0 + 8u * (uint32_t)buf);
@@ -372,9 +381,11 @@ bool view_ok(const MatView &v)
     return v.dim % 64 == 0 && v.rows % v.seq == 0 && v.cols % (v.heads * v.dim) == 0;
 }
 
-template <int MODE>
-int launch(const GemmArgs &g, DeviceState *st, cudaStream_t s)
+template <int MODE, int BN>
+int launch_tile(const GemmArgs &g, DeviceState *st, cudaStream_t s)
 {
+    using C = GemmCfg<BN>;
+    constexpr int BNH = C::BNH, SMEM_BYTES = C::SMEM_BYTES;
     const RowPlan rows = row_plan(g);
     MatView va = g.a, vb = g.b;
     ViewGeom ga = {va.heads, va.seq, va.dim}, gb = {vb.heads, vb.seq, vb.dim};
@@ -412,7 +423,7 @@ int launch(const GemmArgs &g, DeviceState *st, cudaStream_t s)
     p.c_vec = c_rows_aligned(g);
     p.bias = (const __nv_bfloat16 *)g.bias;
     p.status = st->status;
-    auto kern = sm100_gemm_kernel<MODE>;
+    auto kern = sm100_gemm_kernel<MODE, BN>;
     static SmemOptIn opt_in;
     EMBER_CUDA_TRY(opt_in(kern, SMEM_BYTES));
     const long long tiles = (long long)p.tiles_m * p.tiles_n;
@@ -434,13 +445,28 @@ int launch(const GemmArgs &g, DeviceState *st, cudaStream_t s)
     return EMBER_OK;
 }
 
+// Tiles of 128 columns where those of 256 would leave half of the CTA pairs without one: twice the pairs, half
+// the products and half the epilogue each. Beyond that the wider tile is the better one: an MMA of 128 columns
+// and its copies want more shared-memory bandwidth (192 bytes per clock) than there is. Measured: forward and
+// backward of a block of 2 x 500 x 512 (4 to 24 tiles) 127 -> 116 us; with the line at twice as many tiles a block of
+// 2 x 1024 x 1536 (48 to 144 tiles) 224 -> 248 us.
+template <int MODE>
+int launch(const GemmArgs &g, DeviceState *st, cudaStream_t s)
+{
+    const RowPlan rows = row_plan(g);
+    const long long m = MODE == GEMM_TN ? g.m : (long long)rows.batch * rows.seq_pad;
+    const long long tiles = (m + 2 * BM - 1) / (2 * BM) * ((g.n + 255) / 256);
+    const int sms = st->sm_count > 0 ? st->sm_count : 148;
+    return tiles * 2 <= (sms / 2) ? launch_tile<MODE, 128>(g, st, s) : launch_tile<MODE, 256>(g, st, s);
+}
+
 }  // namespace
 
 bool sm100_gemm_supported(const GemmArgs &g)
 {
     if (g.dtype != EMBER_BF16 || g.m <= 0 || g.n <= 0 || g.k <= 0) return false;
     if (g.m > 0x7fffff00LL || g.a.rows > 0x7fffff00LL || g.b.rows > 0x7fffff00LL) return false;  // 32-bit box coordinates
-    if ((g.m + 2 * BM - 1) / (2 * BM) * (long long)((g.n + BN - 1) / BN) > 0x7fffffffLL) return false;
+    if ((g.m + 2 * BM - 1) / (2 * BM) * (long long)((g.n + 255) / 256) > 0x7fffffffLL) return false;
     if (g.c.heads > 0 && (g.c.dim % 8 != 0 || !c_rows_aligned(g))) return false;  // 16-byte output chunks
     if (!view_ok(g.a) || !view_ok(g.b)) return false;
     if (g.mode != GEMM_TN && g.b.heads != 0) return false;  // no caller has a head-major weight
@@ -455,7 +481,7 @@ bool sm100_gemm_supported(const GemmArgs &g)
     const long long padded = (long long)rows.batch * rows.seq_pad;
     const long long total = g.mode == GEMM_TN ? g.k : g.m;
     if ((long long)rows.batch * rows.seq != total || rows.seq * 16LL < rows.seq_pad) return false;
-    return padded <= 0x7fffff00LL && (g.mode == GEMM_TN || (padded + 2 * BM - 1) / (2 * BM) * (long long)((g.n + BN - 1) / BN) <= 0x7fffffffLL);
+    return padded <= 0x7fffff00LL && (g.mode == GEMM_TN || (padded + 2 * BM - 1) / (2 * BM) * (long long)((g.n + 255) / 256) <= 0x7fffffffLL);
 }
 
 // dst (rows x 8*chunks) = src (rows x cols) with zeros past the last column. The source has rows at any
