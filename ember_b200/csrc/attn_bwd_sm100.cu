@@ -1237,6 +1237,7 @@ __global__ void __launch_bounds__(128) dq_finish_kernel(const float *__restrict_
     const size_t unit = tile / nqt;
     const int w = threadIdx.x / 32, lane = threadIdx.x % 32;
     pdl_wait();                      // the accumulator is complete when the single-pass kernel has ended
+    pdl_launch_dependents();
     const int q = lane % 4;          // which 8 columns of the chunk
     const int col = c * 32 + q * 8;
     if (col >= d) return;            // d: elements per dq row in memory (a multiple of 8)
@@ -1329,18 +1330,6 @@ __global__ void __launch_bounds__(256) delta_bf16_rows_kernel(const uint4 *__res
     if (row < rows && c == 0) delta[row] = s;
 }
 
-// EMBER_PDL=0 (read once) launches the backward's kernels without programmatic stream serialization:
-// plain stream order, for comparison or for a tool that cannot follow programmatic edges.
-static int pdl_attr_count()
-{
-    static int v = -1;
-    if (v < 0) {
-        const char *e = getenv("EMBER_PDL");
-        v = (e && e[0] == '0') ? 0 : 1;
-    }
-    return v;
-}
-
 // zero / zero_bytes: the accumulator to clear in the same launch (16-byte aligned, a multiple of 16 bytes), or NULL / 0
 template <int HD>
 int launch_delta_bf16(const AttnArgs &a, float *delta, cudaStream_t s, void *zero = nullptr, size_t zero_bytes = 0)
@@ -1353,7 +1342,7 @@ int launch_delta_bf16(const AttnArgs &a, float *delta, cudaStream_t s, void *zer
     cfg.blockDim = dim3(256);
     cfg.stream = s;
     cfg.attrs = pdl;
-    cfg.numAttrs = pdl_attr_count();
+    cfg.numAttrs = pdl_enabled() ? 1 : 0;
     if (a.d != HD) {
         cfg.gridDim = dim3((unsigned)((rows + 15) / 16));
         EMBER_CUDA_TRY(cudaLaunchKernelEx(&cfg, delta_bf16_rows_kernel, (const uint4 *)a.out, (const uint4 *)a.dout, delta, rows,
@@ -1410,7 +1399,7 @@ int launch_fused_form(const AttnArgs &a, float *delta, float *dq_acc, DeviceStat
     cfg.dynamicSmemBytes = C::SMEM_BYTES;
     cfg.stream = s;
     cfg.attrs = pdl;
-    cfg.numAttrs = pdl_attr_count();
+    cfg.numAttrs = pdl_enabled() ? 1 : 0;
     EMBER_CUDA_TRY(cudaLaunchKernelEx(&cfg, k1, tq, tk, tv, tdo, p));
     cfg.gridDim = dim3((unsigned)((size_t)a.bh * nqt), (unsigned)chunks);
     cfg.blockDim = dim3(128);

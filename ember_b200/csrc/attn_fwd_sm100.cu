@@ -178,9 +178,6 @@ __global__ void __launch_bounds__(FWD_THREADS, 1)
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-    // A kernel launched behind this one with programmatic stream serialization (the backward's delta
-    // kernel) may have its CTAs placed on SMs as they fall idle; it waits for this grid's end itself.
-    pdl_launch_dependents();
     const uint32_t crank = PAIR ? cluster_ctarank() : 0u;  // rank 0 of a pair issues the MMAs
     int bh, rank;
     work_item(p.order, PAIR ? blockIdx.x / 2 : blockIdx.x, bh, rank);
@@ -264,6 +261,10 @@ __global__ void __launch_bounds__(FWD_THREADS, 1)
     if constexpr (PAIR) cluster_sync_all();  // both CTAs' barriers exist before either signals the other's
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    // The kernel launched behind this one may have its CTAs placed on SMs as they fall idle; it waits for this
+    // grid's end itself, as this one does for the kernel before (a projection that writes q, k and v).
+    pdl_launch_dependents();
+    pdl_wait();
 
     if (warp >= 8) {
         reg_dealloc_40();
@@ -703,9 +704,14 @@ int launch_form(const AttnArgs &a, DeviceState *st, cudaStream_t s)
     EMBER_CUDA_TRY(opt_in(kern, C::SMEM_BYTES));
     p.order = make_work_order(a.bh, (a.lq + p.block_rows - 1) / p.block_rows, st->sm_count, ((size_t)a.lq + a.lk) * HD * 2 * 2,  // Q, O, K, V
                               a.causal != 0);
-    dim3 grid((unsigned)(p.order.units * p.order.blocks));
-    kern<<<grid, FWD_THREADS, C::SMEM_BYTES, s>>>(tq, tk, tv, p);
-    EMBER_CUDA_TRY(cudaGetLastError());
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(p.order.units * p.order.blocks));
+    cfg.blockDim = dim3(FWD_THREADS);
+    cfg.dynamicSmemBytes = C::SMEM_BYTES;
+    cfg.stream = s;
+    LaunchAttrs attrs;
+    attrs.pdl().set(cfg);
+    EMBER_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, tq, tk, tv, p));
     return EMBER_OK;
 }
 

@@ -35,6 +35,8 @@ __global__ void __launch_bounds__(256) column_sum_kernel(const MatView a, T *__r
     constexpr int COLS = TX * NV;
     __shared__ float red[TY][COLS + 1];
     __shared__ float total[COLS];
+    pdl_launch_dependents();
+    pdl_wait();
     const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;
     const int rank = splits > 1 ? (int)cluster_ctarank() : 0;
     const int col = ((int)blockIdx.x / splits) * COLS + tx * NV;
@@ -129,13 +131,8 @@ int launch(const MatView &a, T *out, int sms, cudaStream_t s)
     cfg.gridDim = dim3((unsigned)(strips * splits));
     cfg.blockDim = dim3(256);
     cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = splits;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = splits > 1 ? 1 : 0;
+    LaunchAttrs attrs;
+    attrs.cluster((unsigned)splits).pdl().set(cfg);
     EMBER_CUDA_TRY(cudaLaunchKernelEx(&cfg, column_sum_kernel<T, VEC>, a, out, splits));
     return EMBER_OK;
 }

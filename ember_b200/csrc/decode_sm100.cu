@@ -391,6 +391,7 @@ __global__ void __launch_bounds__(128) decode_merge_kernel(const float *__restri
     int first = (int)(begin * ncta / total);
     while (slice_begin(total, first + 1, ncta) <= begin) first++;
     while (slice_begin(total, first, ncta) > begin) first--;
+    pdl_launch_dependents();
     pdl_wait();
     if (slice_begin(total, first + 1, ncta) >= end) return;  // one CTA had all of it and wrote the result
     float mx = -INFINITY;
@@ -445,16 +446,13 @@ int launch(const CacheDecodeArgs &a, DeviceState *st, cudaStream_t s)
     auto kern = decode_sm100_kernel<HD, G>;
     static SmemOptIn opt_in;
     EMBER_CUDA_TRY(opt_in(kern, C::SMEM));
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    LaunchAttrs attrs;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)ncta);
     cfg.blockDim = dim3(THREADS);
     cfg.dynamicSmemBytes = C::SMEM;
     cfg.stream = s;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    attrs.pdl().set(cfg);
     EMBER_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, tq, tk, tv, p));
     // a unit is shared whenever a slice begins inside it
     const long long total = (long long)units * p.tiles;

@@ -101,6 +101,8 @@ __global__ void __launch_bounds__(THREADS) skinny_gemm_kernel(const __grid_const
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    pdl_launch_dependents();
+    pdl_wait();
 
     if (warp == 5) {
         if (lane == 0) {
@@ -213,13 +215,8 @@ int launch_mp(const GemmArgs &g, DeviceState *st, cudaStream_t s)
     cfg.blockDim = dim3(THREADS);
     cfg.dynamicSmemBytes = C::SMEM_BYTES;
     cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = splits;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    LaunchAttrs attrs;
+    attrs.cluster((unsigned)splits).pdl().set(cfg);
     EMBER_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, tw, tx, p));
     return EMBER_OK;
 }

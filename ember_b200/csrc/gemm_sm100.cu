@@ -185,6 +185,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     cluster_sync_all();  // both CTAs' barriers exist before either signals the other's
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    pdl_launch_dependents();
+    pdl_wait();
 
     if (warp == 5) {
         if (lane == 0) {
@@ -434,13 +436,8 @@ int launch_tile(const GemmArgs &g, DeviceState *st, cudaStream_t s)
     cfg.blockDim = dim3(GEMM_THREADS);
     cfg.dynamicSmemBytes = SMEM_BYTES;
     cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;  // consecutive CTAs 2i, 2i+1 form a pair
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    LaunchAttrs attrs;  // consecutive CTAs 2i, 2i+1 form a pair
+    attrs.cluster(2).pdl().set(cfg);
     EMBER_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, ta, tb, p));
     return EMBER_OK;
 }
@@ -490,6 +487,8 @@ bool sm100_gemm_supported(const GemmArgs &g)
 __global__ void __launch_bounds__(256) pack_rows_kernel(const unsigned short *__restrict__ src, uint4 *__restrict__ dst, long long rows,
                                                         int cols, int chunks)
 {
+    ptx::pdl_launch_dependents();
+    ptx::pdl_wait();
     const long long row = (long long)blockIdx.x * 8 + threadIdx.x / 32;
     if (row >= rows) return;
     const int end = min(chunks, ((int)blockIdx.y + 1) * 256);
@@ -524,9 +523,13 @@ __global__ void __launch_bounds__(256) pack_rows_kernel(const unsigned short *__
 int pack_rows(const MatView &v, void *dst, cudaStream_t s)
 {
     const int chunks = (v.cols + 7) / 8;
-    const dim3 grid((unsigned)((v.rows + 7) / 8), (unsigned)((chunks + 255) / 256));
-    pack_rows_kernel<<<grid, 256, 0, s>>>((const unsigned short *)v.ptr, (uint4 *)dst, v.rows, v.cols, chunks);
-    EMBER_CUDA_TRY(cudaGetLastError());
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)((v.rows + 7) / 8), (unsigned)((chunks + 255) / 256));
+    cfg.blockDim = dim3(256);
+    cfg.stream = s;
+    LaunchAttrs attrs;
+    attrs.pdl().set(cfg);
+    EMBER_CUDA_TRY(cudaLaunchKernelEx(&cfg, pack_rows_kernel, (const unsigned short *)v.ptr, (uint4 *)dst, v.rows, v.cols, chunks));
     return EMBER_OK;
 }
 

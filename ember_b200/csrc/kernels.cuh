@@ -7,6 +7,49 @@
 
 namespace ember {
 
+// Programmatic dependent launch: a kernel sets itself up (barriers, tensor memory, descriptors) on SMs that fall
+// idle while the one before it drains, which saves 2 to 3 us a launch in chains of short kernels. Measured with
+// and without it on the projections, the cache and the forward: a token through a 2048-wide block at batch 8
+// 41 -> 31 us, forward and backward of a block of 2 x 1024 x 1536 224 -> 200 us, of 16 units x L2048 92.5 -> 87.2 us.
+// EMBER_PDL=0 (read once) launches every kernel in plain stream order.
+// Rules of the kernels that are launched with it, which make any chain of them safe:
+//   - every thread passes pdl_wait() before it reads or writes global memory (prefetching a tensor map and
+//     setting up barriers and tensor memory may come before), so that a kernel's end implies the end of
+//     all before it (the single-pass backward reads q, k, v and dO earlier: the delta kernel before it passes
+//     pdl_wait() first and lets it start afterwards);
+//   - a kernel that allocates tensor memory passes pdl_launch_dependents() after the allocation: a later kernel's
+//     block can then never hold the columns that an earlier one's, which it waits for, still needs.
+bool pdl_enabled();
+
+struct LaunchAttrs {
+    cudaLaunchAttribute attr[2];
+    int count = 0;
+
+    LaunchAttrs &cluster(unsigned x)
+    {
+        if (x > 1) {
+            attr[count].id = cudaLaunchAttributeClusterDimension;
+            attr[count].val.clusterDim.x = x;
+            attr[count].val.clusterDim.y = 1;
+            attr[count++].val.clusterDim.z = 1;
+        }
+        return *this;
+    }
+    LaunchAttrs &pdl()
+    {
+        if (pdl_enabled()) {
+            attr[count].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            attr[count++].val.programmaticStreamSerializationAllowed = 1;
+        }
+        return *this;
+    }
+    void set(cudaLaunchConfig_t &cfg)
+    {
+        cfg.attrs = attr;
+        cfg.numAttrs = (unsigned)count;
+    }
+};
+
 struct AttnArgs {
     const void *q = nullptr, *k = nullptr, *v = nullptr;
     void *out = nullptr;

@@ -296,6 +296,7 @@ __global__ void __launch_bounds__(256) kv_append_kernel(uint4 *__restrict__ kc, 
                                                         int elems_per_vec, DeviceStatus *status)
 {
     ptx::pdl_launch_dependents();  // the decode kernel behind it may set itself up meanwhile
+    ptx::pdl_wait();
     const size_t total = (size_t)batch * g.kv_heads * n_new * vec_per_row;
     const int limit = g.block_table ? (g.max_blocks << g.page_shift) : g.capacity;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
@@ -470,10 +471,14 @@ int ember_kv_cache_append(void *k_cache, void *v_cache, const void *k_new, const
     const int vec_per_row = d / elems_per_vec;
     const size_t total = (size_t)batch * kv_heads * n_new * vec_per_row;
     const size_t want = (total + 255) / 256, cap = (size_t)(st->sm_count > 0 ? st->sm_count : 148) * 16;
-    kv_append_kernel<<<(int)(want < cap ? want : cap), 256, 0, pick_stream(stream, st)>>>(
-        (uint4 *)k_cache, (uint4 *)v_cache, (const uint4 *)k_new, (const uint4 *)v_new, make_geom(a), batch, n_new, pos,
-        vec_per_row, elems_per_vec, st->status);
-    EMBER_CUDA_TRY(cudaGetLastError());
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(want < cap ? want : cap));
+    cfg.blockDim = dim3(256);
+    cfg.stream = pick_stream(stream, st);
+    LaunchAttrs attrs;
+    attrs.pdl().set(cfg);
+    EMBER_CUDA_TRY(cudaLaunchKernelEx(&cfg, kv_append_kernel, (uint4 *)k_cache, (uint4 *)v_cache, (const uint4 *)k_new, (const uint4 *)v_new,
+                                      make_geom(a), batch, n_new, pos, vec_per_row, elems_per_vec, st->status));
     return EMBER_OK;
 }
 

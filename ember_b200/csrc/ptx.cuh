@@ -332,7 +332,7 @@ __device__ __forceinline__ void mma_ts_lo(uint32_t d_tmem, uint32_t a_tmem, uint
 // CTAs placed (and run whatever does not depend on the kernel before it on the stream) as soon as every
 // CTA of that kernel has passed pdl_launch_dependents(); pdl_wait() then blocks until that kernel has
 // completed and its writes are visible. Launched without the attribute, or after something that is
-// not a kernel, both are no-ops. Used along forward -> delta -> single-pass backward -> dQ finish.
+// not a kernel, both are no-ops. The rules that its users keep stand beside pdl_enabled (kernels.cuh).
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

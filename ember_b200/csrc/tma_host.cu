@@ -1,9 +1,20 @@
 // Host-side construction of TMA tensor maps. The driver's encoder is reached through
-// cudaGetDriverEntryPoint, so the library does not link against libcuda.
+// cudaGetDriverEntryPoint, so the library does not link against libcuda. Also the launch setting they share.
+#include <stdlib.h>
+
 #include "kernels.cuh"
 #include "ptx.cuh"
 
 namespace ember {
+
+bool pdl_enabled()
+{
+    static const bool on = [] {
+        const char *e = getenv("EMBER_PDL");
+        return !(e && e[0] == '0');
+    }();
+    return on;
+}
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                   const cuuint64_t *, const cuuint32_t *, const cuuint32_t *,
