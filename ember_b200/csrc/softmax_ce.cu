@@ -18,6 +18,7 @@
 // accesses otherwise.
 #include "common.cuh"
 #include "kernels.cuh"
+#include "ptx.cuh"
 
 namespace ember {
 
@@ -108,6 +109,8 @@ __global__ void __launch_bounds__(W < 256 ? 256 : W) row_softmax_kernel(const T 
                                                                          T *__restrict__ y, float *__restrict__ row_loss,
                                                                          long long rows, int cols, int cache_elems)
 {
+    ptx::pdl_launch_dependents();
+    ptx::pdl_wait();
     extern __shared__ __align__(16) unsigned char smem_bytes[];
     float *red = reinterpret_cast<float *>(smem_bytes);  // 32 floats
     constexpr int BS = W < 256 ? 256 : W, GROUPS = BS / W, NV = Vec16<T>::NV;
@@ -259,6 +262,8 @@ __global__ void __launch_bounds__(256, 2) row_softmax_regs_kernel(const T *__res
                                                                    T *__restrict__ y, float *__restrict__ row_loss,
                                                                    long long rows, int cols)
 {
+    ptx::pdl_launch_dependents();
+    ptx::pdl_wait();
     __shared__ float red[32];
     constexpr int GROUPS = 256 / W, NV = Vec16<T>::NV;
     constexpr float kLog2e = 1.4426950408889634f;
@@ -375,6 +380,8 @@ __global__ void __launch_bounds__(256, 2) row_softmax_regs_kernel(const T *__res
 // loss = -(sum of the row losses) / rows, added in a fixed order.
 __global__ void __launch_bounds__(BLOCK) loss_finalize_kernel(const float *row_loss, long long rows, float *loss)
 {
+    ptx::pdl_launch_dependents();
+    ptx::pdl_wait();
     __shared__ float red[BLOCK];
     float s = 0.f;
     for (long long r = threadIdx.x; r < rows; r += BLOCK) s += row_loss[r];
@@ -391,6 +398,8 @@ template <typename T, bool VEC>
 __global__ void __launch_bounds__(BLOCK) ce_backward_kernel(const T *__restrict__ probs, const T *__restrict__ target,
                                                             T *__restrict__ grad, size_t total, float inv_n)
 {
+    ptx::pdl_launch_dependents();
+    ptx::pdl_wait();
     constexpr int NV = Vec16<T>::NV;
     if constexpr (VEC) {
         const uint4 *pv = reinterpret_cast<const uint4 *>(probs), *tv = reinterpret_cast<const uint4 *>(target);
@@ -427,7 +436,9 @@ int launch_rows(const T *x, const T *target, T *y, float *row_loss, long long ro
     const int width = row_bytes <= WARP_ROW_MAX_BYTES ? 32 : (row_bytes <= BLOCK_ROW_MAX_BYTES ? 256 : 1024);
     // 16-byte pieces that a row touches (without vec: at most, wherever it starts)
     const long long touched = vec ? cols / NV : ((long long)cols + 2 * NV - 2) / NV;
-    const int width_r = touched <= 16 * 32 ? 32 : 256;
+    // A warp per row, unless there are too few rows for that: up to the 16 warps of this kernel that an SM holds,
+    // rows of 2 KB and more get a block each (a classifier step of 2000 x 1024 x 3001: 155.1 -> 153.9 us).
+    const int width_r = touched <= 16 * 32 && !(touched >= 128 && rows <= 16LL * (sm_count > 0 ? sm_count : 148)) ? 32 : 256;
     if (bases && touched <= 16 * 256 && (vec || cols >= 2 * NV)) {  // the row fits the registers of the threads that own it
         const int groups_r = 256 / width_r;
         const long long need_r = (rows + groups_r - 1) / groups_r;
@@ -436,8 +447,8 @@ int launch_rows(const T *x, const T *target, T *y, float *row_loss, long long ro
         const int pieces = (int)((touched + width_r - 1) / width_r);  // per thread, at most 16 here
 #define EMBER_LAUNCH_REGS(W, NP)                                                                                                  \
     do {                                                                                                                          \
-        if (vec) row_softmax_regs_kernel<T, W, MODE, NP, false><<<grid_r, 256, 0, s>>>(x, target, y, row_loss, rows, cols);       \
-        else row_softmax_regs_kernel<T, W, MODE, NP, true><<<grid_r, 256, 0, s>>>(x, target, y, row_loss, rows, cols);            \
+        auto kern = vec ? row_softmax_regs_kernel<T, W, MODE, NP, false> : row_softmax_regs_kernel<T, W, MODE, NP, true>;         \
+        EMBER_CUDA_TRY(launch_pdl(kern, grid_r, 256, 0, s, x, target, y, row_loss, rows, cols));                                 \
     } while (0)
 #define EMBER_LAUNCH_REGS_W(W)                    \
     do {                                          \
@@ -450,7 +461,6 @@ int launch_rows(const T *x, const T *target, T *y, float *row_loss, long long ro
         if (width_r == 32) EMBER_LAUNCH_REGS_W(32); else EMBER_LAUNCH_REGS_W(256);
 #undef EMBER_LAUNCH_REGS_W
 #undef EMBER_LAUNCH_REGS
-        EMBER_CUDA_TRY(cudaGetLastError());
         return EMBER_OK;
     }
     const int block = width < 256 ? 256 : width, groups = block / width;
@@ -465,7 +475,7 @@ int launch_rows(const T *x, const T *target, T *y, float *row_loss, long long ro
         auto kern = row_softmax_kernel<T, W, MODE, VEC>;                                                        \
         static SmemOptIn opt_in; /* the size varies with the row: the largest any row needs */                   \
         EMBER_CUDA_TRY(opt_in(kern, 128 + CACHE_BYTES));                                                        \
-        kern<<<grid, block, smem, s>>>(x, target, y, row_loss, rows, cols, cache_elems);                         \
+        EMBER_CUDA_TRY(launch_pdl(kern, grid, block, smem, s, x, target, y, row_loss, rows, cols, cache_elems)); \
     } while (0)
     if (width == 32) {
         if (vec) EMBER_LAUNCH_ROWS(32, true); else EMBER_LAUNCH_ROWS(32, false);
@@ -475,7 +485,6 @@ int launch_rows(const T *x, const T *target, T *y, float *row_loss, long long ro
         if (vec) EMBER_LAUNCH_ROWS(1024, true); else EMBER_LAUNCH_ROWS(1024, false);
     }
 #undef EMBER_LAUNCH_ROWS
-    EMBER_CUDA_TRY(cudaGetLastError());
     return EMBER_OK;
 }
 
@@ -541,8 +550,7 @@ int ember_cross_entropy_fwd(const void *pred, const void *target, void *probs, f
         rc = launch_rows<float, MODE_CROSS_ENTROPY>((const float *)pred, (const float *)target, (float *)probs, row_loss,
                                                    rows, cols, st->sm_count, s);
     if (rc) return rc;
-    loss_finalize_kernel<<<1, BLOCK, 0, s>>>(row_loss, rows, loss);
-    EMBER_CUDA_TRY(cudaGetLastError());
+    EMBER_CUDA_TRY(launch_pdl(loss_finalize_kernel, 1, BLOCK, 0, s, row_loss, rows, loss));
     return EMBER_OK;
 }
 
@@ -564,13 +572,13 @@ int ember_cross_entropy_bwd(const void *probs, const void *target, void *grad, l
     const int grid = (int)(want < cap ? want : cap);
     const float inv_n = 1.f / (float)rows;
     if (dtype == EMBER_BF16) {
-        if (vec) ce_backward_kernel<__nv_bfloat16, true><<<grid, BLOCK, 0, s>>>((const __nv_bfloat16 *)probs, (const __nv_bfloat16 *)target, (__nv_bfloat16 *)grad, total, inv_n);
-        else ce_backward_kernel<__nv_bfloat16, false><<<grid, BLOCK, 0, s>>>((const __nv_bfloat16 *)probs, (const __nv_bfloat16 *)target, (__nv_bfloat16 *)grad, total, inv_n);
+        auto kern = vec ? ce_backward_kernel<__nv_bfloat16, true> : ce_backward_kernel<__nv_bfloat16, false>;
+        EMBER_CUDA_TRY(launch_pdl(kern, grid, BLOCK, 0, s, (const __nv_bfloat16 *)probs, (const __nv_bfloat16 *)target,
+                                  (__nv_bfloat16 *)grad, total, inv_n));
     } else {
-        if (vec) ce_backward_kernel<float, true><<<grid, BLOCK, 0, s>>>((const float *)probs, (const float *)target, (float *)grad, total, inv_n);
-        else ce_backward_kernel<float, false><<<grid, BLOCK, 0, s>>>((const float *)probs, (const float *)target, (float *)grad, total, inv_n);
+        auto kern = vec ? ce_backward_kernel<float, true> : ce_backward_kernel<float, false>;
+        EMBER_CUDA_TRY(launch_pdl(kern, grid, BLOCK, 0, s, (const float *)probs, (const float *)target, (float *)grad, total, inv_n));
     }
-    EMBER_CUDA_TRY(cudaGetLastError());
     return EMBER_OK;
 }
 
