@@ -98,6 +98,8 @@ __global__ void __launch_bounds__(256, 2) simt_gemm_kernel(const MatView a, cons
 {
     using OA = Operand<T, MODE != GEMM_TN, FA, C::TM>;
     using OB = Operand<T, MODE == GEMM_NT, FB, C::TN>;
+    ptx::pdl_launch_dependents();
+    ptx::pdl_wait();
     extern __shared__ __align__(16) float sm[];
     float *as = sm, *bs = sm + C::SLAB * C::PA;
     const int rank = splits > 1 ? (int)ptx::cluster_ctarank() : 0;
@@ -244,13 +246,10 @@ int launch_tile(const GemmArgs &g, int splits, cudaStream_t s)
     cfg.blockDim = dim3(256);
     cfg.dynamicSmemBytes = C::FLOATS * sizeof(float);
     cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = splits;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = splits > 1 ? 1 : 0;
+    LaunchAttrs attrs;
+    attrs.cluster((unsigned)splits);
+    if (cfg.gridDim.x <= (unsigned)kPdlMaxGrid) attrs.pdl();
+    attrs.set(cfg);
     EMBER_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, g.a, g.b, g.c, (const T *)g.bias, g.m, g.n, g.k, (int)tiles_n, splits));
     return EMBER_OK;
 }
