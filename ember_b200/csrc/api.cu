@@ -68,6 +68,10 @@ int ember_attention_fwd(const void *q, const void *k, const void *v, void *out, 
     a.scale = scale; a.causal = causal ? 1 : 0; a.dtype = dtype;
     cudaStream_t s = pick_stream(stream, st);
     if (sm100_fwd_supported(a)) return sm100_attention_fwd(a, st, s);
+    if (sm100_f32_fwd_preferred(a, st->sm_count)) {
+        rc = sm100_f32_attention_fwd(a, st, s);
+        if (rc != EMBER_ERR_NOMEM) return rc;  // without memory for the operands' parts: the CUDA cores, which need none
+    }
     return simt_attention_fwd(a, st, s);
 }
 
@@ -100,7 +104,11 @@ int ember_attention_bwd(const void *q, const void *k, const void *v, const void 
         float *acc = det ? nullptr : (float *)((char *)workspace + delta_bytes(batch_heads, lq));
         return sm100_attention_bwd(a, (float *)workspace, acc, det, st, s);
     }
-    return simt_attention_bwd(a, (float *)workspace, st, s);
+    if (sm100_f32_bwd_preferred(a, st->sm_count)) {
+        rc = sm100_f32_attention_bwd(a, (float *)workspace, st, s);
+        if (rc != EMBER_ERR_NOMEM) return rc;
+    }
+    return simt_attention_bwd(a, (float *)workspace, false, st, s);
 }
 
 int ember_set_deterministic(int on)

@@ -1,0 +1,1048 @@
+// Float32 attention on the tensor cores: every operand is the sum of three bf16 parts (split_f32.cuh), a product of
+// two operands six tcgen05 products of their parts, small ones first, accumulated in float32 over at most 64 terms in
+// tensor memory and then added into float32 registers. Probabilities and score gradients are split the same way in
+// registers, so nothing is held or multiplied with less than 24 bits.
+//
+// The CUDA-core kernels (attn_simt.cu) do the same products at the FMA pipe's rate, 128 per clock and SM; six bf16 products for
+// each leave 683 per clock. Measured, 16 units x L1024, causal: d 64 forward 93 -> 29 us, backward 215 -> 61 us (and 6 us of
+// splitting each); d 128, 8 units: 105 -> 56 and 234 -> 103 us. What bounds them now: the compute warps (exponentials and the
+// splitting of 128 x 64 probabilities, 2500 clocks a tile) and the hand-overs between them and the products (1536 to 3456 clocks).
+// Errors against float64 (relative 2-norm, CUDA cores -> here): 16 units x L1024 d 64 causal: o 2.3e-7 -> 0.9e-7, dq 3.3e-7 ->
+// 2.6e-7, dk 7.7e-7 -> 2.9e-7, dv 7.8e-7 -> 2.2e-7, log-sum-exp 3.3e-8 both; 8 x 777 x 1301 d 80: o 6.5e-7 -> 1.3e-7, dq 7.1e-7 -> 3.3e-7, dk
+// 5.7e-7 -> 3.2e-7, dv 5.5e-7 -> 2.7e-7, log-sum-exp 2.9e-8 both.
+//
+// Common to the kernels: 128 rows of one operand belong to a CTA (a row per tensor-memory lane) and lie in tensor memory as
+// the A operand of the score product, tiles of 64 rows of the other operand's planes are streamed by TMA, eight compute
+// warps (two warpgroups) own the rows' softmax, two warps issue, one loads.
+#include <math.h>
+
+#include "common.cuh"
+#include "kernels.cuh"
+#include "ptx.cuh"
+#include "split_f32.cuh"
+
+namespace ember {
+
+namespace {
+
+using namespace ptx;
+
+constexpr int F32_THREADS = 384;       // warps 0-7 compute, 8 and 10 MMA issue, 9 TMA, 11 allocation
+constexpr float LOG2E_T = 1.4426950408889634f;
+constexpr int SUB = 64 * 128;          // 64 rows x 128 bytes: one TMA box
+constexpr int TN = 64;                 // rows of a streamed tile
+
+enum { WF_Q = 301, WF_K, WF_V, WF_S, WF_P, WF_O, WF_OFREE, WF_KEMPTY, WF_VEMPTY, WB_A, WB_B0, WB_B1, WB_S, WB_P, WB_DP, WB_DS, WB_ACC, WB_FREE, WB_E0, WB_E1 };
+
+__device__ __forceinline__ float exp_nat(float x) { return ex2(x * LOG2E_T); }
+
+// e^x of the backward, which has no division by the sum for errors common to a row to cancel in: what the product with log2(e) is
+// rounded by is put back to first order, 2^(y + r) = 2^y (1 + r ln 2). x is finite.
+__device__ __forceinline__ f32x2 exp_pair(f32x2 x)
+{
+    const f32x2 y = mul2(x, pack2(LOG2E_T, LOG2E_T)), neg = mul2(x, pack2(-LOG2E_T, -LOG2E_T));
+    // log2(e) = LOG2E_T + 1.925963e-8
+    const f32x2 r = fma2(x, pack2(1.925963033500e-8f, 1.925963033500e-8f), fma2(x, pack2(LOG2E_T, LOG2E_T), neg));
+    float a, b;
+    unpack2(y, a, b);
+    const f32x2 v = pack2(ex2(a), ex2(b));
+    return fma2(v, mul2(r, pack2(0.69314718f, 0.69314718f)), v);
+}
+
+// The six products of parts, small ones first: (part of A, part of B) = (2, 0) (1, 1) (0, 2) (1, 0) (0, 1) (0, 0), 0 = high. A
+// loop and not straight code: with the four products of a backward step unrolled, issuing and computing warps together outgrew
+// the instruction cache.
+constexpr int PRODUCTS = 6;
+__device__ __forceinline__ uint32_t part_a(int i) { return (0x046u >> (2 * i)) & 3u; }
+__device__ __forceinline__ uint32_t part_b(int i) { return (0x124u >> (2 * i)) & 3u; }
+
+// Row `src` (d columns in memory; null: zeros), columns [col0, col0 + 32 * n32) -> the three parts in tensor memory, part q at
+// column taddr + q * plane.
+__device__ __forceinline__ void row_to_tmem(const float *src, int d, bool vec, int col0, int n32, uint32_t taddr, int plane)
+{
+    for (int h = 0; h < n32; h++) {
+        const int c0 = col0 + h * 32;
+        float v[32];
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const int c = c0 + i * 4;
+            float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (src) {
+                if (vec) {
+                    if (c < d) f = *reinterpret_cast<const float4 *>(src + c);
+                } else {
+                    if (c < d) f.x = src[c];
+                    if (c + 1 < d) f.y = src[c + 1];
+                    if (c + 2 < d) f.z = src[c + 2];
+                    if (c + 3 < d) f.w = src[c + 3];
+                }
+            }
+            v[4 * i] = f.x; v[4 * i + 1] = f.y; v[4 * i + 2] = f.z; v[4 * i + 3] = f.w;
+        }
+        uint32_t a[16], b[16], c[16];
+#pragma unroll
+        for (int i = 0; i < 16; i++) split_pair(pack2(v[2 * i], v[2 * i + 1]), a[i], b[i], c[i]);
+        const uint32_t t = taddr + (uint32_t)(c0 / 2);
+        tmem_st_32x32b_x16(t, a);
+        tmem_st_32x32b_x16(t + plane, b);
+        tmem_st_32x32b_x16(t + 2 * plane, c);
+    }
+    tmem_wait_st();
+}
+
+// 32 values of a row -> their parts in tensor memory: 3 blocks of 16 columns from taddr, part by part. The A operand of 16 values
+// (one MMA) is 8 columns.
+__device__ __forceinline__ void split_to_tmem(const f32x2 *v, uint32_t taddr)
+{
+    uint32_t a[16], b[16], c[16];
+#pragma unroll
+    for (int i = 0; i < 16; i++) split_pair(v[i], a[i], b[i], c[i]);
+    tmem_st_32x32b_x16(taddr, a);
+    tmem_st_32x32b_x16(taddr + 16, b);
+    tmem_st_32x32b_x16(taddr + 32, c);
+}
+
+// Where such a block lies inside a region of 96 columns that held the 64 scores in columns [16, 80): the 32 scores of half h are in
+// [16 + 32 h, 48 + 32 h) and its parts go to [48 h, 48 h + 48), so that a half never overwrites scores of the other.
+constexpr int REGION = 96, SCORES_AT = 16;
+__device__ __forceinline__ constexpr uint32_t part_col(int part, int k16) { return (uint32_t)((k16 / 2) * 48 + part * 16 + (k16 % 2) * 8); }
+
+// A chain of four (or two) MMAs of 16 contraction steps, A in tensor memory (AO* columns further each) or in shared memory (AO* in
+// units of 16 bytes), B BO* further each. Products of parts are short MMAs (64 columns: 32 clocks), so what one costs to issue
+// decides: `elected` is taken once per tile and four MMAs make one asm block (an elect.sync and a branch on the
+// number of steps for each took 85 clocks an MMA).
+#define EMBER_CHAIN_HEAD "{\n.reg .pred p, q;\n.reg .b64 da, db;\n.reg .b32 t, u;\nsetp.ne.b32 q, %4, 0;\nsetp.ne.b32 p, %5, 0;\n"
+template <int A1, int A2, int A3, int B1, int B2, int B3>
+__device__ __forceinline__ void chain_ts(uint32_t d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t elected, uint32_t acc, bool four)
+{
+    if (four)
+        asm volatile(EMBER_CHAIN_HEAD
+                     "mov.b64 db, {%2, %6};\n@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, p;\nsetp.eq.u32 p, 0, 0;\n"
+                     "add.u32 t, %2, %10;\nadd.u32 u, %1, %7;\nmov.b64 db, {t, %6};\n@q tcgen05.mma.cta_group::1.kind::f16 [%0], [u], db, %3, p;\n"
+                     "add.u32 t, %2, %11;\nadd.u32 u, %1, %8;\nmov.b64 db, {t, %6};\n@q tcgen05.mma.cta_group::1.kind::f16 [%0], [u], db, %3, p;\n"
+                     "add.u32 t, %2, %12;\nadd.u32 u, %1, %9;\nmov.b64 db, {t, %6};\n@q tcgen05.mma.cta_group::1.kind::f16 [%0], [u], db, %3, p;\n}\n"
+                     ::"r"(d), "r"(a), "r"(b), "r"(idesc), "r"(elected), "r"(acc), "r"(kDescHiSw128), "n"(A1), "n"(A2), "n"(A3), "n"(B1), "n"(B2), "n"(B3) : "memory");
+    else
+        asm volatile(EMBER_CHAIN_HEAD
+                     "mov.b64 db, {%2, %6};\n@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, p;\nsetp.eq.u32 p, 0, 0;\n"
+                     "add.u32 t, %2, %8;\nadd.u32 u, %1, %7;\nmov.b64 db, {t, %6};\n@q tcgen05.mma.cta_group::1.kind::f16 [%0], [u], db, %3, p;\n}\n"
+                     ::"r"(d), "r"(a), "r"(b), "r"(idesc), "r"(elected), "r"(acc), "r"(kDescHiSw128), "n"(A1), "n"(B1) : "memory");
+}
+template <int A1, int A2, int A3, int B1, int B2, int B3>
+__device__ __forceinline__ void chain_ss(uint32_t d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t elected, uint32_t acc, bool four)
+{
+    if (four)
+        asm volatile(EMBER_CHAIN_HEAD
+                     "mov.b64 db, {%2, %6};\nmov.b64 da, {%1, %6};\n@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\nsetp.eq.u32 p, 0, 0;\n"
+                     "add.u32 t, %2, %10;\nadd.u32 u, %1, %7;\nmov.b64 db, {t, %6};\nmov.b64 da, {u, %6};\n@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n"
+                     "add.u32 t, %2, %11;\nadd.u32 u, %1, %8;\nmov.b64 db, {t, %6};\nmov.b64 da, {u, %6};\n@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n"
+                     "add.u32 t, %2, %12;\nadd.u32 u, %1, %9;\nmov.b64 db, {t, %6};\nmov.b64 da, {u, %6};\n@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n}\n"
+                     ::"r"(d), "r"(a), "r"(b), "r"(idesc), "r"(elected), "r"(acc), "r"(kDescHiSw128), "n"(A1), "n"(A2), "n"(A3), "n"(B1), "n"(B2), "n"(B3) : "memory");
+    else
+        asm volatile(EMBER_CHAIN_HEAD
+                     "mov.b64 db, {%2, %6};\nmov.b64 da, {%1, %6};\n@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\nsetp.eq.u32 p, 0, 0;\n"
+                     "add.u32 t, %2, %8;\nadd.u32 u, %1, %7;\nmov.b64 db, {t, %6};\nmov.b64 da, {u, %6};\n@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n}\n"
+                     ::"r"(d), "r"(a), "r"(b), "r"(idesc), "r"(elected), "r"(acc), "r"(kDescHiSw128), "n"(A1), "n"(B1) : "memory");
+}
+
+// Scores: D (128 x 64) = A * B^T (a tile of 64 rows, HD columns, planes PLANE bytes apart). A in tensor memory, parts HD / 2
+// columns apart, or in shared memory (SS): 128 rows, planes 2 * PLANE bytes apart, 64-column sub-tiles 2 * SUB. The contraction
+// stops at the end of the 32 columns that hold the last of d (zeros past d).
+template <int HD, bool SS>
+__device__ __forceinline__ void mma_scores(uint32_t d, uint32_t a, uint32_t b_smem, int ksteps, uint32_t elected)
+{
+    constexpr uint32_t IDESC = idesc_bf16_f32(128, TN, 0, 0);
+    constexpr int PLANE = HD / 64 * SUB;
+    const uint32_t b_lo = desc_lo(b_smem, 16), a_lo = SS ? desc_lo(a, 16) : a;
+#pragma unroll 1
+    for (int i = 0; i < PRODUCTS; i++) {
+#pragma unroll
+        for (int sub = 0; sub < HD / 64; sub++) {
+            const uint32_t acc = i > 0 || sub > 0, pa = part_a(i), b = b_lo + part_b(i) * (PLANE >> 4) + ((sub * SUB) >> 4);
+            const bool four = ksteps - sub * 4 > 2;
+            if (SS) chain_ss<2, 4, 6, 2, 4, 6>(d, a_lo + pa * ((2 * PLANE) >> 4) + ((sub * 2 * SUB) >> 4), b, IDESC, elected, acc, four);
+            else chain_ts<8, 16, 24, 2, 4, 6>(d, a_lo + pa * (HD / 2) + sub * 32, b, IDESC, elected, acc, four);
+        }
+    }
+}
+// Results: D (128 x n) = P (parts in a region of tensor memory, 64 columns of the product) * B (the tile's 64 rows x n columns).
+template <int HD>
+__device__ __forceinline__ void mma_results(uint32_t d, uint32_t region, uint32_t b_smem, uint32_t idesc, uint32_t elected)
+{
+    constexpr int PLANE = HD / 64 * SUB;
+    const uint32_t b_lo = desc_lo(b_smem, SUB);
+#pragma unroll 1
+    for (int i = 0; i < PRODUCTS; i++)
+        chain_ts<part_col(0, 1), part_col(0, 2), part_col(0, 3), 128, 256, 384>(d, region + part_a(i) * part_col(1, 0), b_lo + part_b(i) * (PLANE >> 4), idesc, elected,
+                                                                                i > 0, true);
+}
+
+// Loads a 64-row tile's three planes.
+template <int HD>
+__device__ __forceinline__ void load_planes(uint32_t dst, const CUtensorMap *map, uint32_t bar, int row, int unit, int units)
+{
+    mbar_arrive_expect_tx(bar, 3 * (HD / 64) * SUB);
+    for (int pl = 0; pl < 3; pl++)
+        for (int s = 0; s < HD / 64; s++) tma_load_3d(dst + (pl * (HD / 64) + s) * SUB, map, bar, s * 64, row, pl * units + unit);
+}
+
+// Adds a partial result's first n columns (rounded up to 32) into registers: acc = acc * alpha + part.
+template <int N32, bool SCALE>
+__device__ __forceinline__ void flush(f32x2 (&acc)[N32 * 16], uint32_t taddr, int n, float alpha)
+{
+    const f32x2 al = pack2(alpha, alpha);
+#pragma unroll
+    for (int c = 0; c < N32; c++) {
+        if (c * 32 < n) {
+            uint32_t u[32];
+            tmem_ld_32x32b_x32(taddr + c * 32, u);
+            tmem_wait_ld();
+#pragma unroll
+            for (int i = 0; i < 16; i++) {
+                const f32x2 part = pack2(__uint_as_float(u[2 * i]), __uint_as_float(u[2 * i + 1]));
+                acc[c * 16 + i] = SCALE ? fma2(acc[c * 16 + i], al, part) : add2(acc[c * 16 + i], part);
+            }
+        }
+    }
+}
+
+template <int N>
+__device__ __forceinline__ void store_cols(float *dst, const f32x2 (&v2)[N / 2], float scale, int col0, int d, bool vec, const void *base, size_t bytes,
+                                           DeviceStatus *status)
+{
+    (void)base; (void)bytes; (void)status;
+#pragma unroll
+    for (int c = 0; c < N; c += 4) {
+        float v[4];
+        unpack2(v2[c / 2], v[0], v[1]);
+        unpack2(v2[c / 2 + 1], v[2], v[3]);
+        if (vec) {
+            if (col0 + c < d && EMBER_STORE_OK(dst + col0 + c, base, bytes, 16, status))
+                *reinterpret_cast<float4 *>(dst + col0 + c) = make_float4(v[0] * scale, v[1] * scale, v[2] * scale, v[3] * scale);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                if (col0 + c + i < d && EMBER_STORE_OK(dst + col0 + c + i, base, bytes, 4, status)) dst[col0 + c + i] = v[i] * scale;
+        }
+    }
+}
+
+// ---------------------------------------------------------------- forward
+// The two warpgroups take the key tiles in turn, each with its own running maximum, sum and output, which are put together at
+// the end: while one forms its probabilities, the tensor core works for the other. Tensor memory: the query rows' parts,
+// scores and probabilities for each warpgroup (at 128 columns over one another), and the partial output.
+// Two warps issue, one the score products and one the others: beside the compute warps, which evict its few instructions from
+// the scheduler's own cache, an issuing warp needs 50 clocks for an MMA that takes 32 (alone 16), and one for both held a tile at 3570 clocks.
+template <int HD>
+struct F32FwdCfg {
+    static constexpr int TILE = 3 * (HD / 64) * SUB;  // 24 or 48 KB
+    static constexpr int KST = HD == 64 ? 3 : 2, VST = KST;
+    static constexpr int OFF_K = 0, OFF_V = KST * TILE, OFF_BAR = OFF_V + VST * TILE;
+    static constexpr int USED = OFF_BAR + 256, SMEM = USED + 1024;
+    // HD 64: one score buffer, read out at once, apart from the probabilities, and a partial output for each warpgroup, added up a
+    // turn later. HD 128: scores under the probabilities, one partial output, added up before the next one's product.
+    static constexpr bool LATE = HD == 64;
+    static constexpr int T_Q = 0, T_S = 3 * HD / 2 + (LATE ? 0 : SCORES_AT), S_STEP = LATE ? 0 : REGION;
+    static constexpr int T_P = LATE ? 3 * HD / 2 + TN : 3 * HD / 2, T_O = T_P + 2 * REGION, O_STEP = LATE ? HD : 0;
+    static_assert(T_O + HD + O_STEP <= 512, "");
+    enum { B_Q, B_KFULL, B_KEMPTY = B_KFULL + KST, B_VFULL = B_KEMPTY + KST, B_VEMPTY = B_VFULL + VST, B_S = B_VEMPTY + VST, B_P = B_S + 2, B_O = B_P + 2, B_OFREE = B_O + 2, B_SREAD = B_OFREE + 2, NUM_BARS };
+};
+
+struct F32FwdParams {
+    const float *q;
+    float *out, *lse;
+    int lq, lk, d, causal;
+    bool vec_q, vec_o;
+    float scale;
+    SplitGuard guard;
+    DeviceStatus *status;
+    WorkOrder order;
+};
+
+template <int HD>
+__global__ void __launch_bounds__(F32_THREADS, 1)
+    sm100_f32_fwd_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v, const F32FwdParams p)
+{
+    using C = F32FwdCfg<HD>;
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    uint8_t *smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
+    const uint32_t bar0 = smem_base + C::OFF_BAR;
+    auto BAR = [&](int i) { return bar0 + 8u * (uint32_t)i; };
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem_gen + C::OFF_BAR + 8 * C::NUM_BARS);
+    volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    int unit, rank;
+    work_item(p.order, blockIdx.x, unit, rank);
+    const int q0 = (p.order.blocks - 1 - rank) * 128, off = p.lk - p.lq;  // heaviest (latest) causal rows first
+    const int n = ((p.causal ? min(p.lk, q0 + 128 + off) : p.lk) + TN - 1) / TN;
+
+    if (threadIdx.x == 0) {
+        *abort_flag = 0;
+        mbar_init(BAR(C::B_Q), 8);
+        for (int s = 0; s < C::KST; s++) { mbar_init(BAR(C::B_KFULL + s), 1); mbar_init(BAR(C::B_KEMPTY + s), 1); }
+        for (int s = 0; s < C::VST; s++) { mbar_init(BAR(C::B_VFULL + s), 1); mbar_init(BAR(C::B_VEMPTY + s), 1); }
+        for (int w = 0; w < 2; w++) {
+            mbar_init(BAR(C::B_S + w), 1);
+            mbar_init(BAR(C::B_P + w), 4);
+            mbar_init(BAR(C::B_O + w), 1);
+            mbar_init(BAR(C::B_OFREE + w), 4);
+        }
+        mbar_init(BAR(C::B_SREAD), 4);
+        fence_mbar_init();
+    }
+    if (warp == 11) {
+        tmem_alloc(smem_u32(tmem_slot), 512);
+        tmem_relinquish();
+    }
+    if (warp == 9 && lane == 0) {
+        prefetch_tensormap(&tm_k);
+        prefetch_tensormap(&tm_v);
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+    pdl_launch_dependents();
+    pdl_wait();
+    const bool leave = split_out_of_range(p.guard, tmem_slot + 2);
+
+    if (leave) {
+        // the kernel behind this one does the work
+    } else if (warp >= 8) {
+        reg_dealloc_40();
+        if (warp == 9 && lane == 0) {
+            // ------------------------------------------------------------ TMA producer
+            int k_issued = 0, v_issued = 0;
+            for (int j = 0; j < n; j++) {
+                const int ks = j % C::KST, vs = j % C::VST;
+                if (!mbar_wait(BAR(C::B_KEMPTY + ks), ((j / C::KST) & 1) ^ 1, abort_flag, p.status, WF_KEMPTY)) break;
+                load_planes<HD>(smem_base + C::OFF_K + ks * C::TILE, &tm_k, BAR(C::B_KFULL + ks), j * TN, unit, p.order.units);
+                k_issued = j + 1;
+                if (!mbar_wait(BAR(C::B_VEMPTY + vs), ((j / C::VST) & 1) ^ 1, abort_flag, p.status, WF_VEMPTY)) break;
+                load_planes<HD>(smem_base + C::OFF_V + vs * C::TILE, &tm_v, BAR(C::B_VFULL + vs), j * TN, unit, p.order.units);
+                v_issued = j + 1;
+            }
+            // do not leave while a copy is still landing in shared memory
+            const long long t0 = clock64();
+            for (int j = max(0, k_issued - C::KST); j < k_issued; j++)
+                while (!mbar_try_wait(BAR(C::B_KFULL + j % C::KST), (j / C::KST) & 1) && clock64() - t0 < kWaitLimitCycles) {}
+            for (int j = max(0, v_issued - C::VST); j < v_issued; j++)
+                while (!mbar_try_wait(BAR(C::B_VFULL + j % C::VST), (j / C::VST) & 1) && clock64() - t0 < kWaitLimitCycles) {}
+        } else if (warp == 8) {
+            // ------------------------------------------------------------ score products
+            const int ksteps = (p.d + 15) / 16;
+            const uint32_t elected = elect_one();
+            bool ok = mbar_wait(BAR(C::B_Q), 0, abort_flag, p.status, WF_Q);
+            for (int j = 0; j < n && ok; j++) {
+                const int w = j & 1;
+                ok = ok && mbar_wait(BAR(C::B_KFULL + j % C::KST), (j / C::KST) & 1, abort_flag, p.status, WF_K);
+                // the last scores here have been read, or (in the same columns) their probabilities multiplied
+                if (C::LATE && j > 0) ok = ok && mbar_wait(BAR(C::B_SREAD), (j - 1) & 1, abort_flag, p.status, WF_P);
+                if (!C::LATE && j > 1) ok = ok && mbar_wait(BAR(C::B_O + w), ((j - 2) >> 1) & 1, abort_flag, p.status, WF_P);
+                tc_fence_after();
+                mma_scores<HD, false>(tmem + C::T_S + w * C::S_STEP, tmem + C::T_Q, smem_base + C::OFF_K + (j % C::KST) * C::TILE, ksteps, elected);
+                tc_commit_elect(BAR(C::B_S + w));
+                tc_commit_elect(BAR(C::B_KEMPTY + j % C::KST));
+            }
+        } else if (warp == 10) {
+            // ------------------------------------------------------------ probabilities x V
+            const uint32_t idesc_o = idesc_bf16_f32(128, (p.d + 15) / 16 * 16, 0, 1);
+            const uint32_t elected = elect_one();
+            bool ok = true;
+            for (int j = 0; j < n && ok; j++) {
+                const int w = j & 1;
+                ok = ok && mbar_wait(BAR(C::B_VFULL + j % C::VST), (j / C::VST) & 1, abort_flag, p.status, WF_V);
+                ok = ok && mbar_wait(BAR(C::B_P + w), (j >> 1) & 1, abort_flag, p.status, WF_P);
+                // the partial output has been added up (LATE: this warpgroup did so before it wrote its probabilities)
+                if (!C::LATE && j > 0) ok = ok && mbar_wait(BAR(C::B_OFREE + (w ^ 1)), ((j - 1) >> 1) & 1, abort_flag, p.status, WF_OFREE);
+                tc_fence_after();
+                mma_results<HD>(tmem + C::T_O + w * C::O_STEP, tmem + C::T_P + w * REGION, smem_base + C::OFF_V + (j % C::VST) * C::TILE, idesc_o, elected);
+                tc_commit_elect(BAR(C::B_O + w));
+                tc_commit_elect(BAR(C::B_VEMPTY + j % C::VST));
+            }
+        }
+    } else {
+        // ---------------------------------------------------------------- softmax and output
+        reg_alloc_232();
+        const int w = warp / 4, r = threadIdx.x % 128, row = q0 + r;
+        const uint32_t lane_sel = (uint32_t)((warp % 4) * 32) << 16;
+        const float *src = row < p.lq ? p.q + ((size_t)unit * p.lq + row) * p.d : nullptr;
+        row_to_tmem(src, p.d, p.vec_q, w * (HD / 2), HD / 64, tmem + lane_sel + C::T_Q, HD / 2);
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(BAR(C::B_Q));
+
+        const uint32_t scores = tmem + lane_sel + C::T_S + w * C::S_STEP, region = tmem + lane_sel + C::T_P + w * REGION, to = tmem + lane_sel + C::T_O + w * C::O_STEP;
+        const int limit_row = p.causal ? min(p.lk - 1, row + off) : p.lk - 1;
+        const int limit_tile = p.causal ? min(p.lk - 1, q0 + off) : p.lk - 1;
+        const int cols = (p.d + 15) / 16 * 16;
+        float m = -INFINITY, l = 0.f, late_alpha = 1.f;
+        int late = -1;  // LATE: the tile whose partial output is still to be added, with this factor for what it is added to
+        f32x2 o[HD / 2];
+#pragma unroll
+        for (int i = 0; i < HD / 2; i++) o[i] = 0;
+        const f32x2 scale2 = pack2(p.scale, p.scale), l2e = pack2(LOG2E_T, LOG2E_T);
+        bool ok = true;
+        for (int j = w; j < n && ok; j += 2) {
+            const int k0 = j * TN;
+            ok = ok && mbar_wait(BAR(C::B_S + w), (j >> 1) & 1, abort_flag, p.status, WF_S);
+            tc_fence_after();
+            f32x2 s[32];
+            {
+                uint32_t u[32], v[32];
+                tmem_ld_32x32b_x32(scores, u);
+                tmem_ld_32x32b_x32(scores + 32, v);
+                tmem_wait_ld();
+#pragma unroll
+                for (int i = 0; i < 16; i++) {
+                    s[i] = mul2(pack2(__uint_as_float(u[2 * i]), __uint_as_float(u[2 * i + 1])), scale2);
+                    s[16 + i] = mul2(pack2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])), scale2);
+                }
+            }
+            if (C::LATE) {
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(BAR(C::B_SREAD));
+            }
+            if (k0 + TN - 1 > limit_tile) {
+#pragma unroll
+                for (int i = 0; i < 32; i++) {
+                    float x, y;
+                    unpack2(s[i], x, y);
+                    s[i] = pack2(k0 + 2 * i > limit_row ? -INFINITY : x, k0 + 2 * i + 1 > limit_row ? -INFINITY : y);
+                }
+            }
+            float m4[4] = {m, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+            for (int i = 0; i < 32; i++) {
+                float x, y;
+                unpack2(s[i], x, y);
+                m4[i & 3] = max3(m4[i & 3], x, y);
+            }
+            const float m_new = fmaxf(max3(m4[0], m4[1], m4[2]), m4[3]);
+            const float ref = m_new == -INFINITY ? 0.f : m_new;  // masked keys alone so far: weights of 0
+            const float alpha = exp_nat(m - ref);
+            m = m_new;
+            const f32x2 ref2 = pack2(ref, ref);
+            f32x2 sum[2] = {0, 0};
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+#pragma unroll
+                for (int i = 0; i < 16; i++) {
+                    float x, y;
+                    unpack2(mul2(sub2(s[h * 16 + i], ref2), l2e), x, y);
+                    s[h * 16 + i] = pack2(ex2(x), ex2(y));
+                    sum[i & 1] = add2(sum[i & 1], s[h * 16 + i]);
+                }
+                if (C::LATE && h == 0 && late >= 0) {  // before the first probabilities: what they overwrite has been multiplied
+                    ok = ok && mbar_wait(BAR(C::B_O + w), (late >> 1) & 1, abort_flag, p.status, WF_O);
+                    tc_fence_after();
+                    flush<HD / 32, true>(o, to, cols, late_alpha);
+                }
+                split_to_tmem(s + h * 16, region + h * 48);
+            }
+            tmem_wait_st();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(BAR(C::B_P + w));
+            {
+                float x, y;
+                unpack2(add2(sum[0], sum[1]), x, y);
+                l = l * alpha + (x + y);
+            }
+            if (C::LATE) {
+                late = j;
+                late_alpha = alpha;
+            } else {
+                ok = ok && mbar_wait(BAR(C::B_O + w), (j >> 1) & 1, abort_flag, p.status, WF_O);
+                tc_fence_after();
+                flush<HD / 32, true>(o, to, cols, alpha);
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(BAR(C::B_OFREE + w));
+            }
+        }
+        if (C::LATE && late >= 0) {
+            ok = ok && mbar_wait(BAR(C::B_O + w), (late >> 1) & 1, abort_flag, p.status, WF_O);
+            tc_fence_after();
+            flush<HD / 32, true>(o, to, cols, late_alpha);
+        }
+        // ---- the two warpgroups' results: each finishes half of the columns, the other half goes to the other one through shared
+        // memory (no copy is in flight any more, and after the barrier no product either)
+        constexpr int HALF = HD / 2, ROWB = HALF * 4;
+        float2 *state = reinterpret_cast<float2 *>(smem_gen);                    // [2][128] maximum and sum
+        uint8_t *xo = smem_gen + 2048;                                           // [2][128][HALF]: the half that warpgroup w finishes
+        named_bar_sync(1, 256);
+        state[w * 128 + r] = make_float2(m, l);
+        {
+            uint8_t *dst = xo + ((w ^ 1) * 128 + r) * ROWB;
+#pragma unroll
+            for (int c = 0; c < HALF / 4; c++) {
+                const int i = 2 * c;
+                const ulonglong2 v = w == 0 ? make_ulonglong2(o[HALF / 2 + i], o[HALF / 2 + i + 1]) : make_ulonglong2(o[i], o[i + 1]);
+                *reinterpret_cast<ulonglong2 *>(dst + (((c & ~7) | ((c ^ r) & 7)) << 4)) = v;
+            }
+        }
+        named_bar_sync(1, 256);
+        const float2 other = state[(w ^ 1) * 128 + r];
+        const float mm = fmaxf(m, other.x);
+        const float a_own = exp_nat(m - mm), a_other = exp_nat(other.x - mm);
+        const float ll = w == 0 ? l * a_own + other.y * a_other : other.y * a_other + l * a_own;
+        const float inv = 1.f / ll;
+        f32x2 res[HALF / 2];
+        {
+            const uint8_t *from = xo + (w * 128 + r) * ROWB;
+            const f32x2 own2 = pack2(a_own, a_own), other2 = pack2(a_other, a_other);
+#pragma unroll
+            for (int c = 0; c < HALF / 4; c++) {
+                const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(from + (((c & ~7) | ((c ^ r) & 7)) << 4));
+                const int i = 2 * c;
+                res[i] = fma2(w == 0 ? o[i] : o[HALF / 2 + i], own2, mul2(v.x, other2));
+                res[i + 1] = fma2(w == 0 ? o[i + 1] : o[HALF / 2 + i + 1], own2, mul2(v.y, other2));
+            }
+        }
+        if (ok && row < p.lq) {
+            const size_t at = (size_t)unit * p.lq + row;
+            store_cols<HALF>(p.out + at * p.d, res, inv, w * HALF, p.d, p.vec_o, p.out, (size_t)p.order.units * p.lq * p.d * 4, p.status);
+            if (p.lse && w == 0 && EMBER_STORE_OK(p.lse + at, p.lse, (size_t)p.order.units * p.lq * 4, 4, p.status)) p.lse[at] = mm + logf(ll);
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 11) tmem_dealloc(tmem, 512);
+}
+
+// ---------------------------------------------------------------- backward
+// Work items (roles). A CTA owns 128 rows of one side and streams the other side's tiles:
+//   DKDV (HD 64)   keys:    S^T = K Q^T, P; dP^T = V dO^T, dS;  dV += P dO, dK += dS Q
+//   DK, DV (HD 128) the same, one result each (tensor memory holds one 128-column result beside the parts)
+//   DQ             queries: S = Q K^T, dP = dO V^T, dS;         dQ += dS K
+// so there is one form: A0 and A1 are the CTA's rows, B0 and B1 the streamed tiles, S = A0 B0^T, dP = A1 B1^T, results P B1 and
+// dS B0. Both products of a tile recompute P from the log-sum-exp; no atomics, results repeat bit for bit.
+// A warpgroup takes 32 of a tile's 64 columns.
+enum Role { R_DKDV = 0, R_DQ = 1, R_DK = 2, R_DV = 3 };
+
+template <int HD>
+struct F32BwdCfg {
+    static constexpr int TILE = 3 * (HD / 64) * SUB;
+    static constexpr int A_BYTES = 2 * TILE;                       // 128 rows (A1 at HD 128)
+    // A ring of 3 pairs of tiles beside A1 (HD 64), one pair (HD 128), or (DV, which needs no A1) 2.
+    static constexpr int MAXST = HD == 64 ? 3 : 2, STAGES = HD == 64 ? 3 : 1;
+    static constexpr int OFF_B = 0, OFF_A1 = STAGES * 2 * TILE;    // TILE pairs, A1
+    static constexpr int OFF_VEC = OFF_A1 + A_BYTES;               // per warp: 32 log-sum-exps, 32 deltas
+    static constexpr int OFF_BAR = OFF_VEC + 8 * 256, USED = OFF_BAR + 256, SMEM = USED + 1024;
+    static_assert(HD == 64 || OFF_VEC == MAXST * 2 * TILE, "");
+    // Columns. HD 64: A0, S, P, dP / dS, two results; S is apart from P, so that the next S does not wait for the product of P
+    // (with A1 in tensor memory and S under P a tile took 5700 clocks). HD 128: A0, S, dP / dS, result; DV: A0, two regions
+    // of S / P, result.
+    static constexpr int T_A0 = 0, T_S = 3 * HD / 2 + (HD == 64 ? 0 : SCORES_AT), T_P = HD == 64 ? 160 : 192, T_D = HD == 64 ? 256 : 288, T_R = HD == 64 ? 352 : 384;
+    enum { B_A, B_FULL0, B_FULL1 = B_FULL0 + MAXST, B_EMPTY0 = B_FULL1 + MAXST, B_EMPTY1 = B_EMPTY0 + MAXST, B_S = B_EMPTY1 + MAXST, B_P, B_DP, B_DS, B_R0, B_R1, B_F0, B_F1, NUM_BARS,
+           B_S1 = B_DP };  // DV: scores of odd tiles (the next tile's may be there before this one's have been waited for)
+    static_assert(8 * NUM_BARS + 16 <= 256, "");
+};
+
+struct F32BwdParams {
+    const float *q, *k, *v, *dout, *lse, *delta;
+    float *dq, *dk, *dv;
+    int units, lq, lk, d, causal;
+    int kblocks, qblocks;
+    bool vec_in, vec_out;
+    float scale;
+    SplitGuard guard;
+    DeviceStatus *status;
+    WorkOrder order;
+};
+
+// Which role and block the rank-th heaviest item of a unit is.
+template <int HD>
+__device__ __forceinline__ void bwd_item(int rank, int kb, int qb, int &role, int &blk)
+{
+    constexpr int NR = HD == 64 ? 2 : 3;
+    const int m = min(kb, qb);
+    if (rank < NR * m) {
+        const int i = rank % NR;
+        blk = rank / NR;
+        role = i == 1 ? R_DQ : HD == 64 ? R_DKDV : i == 0 ? R_DK : R_DV;
+    } else if (qb > kb) {
+        role = R_DQ;
+        blk = m + rank - NR * m;
+    } else if (HD == 64) {
+        role = R_DKDV;
+        blk = m + rank - NR * m;
+    } else {
+        const int i = rank - NR * m;
+        role = i % 2 ? R_DV : R_DK;
+        blk = m + i / 2;
+    }
+}
+
+template <int HD>
+__global__ void __launch_bounds__(F32_THREADS, 1)
+    sm100_f32_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
+                         const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do, const F32BwdParams p)
+{
+    using C = F32BwdCfg<HD>;
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    uint8_t *smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
+    const uint32_t bar0 = smem_base + C::OFF_BAR;
+    auto BAR = [&](int i) { return bar0 + 8u * (uint32_t)i; };
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem_gen + C::OFF_BAR + 8 * C::NUM_BARS);
+    volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    int unit, rank, role, blk;
+    work_item(p.order, blockIdx.x, unit, rank);
+    bwd_item<HD>(rank, p.kblocks, p.qblocks, role, blk);
+    const bool is_q = role == R_DQ;
+    const bool has_p = role == R_DKDV || role == R_DV, has_ds = role != R_DV;  // which results
+    const int off = p.lk - p.lq;
+    const int row0 = (is_q ? p.qblocks - 1 - blk : blk) * 128;  // heaviest first: the last queries, the first keys
+    // the streamed tiles: rows [first, ...) of the other side
+    const int first = is_q || !p.causal ? 0 : max(0, (row0 - off) / TN) * TN;
+    const int end = is_q ? (p.causal ? min(p.lk, row0 + 128 + off) : p.lk) : p.lq;
+    const int n = (end - first + TN - 1) / TN;
+    const int stages = role == R_DV ? 2 : C::STAGES;
+
+    if (threadIdx.x == 0) {
+        *abort_flag = 0;
+        mbar_init(BAR(C::B_A), has_ds ? 9 : 8);  // the compute warps, and the copies of A1
+        for (int s = 0; s < C::MAXST; s++) {
+            mbar_init(BAR(C::B_FULL0 + s), 1);
+            mbar_init(BAR(C::B_FULL1 + s), 1);
+            mbar_init(BAR(C::B_EMPTY0 + s), 1);
+            mbar_init(BAR(C::B_EMPTY1 + s), role == R_DKDV ? 2 : 1);  // read by both issuing warps' products
+        }
+        mbar_init(BAR(C::B_S), 1);
+        mbar_init(BAR(C::B_P), 8);
+        mbar_init(BAR(C::B_DP), 1);
+        mbar_init(BAR(C::B_DS), 8);
+        mbar_init(BAR(C::B_R0), 1);
+        mbar_init(BAR(C::B_R1), 1);
+        mbar_init(BAR(C::B_F0), role == R_DKDV ? 4 : 8);
+        mbar_init(BAR(C::B_F1), 4);
+        fence_mbar_init();
+    }
+    if (warp == 11) {
+        tmem_alloc(smem_u32(tmem_slot), 512);
+        tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+    pdl_launch_dependents();
+    pdl_wait();
+    const bool leave = split_out_of_range(p.guard, tmem_slot + 2);
+
+    const uint32_t t_s = tmem + C::T_S, t_p = tmem + C::T_P, t_d = tmem + C::T_D, t_r = tmem + C::T_R;
+    if (leave) {
+        // the kernel behind this one does the work
+    } else if (warp >= 8) {
+        reg_dealloc_40();
+        if (warp == 9 && lane == 0) {
+            // ------------------------------------------------------------ TMA producer
+            const CUtensorMap *b0 = is_q ? &tm_k : &tm_q, *b1 = is_q ? &tm_v : &tm_do;
+            if (has_ds) {  // A1: 128 rows as boxes of 64
+                const CUtensorMap *a1 = is_q ? &tm_do : &tm_v;
+                mbar_arrive_expect_tx(BAR(C::B_A), C::A_BYTES);
+                for (int pl = 0; pl < 3; pl++)
+                    for (int s = 0; s < HD / 64; s++)
+                        for (int h = 0; h < 2; h++)
+                            tma_load_3d(smem_base + C::OFF_A1 + ((pl * (HD / 64) + s) * 2 + h) * SUB, a1, BAR(C::B_A), s * 64, row0 + h * 64, pl * p.units + unit);
+            }
+            int issued0 = 0, issued1 = 0;
+            for (int j = 0; j < n; j++) {
+                const int s = j % stages, ph = ((j / stages) & 1) ^ 1;
+                const uint32_t dst = smem_base + C::OFF_B + s * 2 * C::TILE;
+                // one pair of tiles alone: B1 is free before B0 is (its product comes before the one that reads B0 last)
+                if (stages == 1 && j > 0) {
+                    if (!mbar_wait(BAR(C::B_EMPTY1), ph, abort_flag, p.status, WB_E1)) break;
+                    load_planes<HD>(dst + C::TILE, b1, BAR(C::B_FULL1), first + j * TN, unit, p.units);
+                    issued1 = j + 1;
+                }
+                if (!mbar_wait(BAR(C::B_EMPTY0 + s), ph, abort_flag, p.status, WB_E0)) break;
+                load_planes<HD>(dst, b0, BAR(C::B_FULL0 + s), first + j * TN, unit, p.units);
+                issued0 = j + 1;
+                if (stages > 1 || j == 0) {
+                    if (!mbar_wait(BAR(C::B_EMPTY1 + s), ph, abort_flag, p.status, WB_E1)) break;
+                    load_planes<HD>(dst + C::TILE, b1, BAR(C::B_FULL1 + s), first + j * TN, unit, p.units);
+                    issued1 = j + 1;
+                }
+            }
+            // do not leave while a copy is still landing in shared memory
+            const long long t0 = clock64();
+            for (int j = max(0, issued0 - stages); j < issued0; j++)
+                while (!mbar_try_wait(BAR(C::B_FULL0 + j % stages), (j / stages) & 1) && clock64() - t0 < kWaitLimitCycles) {}
+            for (int j = max(0, issued1 - stages); j < issued1; j++)
+                while (!mbar_try_wait(BAR(C::B_FULL1 + j % stages), (j / stages) & 1) && clock64() - t0 < kWaitLimitCycles) {}
+            while (has_ds && !mbar_try_wait(BAR(C::B_A), 0) && clock64() - t0 < kWaitLimitCycles) {}
+        } else if (warp == 8) {
+            // ------------------------------------------------------------ S and dP
+            const int ksteps = (p.d + 15) / 16;
+            const uint32_t elected = elect_one();
+            bool ok = mbar_wait(BAR(C::B_A), 0, abort_flag, p.status, WB_A);
+            auto wait = [&](int bar, int phase, int where) { ok = ok && mbar_wait(BAR(bar), phase & 1, abort_flag, p.status, where); };
+            for (int j = 0; j < n && ok; j++) {
+                const int s = j % stages;
+                const uint32_t b0 = smem_base + C::OFF_B + s * 2 * C::TILE;
+                // the scores that these overwrite have been read (DV: their probabilities multiplied)
+                uint32_t at = t_s;
+                int done = C::B_S;
+                wait(C::B_FULL0 + s, j / stages, WB_B0);
+                if (role == R_DV) {  // two regions in turn
+                    at += (j & 1) * REGION;
+                    done = j & 1 ? C::B_S1 : C::B_S;
+                    if (j > 1) wait(j & 1 ? C::B_R1 : C::B_R0, (j - 2) >> 1, WB_ACC);
+                } else if (j > 0) {
+                    wait(C::B_P, j - 1, WB_ACC);
+                }
+                tc_fence_after();
+                mma_scores<HD, false>(at, tmem + C::T_A0, b0, ksteps, elected);
+                tc_commit_elect(BAR(done));
+                if (!has_ds) {
+                    tc_commit_elect(BAR(C::B_EMPTY0 + s));
+                    continue;
+                }
+                wait(C::B_FULL1 + s, j / stages, WB_B1);
+                if (j > 0) wait(role == R_DKDV ? C::B_R1 : C::B_R0, j - 1, WB_ACC);  // over dS
+                tc_fence_after();
+                mma_scores<HD, true>(t_d + SCORES_AT, smem_base + C::OFF_A1, b0 + C::TILE, ksteps, elected);
+                tc_commit_elect(BAR(C::B_DP));
+                tc_commit_elect(BAR(C::B_EMPTY1 + s));
+            }
+        } else if (warp == 10) {
+            // ------------------------------------------------------------ P B1 and dS B0
+            const uint32_t idesc_r = idesc_bf16_f32(128, (p.d + 15) / 16 * 16, 0, 1);
+            const uint32_t elected = elect_one();
+            bool ok = true;
+            auto wait = [&](int bar, int phase, int where) { ok = ok && mbar_wait(BAR(bar), phase & 1, abort_flag, p.status, where); };
+            for (int j = 0; j < n && ok; j++) {
+                const int s = j % stages;
+                const uint32_t b0 = smem_base + C::OFF_B + s * 2 * C::TILE;
+                if (has_p) {
+                    wait(C::B_P, j, WB_P);
+                    wait(C::B_FULL1 + s, j / stages, WB_B1);
+                    if (j > 0) wait(C::B_F0, j - 1, WB_FREE);
+                    tc_fence_after();
+                    mma_results<HD>(t_r, t_p + (role == R_DV ? (j & 1) * REGION : 0), b0 + C::TILE, idesc_r, elected);
+                    tc_commit_elect(BAR(role == R_DV && (j & 1) ? C::B_R1 : C::B_R0));
+                    tc_commit_elect(BAR(C::B_EMPTY1 + s));
+                }
+                if (has_ds) {
+                    wait(C::B_DS, j, WB_DS);
+                    wait(C::B_FULL0 + s, j / stages, WB_B0);
+                    if (j > 0) wait(role == R_DKDV ? C::B_F1 : C::B_F0, j - 1, WB_FREE);
+                    tc_fence_after();
+                    mma_results<HD>(t_r + (role == R_DKDV ? 64 : 0), t_d, b0, idesc_r, elected);
+                    tc_commit_elect(BAR(role == R_DKDV ? C::B_R1 : C::B_R0));
+                    tc_commit_elect(BAR(C::B_EMPTY0 + s));
+                }
+            }
+        }
+    } else {
+        // ---------------------------------------------------------------- probabilities, score gradients, results
+        reg_alloc_232();
+        const int w = warp / 4, r = threadIdx.x % 128, row = row0 + r;
+        const uint32_t lane_sel = (uint32_t)((warp % 4) * 32) << 16;
+        const int rows = is_q ? p.lq : p.lk;
+        const float *a0 = is_q ? p.q : p.k;
+        const size_t row_at = ((size_t)unit * rows + row) * p.d;
+        row_to_tmem(row < rows ? a0 + row_at : nullptr, p.d, p.vec_in, w * (HD / 2), HD / 64, tmem + lane_sel + C::T_A0, HD / 2);
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(BAR(C::B_A));
+
+        const float *lse = p.lse + (size_t)unit * p.lq, *delta = p.delta + (size_t)unit * p.lq;
+        float *vec = reinterpret_cast<float *>(smem_gen + C::OFF_VEC + warp * 256);  // this warp's 32 columns
+        // Negative log-sum-exp and delta of a query; past the end (and where a row has no weight at all) P is 0: finite, since
+        // the exponential below would make NaN of an infinity.
+        auto neg_lse = [&](int qi) {
+            const float x = qi < p.lq ? lse[qi] : 1e30f;
+            return x > 1e30f ? -1e30f : -x;
+        };
+        auto neg_delta = [&](int qi) { return has_ds && qi < p.lq ? -delta[qi] : 0.f; };
+        const float nl_row = is_q ? neg_lse(row) : 0.f, nd_row = is_q ? neg_delta(row) : 0.f;
+        const int cols = (p.d + 15) / 16 * 16;
+        // results in registers: DKDV: warpgroup 0 dV, 1 dK; otherwise half of the columns each
+        f32x2 acc[32];
+#pragma unroll
+        for (int i = 0; i < 32; i++) acc[i] = 0;
+        const f32x2 scale2 = pack2(p.scale, p.scale);
+        const int acc_col0 = role == R_DKDV ? 0 : w * (HD / 2);
+        const int acc_cols = min(role == R_DKDV ? cols : HD / 2, cols - acc_col0);
+        const uint32_t acc_at = t_r + lane_sel + (role == R_DKDV ? w * 64 : acc_col0);
+        const int bar_r = role == R_DKDV && w == 1 ? C::B_R1 : C::B_R0, bar_f = role == R_DKDV && w == 1 ? C::B_F1 : C::B_F0;
+        bool ok = true;
+        auto add_result = [&](int j) {
+            if (role == R_DV) ok = ok && mbar_wait(BAR(j & 1 ? C::B_R1 : C::B_R0), (j >> 1) & 1, abort_flag, p.status, WB_ACC);
+            else ok = ok && mbar_wait(BAR(bar_r), j & 1, abort_flag, p.status, WB_ACC);
+            tc_fence_after();
+            if (acc_cols > 0) flush<2, false>(acc, acc_at, acc_cols, 1.f);
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(BAR(bar_f));
+        };
+        const bool first_flush = role == R_DKDV && w == 0;  // dV(j - 1) is there before S(j), dK(j - 1) about when P(j) is
+        for (int j = 0; j < n && ok; j++) {
+            const int c0 = first + j * TN + w * 32;  // this warpgroup's first column of the tile
+            if (!is_q) {                             // columns are queries
+                __syncwarp();
+                const int qi = c0 + lane;
+                vec[lane] = neg_lse(qi);
+                vec[32 + lane] = neg_delta(qi);
+                __syncwarp();
+            }
+            // which columns are masked: keys past the row's limit, or queries before the row's key
+            const int hi = is_q ? (p.causal ? min(p.lk - 1, row + off) : p.lk - 1) : p.lq - 1;
+            const int lo = !is_q && p.causal ? row - off : 0;
+            const bool edge = is_q ? first + j * TN + TN - 1 > (p.causal ? min(p.lk - 1, row0 + off) : p.lk - 1)
+                                   : p.causal && row0 + 127 - off > first + j * TN;
+            if (j > 0 && first_flush) add_result(j - 1);
+            if (role == R_DV) ok = ok && mbar_wait(BAR(j & 1 ? C::B_S1 : C::B_S), (j >> 1) & 1, abort_flag, p.status, WB_S);
+            else ok = ok && mbar_wait(BAR(C::B_S), j & 1, abort_flag, p.status, WB_S);
+            tc_fence_after();
+            const uint32_t turn = lane_sel + (role == R_DV ? (j & 1) * REGION : 0);
+            f32x2 e[16];
+            {
+                uint32_t u[32];
+                tmem_ld_32x32b_x32(t_s + turn + w * 32, u);
+                tmem_wait_ld();
+#pragma unroll
+                for (int i = 0; i < 16; i += 2) {
+                    const ulonglong2 nl = is_q ? make_ulonglong2(pack2(nl_row, nl_row), pack2(nl_row, nl_row)) : *reinterpret_cast<const ulonglong2 *>(vec + i * 2);
+                    e[i] = exp_pair(fma2(pack2(__uint_as_float(u[2 * i]), __uint_as_float(u[2 * i + 1])), scale2, nl.x));
+                    e[i + 1] = exp_pair(fma2(pack2(__uint_as_float(u[2 * i + 2]), __uint_as_float(u[2 * i + 3])), scale2, nl.y));
+                }
+                if (edge) {
+#pragma unroll
+                    for (int i = 0; i < 16; i++) {
+                        const int c = c0 + 2 * i;
+                        float x, y;
+                        unpack2(e[i], x, y);
+                        e[i] = pack2(c > hi || c < lo ? 0.f : x, c + 1 > hi || c + 1 < lo ? 0.f : y);
+                    }
+                }
+            }
+            if (has_p) {
+                if (role == R_DKDV && w == 1 && j > 0) {  // the last P has been multiplied (warpgroup 0 has waited for dV, DV's S for its region)
+                    ok = ok && mbar_wait(BAR(C::B_R0), (j - 1) & 1, abort_flag, p.status, WB_ACC);
+                    tc_fence_after();
+                }
+                split_to_tmem(e, t_p + turn + w * 48);
+                tmem_wait_st();
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(BAR(C::B_P));  // P is written, or at least S is read
+            if (j > 0 && !first_flush) add_result(j - 1);
+            if (has_ds) {
+                ok = ok && mbar_wait(BAR(C::B_DP), j & 1, abort_flag, p.status, WB_DP);
+                tc_fence_after();
+                uint32_t u[32];
+                tmem_ld_32x32b_x32(t_d + lane_sel + SCORES_AT + w * 32, u);
+                tmem_wait_ld();
+#pragma unroll
+                for (int i = 0; i < 16; i += 2) {
+                    const ulonglong2 nd = is_q ? make_ulonglong2(pack2(nd_row, nd_row), pack2(nd_row, nd_row)) : *reinterpret_cast<const ulonglong2 *>(vec + 32 + i * 2);
+                    e[i] = mul2(e[i], add2(pack2(__uint_as_float(u[2 * i]), __uint_as_float(u[2 * i + 1])), nd.x));
+                    e[i + 1] = mul2(e[i + 1], add2(pack2(__uint_as_float(u[2 * i + 2]), __uint_as_float(u[2 * i + 3])), nd.y));
+                }
+                split_to_tmem(e, t_d + lane_sel + w * 48);
+                tmem_wait_st();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(BAR(C::B_DS));
+            }
+        }
+        if (ok) add_result(n - 1);
+        if (ok && row < rows && acc_cols > 0) {
+            float *dst = is_q ? p.dq : role == R_DKDV ? (w == 0 ? p.dv : p.dk) : role == R_DK ? p.dk : p.dv;
+            const bool is_dv = role == R_DV || (role == R_DKDV && w == 0);
+            store_cols<64>(dst + row_at, acc, is_dv ? 1.f : p.scale, acc_col0, role == R_DKDV ? p.d : min(p.d, acc_col0 + HD / 2), p.vec_out, dst, (size_t)p.units * rows * p.d * 4, p.status);
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 11) tmem_dealloc(tmem, 512);
+}
+
+int plane_map(CUtensorMap *m, const void *planes, int d, int rows, int units)
+{
+    return make_tensor_map_bf16_3d(m, planes, (uint64_t)((d + 7) / 8 * 8), (uint64_t)rows, 3ull * units, 64, 64);
+}
+
+bool vec_rows(const void *a, const void *b, const void *c, const void *d, int cols)
+{
+    return cols % 4 == 0 && (((uintptr_t)a | (uintptr_t)b | (uintptr_t)c | (uintptr_t)d) & 15) == 0;
+}
+
+cudaError_t launch_cfg(cudaLaunchConfig_t &cfg, LaunchAttrs &attrs, long long grid, size_t smem, cudaStream_t s)
+{
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3(F32_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    attrs.pdl().set(cfg);
+    return cudaSuccess;
+}
+
+template <int HD>
+int launch_fwd(const AttnArgs &a, const void *kp, const void *vp, const SplitGuard &guard, DeviceState *st, cudaStream_t s)
+{
+    using C = F32FwdCfg<HD>;
+    CUtensorMap tk, tv;
+    int rc;
+    if ((rc = plane_map(&tk, kp, a.d, a.lk, a.bh)) != EMBER_OK || (rc = plane_map(&tv, vp, a.d, a.lk, a.bh)) != EMBER_OK) return rc;
+    F32FwdParams p = {};
+    p.q = (const float *)a.q;
+    p.out = (float *)a.out;
+    p.lse = a.lse;
+    p.lq = a.lq; p.lk = a.lk; p.d = a.d; p.causal = a.causal;
+    p.vec_q = vec_rows(a.q, nullptr, nullptr, nullptr, a.d);
+    p.vec_o = vec_rows(a.out, nullptr, nullptr, nullptr, a.d);
+    p.scale = a.scale;
+    p.guard = guard;
+    p.status = st->status;
+    p.order = make_work_order(a.bh, (a.lq + 127) / 128, st->sm_count, (size_t)a.lk * a.d * 12 + (size_t)a.lq * a.d * 8, a.causal != 0);
+    auto kern = sm100_f32_fwd_kernel<HD>;
+    static SmemOptIn opt_in;
+    EMBER_CUDA_TRY(opt_in(kern, C::SMEM));
+    cudaLaunchConfig_t cfg = {};
+    LaunchAttrs attrs;
+    launch_cfg(cfg, attrs, (long long)p.order.units * p.order.blocks, C::SMEM, s);
+    EMBER_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, tk, tv, p));
+    return EMBER_OK;
+}
+
+template <int HD>
+int launch_bwd(const AttnArgs &a, const float *delta, const void *qp, const void *kp, const void *vp, const void *gp, const SplitGuard &guard,
+               DeviceState *st, cudaStream_t s)
+{
+    using C = F32BwdCfg<HD>;
+    CUtensorMap tq, tk, tv, tg;
+    int rc;
+    if ((rc = plane_map(&tq, qp, a.d, a.lq, a.bh)) != EMBER_OK || (rc = plane_map(&tk, kp, a.d, a.lk, a.bh)) != EMBER_OK ||
+        (rc = plane_map(&tv, vp, a.d, a.lk, a.bh)) != EMBER_OK || (rc = plane_map(&tg, gp, a.d, a.lq, a.bh)) != EMBER_OK)
+        return rc;
+    F32BwdParams p = {};
+    p.q = (const float *)a.q; p.k = (const float *)a.k; p.v = (const float *)a.v; p.dout = (const float *)a.dout;
+    p.lse = a.lse; p.delta = delta;
+    p.dq = (float *)a.dq; p.dk = (float *)a.dk; p.dv = (float *)a.dv;
+    p.units = a.bh; p.lq = a.lq; p.lk = a.lk; p.d = a.d; p.causal = a.causal;
+    p.kblocks = (a.lk + 127) / 128;
+    p.qblocks = (a.lq + 127) / 128;
+    p.vec_in = vec_rows(a.q, a.k, a.v, a.dout, a.d);
+    p.vec_out = vec_rows(a.dq, a.dk, a.dv, nullptr, a.d);
+    p.scale = a.scale;
+    p.guard = guard;
+    p.status = st->status;
+    p.order = make_work_order(a.bh, (HD == 64 ? 1 : 2) * p.kblocks + p.qblocks, st->sm_count, ((size_t)a.lk + a.lq) * a.d * 24, a.causal != 0);
+    auto kern = sm100_f32_bwd_kernel<HD>;
+    static SmemOptIn opt_in;
+    EMBER_CUDA_TRY(opt_in(kern, C::SMEM));
+    cudaLaunchConfig_t cfg = {};
+    LaunchAttrs attrs;
+    launch_cfg(cfg, attrs, (long long)p.order.units * p.order.blocks, C::SMEM, s);
+    EMBER_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, tq, tk, tv, tg, p));
+    return EMBER_OK;
+}
+
+// Scales beyond 2^20 could take scores of operands below 2^50 to infinity.
+bool takes(const AttnArgs &a) { return a.dtype == EMBER_F32 && a.d <= 128 && fabsf(a.scale) <= 1048576.f && (long long)a.bh * 3 <= 0x7fffffffLL; }
+
+}  // namespace
+
+// Which kernels take a call: both sides' times are estimated, in us, from measured launches. The tensor-core side has a fixed part (the
+// split, three launches, start and end of a CTA) and works in 128-row blocks, so short or few rows stay on the CUDA cores; its
+// planes cost passes over memory that a few rows against long keys do not pay back. Measured, CUDA cores / tensor cores, causal, forward
+// (F) and backward (B):
+//   d 64    8 x 128 F 10 / 19 B 17 / 21    32 x 128 F 12 / 17 B 28 / 23   1 x 256 F 15 / 18 B 26 / 24    32 x 256 F 25 / 21 B 64 / 29
+//           1 x 512 F 25 / 23 B 43 / 33    8 x 1024 F 74 / 34 B 206 / 56  4 x 2048 F 141 / 52 B 393 / 92  512 x 128 F 56 / 66 B 172 / 145
+//   d 128   8 x 256 F 23 / 27 B 52 / 39    1 x 512 F 39 / 34 B 68 / 57    8 x 1024 F 105 / 56 B 234 / 103 4 x 2048 F 197 / 89 B 444 / 182
+//   rows against keys, d 64   512 x 32 x 2048 F 293 / 411 B 1668 / 1165   128 x 32 x 2048 F 121 / 106 B 483 / 318   512 x 64 x 64 F 26 / 44 B 67 / 87
+// The estimates are within a quarter of these.
+namespace {
+struct Shape {
+    double units, lq, lk, d, visible;  // visible: the share of (query, key) pairs under the mask
+    double qb, kb, qt, kt;             // blocks of 128 rows, tiles of 64
+    bool wide;                         // more than 64 columns
+    double dpad;                       // columns the CUDA-core kernels work on
+    explicit Shape(const AttnArgs &a)
+        : units(a.bh), lq(a.lq), lk(a.lk), d(a.d), visible(a.causal ? 1.0 - (a.lq - 1.0) / (2.0 * a.lk) : 1.0), qb((a.lq + 127) / 128), kb((a.lk + 127) / 128),
+          qt((a.lq + 63) / 64), kt((a.lk + 63) / 64), wide(a.d > 64), dpad(a.d <= 32 ? 32 : a.d <= 64 ? 64 : 128)
+    {
+    }
+};
+double longest(double a, double b) { return a > b ? a : b; }
+}  // namespace
+
+bool sm100_f32_fwd_preferred(const AttnArgs &a, int sms)
+{
+    if (!takes(a) || (long long)a.bh * ((a.lq + 127) / 128) > 0x7fffffffLL) return false;
+    const Shape s(a);
+    const double tile = s.wide ? 2.1 : 1.13, cta = s.wide ? 7.0 : 5.5, waves = s.units * s.qb / (sms > 0 ? sms : 148);
+    const double tensor = 10.0 + longest(cta + tile * s.kt, waves * (cta + tile * (s.visible * s.kt + 0.5))) + s.units * s.lk * s.d * 32.0 / 7.5e6;
+    const double rows = (a.lq + 15) / 16 * 16.0;
+    const double cores = 5.0 + s.lk * (s.wide ? 0.0665 : s.dpad > 32 ? 0.041 : 0.028) + 35e-9 * 4.0 * s.units * rows * s.lk * s.dpad * s.visible;
+    return tensor < cores;
+}
+
+bool sm100_f32_bwd_preferred(const AttnArgs &a, int sms)
+{
+    if (!takes(a) || (long long)a.bh * (2 * ((a.lk + 127LL) / 128) + (a.lq + 127) / 128) > 0x7fffffffLL) return false;
+    const Shape s(a);
+    const double tile = s.wide ? 4.9 : 2.29, cta = s.wide ? 9.5 : 6.5, kinds = s.wide ? 2.0 : 1.0, blocks = kinds * s.kb + s.qb;
+    const double mean = s.visible * (kinds * s.kb * s.qt + s.qb * s.kt) / blocks;
+    const double tensor = 8.0 + longest(cta + tile * longest(s.qt, s.kt), s.units * blocks / (sms > 0 ? sms : 148) * (cta + tile * mean)) +
+                          s.units * (s.lq + s.lk) * s.d * 32.0 / 7.5e6;
+    const double rows = 0.57 * s.qt * 64.0 + 0.43 * ((a.lq + 15) / 16 * 16.0);
+    const double cores = 8.0 + longest(s.lq, s.lk) * (s.wide ? 0.117 : s.dpad > 32 ? 0.07 : 0.05) + 33e-9 * 14.0 * s.units * rows * s.lk * s.dpad * s.visible;
+    return tensor < 0.95 * cores;
+}
+
+int sm100_f32_attention_fwd(const AttnArgs &a, DeviceState *st, cudaStream_t s)
+{
+    const long long q_rows = (long long)a.bh * a.lq, k_rows = (long long)a.bh * a.lk;
+    const size_t k_bytes = split_bytes(k_rows, a.d);
+    char *mem = nullptr;
+    if (!scratch_alloc((void **)&mem, kSplitGuardBytes + 2 * k_bytes, s)) return EMBER_ERR_NOMEM;
+    const SplitJob jobs[3] = {{(const float *)a.k, mem, k_rows, a.d}, {(const float *)a.v, mem + k_bytes, k_rows, a.d}, {(const float *)a.q, nullptr, q_rows, a.d}};
+    SplitGuard guard;
+    int rc = split_f32(jobs, 3, nullptr, mem + 2 * k_bytes, &guard, s);
+    if (rc == EMBER_OK)
+        rc = a.d <= 64 ? launch_fwd<64>(a, mem, mem + k_bytes, guard, st, s) : launch_fwd<128>(a, mem, mem + k_bytes, guard, st, s);
+    if (rc == EMBER_OK) {
+        AttnArgs t = a;
+        t.only_if = guard.fallback;
+        rc = simt_attention_fwd(t, st, s);
+    }
+    cudaFreeAsync(mem, s);
+    return rc;
+}
+
+int sm100_f32_attention_bwd(const AttnArgs &a, float *delta, DeviceState *st, cudaStream_t s)
+{
+    const long long q_rows = (long long)a.bh * a.lq, k_rows = (long long)a.bh * a.lk;
+    const size_t q_bytes = split_bytes(q_rows, a.d), k_bytes = split_bytes(k_rows, a.d);
+    char *mem = nullptr;
+    if (!scratch_alloc((void **)&mem, kSplitGuardBytes + 2 * q_bytes + 2 * k_bytes, s)) return EMBER_ERR_NOMEM;
+    char *qp = mem, *gp = qp + q_bytes, *kp = gp + q_bytes, *vp = kp + k_bytes, *words = vp + k_bytes;
+    const SplitJob jobs[4] = {{(const float *)a.q, qp, q_rows, a.d}, {(const float *)a.dout, gp, q_rows, a.d}, {(const float *)a.k, kp, k_rows, a.d}, {(const float *)a.v, vp, k_rows, a.d}};
+    const SplitDelta dl = {(const float *)a.out, (const float *)a.dout, delta, q_rows, a.d};
+    SplitGuard guard;
+    int rc = split_f32(jobs, 4, &dl, words, &guard, s);
+    if (rc == EMBER_OK)
+        rc = a.d <= 64 ? launch_bwd<64>(a, delta, qp, kp, vp, gp, guard, st, s) : launch_bwd<128>(a, delta, qp, kp, vp, gp, guard, st, s);
+    if (rc == EMBER_OK) {
+        AttnArgs t = a;
+        t.only_if = guard.fallback;
+        rc = simt_attention_bwd(t, delta, true, st, s);
+    }
+    cudaFreeAsync(mem, s);
+    return rc;
+}
+
+}  // namespace ember

@@ -1,7 +1,6 @@
 // Attention on the CUDA cores: float32 arithmetic throughout, float32 or bf16 storage, any head
-// dimension up to 128, any sequence lengths. These kernels serve the float32 I/O mode (whose tolerance
-// against the reference is too tight for bf16 tensor-core products) and the bf16 shapes the tcgen05
-// kernels do not take.
+// dimension up to 128, any sequence lengths. These kernels serve small float32 calls, float32 values that the tensor-core
+// kernels (attn_f32_sm100.cu) cannot hold, and the bf16 shapes that the tcgen05 kernels do not take.
 //
 // Bound: the float32 FMA pipe (128 per clock and SM). A product of two 64-row tiles over 64 columns is
 // 2048 SM clocks of it, so everything is arranged to keep operands coming at that rate:
@@ -232,11 +231,13 @@ struct SimtFwd {
     float *lse;
     int bh, lq, lk, d, causal, blocks;
     float scale;
+    const int *only_if;
 };
 
 template <typename T, bool FAST, int DPAD, int R>
 __global__ void __launch_bounds__(NT) simt_fwd_kernel(const SimtFwd p)
 {
+    if (p.only_if && *p.only_if == 0) return;  // the tensor-core kernel before this one did the work
     constexpr int BM = 8 * R, NP = Cols<DPAD>::NP;
     extern __shared__ __align__(1024) char smem[];
     char *Qs = smem, *Ks = Qs + BM * DPAD * 4, *Vs = Ks + TN * DPAD * 4, *Ps = Vs + TN * DPAD * 4;
@@ -336,6 +337,7 @@ struct SimtBwd {
     int bh, lq, lk, d, causal;
     int kblocks, qblocks;  // blocks of 8*R keys (dK, dV) and of 8*R queries (dQ) per unit
     float scale;
+    const int *only_if;
 };
 
 // One launch, two kinds of blocks: the first bh * kblocks own 8*R keys each and form dK and dV over all
@@ -345,6 +347,7 @@ struct SimtBwd {
 template <typename T, bool FAST, int DPAD, int R>
 __global__ void __launch_bounds__(NT) simt_bwd_kernel(const SimtBwd p)
 {
+    if (p.only_if && *p.only_if == 0) return;  // the tensor-core kernel before this one did the work
     constexpr int BM = 8 * R, NP = Cols<DPAD>::NP;
     extern __shared__ __align__(1024) char smem[];
     // A0, A1: this block's rows (K and V, or Q and dO); B0, B1: the streamed 64-row tiles (Q and dO, or K and V)
@@ -479,7 +482,7 @@ int launch_fwd(const AttnArgs &a, cudaStream_t s)
     auto kern = simt_fwd_kernel<T, FAST, DPAD, R>;
     static SmemOptIn opt_in;
     EMBER_CUDA_TRY(opt_in(kern, smem));
-    SimtFwd p = {a.q, a.k, a.v, a.out, a.lse, a.bh, a.lq, a.lk, a.d, a.causal, (a.lq + BM - 1) / BM, a.scale};
+    SimtFwd p = {a.q, a.k, a.v, a.out, a.lse, a.bh, a.lq, a.lk, a.d, a.causal, (a.lq + BM - 1) / BM, a.scale, a.only_if};
     const long long grid = (long long)p.bh * p.blocks;
     if (grid > 0x7fffffffLL) return too_many_blocks();
     kern<<<(unsigned)grid, NT, smem, s>>>(p);
@@ -496,7 +499,7 @@ int launch_bwd(const AttnArgs &a, const float *delta, cudaStream_t s)
     static SmemOptIn opt_in;
     EMBER_CUDA_TRY(opt_in(kern, smem));
     SimtBwd p = {a.q, a.k, a.v, a.dout, a.lse, delta, a.dq, a.dk, a.dv, a.bh, a.lq, a.lk, a.d, a.causal,
-                 (a.lk + BM - 1) / BM, (a.lq + BM - 1) / BM, a.scale};
+                 (a.lk + BM - 1) / BM, (a.lq + BM - 1) / BM, a.scale, a.only_if};
     const long long grid = (long long)p.bh * ((long long)p.kblocks + p.qblocks);
     if (grid > 0x7fffffffLL) return too_many_blocks();
     kern<<<(unsigned)grid, NT, smem, s>>>(p);
@@ -567,13 +570,13 @@ int simt_attention_fwd(const AttnArgs &a, DeviceState *st, cudaStream_t s)
     return a.d <= 64 ? dispatch_fwd<64>(a, sms, s) : dispatch_fwd<128>(a, sms, s);
 }
 
-int simt_attention_bwd(const AttnArgs &a, float *delta, DeviceState *st, cudaStream_t s)
+int simt_attention_bwd(const AttnArgs &a, float *delta, bool delta_made, DeviceState *st, cudaStream_t s)
 {
     if (a.d > 128) {
         set_error("head dimension %d > 128 is not supported", a.d);
         return EMBER_ERR_UNSUPPORTED;
     }
-    const int rc = launch_delta(a, delta, s);
+    const int rc = delta_made ? EMBER_OK : launch_delta(a, delta, s);
     if (rc != EMBER_OK) return rc;
     const int sms = st->sm_count > 0 ? st->sm_count : 148;
     if (a.d <= 32) return dispatch_bwd<32>(a, sms, delta, s);

@@ -77,11 +77,19 @@ struct AttnArgs {
     float scale = 1.f;
     int causal = 0;
     int dtype = EMBER_F32;
+    const int *only_if = nullptr;  // CUDA-core kernels: return at once when this word of device memory is 0
 };
 
 // CUDA-core kernels (attn_simt.cu): float32 math, f32 or bf16 storage, d <= 128.
 int simt_attention_fwd(const AttnArgs &a, DeviceState *st, cudaStream_t s);
-int simt_attention_bwd(const AttnArgs &a, float *delta, DeviceState *st, cudaStream_t s);
+// delta_made: delta holds the rows' sums already
+int simt_attention_bwd(const AttnArgs &a, float *delta, bool delta_made, DeviceState *st, cudaStream_t s);
+// Float32 storage on the tensor cores, each operand as three bf16 parts (attn_f32_sm100.cu). The scratch they allocate may be
+// missing: EMBER_ERR_NOMEM, nothing launched.
+bool sm100_f32_fwd_preferred(const AttnArgs &a, int sms);
+int sm100_f32_attention_fwd(const AttnArgs &a, DeviceState *st, cudaStream_t s);
+bool sm100_f32_bwd_preferred(const AttnArgs &a, int sms);
+int sm100_f32_attention_bwd(const AttnArgs &a, float *delta, DeviceState *st, cudaStream_t s);
 int launch_delta(const AttnArgs &a, float *delta, cudaStream_t s);
 
 // tcgen05 kernels (attn_fwd_sm100.cu / attn_bwd_sm100.cu): bf16 storage, d in {64, 128}.

@@ -1,0 +1,106 @@
+// Float32 operands for the tensor cores. A float32 value is the exact sum of three bf16 values (24 significand
+// bits = 3 x 8): high, middle and low part, each the rounding of what the ones before left over. Of the nine products of
+// two such sums the six largest are formed, all in float32; what is left out is below 2^-26 of the product.
+// The tensor core adds with truncation (a sum keeps 24 bits and loses the rest towards zero; within one MMA, terms are cut
+// at 2^-25 of the largest), so an accumulator that collects a whole contraction drifts: relative error of random sums of 64 /
+// 512 / 2048 terms 6.6e-8 / 4.7e-7 / 2.1e-6. The kernels therefore let it collect 64 terms at most, the
+// small products first, and add it into float32 registers with rounding.
+// Values that the parts cannot hold (infinities, NaN, 2^50 and above, whose sums of products may meet infinities of
+// either sign, and tensors that are tiny throughout, whose parts run into bf16's smallest exponents) are found while the parts are
+// made: the tensor-core kernel then leaves the work to the CUDA-core kernel that is launched behind it and otherwise
+// returns at once.
+#pragma once
+
+#include "common.cuh"
+#include "kernels.cuh"
+#include "ptx.cuh"
+
+namespace ember {
+
+constexpr int kSplitMaxJobs = 4;
+constexpr int kSplitMaxBlocks = 592;               // 4 blocks of 256 threads per SM
+constexpr uint32_t kSplitHuge = 0x58800000u;       // 2^50
+constexpr uint32_t kSplitTiny = 0x0D800000u;       // 2^-100
+
+// What a split launch leaves for the kernels behind it: the largest magnitude (as bits; a NaN is larger than all) that each of
+// its blocks saw, by tensor, and the word through which the tensor-core kernel tells the CUDA-core kernel to run.
+struct SplitGuard {
+    const uint32_t *slots = nullptr;
+    int first[kSplitMaxJobs + 1] = {};  // blocks [first[i], first[i + 1]) saw tensor i
+    int count = 0;
+    int *fallback = nullptr;
+};
+
+#ifdef __CUDACC__
+// Whether any tensor holds values that the parts cannot represent. All threads of the block call it; `word` is shared memory.
+__device__ __forceinline__ bool split_out_of_range(const SplitGuard &g, uint32_t *word)
+{
+    if (threadIdx.x == 0) *word = 0;
+    __syncthreads();
+    uint32_t bits = 0;
+    for (int i = 0; i < g.count; i++)
+        for (int b = g.first[i] + (int)threadIdx.x; b < g.first[i + 1]; b += blockDim.x) {
+            const uint32_t m = g.slots[b];
+            if (m >= kSplitHuge) bits |= 1u;
+            if (m != 0) bits |= 2u << (2 * i);
+            if (m >= kSplitTiny) bits |= 4u << (2 * i);
+        }
+    if (bits) atomicOr(word, bits);
+    __syncthreads();
+    bits = *word;
+    bool out = (bits & 1u) != 0;
+    for (int i = 0; i < g.count; i++) out = out || ((bits >> (1 + 2 * i)) & 3u) == 1u;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *g.fallback = out ? 1 : 0;
+    return out;
+}
+
+// Two neighbouring columns -> one 32-bit word of each part.
+__device__ __forceinline__ void split_pair(float a, float b, uint32_t &hi, uint32_t &mid, uint32_t &lo)
+{
+    hi = ptx::pack_bf16(a, b);
+    a -= __uint_as_float(hi << 16);
+    b -= __uint_as_float(hi & 0xffff0000u);
+    mid = ptx::pack_bf16(a, b);
+    a -= __uint_as_float(mid << 16);
+    b -= __uint_as_float(mid & 0xffff0000u);
+    lo = ptx::pack_bf16(a, b);
+}
+__device__ __forceinline__ void split_pair(ptx::f32x2 v, uint32_t &hi, uint32_t &mid, uint32_t &lo)
+{
+    float a, b;
+    ptx::unpack2(v, a, b);
+    hi = ptx::pack_bf16(a, b);
+    v = ptx::sub2(v, ptx::pack2(__uint_as_float(hi << 16), __uint_as_float(hi & 0xffff0000u)));
+    ptx::unpack2(v, a, b);
+    mid = ptx::pack_bf16(a, b);
+    v = ptx::sub2(v, ptx::pack2(__uint_as_float(mid << 16), __uint_as_float(mid & 0xffff0000u)));
+    ptx::unpack2(v, a, b);
+    lo = ptx::pack_bf16(a, b);
+}
+#endif
+
+// One tensor to split: rows x cols float32, row-major -> three bf16 planes of rows x cols rounded up to 8 (zeros there), one
+// after the other. dst null: only looked through for values out of range.
+struct SplitJob {
+    const float *src = nullptr;
+    void *dst = nullptr;
+    long long rows = 0;
+    int cols = 0;
+};
+// delta[row] = sum of out * dout over the row, made by further blocks of the same launch (the backward needs both before it starts)
+struct SplitDelta {
+    const float *out = nullptr, *dout = nullptr;
+    float *delta = nullptr;
+    long long rows = 0;
+    int cols = 0;
+};
+
+inline size_t split_plane_elems(long long rows, int cols) { return (size_t)rows * ((cols + 7) / 8 * 8); }
+inline size_t split_bytes(long long rows, int cols) { return align_up(3 * split_plane_elems(rows, cols) * 2, 256); }
+// scratch for the guard's words
+constexpr size_t kSplitGuardBytes = (kSplitMaxBlocks + 64) * 4;
+
+// Splits up to four tensors in one launch. guard_mem: kSplitGuardBytes. Any alignment of src; dst 16-byte aligned.
+int split_f32(const SplitJob *jobs, int count, const SplitDelta *delta, void *guard_mem, SplitGuard *guard, cudaStream_t s);
+
+}  // namespace ember

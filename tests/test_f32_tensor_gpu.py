@@ -1,0 +1,138 @@
+"""Float32 attention on the tensor cores (operands as three bf16 parts): edges of its 128-row blocks and 64-row tiles,
+head dimensions that fill the parts' columns partly, rows at any alignment, and the calls that it has to leave to the
+CUDA-core kernels (values that the parts cannot hold, no memory for them), against float64.
+
+Tolerance: products of parts leave out less than 2^-25 of a product and the tensor core's additions lose up to 2^-23 each of
+a partial sum of 64 terms or fewer (at most 4 additions of full size), partial sums are then added in float32: of a sum of n
+terms of order one that is about (4 + sqrt(n / 64)) * 2^-23 of its terms' root sum of squares. 64 * 2^-24 of the largest result
+covers n up to 5000 with the exponentials' 2^-22 and a few units for the log-sum-exp."""
+import numpy as np
+import pytest
+
+import ember_b200 as em
+from conftest import seeded
+from ember_b200 import _lib
+
+pytestmark = pytest.mark.gpu
+REL = 64 * 2.0 ** -24
+
+
+def reference(q, k, v, g, scale, causal):
+    q, k, v, g = (x.astype(np.float64) for x in (q, k, v, g))
+    s = np.einsum("uid,ujd->uij", q, k) * scale
+    if causal:
+        s[:, np.triu(np.ones(s.shape[1:], bool), 1 + s.shape[2] - s.shape[1])] = -np.inf
+    m = s.max(-1, keepdims=True)
+    p = np.exp(s - m)
+    lse = (m + np.log(p.sum(-1, keepdims=True)))
+    p = np.exp(s - lse)
+    o = np.einsum("uij,ujd->uid", p, v)
+    ds = p * (np.einsum("uid,ujd->uij", g, v) - (g * o).sum(-1, keepdims=True)) * scale
+    return o, lse[..., 0], np.einsum("uij,ujd->uid", ds, k), np.einsum("uij,uid->ujd", ds, q), np.einsum("uij,uid->ujd", p, g)
+
+
+def run(q, k, v, g, scale, causal):
+    tq, tk, tv, tg = (em.Tensor(x[None]) if not isinstance(x, em.Tensor) else x for x in (q, k, v, g))
+    o, lse = em.attention_forward(tq, tk, tv, scale, causal)
+    grads = em.attention_backward(tq, tk, tv, o, lse, tg, scale, causal)
+    return [t.to_np()[0] for t in (o, lse, *grads)]
+
+
+def inputs(units, lq, lk, d, seed=1, std=0.5):
+    return [seeded((units, n, d), seed + i, std) for i, n in enumerate((lq, lk, lk, lq))]
+
+
+def close(got, want, rel=REL):
+    for name, a, b in zip(("o", "lse", "dq", "dk", "dv"), got, want):
+        assert np.abs(a - b).max() <= rel * max(1e-30, np.abs(b).max()), name
+
+
+@pytest.mark.parametrize("units,lq,lk,d,causal", [
+    (2, 640, 640, 64, True), (1, 1, 4097, 64, True), (2, 129, 577, 64, False), (1, 511, 513, 64, True), (3, 385, 1025, 64, True),
+    (1, 1300, 1290 + 10, 40, False), (2, 200, 1152, 33, True), (1, 600, 1217, 61, False), (1, 1100, 1100, 8, True), (1, 1090, 1090, 3, False),
+    (1, 512, 512, 128, True), (2, 127, 641, 128, False), (1, 65, 1023, 80, True), (2, 300, 700, 96, True), (1, 577, 577, 101, False), (1, 640, 576, 72, False),
+    (160, 256, 256, 64, True), (40, 256, 256, 128, False),
+])
+def test_edges_of_blocks_and_tiles(units, lq, lk, d, causal):
+    x = inputs(units, lq, lk, d)
+    close(run(*x, d ** -0.5, causal), reference(*x, d ** -0.5, causal))
+
+
+@pytest.mark.parametrize("d", [64, 96, 40])
+@pytest.mark.parametrize("scale", [-0.3, 0.0, 2.0])
+def test_any_scale(d, scale):
+    x = inputs(2, 600, 700, d)
+    close(run(*x, scale, True), reference(*x, scale, True))
+
+
+@pytest.mark.parametrize("d", [64, 128, 40])
+def test_rows_off_the_16_byte_grid(d):
+    """Views one element into a buffer: every operand's rows start at odd multiples of 4 bytes."""
+    x = inputs(2, 520, 530, d)
+    off = []
+    for a in x:
+        flat = np.concatenate([np.zeros(1, np.float32), a.ravel()])
+        off.append(em.Tensor(flat).view(1, (1, *a.shape)))
+    close(run(*off, d ** -0.5, True), reference(*x, d ** -0.5, True))
+
+
+@pytest.mark.parametrize("d", [64, 128])
+def test_lengths_of_one_visible_key(d):
+    """Row 0 of a square causal call sees one key: its output is that key's value, bit for bit (three parts hold a float32 exactly)."""
+    q, k, v, g = inputs(1, 640, 640, d)
+    o = run(q, k, v, g, d ** -0.5, True)[0]
+    assert np.array_equal(o[0, 0], v[0, 0])
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("which", [0, 1, 2, 3])
+@pytest.mark.parametrize("value", [np.inf, np.nan, 3e38])
+def test_values_that_the_parts_cannot_hold(d, which, value):
+    """One such element anywhere: infinities and NaN where a call without memory for the parts (the CUDA-core kernels alone) has
+    them, and the same numbers elsewhere."""
+    x = inputs(2, 520, 600, d)
+    x[which][1, 300, 5] = value
+    L = _lib.lib()
+    got = run(*x, d ** -0.5, False)
+    L.ember_selftest_fail_scratch(2)
+    want = run(*x, d ** -0.5, False)
+    assert L.ember_selftest_fail_scratch(0) == 0  # both calls asked for that memory
+    if value == 3e38:  # times score gradients that are nothing but the rounding of what cancels there: not dq and dk
+        got, want = ([t[0], t[1], t[4]] for t in (got, want))
+    for a, b in zip(got, want):
+        fine = np.isfinite(b)
+        assert np.array_equal(fine, np.isfinite(a)) and np.array_equal(a[~fine], b[~fine], equal_nan=True)
+        for u in range(2):  # the element's own unit by its own largest value
+            f = fine[u]
+            assert not f.any() or np.abs(a[u][f].astype(np.float64) - b[u][f]).max() <= REL * np.abs(b[u][f].astype(np.float64)).max()
+
+
+@pytest.mark.parametrize("d", [64, 128])
+def test_tensors_of_tiny_values_keep_their_precision(d):
+    """Upstream gradients of 1e-33: their low parts would fall under bf16's smallest values."""
+    q, k, v, g = inputs(2, 520, 600, d)
+    g *= np.float32(2e-33)
+    close(run(q, k, v, g, d ** -0.5, False), reference(q, k, v, g, d ** -0.5, False))
+
+
+def test_zeros_stay_on_the_tensor_cores_and_give_means():
+    q, k, v, g = inputs(2, 520, 600, 64)
+    q[:] = 0
+    close(run(q, k, v, g, 0.125, False), reference(q, k, v, g, 0.125, False))
+
+
+def test_without_memory_for_the_parts():
+    x = inputs(2, 600, 600, 64)
+    L = _lib.lib()
+    L.ember_selftest_fail_scratch(2)
+    got = run(*x, 0.125, True)
+    L.ember_selftest_fail_scratch(0)
+    close(got, reference(*x, 0.125, True))
+
+
+@pytest.mark.parametrize("d", [64, 128])
+def test_results_repeat_bit_for_bit(d):
+    x = inputs(3, 700, 900, d)
+    first = run(*x, d ** -0.5, True)
+    for _ in range(3):
+        assert all(np.array_equal(a, b) for a, b in zip(first, run(*x, d ** -0.5, True)))
