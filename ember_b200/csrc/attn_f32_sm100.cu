@@ -49,13 +49,6 @@ __device__ __forceinline__ f32x2 exp_pair(f32x2 x)
     return fma2(v, mul2(r, pack2(0.69314718f, 0.69314718f)), v);
 }
 
-// The six products of parts, small ones first: (part of A, part of B) = (2, 0) (1, 1) (0, 2) (1, 0) (0, 1) (0, 0), 0 = high. A
-// loop and not straight code: with the four products of a backward step unrolled, issuing and computing warps together outgrew
-// the instruction cache.
-constexpr int PRODUCTS = 6;
-__device__ __forceinline__ uint32_t part_a(int i) { return (0x046u >> (2 * i)) & 3u; }
-__device__ __forceinline__ uint32_t part_b(int i) { return (0x124u >> (2 * i)) & 3u; }
-
 // Row `src` (d columns in memory; null: zeros), columns [col0, col0 + 32 * n32) -> the three parts in tensor memory, part q at
 // column taddr + q * plane.
 __device__ __forceinline__ void row_to_tmem(const float *src, int d, bool vec, int col0, int n32, uint32_t taddr, int plane)
@@ -155,10 +148,10 @@ __device__ __forceinline__ void mma_scores(uint32_t d, uint32_t a, uint32_t b_sm
     constexpr int PLANE = HD / 64 * SUB;
     const uint32_t b_lo = desc_lo(b_smem, 16), a_lo = SS ? desc_lo(a, 16) : a;
 #pragma unroll 1
-    for (int i = 0; i < PRODUCTS; i++) {
+    for (int i = 0; i < kSplitProducts; i++) {
 #pragma unroll
         for (int sub = 0; sub < HD / 64; sub++) {
-            const uint32_t acc = i > 0 || sub > 0, pa = part_a(i), b = b_lo + part_b(i) * (PLANE >> 4) + ((sub * SUB) >> 4);
+            const uint32_t acc = i > 0 || sub > 0, pa = split_part_a(i), b = b_lo + split_part_b(i) * (PLANE >> 4) + ((sub * SUB) >> 4);
             const bool four = ksteps - sub * 4 > 2;
             if (SS) chain_ss<2, 4, 6, 2, 4, 6>(d, a_lo + pa * ((2 * PLANE) >> 4) + ((sub * 2 * SUB) >> 4), b, IDESC, elected, acc, four);
             else chain_ts<8, 16, 24, 2, 4, 6>(d, a_lo + pa * (HD / 2) + sub * 32, b, IDESC, elected, acc, four);
@@ -172,8 +165,8 @@ __device__ __forceinline__ void mma_results(uint32_t d, uint32_t region, uint32_
     constexpr int PLANE = HD / 64 * SUB;
     const uint32_t b_lo = desc_lo(b_smem, SUB);
 #pragma unroll 1
-    for (int i = 0; i < PRODUCTS; i++)
-        chain_ts<part_col(0, 1), part_col(0, 2), part_col(0, 3), 128, 256, 384>(d, region + part_a(i) * part_col(1, 0), b_lo + part_b(i) * (PLANE >> 4), idesc, elected,
+    for (int i = 0; i < kSplitProducts; i++)
+        chain_ts<part_col(0, 1), part_col(0, 2), part_col(0, 3), 128, 256, 384>(d, region + split_part_a(i) * part_col(1, 0), b_lo + split_part_b(i) * (PLANE >> 4), idesc, elected,
                                                                                 i > 0, true);
 }
 

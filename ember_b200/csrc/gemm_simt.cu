@@ -1,7 +1,6 @@
 // CUDA-core matrix products for the Linear layers: float32 arithmetic, f32 or bf16 storage, any
-// shape and any view (row-major or head-major operands). This is the float32 mode of the layers
-// (bf16 tensor-core products would use up its 1e-3 tolerance) and the path for shapes the tcgen05
-// kernel does not take.
+// shape and any view (row-major or head-major operands): small float32 products, float32 values that the tensor-core
+// kernel's planes (gemm_f32_sm100.cu) cannot hold, and shapes that the tcgen05 kernels do not take.
 #include "common.cuh"
 #include "kernels.cuh"
 #include "ptx.cuh"
@@ -95,23 +94,17 @@ __device__ __forceinline__ void st4(__nv_bfloat16 *p, const float (&v)[4])
     *reinterpret_cast<uint2 *>(p) = make_uint2(ptx::pack_bf16(v[0], v[1]), ptx::pack_bf16(v[2], v[3]));
 }
 
-__device__ __forceinline__ float4 ld_cluster4(uint32_t addr)
-{
-    float4 v;
-    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
-    return v;
-}
-
 // CV: results are stored four columns at a time, else neighbouring columns by neighbouring threads.
 template <typename T, int MODE, bool FA, bool FB, bool CV, typename C>
 __global__ void __launch_bounds__(C::NT, 512 / C::NT) simt_gemm_kernel(const MatView a, const MatView b, const MatView c, const T *bias,
                                                         const long long m, const int n, const int k, const int tiles_n,
-                                                        const int splits)
+                                                        const int splits, const int *only_if)
 {
     using OA = Operand<T, MODE != GEMM_TN, FA, C::TM>;
     using OB = Operand<T, MODE == GEMM_NT, FB, C::TN>;
     ptx::pdl_launch_dependents();
     ptx::pdl_wait();
+    if (only_if && *only_if == 0) return;  // the tensor-core kernel before this one did the work
     extern __shared__ __align__(16) float sm[];
     float *as = sm, *bs = sm + C::SLAB * C::PA;
     const int rank = splits > 1 ? (int)ptx::cluster_ctarank() : 0;
@@ -263,8 +256,8 @@ __global__ void __launch_bounds__(C::NT, 512 / C::NT) simt_gemm_kernel(const Mat
             ptx::cluster_sync_all();
             for (int e = rank * 256 + threadIdx.x; e < C::TM * C::TN / 4; e += splits * 256) {
                 const uint32_t at = ptx::smem_u32(sm + e / (C::TN / 4) * C::PITCH + e % (C::TN / 4) * 4);
-                float4 s = ld_cluster4(ptx::map_to_cta(at, 0));
-                for (int r = 1; r < splits; r++) add4(s, ld_cluster4(ptx::map_to_cta(at, (uint32_t)r)));
+                float4 s = ptx::ld_cluster4(ptx::map_to_cta(at, 0));
+                for (int r = 1; r < splits; r++) add4(s, ptx::ld_cluster4(ptx::map_to_cta(at, (uint32_t)r)));
                 store(e, s);
             }
             ptx::cluster_sync_all();  // nobody reads this block's shared memory any more
@@ -297,7 +290,7 @@ int launch_store(const GemmArgs &g, int splits, cudaStream_t s)
     attrs.cluster((unsigned)splits);
     if (cfg.gridDim.x <= (unsigned)kPdlMaxGrid) attrs.pdl();
     attrs.set(cfg);
-    EMBER_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, g.a, g.b, g.c, (const T *)g.bias, g.m, g.n, g.k, (int)tiles_n, splits));
+    EMBER_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, g.a, g.b, g.c, (const T *)g.bias, g.m, g.n, g.k, (int)tiles_n, splits, g.only_if));
     return EMBER_OK;
 }
 

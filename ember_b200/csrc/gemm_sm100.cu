@@ -25,6 +25,7 @@
 // one whose contraction index runs across rows (MN-major: A of TN, B of NN/TN) is stored as
 // sub-tiles of 64 k-rows x 64 columns, 8 KB apart.
 #include "common.cuh"
+#include "gemm_tiles.cuh"
 #include "kernels.cuh"
 #include "ptx.cuh"
 
@@ -34,11 +35,10 @@ namespace {
 
 using namespace ptx;
 
-constexpr int BM = 128, BK = 64, STAGES = 6;  // BM: rows per CTA; a pair covers 2 * BM
+constexpr int STAGES = 6;
 constexpr int A_BYTES = BM * BK * 2;
 constexpr int SUB_BYTES = 64 * 128;           // 64 rows x 128 bytes
 constexpr int GEMM_THREADS = 192;
-constexpr int GROUP_M = 16;                   // tiles that share B columns run together
 
 // BN: columns of a pair's tile, 256, or 128 for results of few tiles: see launch.
 template <int BN>
@@ -55,11 +55,6 @@ struct GemmCfg {
 enum { B_FULL = 0, B_EMPTY = B_FULL + STAGES, B_ACCFULL = B_EMPTY + STAGES, B_ACCEMPTY = B_ACCFULL + 2, NUM_BARS = B_ACCEMPTY + 2 };
 enum { WG_EMPTY = 201, WG_FULL, WG_ACCEMPTY, WG_ACCFULL, WG_SMEM };
 
-// seq: rows from one batch entry to the next in the TILE's row space, see GemmParams::seq_pad
-struct ViewGeom {
-    int heads, seq, dim;
-};
-
 struct GemmParams {
     int n, kblocks;
     int tiles_m, tiles_n;
@@ -73,57 +68,6 @@ struct GemmParams {
     const __nv_bfloat16 *bias;
     DeviceStatus *status;
 };
-
-// TMA coordinates of a 64-column box of a view, walked along the contraction index. The producer
-// computes coordinates on the critical path of every stage, so the divisions that split a row into
-// (batch, position) and a column into (part, head, element) are done once per tile and the walk
-// itself only adds and carries (all steps are 64; the padded seq is a multiple of 64, dim too unless
-// there is a single head: a row-major matrix walked by batch entries).
-struct BoxWalker {
-    int c0, c1, c2, c3, c4;  // column | element, row | position, head, batch, part
-    int heads, seq, dim;
-
-    __device__ __forceinline__ void init(const ViewGeom &g, int row0, int col0)
-    {
-        heads = g.heads;
-        seq = g.seq;
-        dim = g.dim;
-        if (heads == 0) {
-            c0 = col0; c1 = row0; c2 = c3 = c4 = 0;
-        } else {
-            c3 = row0 / seq; c1 = row0 - c3 * seq;
-            const int ph = col0 / dim;
-            c0 = col0 - ph * dim;
-            c4 = ph / heads; c2 = ph - c4 * heads;
-        }
-    }
-    __device__ __forceinline__ void step_rows()  // 64 rows further
-    {
-        c1 += 64;
-        if (heads != 0 && c1 >= seq) { c1 -= seq; c3++; }
-    }
-    __device__ __forceinline__ void step_cols()  // 64 columns further
-    {
-        c0 += 64;
-        if (heads != 0 && c0 >= dim) {
-            c0 = 0;
-            if (++c2 >= heads) { c2 = 0; c4++; }
-        }
-    }
-    __device__ __forceinline__ void load(uint32_t dst, const CUtensorMap *map, uint32_t bar) const
-    {
-        tma_load_5d_pair(dst, map, bar, c0, c1, c2, c3, c4);
-    }
-};
-
-__device__ __forceinline__ void tile_coords(const GemmParams &p, int tile, int &tm, int &tn)
-{
-    const int per_group = GROUP_M * p.tiles_n;
-    const int g = tile / per_group, rem = tile - g * per_group;
-    const int rows_here = min(GROUP_M, p.tiles_m - g * GROUP_M);
-    tn = rem / rows_here;
-    tm = g * GROUP_M + (rem - tn * rows_here);
-}
 
 template <int MODE, int BN>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
@@ -195,7 +139,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
             bool ok = true;
             for (int tile = pair; tile < num_tiles && ok; tile += npairs) {
                 int tm, tn;
-                tile_coords(p, tile, tm, tn);
+                tile_coords(p.tiles_m, p.tiles_n, tile, tm, tn);
                 const int m0 = tm * 2 * BM + (int)rank * BM, n0 = tn * BN + (int)rank * BNH;  // this CTA's A rows and B columns
                 constexpr int NA = MODE == GEMM_TN ? BM / 64 : 1, NB = MODE == GEMM_NT ? 1 : BNH / 64;
                 BoxWalker wa[NA], wb[NB];
@@ -268,7 +212,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
         bool ok = true;
         for (int tile = pair; tile < num_tiles; tile += npairs, tcount++) {
             int tm, tn;
-            tile_coords(p, tile, tm, tn);
+            tile_coords(p.tiles_m, p.tiles_n, tile, tm, tn);
             const int buf = tcount & 1;
             const int m0 = (tm * 2 + (int)rank) * BM, entry = m0 / p.seq_pad, l0 = m0 - entry * p.seq_pad;
             const int rows_valid = entry < p.batch ? min(BM, p.seq - l0) : 0;  // may be <= 0: padding alone
@@ -352,36 +296,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     if (warp == 4) tmem_dealloc_pair(tmem, 512);
 }
 
-// The batch entries the rows of a product are walked by. A head-major view whose seq is a multiple of the
-// boxes' rows can be tiled as if its rows were consecutive; otherwise tiles (NN, NT: rows of A and C) or
-// contraction steps (TN: rows of A and B) stop at the end of each entry, the copy engine fills the rest
-// of the box with zeros, and what is computed for them is not stored. A row-major view on the same row
-// axis is then described as one head of `cols` columns, so that its boxes end there too (with rows of the
-// next entry in their place, an infinity among those would meet the other operand's zeros).
-struct RowPlan {
-    bool by_entry;
-    int batch, seq, seq_pad;
-};
-
-RowPlan row_plan(const GemmArgs &g)
-{
-    const MatView *axis[2] = {&g.a, g.mode == GEMM_TN ? &g.b : &g.c};
-    const long long rows = g.mode == GEMM_TN ? g.k : g.m;
-    const int box = g.mode == GEMM_TN ? BK : BM;
-    for (const MatView *v : axis)
-        if (v->heads > 0 && v->seq % box != 0) return {true, (int)(rows / v->seq), v->seq, (v->seq + box - 1) / box * box};
-    return {false, 1, (int)rows, (int)((rows + 2 * BM - 1) / (2 * BM) * (2 * BM))};
-}
-
 bool c_rows_aligned(const GemmArgs &g) { return g.n % 8 == 0 && ((uintptr_t)g.c.ptr & 15) == 0; }
-
-bool view_ok(const MatView &v)
-{
-    if (((uintptr_t)v.ptr & 15) != 0) return false;
-    if (v.heads == 0) return v.cols % 8 == 0;
-    // head-major: a box of 64 columns must stay inside one head
-    return v.dim % 64 == 0 && v.rows % v.seq == 0 && v.cols % (v.heads * v.dim) == 0;
-}
 
 template <int MODE, int BN>
 int launch_tile(const GemmArgs &g, DeviceState *st, cudaStream_t s)

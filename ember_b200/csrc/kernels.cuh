@@ -165,6 +165,7 @@ struct GemmArgs {
     long long m = 0;
     int n = 0, k = 0;
     int dtype = EMBER_F32;
+    const int *only_if = nullptr;  // CUDA-core kernel: return at once when this word of device memory is 0
 };
 
 // CUDA-core kernels (gemm_simt.cu): float32 math, any shape and view.
@@ -180,6 +181,13 @@ int pack_rows(const MatView &v, void *dst, cudaStream_t s);
 bool sm100_skinny_gemm_supported(const GemmArgs &g);
 bool sm100_skinny_gemm_preferred(const GemmArgs &g);  // quicker than sm100_gemm, where that takes the product too
 int sm100_skinny_gemm(const GemmArgs &g, DeviceState *st, cudaStream_t s);
-int make_tensor_map_bf16_view(CUtensorMap *map, const MatView &v, uint32_t box_cols, uint32_t box_rows);
+// planes: so many copies of the view one after the other, counted along the parts
+int make_tensor_map_bf16_view(CUtensorMap *map, const MatView &v, uint32_t box_cols, uint32_t box_rows, int planes = 1);
+// Float32 storage on the tensor cores, operands as three bf16 planes each (gemm_f32_sm100.cu, split_f32.cuh): a row-major view's rows
+// padded to 8 columns. _us: an estimate of the time, without the splitting.
+struct SplitGuard;
+bool sm100_f32_gemm_supported(const GemmArgs &g);
+double sm100_f32_gemm_us(const GemmArgs &g, int sms);
+int sm100_f32_gemm(const GemmArgs &g, const void *a_planes, const void *b_planes, const SplitGuard &guard, DeviceState *st, cudaStream_t s);
 
 }  // namespace ember

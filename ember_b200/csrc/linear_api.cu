@@ -3,6 +3,7 @@
 // kernel (float32 mode and everything else).
 #include "common.cuh"
 #include "kernels.cuh"
+#include "split_f32.cuh"
 
 using namespace ember;
 
@@ -118,6 +119,86 @@ bool worth_packing(const GemmArgs &g)
     return sm100_skinny_gemm_supported(t) || sm100_gemm_supported(t);
 }
 
+// Float32 products on the tensor cores (gemm_f32_sm100.cu): the operands' planes are made in one launch for all products of an
+// entry point, and the CUDA-core kernels behind them return at once unless an operand holds values that planes cannot.
+//
+// Which side takes a call: both times are estimated, in us. The tensor-core side starts at 17.5 for one product (split, product, the launch
+// that returns) and 33 for two, splitting costs a pass (10 bytes an element at 5 TB/s), its tiles are 256 rows; the CUDA cores
+// run at 40 TFLOP/s where tiles of 128 x 128 fill the SMs, at 17 to 34 below. Measured, CUDA cores / tensor cores, forward and both gradients
+// (rows x contraction x columns):
+//   300^3 10 / 18, 21 / 35      512^3 17 / 17, 35 / 33          1024^3 66 / 24, 153 / 46       2048^3 415 / 85, 831 / 168
+//   256 x 1024 x 1000 30 / 18, 50 / 36      8192 x 64 x 1000 30 / 22, 128 / 80     4000 x 512 x 200 35 / 20, 87 / 50    2000 x 1024 x 3001 354 / 84, 1003 / 161
+//   8192 x 512 x 64 34 / 22, 47 / 66        64 x 2048 x 8192 125 / 84, 183 / 155   32 x 1024 x 16384 61 / 75, 103 / 155
+constexpr double kSplitUsPerByte = 1.0 / 5e6;
+
+double simt_f32_us(const GemmArgs &g, int sms)
+{
+    const bool full = (double)((g.m + 127) / 128) * ((g.n + 127) / 128) >= sms;
+    return 6.0 + 2.0 * (double)g.m * g.n * g.k / (full ? 4e7 : 2.4e7);
+}
+
+struct F32Products {
+    GemmArgs g[2];
+    int count = 0;
+    MatView ops[3];
+    int nops = 0;
+
+    int operand(const MatView &v)
+    {
+        for (int i = 0; i < nops; i++)
+            if (ops[i].ptr == v.ptr && ops[i].rows == v.rows && ops[i].cols == v.cols && ops[i].heads == v.heads) return i;
+        ops[nops] = v;
+        return nops++;
+    }
+    void add(const GemmArgs &p)
+    {
+        g[count++] = p;
+        operand(p.a);
+        operand(p.b);
+    }
+    bool preferred(int sms)
+    {
+        if (count == 0) return false;
+        double tensor = count > 1 ? 20.0 : 12.0, cores = 0;
+        for (int i = 0; i < count; i++) {
+            if (!sm100_f32_gemm_supported(g[i])) return false;
+            tensor += sm100_f32_gemm_us(g[i], sms);
+            cores += simt_f32_us(g[i], sms);
+        }
+        for (int i = 0; i < nops; i++) tensor += (double)ops[i].rows * ops[i].cols * 10.0 * kSplitUsPerByte;
+        if (tensor < (count > 1 ? 33.0 : 17.5)) tensor = count > 1 ? 33.0 : 17.5;
+        return tensor < cores;
+    }
+    // EMBER_ERR_NOMEM: no memory for the planes, nothing launched
+    int run(DeviceState *st, cudaStream_t s)
+    {
+        size_t at[3], bytes = 0;
+        for (int i = 0; i < nops; i++) {
+            at[i] = bytes;
+            bytes += split_bytes(ops[i].rows, ops[i].cols);
+        }
+        char *mem = nullptr;
+        if (!scratch_alloc((void **)&mem, bytes + kSplitGuardBytes, s)) return EMBER_ERR_NOMEM;
+        SplitJob jobs[3];
+        for (int i = 0; i < nops; i++) {
+            jobs[i].src = (const float *)ops[i].ptr;
+            jobs[i].dst = mem + at[i];
+            jobs[i].rows = ops[i].rows;  // a head-major tensor is as many elements in a row, of which planes keep the order
+            jobs[i].cols = ops[i].cols;
+        }
+        SplitGuard guard;
+        int rc = split_f32(jobs, nops, nullptr, mem + bytes, &guard, s);
+        for (int i = 0; i < count && rc == EMBER_OK; i++) rc = sm100_f32_gemm(g[i], mem + at[operand(g[i].a)], mem + at[operand(g[i].b)], guard, st, s);
+        for (int i = 0; i < count && rc == EMBER_OK; i++) {
+            GemmArgs t = g[i];
+            t.only_if = guard.fallback;
+            rc = simt_gemm(t, st, s);
+        }
+        cudaFreeAsync(mem, s);
+        return rc;
+    }
+};
+
 int run(GemmArgs g, DeviceState *st, cudaStream_t s, PackedOperands &packed)
 {
     if (worth_packing(g)) {
@@ -155,6 +236,9 @@ int ember_linear_fwd(const void *x, const void *w, const void *bias, void *y, lo
     g.bias = bias;
     g.m = m; g.n = n; g.k = k; g.dtype = dtype;
     PackedOperands packed(pick_stream(stream, st));
+    F32Products f32;
+    if (dtype == EMBER_F32) f32.add(g);
+    if (f32.preferred(st->sm_count) && (rc = f32.run(st, packed.stream)) != EMBER_ERR_NOMEM) return rc;
     return run(g, st, packed.stream, packed);
 }
 
@@ -172,25 +256,28 @@ int ember_linear_bwd(const void *x, const void *w, const void *dy, void *dx, voi
     cudaStream_t s = pick_stream(stream, st);
     PackedOperands packed(s);
     const MatView vx = view(x, m, k, x_heads, sh), vdy = view(dy, m, n, y_heads, sh);
-    if (dw) {  // grad_w (k x n) = x^T dy
-        GemmArgs g;
-        g.mode = GEMM_TN;
-        g.a = vx;
-        g.b = vdy;
-        g.c = view(dw, k, n, 0, sh);
-        g.m = k; g.n = n; g.k = (int)m; g.dtype = dtype;
-        if ((rc = run(g, st, s, packed)) != EMBER_OK) return rc;
+    GemmArgs gw, gx;
+    gw.mode = GEMM_TN;  // grad_w (k x n) = x^T dy
+    gw.a = vx;
+    gw.b = vdy;
+    gw.c = view(dw, k, n, 0, sh);
+    gw.m = k; gw.n = n; gw.k = (int)m; gw.dtype = dtype;
+    gx.mode = GEMM_NT;  // grad_x (m x k) = dy w^T
+    gx.a = vdy;
+    gx.b = view(w, k, n, 0, sh);
+    gx.c = view(dx, m, k, x_heads, sh);
+    gx.m = m; gx.n = k; gx.k = n; gx.dtype = dtype;
+    F32Products f32;
+    if (dtype == EMBER_F32 && dw) f32.add(gw);
+    if (dtype == EMBER_F32 && dx) f32.add(gx);
+    bool done = false;
+    if (f32.preferred(st->sm_count)) {
+        if ((rc = f32.run(st, s)) != EMBER_OK && rc != EMBER_ERR_NOMEM) return rc;
+        done = rc == EMBER_OK;
     }
+    if (!done && dw && (rc = run(gw, st, s, packed)) != EMBER_OK) return rc;
     if (db && (rc = column_sums(vdy, db, dtype, st, s)) != EMBER_OK) return rc;  // grad_b = sum(dy, axis 0)
-    if (dx) {  // grad_x (m x k) = dy w^T
-        GemmArgs g;
-        g.mode = GEMM_NT;
-        g.a = vdy;
-        g.b = view(w, k, n, 0, sh);
-        g.c = view(dx, m, k, x_heads, sh);
-        g.m = m; g.n = k; g.k = n; g.dtype = dtype;
-        if ((rc = run(g, st, s, packed)) != EMBER_OK) return rc;
-    }
+    if (!done && dx && (rc = run(gx, st, s, packed)) != EMBER_OK) return rc;
     return EMBER_OK;
 }
 

@@ -54,6 +54,13 @@ __device__ __forceinline__ bool split_out_of_range(const SplitGuard &g, uint32_t
     return out;
 }
 
+// The six products of parts, small ones first: (part of A, part of B) = (2, 0) (1, 1) (0, 2) (1, 0) (0, 1) (0, 0), 0 = high. A
+// loop and not straight code: with the four products of a backward step unrolled, issuing and computing warps together outgrew
+// the instruction cache.
+constexpr int kSplitProducts = 6;
+__device__ __forceinline__ uint32_t split_part_a(int i) { return (0x046u >> (2 * i)) & 3u; }
+__device__ __forceinline__ uint32_t split_part_b(int i) { return (0x124u >> (2 * i)) & 3u; }
+
 // Two neighbouring columns -> one 32-bit word of each part.
 __device__ __forceinline__ void split_pair(float a, float b, uint32_t &hi, uint32_t &mid, uint32_t &lo)
 {

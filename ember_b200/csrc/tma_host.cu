@@ -65,7 +65,7 @@ int make_tensor_map_bf16_3d(CUtensorMap *map, const void *base, uint64_t inner, 
 // A matrix view as a 5-D TMA tensor (innermost first): row-major (cols, rows, 1, 1, 1); head-major
 // (dim, seq, heads, batch, parts). Boxes of box_rows x box_cols elements (box_cols * 2 bytes = 128)
 // along the two innermost dimensions, 128-byte swizzle, zero fill outside.
-int make_tensor_map_bf16_view(CUtensorMap *map, const MatView &v, uint32_t box_cols, uint32_t box_rows)
+int make_tensor_map_bf16_view(CUtensorMap *map, const MatView &v, uint32_t box_cols, uint32_t box_rows, int planes)
 {
     EncodeTiledFn fn = encode_fn();
     if (!fn) {
@@ -76,7 +76,8 @@ int make_tensor_map_bf16_view(CUtensorMap *map, const MatView &v, uint32_t box_c
     if (v.heads == 0) {
         dims[0] = (cuuint64_t)v.cols;
         dims[1] = (cuuint64_t)v.rows;
-        dims[2] = dims[3] = dims[4] = 1;
+        dims[2] = dims[3] = 1;
+        dims[4] = (cuuint64_t)planes;
         strides[0] = (cuuint64_t)v.cols * 2;
         strides[1] = strides[2] = strides[3] = (cuuint64_t)v.cols * 2 * (cuuint64_t)v.rows;
     } else {
@@ -85,7 +86,7 @@ int make_tensor_map_bf16_view(CUtensorMap *map, const MatView &v, uint32_t box_c
         dims[1] = (cuuint64_t)v.seq;
         dims[2] = (cuuint64_t)v.heads;
         dims[3] = batch;
-        dims[4] = parts;
+        dims[4] = parts * planes;
         strides[0] = (cuuint64_t)v.dim * 2;
         strides[1] = strides[0] * (cuuint64_t)v.seq;
         strides[2] = strides[1] * (cuuint64_t)v.heads;
