@@ -183,6 +183,9 @@ bool sm100_skinny_gemm_preferred(const GemmArgs &g);  // quicker than sm100_gemm
 int sm100_skinny_gemm(const GemmArgs &g, DeviceState *st, cudaStream_t s);
 // planes: so many copies of the view one after the other, counted along the parts
 int make_tensor_map_bf16_view(CUtensorMap *map, const MatView &v, uint32_t box_cols, uint32_t box_rows, int planes = 1);
+// Float32, at most 16 rows, y = x w + b (gemm_skinny_f32.cu): a decode step's projections on the CUDA cores.
+bool skinny_f32_supported(const GemmArgs &g);
+int skinny_f32_gemm(const GemmArgs &g, DeviceState *st, cudaStream_t s);
 // Float32 storage on the tensor cores, operands as three bf16 planes each (gemm_f32_sm100.cu, split_f32.cuh): a row-major view's rows
 // padded to 8 columns. _us: an estimate of the time, without the splitting.
 struct SplitGuard;

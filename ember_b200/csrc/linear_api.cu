@@ -212,6 +212,7 @@ int run(GemmArgs g, DeviceState *st, cudaStream_t s, PackedOperands &packed)
     const bool large = sm100_gemm_supported(g);
     if (sm100_skinny_gemm_supported(g) && (!large || sm100_skinny_gemm_preferred(g))) return sm100_skinny_gemm(g, st, s);
     if (large) return sm100_gemm(g, st, s);
+    if (skinny_f32_supported(g)) return skinny_f32_gemm(g, st, s);
     return simt_gemm(g, st, s);
 }
 
@@ -237,7 +238,7 @@ int ember_linear_fwd(const void *x, const void *w, const void *bias, void *y, lo
     g.m = m; g.n = n; g.k = k; g.dtype = dtype;
     PackedOperands packed(pick_stream(stream, st));
     F32Products f32;
-    if (dtype == EMBER_F32) f32.add(g);
+    if (dtype == EMBER_F32 && !skinny_f32_supported(g)) f32.add(g);
     if (f32.preferred(st->sm_count) && (rc = f32.run(st, packed.stream)) != EMBER_ERR_NOMEM) return rc;
     return run(g, st, packed.stream, packed);
 }

@@ -49,6 +49,12 @@ def test_head_major_operands(batch, seq, heads, dim):
         assert np.abs(a - r).max() <= 1e-5 * np.abs(r).max()
 
 
+@pytest.mark.parametrize("m,n,k", [(1, 64, 64), (3, 68, 65), (4, 1000, 512), (5, 64, 2048), (8, 1540, 100), (9, 204, 8192), (13, 2048, 513), (16, 6144, 1030), (16, 64, 1023), (2, 4100, 4099)])
+def test_few_rows(m, n, k):
+    """The kernel that streams w: every number of rows' form, contractions that leave rounds and the cluster's parts uneven."""
+    check(m, n, k)
+
+
 def test_one_hot_rows_pick_rows_of_w_bit_for_bit():
     """Three planes hold a float32 exactly, and so does the sum of its products with one."""
     w = seeded((1024, 1032), 1)
