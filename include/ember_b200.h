@@ -13,7 +13,9 @@
  *     lse: (batch_heads, lq) float32, natural-log log-sum-exp of the scaled,
  *     masked scores of each query row.
  *   - dtype selects the storage type of q/k/v/out/dout/dq/dk/dv: EMBER_F32 or
- *     EMBER_BF16. Softmax and all accumulation are float32 in both modes.
+ *     EMBER_BF16. Softmax and all accumulation are float32 in both modes. Float32 forwards and backwards
+ *     of some size take temporary device memory (6 bytes per element of their inputs) from the stream's pool and
+ *     free it in stream order (under stream capture: memory nodes); where there is none they run without.
  *   - causal != 0 masks key j for query i when j > i + (lk - lq) (lower
  *     triangle aligned to the bottom-right corner; requires lq <= lk). This is
  *     the additive {0,-inf} mask the reference would need a broadcast add for
@@ -247,7 +249,8 @@ EMBER_API int ember_gather_outputs(void *out_full, const void *out_slab, size_t 
  *
  * x is a logical (m, k) matrix, w is (k, n) row-major as the reference stores it (in_features,
  * out_features), bias has n elements (or NULL), y is (m, n). dtype selects storage as for attention
- * (float32 arithmetic on CUDA cores for EMBER_F32; bf16 tensor-core products with float32
+ * (EMBER_F32: float32 arithmetic on CUDA cores, or, by size, each operand as three bf16 parts on the tensor cores, which hold
+ * a float32 exactly; bf16 tensor-core products with float32
  * accumulation for EMBER_BF16 when the shapes allow, else float32 arithmetic on bf16 storage).
  *
  * Head-major operands, so that no transpose runs between a projection and attention:
