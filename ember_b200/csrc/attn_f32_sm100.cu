@@ -14,6 +14,7 @@
 // Common to the kernels: 128 rows of one operand belong to a CTA (a row per tensor-memory lane) and lie in tensor memory as
 // the A operand of the score product, tiles of 64 rows of the other operand's planes are streamed by TMA, eight compute
 // warps (two warpgroups) own the rows' softmax, two warps issue, one loads.
+#include <float.h>
 #include <math.h>
 
 #include "common.cuh"
@@ -37,7 +38,8 @@ enum { WF_Q = 301, WF_K, WF_V, WF_S, WF_P, WF_O, WF_OFREE, WF_KEMPTY, WF_VEMPTY,
 __device__ __forceinline__ float exp_nat(float x) { return ex2(x * LOG2E_T); }
 
 // e^x of the backward, which has no division by the sum for errors common to a row to cancel in: what the product with log2(e) is
-// rounded by is put back to first order, 2^(y + r) = 2^y (1 + r ln 2). x is finite.
+// rounded by is put back to first order, 2^(y + r) = 2^y (1 + r ln 2). x log2(e) is finite (kMostScore), and x at most a rounding
+// error of a score above 0, since scores come out as the forward's did.
 __device__ __forceinline__ f32x2 exp_pair(f32x2 x)
 {
     const f32x2 y = mul2(x, pack2(LOG2E_T, LOG2E_T)), neg = mul2(x, pack2(-LOG2E_T, -LOG2E_T));
@@ -140,9 +142,9 @@ __device__ __forceinline__ void chain_ss(uint32_t d, uint32_t a, uint32_t b, uin
 
 // Scores: D (128 x 64) = A * B^T (a tile of 64 rows, HD columns, planes PLANE bytes apart). A in tensor memory, parts HD / 2
 // columns apart, or in shared memory (SS): 128 rows, planes 2 * PLANE bytes apart, 64-column sub-tiles 2 * SUB. The contraction
-// stops at the end of the 32 columns that hold the last of d (zeros past d).
+// stops at the end of the 32 columns that hold the last of d (zeros past d). `mirrored`: the tile is the queries' and A the keys'.
 template <int HD, bool SS>
-__device__ __forceinline__ void mma_scores(uint32_t d, uint32_t a, uint32_t b_smem, int ksteps, uint32_t elected)
+__device__ __forceinline__ void mma_scores(uint32_t d, uint32_t a, uint32_t b_smem, int ksteps, uint32_t elected, bool mirrored)
 {
     constexpr uint32_t IDESC = idesc_bf16_f32(128, TN, 0, 0);
     constexpr int PLANE = HD / 64 * SUB;
@@ -151,7 +153,7 @@ __device__ __forceinline__ void mma_scores(uint32_t d, uint32_t a, uint32_t b_sm
     for (int i = 0; i < kSplitProducts; i++) {
 #pragma unroll
         for (int sub = 0; sub < HD / 64; sub++) {
-            const uint32_t acc = i > 0 || sub > 0, pa = split_part_a(i), b = b_lo + split_part_b(i) * (PLANE >> 4) + ((sub * SUB) >> 4);
+            const uint32_t acc = i > 0 || sub > 0, pa = split_part_a(i, mirrored), b = b_lo + split_part_b(i, mirrored) * (PLANE >> 4) + ((sub * SUB) >> 4);
             const bool four = ksteps - sub * 4 > 2;
             if (SS) chain_ss<2, 4, 6, 2, 4, 6>(d, a_lo + pa * ((2 * PLANE) >> 4) + ((sub * 2 * SUB) >> 4), b, IDESC, elected, acc, four);
             else chain_ts<8, 16, 24, 2, 4, 6>(d, a_lo + pa * (HD / 2) + sub * 32, b, IDESC, elected, acc, four);
@@ -335,7 +337,7 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
                 if (C::LATE && j > 0) ok = ok && mbar_wait(BAR(C::B_SREAD), (j - 1) & 1, abort_flag, p.status, WF_P);
                 if (!C::LATE && j > 1) ok = ok && mbar_wait(BAR(C::B_O + w), ((j - 2) >> 1) & 1, abort_flag, p.status, WF_P);
                 tc_fence_after();
-                mma_scores<HD, false>(tmem + C::T_S + w * C::S_STEP, tmem + C::T_Q, smem_base + C::OFF_K + (j % C::KST) * C::TILE, ksteps, elected);
+                mma_scores<HD, false>(tmem + C::T_S + w * C::S_STEP, tmem + C::T_Q, smem_base + C::OFF_K + (j % C::KST) * C::TILE, ksteps, elected, false);
                 tc_commit_elect(BAR(C::B_S + w));
                 tc_commit_elect(BAR(C::B_KEMPTY + j % C::KST));
             }
@@ -693,7 +695,7 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
                     wait(C::B_P, j - 1, WB_ACC);
                 }
                 tc_fence_after();
-                mma_scores<HD, false>(at, tmem + C::T_A0, b0, ksteps, elected);
+                mma_scores<HD, false>(at, tmem + C::T_A0, b0, ksteps, elected, !is_q);  // the forward's scores, bit for bit
                 tc_commit_elect(BAR(done));
                 if (!has_ds) {
                     tc_commit_elect(BAR(C::B_EMPTY0 + s));
@@ -702,7 +704,7 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
                 wait(C::B_FULL1 + s, j / stages, WB_B1);
                 if (j > 0) wait(role == R_DKDV ? C::B_R1 : C::B_R0, j - 1, WB_ACC);  // over dS
                 tc_fence_after();
-                mma_scores<HD, true>(t_d + SCORES_AT, smem_base + C::OFF_A1, b0 + C::TILE, ksteps, elected);
+                mma_scores<HD, true>(t_d + SCORES_AT, smem_base + C::OFF_A1, b0 + C::TILE, ksteps, elected, false);
                 tc_commit_elect(BAR(C::B_DP));
                 tc_commit_elect(BAR(C::B_EMPTY1 + s));
             }
@@ -751,7 +753,7 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
         const float *lse = p.lse + (size_t)unit * p.lq, *delta = p.delta + (size_t)unit * p.lq;
         float *vec = reinterpret_cast<float *>(smem_gen + C::OFF_VEC + warp * 256);  // this warp's 32 columns
         // Negative log-sum-exp and delta of a query; past the end (and where a row has no weight at all) P is 0: finite, since
-        // the exponential below would make NaN of an infinity.
+        // the exponential below would make NaN of an infinity, and beyond every score (kMostScore).
         auto neg_lse = [&](int qi) {
             const float x = qi < p.lq ? lse[qi] : 1e30f;
             return x > 1e30f ? -1e30f : -x;
@@ -943,6 +945,13 @@ int launch_bwd(const AttnArgs &a, const float *delta, const void *qp, const void
     return EMBER_OK;
 }
 
+// What scores may reach (columns x the largest elements of q and k x scale) before the CUDA cores take over. 2^96 keeps them below the
+// 1e30 that stands for an infinite log-sum-exp. The backward's weights e^(score - log-sum-exp) carry the score's rounding error, unless
+// forward and backward form the same bits: both tensor-core kernels do, both CUDA-core kernels do, one of each does not (values'
+// gradients off by 1e-4 of their norm at scores of 1e4, 7e-3 at 1e6, NaN at 1e12). Where sizes send the two directions to different
+// kernels, 2^12 keeps that below 5e-4.
+constexpr double kMostScore = 7.9e28, kMostScoreMixed = 4096;
+
 // Scales beyond 2^20 could take scores of operands below 2^50 to infinity.
 bool takes(const AttnArgs &a) { return a.dtype == EMBER_F32 && a.d <= 128 && fabsf(a.scale) <= 1048576.f && (long long)a.bh * 3 <= 0x7fffffffLL; }
 
@@ -996,6 +1005,16 @@ bool sm100_f32_bwd_preferred(const AttnArgs &a, int sms)
     return tensor < 0.95 * cores;
 }
 
+namespace {
+// The guard's limit for the largest elements of q and k.
+float score_limit(const AttnArgs &a, int sms)
+{
+    const double most = sm100_f32_fwd_preferred(a, sms) && sm100_f32_bwd_preferred(a, sms) ? kMostScore : kMostScoreMixed;
+    const double limit = a.scale != 0 ? most / (a.d * fabs((double)a.scale)) : FLT_MAX;
+    return limit < FLT_MAX ? (float)limit : FLT_MAX;
+}
+}  // namespace
+
 int sm100_f32_attention_fwd(const AttnArgs &a, DeviceState *st, cudaStream_t s)
 {
     const long long q_rows = (long long)a.bh * a.lq, k_rows = (long long)a.bh * a.lk;
@@ -1005,6 +1024,8 @@ int sm100_f32_attention_fwd(const AttnArgs &a, DeviceState *st, cudaStream_t s)
     const SplitJob jobs[3] = {{(const float *)a.k, mem, k_rows, a.d}, {(const float *)a.v, mem + k_bytes, k_rows, a.d}, {(const float *)a.q, nullptr, q_rows, a.d}};
     SplitGuard guard;
     int rc = split_f32(jobs, 3, nullptr, mem + 2 * k_bytes, &guard, s);
+    guard.pair[1] = 2;  // k or q, and the other one
+    guard.pair_limit = score_limit(a, st->sm_count);
     if (rc == EMBER_OK)
         rc = a.d <= 64 ? launch_fwd<64>(a, mem, mem + k_bytes, guard, st, s) : launch_fwd<128>(a, mem, mem + k_bytes, guard, st, s);
     if (rc == EMBER_OK) {
@@ -1027,6 +1048,8 @@ int sm100_f32_attention_bwd(const AttnArgs &a, float *delta, DeviceState *st, cu
     const SplitDelta dl = {(const float *)a.out, (const float *)a.dout, delta, q_rows, a.d};
     SplitGuard guard;
     int rc = split_f32(jobs, 4, &dl, words, &guard, s);
+    guard.pair[1] = 2;  // k or q, and the other one
+    guard.pair_limit = score_limit(a, st->sm_count);
     if (rc == EMBER_OK)
         rc = a.d <= 64 ? launch_bwd<64>(a, delta, qp, kp, vp, gp, guard, st, s) : launch_bwd<128>(a, delta, qp, kp, vp, gp, guard, st, s);
     if (rc == EMBER_OK) {

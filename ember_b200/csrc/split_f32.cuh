@@ -29,37 +29,45 @@ struct SplitGuard {
     int first[kSplitMaxJobs + 1] = {};  // blocks [first[i], first[i + 1]) saw tensor i
     int count = 0;
     int *fallback = nullptr;
+    // Largest product of tensors pair[0]'s and pair[1]'s largest magnitudes that the kernel takes (attention: what it could score).
+    int pair[2] = {};
+    float pair_limit = 0;  // 0: any
 };
 
 #ifdef __CUDACC__
-// Whether any tensor holds values that the parts cannot represent. All threads of the block call it; `word` is shared memory.
-__device__ __forceinline__ bool split_out_of_range(const SplitGuard &g, uint32_t *word)
+// Whether any tensor holds values that the parts cannot represent, or the pair's product is beyond its limit. All threads of the block
+// call it; `words` is shared memory, kSplitMaxJobs words.
+__device__ __forceinline__ bool split_out_of_range(const SplitGuard &g, uint32_t *words)
 {
-    if (threadIdx.x == 0) *word = 0;
+    if (threadIdx.x < kSplitMaxJobs) words[threadIdx.x] = 0;
     __syncthreads();
-    uint32_t bits = 0;
-    for (int i = 0; i < g.count; i++)
-        for (int b = g.first[i] + (int)threadIdx.x; b < g.first[i + 1]; b += blockDim.x) {
-            const uint32_t m = g.slots[b];
-            if (m >= kSplitHuge) bits |= 1u;
-            if (m != 0) bits |= 2u << (2 * i);
-            if (m >= kSplitTiny) bits |= 4u << (2 * i);
-        }
-    if (bits) atomicOr(word, bits);
+    uint32_t m[kSplitMaxJobs] = {};
+#pragma unroll 2
+    for (int b = (int)threadIdx.x; b < g.first[g.count]; b += blockDim.x) {
+        const uint32_t v = g.slots[b];
+#pragma unroll
+        for (int i = 0; i < kSplitMaxJobs; i++)
+            if (i < g.count && b >= g.first[i] && b < g.first[i + 1]) m[i] = max(m[i], v);
+    }
+#pragma unroll
+    for (int i = 0; i < kSplitMaxJobs; i++) {
+        m[i] = __reduce_max_sync(0xffffffffu, m[i]);
+        if (threadIdx.x % 32 == 0 && m[i] != 0) atomicMax(&words[i], m[i]);
+    }
     __syncthreads();
-    bits = *word;
-    bool out = (bits & 1u) != 0;
-    for (int i = 0; i < g.count; i++) out = out || ((bits >> (1 + 2 * i)) & 3u) == 1u;
+    bool out = g.pair_limit > 0 && !(__uint_as_float(words[g.pair[0]]) * __uint_as_float(words[g.pair[1]]) <= g.pair_limit);
+    for (int i = 0; i < g.count; i++) out = out || words[i] >= kSplitHuge || (words[i] != 0 && words[i] < kSplitTiny);
     if (blockIdx.x == 0 && threadIdx.x == 0) *g.fallback = out ? 1 : 0;
     return out;
 }
 
 // The six products of parts, small ones first: (part of A, part of B) = (2, 0) (1, 1) (0, 2) (1, 0) (0, 1) (0, 0), 0 = high. A
 // loop and not straight code: with the four products of a backward step unrolled, issuing and computing warps together outgrew
-// the instruction cache.
+// the instruction cache. With the two operands exchanged and `mirrored` the same six come in the same order, so that a product and its
+// transpose are the same bits.
 constexpr int kSplitProducts = 6;
-__device__ __forceinline__ uint32_t split_part_a(int i) { return (0x046u >> (2 * i)) & 3u; }
-__device__ __forceinline__ uint32_t split_part_b(int i) { return (0x124u >> (2 * i)) & 3u; }
+__device__ __forceinline__ uint32_t split_part_a(int i, bool mirrored = false) { return ((mirrored ? 0x124u : 0x046u) >> (2 * i)) & 3u; }
+__device__ __forceinline__ uint32_t split_part_b(int i, bool mirrored = false) { return ((mirrored ? 0x046u : 0x124u) >> (2 * i)) & 3u; }
 
 // Two neighbouring columns -> one 32-bit word of each part.
 __device__ __forceinline__ void split_pair(float a, float b, uint32_t &hi, uint32_t &mid, uint32_t &lo)

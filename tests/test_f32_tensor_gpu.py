@@ -115,6 +115,31 @@ def test_tensors_of_tiny_values_keep_their_precision(d):
     close(run(q, k, v, g, d ** -0.5, False), reference(q, k, v, g, d ** -0.5, False))
 
 
+@pytest.mark.parametrize("units,lq,lk,d", [(2, 520, 600, 64), (2, 520, 600, 128), (1, 600, 600, 40), (1, 200, 512, 64), (64, 128, 128, 64)])
+@pytest.mark.parametrize("size", [10.0, 30.0, 1e3, 1e5, 1e8, 4e14])
+def test_large_scores_leave_the_largest_a_weight_of_one(units, lq, lk, d, size):
+    """Elements of +-size: query i scores 10 times its other keys with key i + lk - lq, whose weight is 1 to the last bit wherever forward
+    and backward round scores alike. That key's value is the output, its gradient the upstream gradient. Scores' rounding errors may reach
+    the weight where the two run on different kernels, up to the 2^12 at which those calls stay on the CUDA cores: 2^-10 then (a few units
+    of 2^-23 of a score)."""
+    rng = np.random.default_rng(5)
+    k = np.where(rng.standard_normal((units, lk, d)) < 0, -1, 1) * rng.uniform(0.75, 1.25, (units, lk, d)) * size
+    k = k.astype(np.float32)
+    q = (k[:, lk - lq:] * np.float32(1.37)).astype(np.float32)
+    v, g = seeded((units, lk, d), 2), seeded((units, lq, d), 3)
+    scale = 0.25 if d == 40 else 0.125
+    s = (q[0].astype(np.float64) @ k[0].T.astype(np.float64)) * scale
+    best = s[np.arange(lq), np.arange(lq) + lk - lq]
+    s[np.arange(lq), np.arange(lq) + lk - lq] = -np.inf
+    assert (best - s.max(1)).min() > 40
+    o, lse, dq, dk, dv = run(q, k, v, g, scale, False)
+    rel = 2.0 ** -10 if units == 64 or lq == 200 else 2.0 ** -20
+    assert np.abs(o - v[:, lk - lq:]).max() <= 2.0 ** -20 * np.abs(v).max()
+    assert np.abs(lse[0] - best).max() <= 2.0 ** -20 * best.max()
+    assert np.abs(dv[:, lk - lq:] - g).max() <= rel * np.abs(g).max()
+    assert np.isfinite(dq).all() and np.isfinite(dk).all()
+
+
 def test_zeros_stay_on_the_tensor_cores_and_give_means():
     q, k, v, g = inputs(2, 520, 600, 64)
     q[:] = 0
