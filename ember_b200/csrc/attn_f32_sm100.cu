@@ -1,7 +1,8 @@
 // Float32 attention on the tensor cores: every operand is the sum of three bf16 parts (split_f32.cuh), a product of
 // two operands six tcgen05 products of their parts, small ones first, accumulated in float32 over at most 64 terms in
 // tensor memory and then added into float32 registers. Probabilities and score gradients are split the same way in
-// registers, so nothing is held or multiplied with less than 24 bits.
+// registers, so nothing is held or multiplied with less than 24 bits. Parts are of 2^20 times a value (a power of its own for score
+// gradients), so that small ones keep all of theirs; where a result leaves the accumulators that is undone.
 //
 // The CUDA-core kernels (attn_simt.cu) do the same products at the FMA pipe's rate, 128 per clock and SM; six bf16 products for
 // each leave 683 per clock. Measured, 16 units x L1024, causal: d 64 forward 93 -> 29 us, backward 215 -> 61 us (and 6 us of
@@ -76,7 +77,7 @@ __device__ __forceinline__ void row_to_tmem(const float *src, int d, bool vec, i
         }
         uint32_t a[16], b[16], c[16];
 #pragma unroll
-        for (int i = 0; i < 16; i++) split_pair(pack2(v[2 * i], v[2 * i + 1]), a[i], b[i], c[i]);
+        for (int i = 0; i < 16; i++) split_pair(pack2(v[2 * i] * kSplitUp, v[2 * i + 1] * kSplitUp), a[i], b[i], c[i]);
         const uint32_t t = taddr + (uint32_t)(c0 / 2);
         tmem_st_32x32b_x16(t, a);
         tmem_st_32x32b_x16(t + plane, b);
@@ -86,12 +87,13 @@ __device__ __forceinline__ void row_to_tmem(const float *src, int d, bool vec, i
 }
 
 // 32 values of a row -> their parts in tensor memory: 3 blocks of 16 columns from taddr, part by part. The A operand of 16 values
-// (one MMA) is 8 columns.
+// (one MMA) is 8 columns. UP: of 2^20 times the values.
+template <bool UP>
 __device__ __forceinline__ void split_to_tmem(const f32x2 *v, uint32_t taddr)
 {
     uint32_t a[16], b[16], c[16];
 #pragma unroll
-    for (int i = 0; i < 16; i++) split_pair(v[i], a[i], b[i], c[i]);
+    for (int i = 0; i < 16; i++) split_pair(UP ? mul2(v[i], pack2(kSplitUp, kSplitUp)) : v[i], a[i], b[i], c[i]);
     tmem_st_32x32b_x16(taddr, a);
     tmem_st_32x32b_x16(taddr + 16, b);
     tmem_st_32x32b_x16(taddr + 32, c);
@@ -202,7 +204,7 @@ __device__ __forceinline__ void flush(f32x2 (&acc)[N32 * 16], uint32_t taddr, in
 }
 
 template <int N>
-__device__ __forceinline__ void store_cols(float *dst, const f32x2 (&v2)[N / 2], float scale, int col0, int d, bool vec, const void *base, size_t bytes,
+__device__ __forceinline__ void store_cols(float *dst, const f32x2 (&v2)[N / 2], float down, float scale, int col0, int d, bool vec, const void *base, size_t bytes,
                                            DeviceStatus *status)
 {
     (void)base; (void)bytes; (void)status;
@@ -211,13 +213,15 @@ __device__ __forceinline__ void store_cols(float *dst, const f32x2 (&v2)[N / 2],
         float v[4];
         unpack2(v2[c / 2], v[0], v[1]);
         unpack2(v2[c / 2 + 1], v[2], v[3]);
+#pragma unroll
+        for (int i = 0; i < 4; i++) v[i] = v[i] * down * scale;
         if (vec) {
             if (col0 + c < d && EMBER_STORE_OK(dst + col0 + c, base, bytes, 16, status))
-                *reinterpret_cast<float4 *>(dst + col0 + c) = make_float4(v[0] * scale, v[1] * scale, v[2] * scale, v[3] * scale);
+                *reinterpret_cast<float4 *>(dst + col0 + c) = make_float4(v[0], v[1], v[2], v[3]);
         } else {
 #pragma unroll
             for (int i = 0; i < 4; i++)
-                if (col0 + c + i < d && EMBER_STORE_OK(dst + col0 + c + i, base, bytes, 4, status)) dst[col0 + c + i] = v[i] * scale;
+                if (col0 + c + i < d && EMBER_STORE_OK(dst + col0 + c + i, base, bytes, 4, status)) dst[col0 + c + i] = v[i];
         }
     }
 }
@@ -378,7 +382,7 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
         f32x2 o[HD / 2];
 #pragma unroll
         for (int i = 0; i < HD / 2; i++) o[i] = 0;
-        const f32x2 scale2 = pack2(p.scale, p.scale), l2e = pack2(LOG2E_T, LOG2E_T);
+        const f32x2 scale2 = pack2(p.scale * kSplitDown2, p.scale * kSplitDown2), l2e = pack2(LOG2E_T, LOG2E_T);
         bool ok = true;
         for (int j = w; j < n && ok; j += 2) {
             const int k0 = j * TN;
@@ -436,7 +440,7 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
                     tc_fence_after();
                     flush<HD / 32, true>(o, to, cols, late_alpha);
                 }
-                split_to_tmem(s + h * 16, region + h * 48);
+                split_to_tmem<true>(s + h * 16, region + h * 48);
             }
             tmem_wait_st();
             tc_fence_before();
@@ -500,7 +504,7 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
         }
         if (ok && row < p.lq) {
             const size_t at = (size_t)unit * p.lq + row;
-            store_cols<HALF>(p.out + at * p.d, res, inv, w * HALF, p.d, p.vec_o, p.out, (size_t)p.order.units * p.lq * p.d * 4, p.status);
+            store_cols<HALF>(p.out + at * p.d, res, kSplitDown2, inv, w * HALF, p.d, p.vec_o, p.out, (size_t)p.order.units * p.lq * p.d * 4, p.status);
             if (p.lse && w == 0 && EMBER_STORE_OK(p.lse + at, p.lse, (size_t)p.order.units * p.lq * 4, 4, p.status)) p.lse[at] = mm + logf(ll);
         }
     }
@@ -535,7 +539,7 @@ struct F32BwdCfg {
     static constexpr int T_A0 = 0, T_S = 3 * HD / 2 + (HD == 64 ? 0 : SCORES_AT), T_P = HD == 64 ? 160 : 192, T_D = HD == 64 ? 256 : 288, T_R = HD == 64 ? 352 : 384;
     enum { B_A, B_FULL0, B_FULL1 = B_FULL0 + MAXST, B_EMPTY0 = B_FULL1 + MAXST, B_EMPTY1 = B_EMPTY0 + MAXST, B_S = B_EMPTY1 + MAXST, B_P, B_DP, B_DS, B_R0, B_R1, B_F0, B_F1, NUM_BARS,
            B_S1 = B_DP };  // DV: scores of odd tiles (the next tile's may be there before this one's have been waited for)
-    static_assert(8 * NUM_BARS + 16 <= 256, "");
+    static_assert(8 * NUM_BARS + 8 + 4 * kSplitMaxTensors <= 256, "");
 };
 
 struct F32BwdParams {
@@ -758,14 +762,22 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
             const float x = qi < p.lq ? lse[qi] : 1e30f;
             return x > 1e30f ? -1e30f : -x;
         };
-        auto neg_delta = [&](int qi) { return has_ds && qi < p.lq ? -delta[qi] : 0.f; };
+        // Score gradients, products of four tensors' values, are split as 2^ds_shift times themselves: the range in which their
+        // products' sums stay well inside float32 (with weights up to 2^20) depends on those tensors (0 to 4: q, dO, k, v, delta).
+        const uint32_t *most = tmem_slot + 2;
+        const int e_dp = max(split_exponent(most[1]) + split_exponent(most[3]) + 7, split_exponent(most[4])) + 1;
+        const int e_sum = max(0, max(split_exponent(most[0]), split_exponent(most[2])) + kSplitShift + 32 - __clz(max(p.lq, p.lk)));
+        const int ds_shift = max(-60, min(100, 100 - e_dp - e_sum));
+        const float ds_up = __int_as_float((127 + ds_shift) << 23), ds_down = __int_as_float((127 - ds_shift - kSplitShift) << 23);
+        const f32x2 dp_scale2 = pack2(ds_up * kSplitDown2, ds_up * kSplitDown2);
+        auto neg_delta = [&](int qi) { return has_ds && qi < p.lq ? -delta[qi] * ds_up : 0.f; };
         const float nl_row = is_q ? neg_lse(row) : 0.f, nd_row = is_q ? neg_delta(row) : 0.f;
         const int cols = (p.d + 15) / 16 * 16;
         // results in registers: DKDV: warpgroup 0 dV, 1 dK; otherwise half of the columns each
         f32x2 acc[32];
 #pragma unroll
         for (int i = 0; i < 32; i++) acc[i] = 0;
-        const f32x2 scale2 = pack2(p.scale, p.scale);
+        const f32x2 scale2 = pack2(p.scale * kSplitDown2, p.scale * kSplitDown2);
         const int acc_col0 = role == R_DKDV ? 0 : w * (HD / 2);
         const int acc_cols = min(role == R_DKDV ? cols : HD / 2, cols - acc_col0);
         const uint32_t acc_at = t_r + lane_sel + (role == R_DKDV ? w * 64 : acc_col0);
@@ -826,7 +838,7 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
                     ok = ok && mbar_wait(BAR(C::B_R0), (j - 1) & 1, abort_flag, p.status, WB_ACC);
                     tc_fence_after();
                 }
-                split_to_tmem(e, t_p + turn + w * 48);
+                split_to_tmem<true>(e, t_p + turn + w * 48);
                 tmem_wait_st();
             }
             tc_fence_before();
@@ -842,10 +854,10 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
 #pragma unroll
                 for (int i = 0; i < 16; i += 2) {
                     const ulonglong2 nd = is_q ? make_ulonglong2(pack2(nd_row, nd_row), pack2(nd_row, nd_row)) : *reinterpret_cast<const ulonglong2 *>(vec + 32 + i * 2);
-                    e[i] = mul2(e[i], add2(pack2(__uint_as_float(u[2 * i]), __uint_as_float(u[2 * i + 1])), nd.x));
-                    e[i + 1] = mul2(e[i + 1], add2(pack2(__uint_as_float(u[2 * i + 2]), __uint_as_float(u[2 * i + 3])), nd.y));
+                    e[i] = mul2(e[i], fma2(pack2(__uint_as_float(u[2 * i]), __uint_as_float(u[2 * i + 1])), dp_scale2, nd.x));
+                    e[i + 1] = mul2(e[i + 1], fma2(pack2(__uint_as_float(u[2 * i + 2]), __uint_as_float(u[2 * i + 3])), dp_scale2, nd.y));
                 }
-                split_to_tmem(e, t_d + lane_sel + w * 48);
+                split_to_tmem<false>(e, t_d + lane_sel + w * 48);
                 tmem_wait_st();
                 tc_fence_before();
                 __syncwarp();
@@ -856,7 +868,7 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
         if (ok && row < rows && acc_cols > 0) {
             float *dst = is_q ? p.dq : role == R_DKDV ? (w == 0 ? p.dv : p.dk) : role == R_DK ? p.dk : p.dv;
             const bool is_dv = role == R_DV || (role == R_DKDV && w == 0);
-            store_cols<64>(dst + row_at, acc, is_dv ? 1.f : p.scale, acc_col0, role == R_DKDV ? p.d : min(p.d, acc_col0 + HD / 2), p.vec_out, dst, (size_t)p.units * rows * p.d * 4, p.status);
+            store_cols<64>(dst + row_at, acc, is_dv ? kSplitDown2 : ds_down, is_dv ? 1.f : p.scale, acc_col0, role == R_DKDV ? p.d : min(p.d, acc_col0 + HD / 2), p.vec_out, dst, (size_t)p.units * rows * p.d * 4, p.status);
         }
     }
     tc_fence_before();
@@ -952,8 +964,12 @@ int launch_bwd(const AttnArgs &a, const float *delta, const void *qp, const void
 // kernels, 2^12 keeps that below 5e-4.
 constexpr double kMostScore = 7.9e28, kMostScoreMixed = 4096;
 
-// Scales beyond 2^20 could take scores of operands below 2^50 to infinity.
-bool takes(const AttnArgs &a) { return a.dtype == EMBER_F32 && a.d <= 128 && fabsf(a.scale) <= 1048576.f && (long long)a.bh * 3 <= 0x7fffffffLL; }
+// Scales below 2^-60 times 2^-40 (the parts' factors) would end in float32's smallest exponents, those beyond 2^20 could take scores
+// of operands below 2^28 to the limit above.
+bool takes(const AttnArgs &a)
+{
+    return a.dtype == EMBER_F32 && a.d <= 128 && fabsf(a.scale) <= 1048576.f && (a.scale == 0 || fabsf(a.scale) >= 8.7e-19f) && (long long)a.bh * 3 <= 0x7fffffffLL;
+}
 
 }  // namespace
 

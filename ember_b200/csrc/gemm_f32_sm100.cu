@@ -241,11 +241,14 @@ __global__ void __launch_bounds__(THREADS, 1)
             auto bias4 = [&](int col) {
                 return p.bias ? make_float4(p.bias[col], p.bias[col + 1], p.bias[col + 2], p.bias[col + 3]) : make_float4(0.f, 0.f, 0.f, 0.f);
             };
+            auto with_bias = [](const float4 &v, const float4 &b) {
+                return make_float4(fmaf(v.x, kSplitDown2, b.x), fmaf(v.y, kSplitDown2, b.y), fmaf(v.z, kSplitDown2, b.z), fmaf(v.w, kSplitDown2, b.w));
+            };
             auto store1 = [&](float *dst, int col, const float4 &v) {  // columns one by one (row-major)
                 const float x[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
                 for (int i = 0; i < 4; i++)
-                    if (col + i < p.n) dst[i] = x[i] + (p.bias ? p.bias[col + i] : 0.f);
+                    if (col + i < p.n) dst[i] = fmaf(x[i], kSplitDown2, p.bias ? p.bias[col + i] : 0.f);
             };
             const int rows_here = ok ? rows_valid : 0;
             if (BN == 128 && p.splits == 1) {
@@ -259,8 +262,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                         unpack2(acc[2 * q + 1], v.z, v.w);
                         if (col + q * 4 >= p.n) continue;
                         if (p.c_vec) {
-                            const float4 b = bias4(col + q * 4);
-                            *reinterpret_cast<float4 *>(dst + q * 4) = make_float4(v.x + b.x, v.y + b.y, v.z + b.z, v.w + b.w);
+                            *reinterpret_cast<float4 *>(dst + q * 4) = with_bias(v, bias4(col + q * 4));
                         } else {
                             store1(dst + q * 4, col + q * 4, v);
                         }
@@ -283,9 +285,8 @@ __global__ void __launch_bounds__(THREADS, 1)
                         const float4 b = bias4(col);
 #pragma unroll 4
                         for (int i = 0; i < 8; i++) {
-                            float4 v = *reinterpret_cast<const float4 *>(from + i * 512 + (((lane % 8) ^ ((i * 4 + lane / 8) & 7)) << 4));
-                            v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w;
-                            if (first + i * 4 < rows_here) *reinterpret_cast<float4 *>(dst + (size_t)(i * 4) * row_stride) = v;
+                            const float4 v = *reinterpret_cast<const float4 *>(from + i * 512 + (((lane % 8) ^ ((i * 4 + lane / 8) & 7)) << 4));
+                            if (first + i * 4 < rows_here) *reinterpret_cast<float4 *>(dst + (size_t)(i * 4) * row_stride) = with_bias(v, b);
                         }
                     } else {
 #pragma unroll 1
@@ -318,8 +319,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                     if (row >= rows_here || col >= p.n) continue;
                     float *dst = column(col) + (size_t)row * row_stride;
                     if (p.c_vec) {
-                        const float4 b = bias4(col);
-                        *reinterpret_cast<float4 *>(dst) = make_float4(v.x + b.x, v.y + b.y, v.z + b.z, v.w + b.w);
+                        *reinterpret_cast<float4 *>(dst) = with_bias(v, bias4(col));
                     } else {
                         store1(dst, col, v);
                     }

@@ -14,6 +14,18 @@ struct SplitParams {
     int delta_blocks;
 };
 
+// The largest magnitude that this block saw, into its slot.
+__device__ __forceinline__ void report(uint32_t *slots, uint32_t amax)
+{
+    __shared__ uint32_t most;
+    if (threadIdx.x == 0) most = 0;
+    __syncthreads();
+    amax = __reduce_max_sync(0xffffffffu, amax);
+    if (threadIdx.x % 32 == 0) atomicMax(&most, amax);
+    __syncthreads();
+    if (threadIdx.x == 0) slots[blockIdx.x] = most;
+}
+
 // Bound: one pass over memory, 4 bytes read and 6 written per element, mostly within L2 (the next kernel reads the planes at
 // once). A thread makes 8 columns of the three planes (16-byte stores); a block takes every n-th piece of its tensor.
 __global__ void __launch_bounds__(256) split_f32_kernel(const SplitParams p)
@@ -27,6 +39,7 @@ __global__ void __launch_bounds__(256) split_f32_kernel(const SplitParams p)
         const int lane = threadIdx.x % 16;
         const bool vec = d.cols % 4 == 0 && (((uintptr_t)d.out | (uintptr_t)d.dout) & 15) == 0;
         const long long step = (long long)p.delta_blocks * 16;
+        uint32_t amax = 0;
         for (long long row0 = (long long)((int)blockIdx.x - total) * 16; row0 < d.rows; row0 += step) {
             const long long row = row0 + threadIdx.x / 16;
             float s = 0.f;
@@ -43,8 +56,12 @@ __global__ void __launch_bounds__(256) split_f32_kernel(const SplitParams p)
             }
 #pragma unroll
             for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-            if (row < d.rows && lane == 0) d.delta[row] = s;
+            if (row < d.rows && lane == 0) {
+                d.delta[row] = s;
+                amax = max(amax, __float_as_uint(s) & 0x7fffffffu);
+            }
         }
+        report(p.slots, amax);
         return;
     }
     int j = 0;
@@ -74,18 +91,12 @@ __global__ void __launch_bounds__(256) split_f32_kernel(const SplitParams p)
         for (int i = 0; i < 8; i++) amax = max(amax, __float_as_uint(v[i]) & 0x7fffffffu);
         if (!dst) continue;
 #pragma unroll
-        for (int i = 0; i < 4; i++) split_pair(v[2 * i], v[2 * i + 1], h[i], m[i], l[i]);
+        for (int i = 0; i < 4; i++) split_pair(v[2 * i] * kSplitUp, v[2 * i + 1] * kSplitUp, h[i], m[i], l[i]);
         dst[c] = make_uint4(h[0], h[1], h[2], h[3]);
         dst[chunks + c] = make_uint4(m[0], m[1], m[2], m[3]);
         dst[2 * chunks + c] = make_uint4(l[0], l[1], l[2], l[3]);
     }
-    __shared__ uint32_t most;
-    if (threadIdx.x == 0) most = 0;
-    __syncthreads();
-    amax = __reduce_max_sync(0xffffffffu, amax);
-    if (threadIdx.x % 32 == 0) atomicMax(&most, amax);
-    __syncthreads();
-    if (threadIdx.x == 0) p.slots[blockIdx.x] = most;
+    report(p.slots, amax);
 }
 
 }  // namespace
@@ -115,7 +126,11 @@ int split_f32(const SplitJob *jobs, int count, const SplitDelta *delta, void *gu
     guard->slots = p.slots;
     guard->count = count;
     for (int i = 0; i <= count; i++) guard->first[i] = p.first[i];
-    guard->fallback = (int *)guard_mem + kSplitMaxBlocks;
+    if (delta) {
+        guard->delta_at = guard->count++;
+        guard->first[guard->count] = p.first[count] + p.delta_blocks;
+    }
+    guard->fallback = (int *)guard_mem + 2 * kSplitMaxBlocks;
     EMBER_CUDA_TRY(launch_pdl(split_f32_kernel, p.first[count] + p.delta_blocks, 256, 0, s, p));
     return EMBER_OK;
 }

@@ -5,10 +5,12 @@
 // at 2^-25 of the largest), so an accumulator that collects a whole contraction drifts: relative error of random sums of 64 /
 // 512 / 2048 terms 6.6e-8 / 4.7e-7 / 2.1e-6. The kernels therefore let it collect 64 terms at most, the
 // small products first, and add it into float32 registers with rounding.
-// Values that the parts cannot hold (infinities, NaN, 2^50 and above, whose sums of products may meet infinities of
-// either sign, and tensors that are tiny throughout, whose parts run into bf16's smallest exponents) are found while the parts are
-// made: the tensor-core kernel then leaves the work to the CUDA-core kernel that is launched behind it and otherwise
-// returns at once.
+// Parts are made of the value times 2^20: bf16 ends at 2^-133, where the low part of a value below 2^-110 would lose its last bits
+// (a row of 1e-36 beside ordinary ones: 3e-5 of its results); 2^20 times the smallest float32 is held exactly. What is made of parts is
+// divided by the powers of two again where it leaves the accumulators.
+// Values that the parts cannot hold (infinities, NaN, 2^28 and above, whose sums of 2^31 products times 2^40 may pass float32) are
+// found while the parts are made: the tensor-core kernel then leaves the work to the CUDA-core kernel that is launched behind it and
+// otherwise returns at once.
 #pragma once
 
 #include "common.cuh"
@@ -19,15 +21,18 @@ namespace ember {
 
 constexpr int kSplitMaxJobs = 4;
 constexpr int kSplitMaxBlocks = 592;               // 4 blocks of 256 threads per SM
-constexpr uint32_t kSplitHuge = 0x58800000u;       // 2^50
-constexpr uint32_t kSplitTiny = 0x0D800000u;       // 2^-100
+constexpr int kSplitMaxTensors = kSplitMaxJobs + 1;  // delta's largest magnitude is reported as well
+constexpr uint32_t kSplitHuge = 0x4D800000u;       // 2^28
+constexpr uint32_t kSplitHugeDelta = 0x67800000u;  // 2^80
+constexpr int kSplitShift = 20;
+constexpr float kSplitUp = 1048576.f, kSplitDown2 = 1.f / 1048576.f / 1048576.f;  // a part's factor, and what undoes it in a product of two
 
 // What a split launch leaves for the kernels behind it: the largest magnitude (as bits; a NaN is larger than all) that each of
 // its blocks saw, by tensor, and the word through which the tensor-core kernel tells the CUDA-core kernel to run.
 struct SplitGuard {
     const uint32_t *slots = nullptr;
-    int first[kSplitMaxJobs + 1] = {};  // blocks [first[i], first[i + 1]) saw tensor i
-    int count = 0;
+    int first[kSplitMaxTensors + 1] = {};  // blocks [first[i], first[i + 1]) saw tensor i; the last may be delta
+    int count = 0, delta_at = -1;
     int *fallback = nullptr;
     // Largest product of tensors pair[0]'s and pair[1]'s largest magnitudes that the kernel takes (attention: what it could score).
     int pair[2] = {};
@@ -36,30 +41,33 @@ struct SplitGuard {
 
 #ifdef __CUDACC__
 // Whether any tensor holds values that the parts cannot represent, or the pair's product is beyond its limit. All threads of the block
-// call it; `words` is shared memory, kSplitMaxJobs words.
+// call it; `words` is shared memory, kSplitMaxTensors words, in which the tensors' largest magnitudes stay (as bits).
 __device__ __forceinline__ bool split_out_of_range(const SplitGuard &g, uint32_t *words)
 {
-    if (threadIdx.x < kSplitMaxJobs) words[threadIdx.x] = 0;
+    if (threadIdx.x < kSplitMaxTensors) words[threadIdx.x] = 0;
     __syncthreads();
-    uint32_t m[kSplitMaxJobs] = {};
+    uint32_t m[kSplitMaxTensors] = {};
 #pragma unroll 2
     for (int b = (int)threadIdx.x; b < g.first[g.count]; b += blockDim.x) {
         const uint32_t v = g.slots[b];
 #pragma unroll
-        for (int i = 0; i < kSplitMaxJobs; i++)
+        for (int i = 0; i < kSplitMaxTensors; i++)
             if (i < g.count && b >= g.first[i] && b < g.first[i + 1]) m[i] = max(m[i], v);
     }
 #pragma unroll
-    for (int i = 0; i < kSplitMaxJobs; i++) {
+    for (int i = 0; i < kSplitMaxTensors; i++) {
         m[i] = __reduce_max_sync(0xffffffffu, m[i]);
         if (threadIdx.x % 32 == 0 && m[i] != 0) atomicMax(&words[i], m[i]);
     }
     __syncthreads();
     bool out = g.pair_limit > 0 && !(__uint_as_float(words[g.pair[0]]) * __uint_as_float(words[g.pair[1]]) <= g.pair_limit);
-    for (int i = 0; i < g.count; i++) out = out || words[i] >= kSplitHuge || (words[i] != 0 && words[i] < kSplitTiny);
+    for (int i = 0; i < g.count; i++) out = out || words[i] >= (i == g.delta_at ? kSplitHugeDelta : kSplitHuge);
     if (blockIdx.x == 0 && threadIdx.x == 0) *g.fallback = out ? 1 : 0;
     return out;
 }
+
+// A power of two above a magnitude given as bits: its exponent.
+__device__ __forceinline__ int split_exponent(uint32_t bits) { return (int)(bits >> 23) - 126; }
 
 // The six products of parts, small ones first: (part of A, part of B) = (2, 0) (1, 1) (0, 2) (1, 0) (0, 1) (0, 0), 0 = high. A
 // loop and not straight code: with the four products of a backward step unrolled, issuing and computing warps together outgrew
@@ -94,7 +102,7 @@ __device__ __forceinline__ void split_pair(ptx::f32x2 v, uint32_t &hi, uint32_t 
 }
 #endif
 
-// One tensor to split: rows x cols float32, row-major -> three bf16 planes of rows x cols rounded up to 8 (zeros there), one
+// One tensor to split: rows x cols float32, row-major -> three bf16 planes (of 2^20 times its values) of rows x cols rounded up to 8 (zeros there), one
 // after the other. dst null: only looked through for values out of range.
 struct SplitJob {
     const float *src = nullptr;
@@ -113,7 +121,7 @@ struct SplitDelta {
 inline size_t split_plane_elems(long long rows, int cols) { return (size_t)rows * ((cols + 7) / 8 * 8); }
 inline size_t split_bytes(long long rows, int cols) { return align_up(3 * split_plane_elems(rows, cols) * 2, 256); }
 // scratch for the guard's words
-constexpr size_t kSplitGuardBytes = (kSplitMaxBlocks + 64) * 4;
+constexpr size_t kSplitGuardBytes = (2 * kSplitMaxBlocks + 64) * 4;
 
 // Splits up to four tensors in one launch. guard_mem: kSplitGuardBytes. Any alignment of src; dst 16-byte aligned.
 int split_f32(const SplitJob *jobs, int count, const SplitDelta *delta, void *guard_mem, SplitGuard *guard, cudaStream_t s);

@@ -140,6 +140,29 @@ def test_large_scores_leave_the_largest_a_weight_of_one(units, lq, lk, d, size):
     assert np.isfinite(dq).all() and np.isfinite(dk).all()
 
 
+@pytest.mark.parametrize("d", [64, 128, 40])
+def test_tiny_rows_keep_their_precision(d):
+    """A row of upstream gradients, one of values and a key whose every weight is about e^-85, far below the rest: each row of results that
+    they alone make by its own largest value. 2^-14 for the key: its scores' rounding errors, 85 * 2^-23 each, reach its weights."""
+    q, k, v, g = inputs(2, 520, 600, d)
+    g[1, 5] *= np.float32(2e-37)
+    q[:, :, 0], k[0, 9] = 4, 0
+    k[0, 9, 0] = -79 / (4 * d ** -0.5)
+    o, lse, dq, dk, dv = run(q, k, v, g, d ** -0.5, False)
+    ro, rl, rq, rk, rv = reference(q, k, v, g, d ** -0.5, False)
+    for a, b, rel in ((dq[1, 5], rq[1, 5], REL), (dv[0, 9], rv[0, 9], 2.0 ** -14), (o, ro, REL), (dk, rk, REL)):
+        assert np.abs(a - b).max() <= rel * np.abs(b).max()
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("sizes", [(1, 1, 1e-18, 1e-18), (1e-18, 1e15, 1e-10, 1e-20), (1, 1, 1e-30, 1e5), (1e6, 1e-7, 1e7, 1e7), (1, 1, 1, 1e-33)])
+def test_sizes_of_the_tensors(d, sizes):
+    """Score gradients near both ends of float32."""
+    q, k, v, g = (a * np.float32(s) for a, s in zip(inputs(2, 520, 600, d), sizes))
+    for a, b in zip(run(q, k, v, g, d ** -0.5, True), reference(q, k, v, g, d ** -0.5, True)):
+        assert np.abs(a - b).max() <= REL * np.abs(b).max() + 2.0 ** -140  # 2^9 of the smallest float32
+
+
 def test_zeros_stay_on_the_tensor_cores_and_give_means():
     q, k, v, g = inputs(2, 520, 600, 64)
     q[:] = 0

@@ -87,6 +87,27 @@ def test_tiny_values_keep_their_precision():
     check(520, 1000, 1024, x=seeded((520, 1024), 1) * np.float32(1e-33))
 
 
+def test_tiny_rows_and_columns_keep_their_precision():
+    """A row of x, one of g and a column of w far below the rest, down to where bf16 has no digits left: each result by its own largest value."""
+    for size in (1e-33, 1e-36, 1e-37):
+        x, w, g = seeded((520, 1024), 1), seeded((1024, 1000), 2), seeded((520, 1000), 3)
+        x[7] *= np.float32(size)
+        g[5] *= np.float32(size)
+        w[:, 11] *= np.float32(size)
+        y, gx, gw = (t.to_np() for t in (em.linear_forward(em.Tensor(x), em.Tensor(w), None), *em.linear_backward(em.Tensor(x), em.Tensor(w), em.Tensor(g), need_grad_b=False)[:2]))
+        x, w, g = (a.astype(np.float64) for a in (x, w, g))
+        for a, r in ((y[7], np.delete(x[7] @ w, 11)), (np.delete(y[:, 11], 7), np.delete(x, 7, 0) @ w[:, 11]), (gx[5], g[5] @ w.T), (gw, x.T @ g)):
+            a = np.delete(a, 11) if a.shape == (1000,) else a
+            assert np.abs(a - r).max() <= 1e-5 * np.abs(r).max()
+
+
+def test_small_products_keep_their_precision():
+    """Operands of 1e-18: their products are near the smallest float32, those of their parts below it."""
+    x, w = seeded((520, 1024), 1) * np.float32(1e-18), seeded((1024, 1000), 2) * np.float32(1e-18)
+    r = x.astype(np.float64) @ w.astype(np.float64)
+    assert np.abs(em.linear_forward(em.Tensor(x), em.Tensor(w), None).to_np() - r).max() <= 1e-5 * np.abs(r).max()
+
+
 def test_without_memory_for_the_planes():
     L = _lib.lib()
     L.ember_selftest_fail_scratch(2)
