@@ -34,7 +34,7 @@ constexpr float LOG2E_T = 1.4426950408889634f;
 constexpr int SUB = 64 * 128;          // 64 rows x 128 bytes: one TMA box
 constexpr int TN = 64;                 // rows of a streamed tile
 
-enum { WF_Q = 301, WF_K, WF_V, WF_S, WF_P, WF_O, WF_OFREE, WF_KEMPTY, WF_VEMPTY, WB_A, WB_B0, WB_B1, WB_S, WB_P, WB_DP, WB_DS, WB_ACC, WB_FREE, WB_E0, WB_E1 };
+enum { WF_Q = 301, WF_K, WF_V, WF_S, WF_P, WF_O, WF_OFREE, WF_KEMPTY, WF_VEMPTY, WB_A, WB_B0, WB_B1, WB_S, WB_P, WB_DP, WB_DS, WB_ACC, WB_FREE, WB_E0, WB_E1, WB_SMEM };
 
 __device__ __forceinline__ float exp_nat(float x) { return ex2(x * LOG2E_T); }
 
@@ -53,8 +53,8 @@ __device__ __forceinline__ f32x2 exp_pair(f32x2 x)
 }
 
 // Row `src` (d columns in memory; null: zeros), columns [col0, col0 + 32 * n32) -> the three parts in tensor memory, part q at
-// column taddr + q * plane.
-__device__ __forceinline__ void row_to_tmem(const float *src, int d, bool vec, int col0, int n32, uint32_t taddr, int plane)
+// column taddr + q * plane, or the low part (`low` given) in shared memory: row r of sub-tiles of 128 rows x 64 columns, as TMA would lay them.
+__device__ __forceinline__ void row_to_tmem(const float *src, int d, bool vec, int col0, int n32, uint32_t taddr, int plane, uint8_t *low, int r)
 {
     for (int h = 0; h < n32; h++) {
         const int c0 = col0 + h * 32;
@@ -81,14 +81,32 @@ __device__ __forceinline__ void row_to_tmem(const float *src, int d, bool vec, i
         const uint32_t t = taddr + (uint32_t)(c0 / 2);
         tmem_st_32x32b_x16(t, a);
         tmem_st_32x32b_x16(t + plane, b);
-        tmem_st_32x32b_x16(t + 2 * plane, c);
+        if (low) {
+            uint8_t *row = low + c0 / 64 * (2 * SUB) + r * 128;
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                *reinterpret_cast<uint4 *>(row + (((c0 % 64 / 8 + i) ^ (r & 7)) << 4)) = make_uint4(c[4 * i], c[4 * i + 1], c[4 * i + 2], c[4 * i + 3]);
+        } else {
+            tmem_st_32x32b_x16(t + 2 * plane, c);
+        }
     }
+    if (low) fence_proxy_async();
     tmem_wait_st();
 }
 
-// 32 values of a row -> their parts in tensor memory: 3 blocks of 16 columns from taddr, part by part. The A operand of 16 values
-// (one MMA) is 8 columns. UP: of 2^20 times the values.
-template <bool UP>
+// Scores, and the parts of what is made of them, share a region of tensor memory; of a tile's 64 columns each half may belong to
+// other threads, so the parts of one may not overwrite scores of the other. 32 values of a part are 16 columns, the A operand of one MMA (16
+// values) 8. One accumulator: 64 scores in columns [16, 80) of 96; the parts of half h in [48 h, 48 h + 48). TWO side by side (the first 64
+// columns of the contraction, and the others) in 128; the parts of half h in 16 columns each from 32 h, 32 h + 16 and 64 + 32 h.
+template <bool TWO>
+struct Region {
+    static constexpr int COLS = TWO ? 128 : 96, SCORES = TWO ? 0 : 16, HALF = TWO ? 32 : 48, LOW = TWO ? 64 : 32;
+    static __device__ __forceinline__ constexpr uint32_t step(int k16) { return (uint32_t)((k16 / 2) * HALF + (k16 % 2) * 8); }
+    static __device__ __forceinline__ uint32_t part(uint32_t q) { return q == 2 ? LOW : q * 16; }
+};
+
+// 32 values of a row -> their parts in tensor memory, in a half of a region. UP: of 2^20 times the values.
+template <typename R, bool UP>
 __device__ __forceinline__ void split_to_tmem(const f32x2 *v, uint32_t taddr)
 {
     uint32_t a[16], b[16], c[16];
@@ -96,82 +114,84 @@ __device__ __forceinline__ void split_to_tmem(const f32x2 *v, uint32_t taddr)
     for (int i = 0; i < 16; i++) split_pair(UP ? mul2(v[i], pack2(kSplitUp, kSplitUp)) : v[i], a[i], b[i], c[i]);
     tmem_st_32x32b_x16(taddr, a);
     tmem_st_32x32b_x16(taddr + 16, b);
-    tmem_st_32x32b_x16(taddr + 32, c);
+    tmem_st_32x32b_x16(taddr + R::LOW, c);
 }
 
-// Where such a block lies inside a region of 96 columns that held the 64 scores in columns [16, 80): the 32 scores of half h are in
-// [16 + 32 h, 48 + 32 h) and its parts go to [48 h, 48 h + 48), so that a half never overwrites scores of the other.
-constexpr int REGION = 96, SCORES_AT = 16;
-__device__ __forceinline__ constexpr uint32_t part_col(int part, int k16) { return (uint32_t)((k16 / 2) * 48 + part * 16 + (k16 % 2) * 8); }
+// 32 neighbouring scores of a row, as pairs. ADD: added to those that are there.
+template <bool ADD>
+__device__ __forceinline__ void load_scores(uint32_t taddr, f32x2 *s)
+{
+    uint32_t u[32];
+    tmem_ld_32x32b_x32(taddr, u);
+    tmem_wait_ld();
+#pragma unroll
+    for (int i = 0; i < 16; i++) {
+        const f32x2 x = pack2(__uint_as_float(u[2 * i]), __uint_as_float(u[2 * i + 1]));
+        s[i] = ADD ? add2(s[i], x) : x;
+    }
+}
 
-// A chain of four (or two) MMAs of 16 contraction steps, A in tensor memory (AO* columns further each) or in shared memory (AO* in
+// A chain of four or (four == 0) two MMAs of 16 contraction steps, A in tensor memory (AO* columns further each) or in shared memory (AO* in
 // units of 16 bytes), B BO* further each. Products of parts are short MMAs (64 columns: 32 clocks), so what one costs to issue
 // decides: `elected` is taken once per tile and four MMAs make one asm block (an elect.sync and a branch on the
-// number of steps for each took 85 clocks an MMA).
+// number of steps for each took 85 clocks an MMA), and the last two are predicated off where two do (a second asm block for that: 4 us
+// of the forward's 37 at 16 units x L1024 d 64).
 #define EMBER_CHAIN_HEAD "{\n.reg .pred p, q;\n.reg .b64 da, db;\n.reg .b32 t, u;\nsetp.ne.b32 q, %4, 0;\nsetp.ne.b32 p, %5, 0;\n"
+#define EMBER_CHAIN_REST "setp.ne.and.b32 q, %13, 0, q;\n"
 template <int A1, int A2, int A3, int B1, int B2, int B3>
-__device__ __forceinline__ void chain_ts(uint32_t d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t elected, uint32_t acc, bool four)
+__device__ __forceinline__ void chain_ts(uint32_t d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t elected, uint32_t acc, uint32_t four)
 {
-    if (four)
-        asm volatile(EMBER_CHAIN_HEAD
-                     "mov.b64 db, {%2, %6};\n@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, p;\nsetp.eq.u32 p, 0, 0;\n"
-                     "add.u32 t, %2, %10;\nadd.u32 u, %1, %7;\nmov.b64 db, {t, %6};\n@q tcgen05.mma.cta_group::1.kind::f16 [%0], [u], db, %3, p;\n"
-                     "add.u32 t, %2, %11;\nadd.u32 u, %1, %8;\nmov.b64 db, {t, %6};\n@q tcgen05.mma.cta_group::1.kind::f16 [%0], [u], db, %3, p;\n"
-                     "add.u32 t, %2, %12;\nadd.u32 u, %1, %9;\nmov.b64 db, {t, %6};\n@q tcgen05.mma.cta_group::1.kind::f16 [%0], [u], db, %3, p;\n}\n"
-                     ::"r"(d), "r"(a), "r"(b), "r"(idesc), "r"(elected), "r"(acc), "r"(kDescHiSw128), "n"(A1), "n"(A2), "n"(A3), "n"(B1), "n"(B2), "n"(B3) : "memory");
-    else
-        asm volatile(EMBER_CHAIN_HEAD
-                     "mov.b64 db, {%2, %6};\n@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, p;\nsetp.eq.u32 p, 0, 0;\n"
-                     "add.u32 t, %2, %8;\nadd.u32 u, %1, %7;\nmov.b64 db, {t, %6};\n@q tcgen05.mma.cta_group::1.kind::f16 [%0], [u], db, %3, p;\n}\n"
-                     ::"r"(d), "r"(a), "r"(b), "r"(idesc), "r"(elected), "r"(acc), "r"(kDescHiSw128), "n"(A1), "n"(B1) : "memory");
+    asm volatile(EMBER_CHAIN_HEAD
+                 "mov.b64 db, {%2, %6};\n@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, p;\nsetp.eq.u32 p, 0, 0;\n"
+                 "add.u32 t, %2, %10;\nadd.u32 u, %1, %7;\nmov.b64 db, {t, %6};\n@q tcgen05.mma.cta_group::1.kind::f16 [%0], [u], db, %3, p;\n" EMBER_CHAIN_REST
+                 "add.u32 t, %2, %11;\nadd.u32 u, %1, %8;\nmov.b64 db, {t, %6};\n@q tcgen05.mma.cta_group::1.kind::f16 [%0], [u], db, %3, p;\n"
+                 "add.u32 t, %2, %12;\nadd.u32 u, %1, %9;\nmov.b64 db, {t, %6};\n@q tcgen05.mma.cta_group::1.kind::f16 [%0], [u], db, %3, p;\n}\n"
+                 ::"r"(d), "r"(a), "r"(b), "r"(idesc), "r"(elected), "r"(acc), "r"(kDescHiSw128), "n"(A1), "n"(A2), "n"(A3), "n"(B1), "n"(B2), "n"(B3), "r"(four) : "memory");
 }
 template <int A1, int A2, int A3, int B1, int B2, int B3>
-__device__ __forceinline__ void chain_ss(uint32_t d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t elected, uint32_t acc, bool four)
+__device__ __forceinline__ void chain_ss(uint32_t d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t elected, uint32_t acc, uint32_t four)
 {
-    if (four)
-        asm volatile(EMBER_CHAIN_HEAD
-                     "mov.b64 db, {%2, %6};\nmov.b64 da, {%1, %6};\n@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\nsetp.eq.u32 p, 0, 0;\n"
-                     "add.u32 t, %2, %10;\nadd.u32 u, %1, %7;\nmov.b64 db, {t, %6};\nmov.b64 da, {u, %6};\n@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n"
-                     "add.u32 t, %2, %11;\nadd.u32 u, %1, %8;\nmov.b64 db, {t, %6};\nmov.b64 da, {u, %6};\n@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n"
-                     "add.u32 t, %2, %12;\nadd.u32 u, %1, %9;\nmov.b64 db, {t, %6};\nmov.b64 da, {u, %6};\n@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n}\n"
-                     ::"r"(d), "r"(a), "r"(b), "r"(idesc), "r"(elected), "r"(acc), "r"(kDescHiSw128), "n"(A1), "n"(A2), "n"(A3), "n"(B1), "n"(B2), "n"(B3) : "memory");
-    else
-        asm volatile(EMBER_CHAIN_HEAD
-                     "mov.b64 db, {%2, %6};\nmov.b64 da, {%1, %6};\n@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\nsetp.eq.u32 p, 0, 0;\n"
-                     "add.u32 t, %2, %8;\nadd.u32 u, %1, %7;\nmov.b64 db, {t, %6};\nmov.b64 da, {u, %6};\n@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n}\n"
-                     ::"r"(d), "r"(a), "r"(b), "r"(idesc), "r"(elected), "r"(acc), "r"(kDescHiSw128), "n"(A1), "n"(B1) : "memory");
+    asm volatile(EMBER_CHAIN_HEAD
+                 "mov.b64 db, {%2, %6};\nmov.b64 da, {%1, %6};\n@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\nsetp.eq.u32 p, 0, 0;\n"
+                 "add.u32 t, %2, %10;\nadd.u32 u, %1, %7;\nmov.b64 db, {t, %6};\nmov.b64 da, {u, %6};\n@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n" EMBER_CHAIN_REST
+                 "add.u32 t, %2, %11;\nadd.u32 u, %1, %8;\nmov.b64 db, {t, %6};\nmov.b64 da, {u, %6};\n@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n"
+                 "add.u32 t, %2, %12;\nadd.u32 u, %1, %9;\nmov.b64 db, {t, %6};\nmov.b64 da, {u, %6};\n@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n}\n"
+                 ::"r"(d), "r"(a), "r"(b), "r"(idesc), "r"(elected), "r"(acc), "r"(kDescHiSw128), "n"(A1), "n"(A2), "n"(A3), "n"(B1), "n"(B2), "n"(B3), "r"(four) : "memory");
 }
 
-// Scores: D (128 x 64) = A * B^T (a tile of 64 rows, HD columns, planes PLANE bytes apart). A in tensor memory, parts HD / 2
-// columns apart, or in shared memory (SS): 128 rows, planes 2 * PLANE bytes apart, 64-column sub-tiles 2 * SUB. The contraction
+// Scores: D (128 x 64) = A * B^T over the 64-column sub-tiles [sub0, sub1) of the contraction, each into 64 columns of its own: an
+// accumulator collects no more (128 terms of one sign lost 1.9e-7 of their sum to the truncation, in two accumulators 1.1e-7). B: a
+// tile of 64 rows, planes PLANE bytes apart. A: A_TMEM tensor memory, parts HD / 2 columns apart; A_LOW the same, but the low part in
+// shared memory at low_smem; A_SMEM all of it in shared memory: 128 rows, planes 2 * PLANE bytes apart, sub-tiles 2 * SUB. The contraction
 // stops at the end of the 32 columns that hold the last of d (zeros past d). `mirrored`: the tile is the queries' and A the keys'.
-template <int HD, bool SS>
-__device__ __forceinline__ void mma_scores(uint32_t d, uint32_t a, uint32_t b_smem, int ksteps, uint32_t elected, bool mirrored)
+enum AKind { A_TMEM, A_LOW, A_SMEM };
+template <int HD, AKind KIND>
+__device__ __forceinline__ void mma_scores(uint32_t d, uint32_t a, uint32_t low_smem, uint32_t b_smem, int sub0, int sub1, int ksteps, uint32_t elected, bool mirrored)
 {
     constexpr uint32_t IDESC = idesc_bf16_f32(128, TN, 0, 0);
     constexpr int PLANE = HD / 64 * SUB;
-    const uint32_t b_lo = desc_lo(b_smem, 16), a_lo = SS ? desc_lo(a, 16) : a;
+    const uint32_t b_lo = desc_lo(b_smem, 16), a_lo = KIND == A_SMEM ? desc_lo(a, 16) : a, low = desc_lo(low_smem, 16);
 #pragma unroll 1
     for (int i = 0; i < kSplitProducts; i++) {
+        const uint32_t pa = split_part_a(i, mirrored), b = b_lo + split_part_b(i, mirrored) * (PLANE >> 4);
 #pragma unroll
-        for (int sub = 0; sub < HD / 64; sub++) {
-            const uint32_t acc = i > 0 || sub > 0, pa = split_part_a(i, mirrored), b = b_lo + split_part_b(i, mirrored) * (PLANE >> 4) + ((sub * SUB) >> 4);
-            const bool four = ksteps - sub * 4 > 2;
-            if (SS) chain_ss<2, 4, 6, 2, 4, 6>(d, a_lo + pa * ((2 * PLANE) >> 4) + ((sub * 2 * SUB) >> 4), b, IDESC, elected, acc, four);
-            else chain_ts<8, 16, 24, 2, 4, 6>(d, a_lo + pa * (HD / 2) + sub * 32, b, IDESC, elected, acc, four);
+        for (int sub = sub0; sub < sub1; sub++) {
+            const uint32_t at = d + (sub - sub0) * 64, four = ksteps - sub * 4 > 2, bs = b + ((sub * SUB) >> 4);
+            if (KIND == A_SMEM) chain_ss<2, 4, 6, 2, 4, 6>(at, a_lo + pa * ((2 * PLANE) >> 4) + ((sub * 2 * SUB) >> 4), bs, IDESC, elected, i > 0, four);
+            else if (KIND == A_LOW && pa == 2) chain_ss<2, 4, 6, 2, 4, 6>(at, low + ((sub * 2 * SUB) >> 4), bs, IDESC, elected, i > 0, four);
+            else chain_ts<8, 16, 24, 2, 4, 6>(at, a_lo + pa * (HD / 2) + sub * 32, bs, IDESC, elected, i > 0, four);
         }
     }
 }
 // Results: D (128 x n) = P (parts in a region of tensor memory, 64 columns of the product) * B (the tile's 64 rows x n columns).
-template <int HD>
+template <int HD, typename R>
 __device__ __forceinline__ void mma_results(uint32_t d, uint32_t region, uint32_t b_smem, uint32_t idesc, uint32_t elected)
 {
     constexpr int PLANE = HD / 64 * SUB;
     const uint32_t b_lo = desc_lo(b_smem, SUB);
 #pragma unroll 1
     for (int i = 0; i < kSplitProducts; i++)
-        chain_ts<part_col(0, 1), part_col(0, 2), part_col(0, 3), 128, 256, 384>(d, region + split_part_a(i) * part_col(1, 0), b_lo + split_part_b(i) * (PLANE >> 4), idesc, elected,
-                                                                                i > 0, true);
+        chain_ts<R::step(1), R::step(2), R::step(3), 128, 256, 384>(d, region + R::part(split_part_a(i)), b_lo + split_part_b(i) * (PLANE >> 4), idesc, elected, i > 0, true);
 }
 
 // Loads a 64-row tile's three planes.
@@ -239,10 +259,13 @@ struct F32FwdCfg {
     static constexpr int OFF_K = 0, OFF_V = KST * TILE, OFF_BAR = OFF_V + VST * TILE;
     static constexpr int USED = OFF_BAR + 256, SMEM = USED + 1024;
     // HD 64: one score buffer, read out at once, apart from the probabilities, and a partial output for each warpgroup, added up a
-    // turn later. HD 128: scores under the probabilities, one partial output, added up before the next one's product.
+    // turn later. HD 128: scores under the probabilities, formed and read in two halves of the contraction one after the other (side
+    // by side they fit only with the queries' low part in shared memory, and a product with that, between others, held a tile up for 800
+    // clocks: 1 x 32 x 2048, 87 us against 81), one partial output, added up before the next one's product.
     static constexpr bool LATE = HD == 64;
-    static constexpr int T_Q = 0, T_S = 3 * HD / 2 + (LATE ? 0 : SCORES_AT), S_STEP = LATE ? 0 : REGION;
-    static constexpr int T_P = LATE ? 3 * HD / 2 + TN : 3 * HD / 2, T_O = T_P + 2 * REGION, O_STEP = LATE ? HD : 0;
+    using R = Region<false>;
+    static constexpr int T_Q = 0, T_S = 3 * HD / 2 + (LATE ? 0 : R::SCORES), T_P = 3 * HD / 2 + (LATE ? TN : 0), S_STEP = LATE ? 0 : R::COLS;
+    static constexpr int T_O = T_P + 2 * R::COLS, O_STEP = LATE ? HD : 0;
     static_assert(T_O + HD + O_STEP <= 512, "");
     enum { B_Q, B_KFULL, B_KEMPTY = B_KFULL + KST, B_VFULL = B_KEMPTY + KST, B_VEMPTY = B_VFULL + VST, B_S = B_VEMPTY + VST, B_P = B_S + 2, B_O = B_P + 2, B_OFREE = B_O + 2, B_SREAD = B_OFREE + 2, NUM_BARS };
 };
@@ -341,8 +364,14 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
                 if (C::LATE && j > 0) ok = ok && mbar_wait(BAR(C::B_SREAD), (j - 1) & 1, abort_flag, p.status, WF_P);
                 if (!C::LATE && j > 1) ok = ok && mbar_wait(BAR(C::B_O + w), ((j - 2) >> 1) & 1, abort_flag, p.status, WF_P);
                 tc_fence_after();
-                mma_scores<HD, false>(tmem + C::T_S + w * C::S_STEP, tmem + C::T_Q, smem_base + C::OFF_K + (j % C::KST) * C::TILE, ksteps, elected, false);
-                tc_commit_elect(BAR(C::B_S + w));
+                for (int sub = 0; sub < HD / 64 && ok; sub++) {
+                    if (sub > 0) {
+                        ok = mbar_wait(BAR(C::B_SREAD), j & 1, abort_flag, p.status, WF_P);
+                        tc_fence_after();
+                    }
+                    mma_scores<HD, A_TMEM>(tmem + C::T_S + w * C::S_STEP, tmem + C::T_Q, 0, smem_base + C::OFF_K + (j % C::KST) * C::TILE, sub, sub + 1, ksteps, elected, false);
+                    tc_commit_elect(BAR(C::B_S + w));
+                }
                 tc_commit_elect(BAR(C::B_KEMPTY + j % C::KST));
             }
         } else if (warp == 10) {
@@ -357,7 +386,7 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
                 // the partial output has been added up (LATE: this warpgroup did so before it wrote its probabilities)
                 if (!C::LATE && j > 0) ok = ok && mbar_wait(BAR(C::B_OFREE + (w ^ 1)), ((j - 1) >> 1) & 1, abort_flag, p.status, WF_OFREE);
                 tc_fence_after();
-                mma_results<HD>(tmem + C::T_O + w * C::O_STEP, tmem + C::T_P + w * REGION, smem_base + C::OFF_V + (j % C::VST) * C::TILE, idesc_o, elected);
+                mma_results<HD, typename C::R>(tmem + C::T_O + w * C::O_STEP, tmem + C::T_P + w * C::R::COLS, smem_base + C::OFF_V + (j % C::VST) * C::TILE, idesc_o, elected);
                 tc_commit_elect(BAR(C::B_O + w));
                 tc_commit_elect(BAR(C::B_VEMPTY + j % C::VST));
             }
@@ -368,12 +397,12 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
         const int w = warp / 4, r = threadIdx.x % 128, row = q0 + r;
         const uint32_t lane_sel = (uint32_t)((warp % 4) * 32) << 16;
         const float *src = row < p.lq ? p.q + ((size_t)unit * p.lq + row) * p.d : nullptr;
-        row_to_tmem(src, p.d, p.vec_q, w * (HD / 2), HD / 64, tmem + lane_sel + C::T_Q, HD / 2);
+        row_to_tmem(src, p.d, p.vec_q, w * (HD / 2), HD / 64, tmem + lane_sel + C::T_Q, HD / 2, nullptr, r);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(BAR(C::B_Q));
 
-        const uint32_t scores = tmem + lane_sel + C::T_S + w * C::S_STEP, region = tmem + lane_sel + C::T_P + w * REGION, to = tmem + lane_sel + C::T_O + w * C::O_STEP;
+        const uint32_t scores = tmem + lane_sel + C::T_S + w * C::S_STEP, region = tmem + lane_sel + C::T_P + w * C::R::COLS, to = tmem + lane_sel + C::T_O + w * C::O_STEP;
         const int limit_row = p.causal ? min(p.lk - 1, row + off) : p.lk - 1;
         const int limit_tile = p.causal ? min(p.lk - 1, q0 + off) : p.lk - 1;
         const int cols = (p.d + 15) / 16 * 16;
@@ -386,25 +415,22 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
         bool ok = true;
         for (int j = w; j < n && ok; j += 2) {
             const int k0 = j * TN;
-            ok = ok && mbar_wait(BAR(C::B_S + w), (j >> 1) & 1, abort_flag, p.status, WF_S);
+            ok = ok && mbar_wait(BAR(C::B_S + w), C::LATE ? (j >> 1) & 1 : 0, abort_flag, p.status, WF_S);
             tc_fence_after();
             f32x2 s[32];
-            {
-                uint32_t u[32], v[32];
-                tmem_ld_32x32b_x32(scores, u);
-                tmem_ld_32x32b_x32(scores + 32, v);
-                tmem_wait_ld();
+            load_scores<false>(scores, s);
+            load_scores<false>(scores + 32, s + 16);
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(BAR(C::B_SREAD));
+            if (!C::LATE) {  // the other half of the contraction
+                ok = ok && mbar_wait(BAR(C::B_S + w), 1, abort_flag, p.status, WF_S);
+                tc_fence_after();
+                load_scores<true>(scores, s);
+                load_scores<true>(scores + 32, s + 16);
+            }
 #pragma unroll
-                for (int i = 0; i < 16; i++) {
-                    s[i] = mul2(pack2(__uint_as_float(u[2 * i]), __uint_as_float(u[2 * i + 1])), scale2);
-                    s[16 + i] = mul2(pack2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])), scale2);
-                }
-            }
-            if (C::LATE) {
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(BAR(C::B_SREAD));
-            }
+            for (int i = 0; i < 32; i++) s[i] = mul2(s[i], scale2);
             if (k0 + TN - 1 > limit_tile) {
 #pragma unroll
                 for (int i = 0; i < 32; i++) {
@@ -440,7 +466,7 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
                     tc_fence_after();
                     flush<HD / 32, true>(o, to, cols, late_alpha);
                 }
-                split_to_tmem<true>(s + h * 16, region + h * 48);
+                split_to_tmem<typename C::R, true>(s + h * 16, region + h * C::R::HALF);
             }
             tmem_wait_st();
             tc_fence_before();
@@ -530,13 +556,17 @@ struct F32BwdCfg {
     // A ring of 3 pairs of tiles beside A1 (HD 64), one pair (HD 128), or (DV, which needs no A1) 2.
     static constexpr int MAXST = HD == 64 ? 3 : 2, STAGES = HD == 64 ? 3 : 1;
     static constexpr int OFF_B = 0, OFF_A1 = STAGES * 2 * TILE;    // TILE pairs, A1
-    static constexpr int OFF_VEC = OFF_A1 + A_BYTES;               // per warp: 32 log-sum-exps, 32 deltas
-    static constexpr int OFF_BAR = OFF_VEC + 8 * 256, USED = OFF_BAR + 256, SMEM = USED + 1024;
-    static_assert(HD == 64 || OFF_VEC == MAXST * 2 * TILE, "");
+    static constexpr int OFF_LOW = OFF_A1 + A_BYTES;               // HD 128: the low parts of A0
+    static constexpr int OFF_VEC = OFF_LOW + (HD == 64 ? 0 : 4 * SUB);  // per warp: 32 log-sum-exps, 32 deltas
+    static constexpr int OFF_BAR = OFF_VEC + 8 * 256, USED = OFF_BAR + 256;
+    static constexpr int SMEM = HD == 64 ? USED + 1024 : 232448;   // 128: the base is checked in the kernel
+    static_assert(HD == 64 || OFF_LOW == MAXST * 2 * TILE, "");
     // Columns. HD 64: A0, S, P, dP / dS, two results; S is apart from P, so that the next S does not wait for the product of P
     // (with A1 in tensor memory and S under P a tile took 5700 clocks). HD 128: A0, S, dP / dS, result; DV: A0, two regions
-    // of S / P, result.
-    static constexpr int T_A0 = 0, T_S = 3 * HD / 2 + (HD == 64 ? 0 : SCORES_AT), T_P = HD == 64 ? 160 : 192, T_D = HD == 64 ? 256 : 288, T_R = HD == 64 ? 352 : 384;
+    // of S / P, result; two accumulators of S and dP each leave no room for A0's low part, which lies in shared memory (the products of
+    // both halves with a part of A come one after the other: 16 x 1024 x 2048 d 128 488 us, half after half 507).
+    using R = Region<HD == 128>;
+    static constexpr int T_A0 = 0, T_S = HD == 64 ? 96 : 128, T_P = HD == 64 ? 160 : 128, T_D = 256, T_R = T_D + R::COLS;
     enum { B_A, B_FULL0, B_FULL1 = B_FULL0 + MAXST, B_EMPTY0 = B_FULL1 + MAXST, B_EMPTY1 = B_EMPTY0 + MAXST, B_S = B_EMPTY1 + MAXST, B_P, B_DP, B_DS, B_R0, B_R1, B_F0, B_F1, NUM_BARS,
            B_S1 = B_DP };  // DV: scores of odd tiles (the next tile's may be there before this one's have been waited for)
     static_assert(8 * NUM_BARS + 8 + 4 * kSplitMaxTensors <= 256, "");
@@ -583,9 +613,21 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
                          const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do, const F32BwdParams p)
 {
     using C = F32BwdCfg<HD>;
-    extern __shared__ uint8_t smem_raw[];
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t *smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
+    if (HD == 128) {  // every thread takes the same decision, before any barrier exists
+        uint32_t dyn;
+        asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn));
+        if (smem_base + C::USED > smem_u32(smem_raw) + dyn) {
+            if (threadIdx.x == 0 && atomicCAS(&p.status->code, 0, EMBER_ERR_UNSUPPORTED) == 0) {
+                p.status->where = WB_SMEM;
+                p.status->block = blockIdx.x;
+                p.status->extra = (int)(smem_base - smem_u32(smem_raw));
+            }
+            return;
+        }
+    }
     const uint32_t bar0 = smem_base + C::OFF_BAR;
     auto BAR = [&](int i) { return bar0 + 8u * (uint32_t)i; };
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem_gen + C::OFF_BAR + 8 * C::NUM_BARS);
@@ -692,14 +734,14 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
                 int done = C::B_S;
                 wait(C::B_FULL0 + s, j / stages, WB_B0);
                 if (role == R_DV) {  // two regions in turn
-                    at += (j & 1) * REGION;
+                    at += (j & 1) * C::R::COLS;
                     done = j & 1 ? C::B_S1 : C::B_S;
                     if (j > 1) wait(j & 1 ? C::B_R1 : C::B_R0, (j - 2) >> 1, WB_ACC);
                 } else if (j > 0) {
                     wait(C::B_P, j - 1, WB_ACC);
                 }
                 tc_fence_after();
-                mma_scores<HD, false>(at, tmem + C::T_A0, b0, ksteps, elected, !is_q);  // the forward's scores, bit for bit
+                mma_scores<HD, HD == 64 ? A_TMEM : A_LOW>(at, tmem + C::T_A0, smem_base + C::OFF_LOW, b0, 0, HD / 64, ksteps, elected, !is_q);  // the forward's scores, bit for bit
                 tc_commit_elect(BAR(done));
                 if (!has_ds) {
                     tc_commit_elect(BAR(C::B_EMPTY0 + s));
@@ -708,7 +750,7 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
                 wait(C::B_FULL1 + s, j / stages, WB_B1);
                 if (j > 0) wait(role == R_DKDV ? C::B_R1 : C::B_R0, j - 1, WB_ACC);  // over dS
                 tc_fence_after();
-                mma_scores<HD, true>(t_d + SCORES_AT, smem_base + C::OFF_A1, b0 + C::TILE, ksteps, elected, false);
+                mma_scores<HD, A_SMEM>(t_d + C::R::SCORES, smem_base + C::OFF_A1, 0, b0 + C::TILE, 0, HD / 64, ksteps, elected, false);
                 tc_commit_elect(BAR(C::B_DP));
                 tc_commit_elect(BAR(C::B_EMPTY1 + s));
             }
@@ -726,7 +768,7 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
                     wait(C::B_FULL1 + s, j / stages, WB_B1);
                     if (j > 0) wait(C::B_F0, j - 1, WB_FREE);
                     tc_fence_after();
-                    mma_results<HD>(t_r, t_p + (role == R_DV ? (j & 1) * REGION : 0), b0 + C::TILE, idesc_r, elected);
+                    mma_results<HD, typename C::R>(t_r, t_p + (role == R_DV ? (j & 1) * C::R::COLS : 0), b0 + C::TILE, idesc_r, elected);
                     tc_commit_elect(BAR(role == R_DV && (j & 1) ? C::B_R1 : C::B_R0));
                     tc_commit_elect(BAR(C::B_EMPTY1 + s));
                 }
@@ -735,7 +777,7 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
                     wait(C::B_FULL0 + s, j / stages, WB_B0);
                     if (j > 0) wait(role == R_DKDV ? C::B_F1 : C::B_F0, j - 1, WB_FREE);
                     tc_fence_after();
-                    mma_results<HD>(t_r + (role == R_DKDV ? 64 : 0), t_d, b0, idesc_r, elected);
+                    mma_results<HD, typename C::R>(t_r + (role == R_DKDV ? 64 : 0), t_d, b0, idesc_r, elected);
                     tc_commit_elect(BAR(role == R_DKDV ? C::B_R1 : C::B_R0));
                     tc_commit_elect(BAR(C::B_EMPTY0 + s));
                 }
@@ -749,7 +791,7 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
         const int rows = is_q ? p.lq : p.lk;
         const float *a0 = is_q ? p.q : p.k;
         const size_t row_at = ((size_t)unit * rows + row) * p.d;
-        row_to_tmem(row < rows ? a0 + row_at : nullptr, p.d, p.vec_in, w * (HD / 2), HD / 64, tmem + lane_sel + C::T_A0, HD / 2);
+        row_to_tmem(row < rows ? a0 + row_at : nullptr, p.d, p.vec_in, w * (HD / 2), HD / 64, tmem + lane_sel + C::T_A0, HD / 2, HD == 64 ? nullptr : smem_gen + C::OFF_LOW, r);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(BAR(C::B_A));
@@ -811,17 +853,16 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
             if (role == R_DV) ok = ok && mbar_wait(BAR(j & 1 ? C::B_S1 : C::B_S), (j >> 1) & 1, abort_flag, p.status, WB_S);
             else ok = ok && mbar_wait(BAR(C::B_S), j & 1, abort_flag, p.status, WB_S);
             tc_fence_after();
-            const uint32_t turn = lane_sel + (role == R_DV ? (j & 1) * REGION : 0);
+            const uint32_t turn = lane_sel + (role == R_DV ? (j & 1) * C::R::COLS : 0);
             f32x2 e[16];
             {
-                uint32_t u[32];
-                tmem_ld_32x32b_x32(t_s + turn + w * 32, u);
-                tmem_wait_ld();
+                load_scores<false>(t_s + turn + w * 32, e);
+                if (HD == 128) load_scores<true>(t_s + turn + 64 + w * 32, e);
 #pragma unroll
                 for (int i = 0; i < 16; i += 2) {
                     const ulonglong2 nl = is_q ? make_ulonglong2(pack2(nl_row, nl_row), pack2(nl_row, nl_row)) : *reinterpret_cast<const ulonglong2 *>(vec + i * 2);
-                    e[i] = exp_pair(fma2(pack2(__uint_as_float(u[2 * i]), __uint_as_float(u[2 * i + 1])), scale2, nl.x));
-                    e[i + 1] = exp_pair(fma2(pack2(__uint_as_float(u[2 * i + 2]), __uint_as_float(u[2 * i + 3])), scale2, nl.y));
+                    e[i] = exp_pair(fma2(e[i], scale2, nl.x));
+                    e[i + 1] = exp_pair(fma2(e[i + 1], scale2, nl.y));
                 }
                 if (edge) {
 #pragma unroll
@@ -838,7 +879,7 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
                     ok = ok && mbar_wait(BAR(C::B_R0), (j - 1) & 1, abort_flag, p.status, WB_ACC);
                     tc_fence_after();
                 }
-                split_to_tmem<true>(e, t_p + turn + w * 48);
+                split_to_tmem<typename C::R, true>(e, t_p + turn + w * C::R::HALF);
                 tmem_wait_st();
             }
             tc_fence_before();
@@ -848,16 +889,16 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
             if (has_ds) {
                 ok = ok && mbar_wait(BAR(C::B_DP), j & 1, abort_flag, p.status, WB_DP);
                 tc_fence_after();
-                uint32_t u[32];
-                tmem_ld_32x32b_x32(t_d + lane_sel + SCORES_AT + w * 32, u);
-                tmem_wait_ld();
+                f32x2 dp[16];
+                load_scores<false>(t_d + lane_sel + C::R::SCORES + w * 32, dp);
+                if (HD == 128) load_scores<true>(t_d + lane_sel + 64 + w * 32, dp);
 #pragma unroll
                 for (int i = 0; i < 16; i += 2) {
                     const ulonglong2 nd = is_q ? make_ulonglong2(pack2(nd_row, nd_row), pack2(nd_row, nd_row)) : *reinterpret_cast<const ulonglong2 *>(vec + 32 + i * 2);
-                    e[i] = mul2(e[i], fma2(pack2(__uint_as_float(u[2 * i]), __uint_as_float(u[2 * i + 1])), dp_scale2, nd.x));
-                    e[i + 1] = mul2(e[i + 1], fma2(pack2(__uint_as_float(u[2 * i + 2]), __uint_as_float(u[2 * i + 3])), dp_scale2, nd.y));
+                    e[i] = mul2(e[i], fma2(dp[i], dp_scale2, nd.x));
+                    e[i + 1] = mul2(e[i + 1], fma2(dp[i + 1], dp_scale2, nd.y));
                 }
-                split_to_tmem<false>(e, t_d + lane_sel + w * 48);
+                split_to_tmem<typename C::R, false>(e, t_d + lane_sel + w * C::R::HALF);
                 tmem_wait_st();
                 tc_fence_before();
                 __syncwarp();
