@@ -44,6 +44,30 @@ MatView view(const void *p, long long rows, int cols, int heads, const LinearSha
     return v;
 }
 
+// The three products of a layer: y (m x n) = x w, grad_w (k x n) = x^T dy, grad_x (m x k) = dy w^T.
+enum { FORWARD = 0, GRAD_W = 1, GRAD_X = 2 };
+
+GemmArgs product_of(int product, const LinearShape &s, const void *x, const void *w, const void *y_or_dy, const void *out)
+{
+    const MatView vx = view(x, s.m, s.k, s.x_heads, s), vw = view(w, s.k, s.n, 0, s), vdy = view(y_or_dy, s.m, s.n, s.y_heads, s);
+    GemmArgs g;
+    g.dtype = s.dtype;
+    if (product == GRAD_W) {
+        g.mode = GEMM_TN;
+        g.a = vx; g.b = vdy; g.c = view(out, s.k, s.n, 0, s);
+        g.m = s.k; g.n = s.n; g.k = (int)s.m;
+    } else if (product == GRAD_X) {
+        g.mode = GEMM_NT;
+        g.a = vdy; g.b = vw; g.c = view(out, s.m, s.k, s.x_heads, s);
+        g.m = s.m; g.n = s.k; g.k = s.n;
+    } else {
+        g.mode = GEMM_NN;
+        g.a = vx; g.b = vw; g.c = vdy;
+        g.m = s.m; g.n = s.n; g.k = s.k;
+    }
+    return g;
+}
+
 // Copies of operands whose rows are no multiple of 16 bytes (a vocabulary of 50257 columns, say), padded with
 // zeros to rows that the copy engine can fetch. They live for one entry point's call, so that the two
 // gradients of a backward call share the copy of dy, and are freed in stream order.
@@ -229,13 +253,8 @@ int ember_linear_fwd(const void *x, const void *w, const void *bias, void *y, lo
     EMBER_REQUIRE(x && w && y, "ember_linear_fwd: NULL tensor pointer");
     DeviceState *st = device_state();
     if (!st) return EMBER_ERR_CUDA;
-    GemmArgs g;
-    g.mode = GEMM_NN;
-    g.a = view(x, m, k, x_heads, sh);
-    g.b = view(w, k, n, 0, sh);
-    g.c = view(y, m, n, y_heads, sh);
+    GemmArgs g = product_of(FORWARD, sh, x, w, y, nullptr);
     g.bias = bias;
-    g.m = m; g.n = n; g.k = k; g.dtype = dtype;
     PackedOperands packed(pick_stream(stream, st));
     F32Products f32;
     if (dtype == EMBER_F32 && !skinny_f32_supported(g)) f32.add(g);
@@ -256,18 +275,7 @@ int ember_linear_bwd(const void *x, const void *w, const void *dy, void *dx, voi
     if (!st) return EMBER_ERR_CUDA;
     cudaStream_t s = pick_stream(stream, st);
     PackedOperands packed(s);
-    const MatView vx = view(x, m, k, x_heads, sh), vdy = view(dy, m, n, y_heads, sh);
-    GemmArgs gw, gx;
-    gw.mode = GEMM_TN;  // grad_w (k x n) = x^T dy
-    gw.a = vx;
-    gw.b = vdy;
-    gw.c = view(dw, k, n, 0, sh);
-    gw.m = k; gw.n = n; gw.k = (int)m; gw.dtype = dtype;
-    gx.mode = GEMM_NT;  // grad_x (m x k) = dy w^T
-    gx.a = vdy;
-    gx.b = view(w, k, n, 0, sh);
-    gx.c = view(dx, m, k, x_heads, sh);
-    gx.m = m; gx.n = k; gx.k = n; gx.dtype = dtype;
+    const GemmArgs gw = product_of(GRAD_W, sh, x, w, dy, dw), gx = product_of(GRAD_X, sh, x, w, dy, dx);
     F32Products f32;
     if (dtype == EMBER_F32 && dw) f32.add(gw);
     if (dtype == EMBER_F32 && dx) f32.add(gx);
@@ -277,7 +285,7 @@ int ember_linear_bwd(const void *x, const void *w, const void *dy, void *dx, voi
         done = rc == EMBER_OK;
     }
     if (!done && dw && (rc = run(gw, st, s, packed)) != EMBER_OK) return rc;
-    if (db && (rc = column_sums(vdy, db, dtype, st, s)) != EMBER_OK) return rc;  // grad_b = sum(dy, axis 0)
+    if (db && (rc = column_sums(gw.b, db, dtype, st, s)) != EMBER_OK) return rc;  // grad_b = sum(dy, axis 0)
     if (!done && dx && (rc = run(gx, st, s, packed)) != EMBER_OK) return rc;
     return EMBER_OK;
 }
@@ -285,24 +293,25 @@ int ember_linear_bwd(const void *x, const void *w, const void *dy, void *dx, voi
 const char *ember_linear_kernel_name(int product, long long m, int n, int k, int dtype, int x_heads, int y_heads,
                                      int seq, int head_dim)
 {
-    // Pointers do not matter for the answer except for their alignment; an aligned dummy stands in.
-    static const uintptr_t dummy = 256;
+    // Pointers do not matter for the answer except for their alignment; aligned stand-ins, one for each tensor.
+    const void *at[4];
+    for (int i = 0; i < 4; i++) at[i] = (const void *)(uintptr_t)(256 * (i + 1));
     const LinearShape sh = {m, n, k, dtype, x_heads, y_heads, seq, head_dim};
-    const void *p = (const void *)dummy;
-    GemmArgs g;
-    g.dtype = dtype;
-    if (product == 1) {  // grad_w
-        g.mode = GEMM_TN;
-        g.a = view(p, m, k, x_heads, sh); g.b = view(p, m, n, y_heads, sh); g.c = view(p, k, n, 0, sh);
-        g.m = k; g.n = n; g.k = (int)m;
-    } else if (product == 2) {  // grad_x
-        g.mode = GEMM_NT;
-        g.a = view(p, m, n, y_heads, sh); g.b = view(p, k, n, 0, sh); g.c = view(p, m, k, x_heads, sh);
-        g.m = m; g.n = k; g.k = n;
-    } else {  // forward
-        g.mode = GEMM_NN;
-        g.a = view(p, m, k, x_heads, sh); g.b = view(p, k, n, 0, sh); g.c = view(p, m, n, y_heads, sh);
-        g.m = m; g.n = n; g.k = k;
+    const GemmArgs g = product_of(product, sh, at[0], at[1], at[2], at[3]);
+    if (dtype == EMBER_F32) {
+        int dev = 0, sms = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+            cudaGetLastError();
+            sms = 148;
+        }
+        F32Products f32;
+        if (product == FORWARD) {
+            if (!skinny_f32_supported(g)) f32.add(g);
+        } else {
+            f32.add(product_of(GRAD_W, sh, at[0], at[1], at[2], at[3]));
+            f32.add(product_of(GRAD_X, sh, at[0], at[1], at[2], at[3]));
+        }
+        return f32.preferred(sms) ? "sm100_tcgen05" : "simt_f32";
     }
     return worth_packing(g) || sm100_skinny_gemm_supported(g) || sm100_gemm_supported(g) ? "sm100_tcgen05" : "simt_f32";
 }

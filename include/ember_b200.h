@@ -216,7 +216,9 @@ EMBER_API int ember_work_order_item(int units, int blocks, int sm_count, size_t 
                                     int index, int *unit, int *rank);
 
 /* Name of the kernel family the forward/backward dispatcher picks for these
- * arguments: "sm100_tcgen05" or "simt_f32". For tests and the benchmark. */
+ * arguments with EMBER_BF16: "sm100_tcgen05" or "simt_f32". For tests and the benchmark. EMBER_F32: always
+ * "simt_f32", the family that takes every call; which of them run on the tensor cores instead depends on
+ * batch_heads and causal as well, which are not arguments here. */
 EMBER_API const char *ember_attention_kernel_name(int op, int lq, int lk, int d, int dtype);
 
 /* ---- Optional gather of the per-rank output slabs (no counterpart in the reference, which has no
@@ -274,7 +276,9 @@ EMBER_API int ember_linear_bwd(const void *x, const void *w, const void *grad_y,
                                void *grad_b, long long m, int n, int k, int dtype, int x_heads, int y_heads,
                                int seq, int head_dim, void *stream);
 /* Kernel family the dispatcher picks for one of the three products (0 forward, 1 grad_w,
- * 2 grad_x) with 16-byte aligned pointers: "sm100_tcgen05" or "simt_f32". */
+ * 2 grad_x) with 16-byte aligned pointers: "sm100_tcgen05" or "simt_f32". Float32 gradients: of a call
+ * that asks for both. Float32 values that the tensor-core kernel cannot hold, and calls without memory for
+ * its operands, run on the CUDA cores all the same. */
 EMBER_API const char *ember_linear_kernel_name(int product, long long m, int n, int k, int dtype, int x_heads,
                                                int y_heads, int seq, int head_dim);
 

@@ -61,6 +61,18 @@ def test_kernel_dispatch_names():
     assert L.ember_attention_kernel_name(_lib.EMBER_OP_FWD, 128, 128, 100, _lib.EMBER_BF16) == b"simt_f32"
 
 
+@pytest.mark.parametrize("m,n,k,names", [
+    (2048, 2048, 2048, "ttt"), (2000, 3001, 1024, "ttt"), (300, 300, 300, "sss"), (1, 8192, 8192, "sss"), (16, 16384, 1024, "sss"),
+    (1000, 1000, 1000, "ttt"), (32, 16384, 1024, "sss"), (8192, 64, 512, "tss"),
+])
+def test_float32_products_are_named_after_the_kernels_that_take_them(m, n, k, names):
+    """By measured times: small products, few rows and gradients whose two products together do not pay for the splitting stay on the CUDA cores."""
+    L = _lib.lib()
+    family = {"t": b"sm100_tcgen05", "s": b"simt_f32"}
+    for product, want in enumerate(names):
+        assert L.ember_linear_kernel_name(product, m, n, k, _lib.EMBER_F32, 0, 0, 0, 0) == family[want], product
+
+
 def _fake(shape, dtype="float32"):
     return Tensor._from_core(None, shape, dtype)
 
