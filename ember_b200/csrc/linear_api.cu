@@ -147,7 +147,7 @@ bool worth_packing(const GemmArgs &g)
 // entry point, and the CUDA-core kernels behind them return at once unless an operand holds values that planes cannot.
 //
 // Which side takes a call: both times are estimated, in us. The tensor-core side starts at 17.5 for one product (split, product, the launch
-// that returns) and 33 for two, splitting costs a pass (10 bytes an element at 5 TB/s), its tiles are 256 rows; the CUDA cores
+// that returns) and 33 for two, splitting costs a pass (4 bytes read and 6 written an element, rows written as multiples of 8, at 5 TB/s), its tiles are 256 rows; the CUDA cores
 // run at 40 TFLOP/s where tiles of 128 x 128 fill the SMs, at 17 to 34 below. Measured, CUDA cores / tensor cores, forward and both gradients
 // (rows x contraction x columns):
 //   300^3 10 / 18, 21 / 35      512^3 17 / 17, 35 / 33          1024^3 66 / 24, 153 / 46       2048^3 415 / 85, 831 / 168
@@ -189,7 +189,7 @@ struct F32Products {
             tensor += sm100_f32_gemm_us(g[i], sms);
             cores += simt_f32_us(g[i], sms);
         }
-        for (int i = 0; i < nops; i++) tensor += (double)ops[i].rows * ops[i].cols * 10.0 * kSplitUsPerByte;
+        for (int i = 0; i < nops; i++) tensor += (4.0 * ops[i].rows * ops[i].cols + 6.0 * split_plane_elems(ops[i].rows, ops[i].cols)) * kSplitUsPerByte;
         if (tensor < (count > 1 ? 33.0 : 17.5)) tensor = count > 1 ? 33.0 : 17.5;
         return tensor < cores;
     }
