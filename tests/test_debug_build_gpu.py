@@ -1,6 +1,6 @@
 """GPU test of the bounds-checked debug build (``libember_b200_dbg.so``, -DEMBER_BOUNDS_CHECK): the
-tensor-core attention kernels run with every global store checked against its tensor's extent, over
-lengths below, at and above the tile sizes; no store may be reported, and the results match the oracle.
+tensor-core attention kernels, bf16 and float32, run with every global store checked against its tensor's extent, over
+lengths below, at and above the tile sizes; no store may be reported, and the results match the oracle (float32: the CUDA-core kernels).
 A child process loads the debug library through EMBER_B200_LIB (one process, one build of the library).
 Skipped when the debug library has not been built (`python -m ember_b200.build --bounds`)."""
 import os
@@ -49,6 +49,32 @@ for D in (64, 128):
             assert np.abs(o.float().cpu().numpy() - ro).max() <= 2e-2
             for got, ref in zip((dq, dk, dv), cpu_oracle.attention_bwd(host[0][:n], host[1][:n], host[2][:n], host[3][:n], None, bool(causal))):
                 assert np.abs(got.float().cpu().numpy() - ref).max() <= 2e-2 * max(np.abs(ref).max(), 1e-6)
+# float32 on the tensor cores: lengths and columns around the 128-row blocks and 64-row tiles
+asked = 0
+for D, lq, lk in ((64, 512, 513), (64, 577, 640), (128, 511, 577), (128, 640, 640), (80, 385, 700), (33, 600, 601), (61, 129, 1100)):
+    x = [seeded((n, D), s, 0.5) for s, n in ((1, lq), (2, lk), (3, lk), (4, lq))]
+    q, k, v, do = (torch.from_numpy(a).to(dev) for a in x)
+    for causal in (0, 1):
+        def step():
+            o, dq, dk, dv = (torch.empty((n, D), device=dev) for n in (lq, lq, lk, lk))
+            lse = torch.empty((lq,), device=dev)
+            wsn = L.ember_attention_workspace_bytes(_lib.EMBER_OP_BWD, 1, lq, lk, D, 0, 0)
+            ws = torch.empty(wsn, device=dev, dtype=torch.uint8)
+            sc = 1.0 / math.sqrt(D)
+            _lib.check(L.ember_attention_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(), 1, lq, lk, D, sc, causal, 0, sp))
+            _lib.check(L.ember_attention_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(), do.data_ptr(),
+                                             dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), 1, lq, lk, D, sc, causal, 0, ws.data_ptr(), wsn, sp))
+            where = ctypes.c_int(0)
+            rc = L.ember_check_device_status(sp, ctypes.byref(where))
+            assert rc == 0, (D, lq, lk, causal, where.value, L.ember_last_error())
+            return [t.cpu().numpy() for t in (o, dq, dk, dv)]
+        got = step()
+        L.ember_selftest_fail_scratch(8)
+        cores = step()
+        asked += 8 - L.ember_selftest_fail_scratch(0)
+        for a, b in zip(got, cores):
+            assert np.abs(a - b).max() <= 64 * 2.0 ** -24 * np.abs(b).max()
+assert asked == 28, asked  # forward and backward of all 14 asked for the memory that the tensor-core kernels need
 print("debug build ok")
 """
 

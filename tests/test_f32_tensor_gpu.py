@@ -2,15 +2,17 @@
 head dimensions that fill the parts' columns partly, rows at any alignment, and the calls that it has to leave to the
 CUDA-core kernels (values that the parts cannot hold, no memory for them), against float64.
 
-Tolerance: products of parts leave out less than 2^-25 of a product and the tensor core's additions lose up to 2^-23 each of
+Tolerance: products of parts leave out less than 2^-24 of a product and the tensor core's additions lose up to 2^-23 each of
 a partial sum of 64 terms or fewer (at most 4 additions of full size), partial sums are then added in float32: of a sum of n
 terms of order one that is about (4 + sqrt(n / 64)) * 2^-23 of its terms' root sum of squares. 64 * 2^-24 of the largest result
 covers n up to 5000 with the exponentials' 2^-22 and a few units for the log-sum-exp."""
+import ctypes
+
 import numpy as np
 import pytest
 
 import ember_b200 as em
-from conftest import seeded
+from conftest import Guarded, seeded
 from ember_b200 import _lib
 
 pytestmark = pytest.mark.gpu
@@ -38,6 +40,14 @@ def run(q, k, v, g, scale, causal):
     return [t.to_np()[0] for t in (o, lse, *grads)]
 
 
+def on_the_cuda_cores(*args):
+    """The same without memory for the parts, and how many of the two calls (forward, backward) asked for it: those on the tensor cores."""
+    L = _lib.lib()
+    L.ember_selftest_fail_scratch(8)
+    got = run(*args)
+    return got, 8 - L.ember_selftest_fail_scratch(0)
+
+
 def inputs(units, lq, lk, d, seed=1, std=0.5):
     return [seeded((units, n, d), seed + i, std) for i, n in enumerate((lq, lk, lk, lq))]
 
@@ -55,7 +65,77 @@ def close(got, want, rel=REL):
 ])
 def test_edges_of_blocks_and_tiles(units, lq, lk, d, causal):
     x = inputs(units, lq, lk, d)
-    close(run(*x, d ** -0.5, causal), reference(*x, d ** -0.5, causal))
+    want = reference(*x, d ** -0.5, causal)
+    close(run(*x, d ** -0.5, causal), want)
+    cores, asked = on_the_cuda_cores(*x, d ** -0.5, causal)
+    assert asked == 2
+    close(cores, want)
+
+
+@pytest.mark.parametrize("units,lq,lk,d,causal", [(2, 513, 640, 64, True), (1, 1300, 1300, 40, False), (1, 577, 600, 101, False), (2, 300, 700, 96, True), (1, 1090, 1090, 3, False)])
+def test_nothing_is_written_outside_the_results(units, lq, lk, d, causal):
+    torch = pytest.importorskip("torch")
+    L = _lib.lib()
+    dev = torch.device("cuda", 0)
+    x = inputs(units, lq, lk, d)
+    q, k, v, g = (torch.from_numpy(a).to(dev) for a in x)
+    o, lse, dq, dk, dv = (Guarded(torch, shape, torch.float32, dev) for shape in ((units, lq, d), (units, lq), (units, lq, d), (units, lk, d), (units, lk, d)))
+    n = L.ember_attention_workspace_bytes(_lib.EMBER_OP_BWD, units, lq, lk, d, 0, 0)
+    ws = Guarded(torch, (n,), torch.uint8, dev)
+    s = torch.cuda.Stream(device=dev)
+    s.wait_stream(torch.cuda.current_stream(dev))
+    sp = ctypes.c_void_p(s.cuda_stream)
+    ptr = lambda t: (t.t if isinstance(t, Guarded) else t).data_ptr()  # noqa: E731
+    _lib.check(L.ember_attention_fwd(*map(ptr, (q, k, v, o, lse)), units, lq, lk, d, d ** -0.5, int(causal), 0, sp))
+    _lib.check(L.ember_attention_bwd(*map(ptr, (q, k, v, o, lse, g, dq, dk, dv)), units, lq, lk, d, d ** -0.5, int(causal), 0, ptr(ws), n, sp))
+    s.synchronize()
+    for t in (o, lse, dq, dk, dv, ws):
+        t.check()
+    close([t.t.cpu().numpy() for t in (o, lse, dq, dk, dv)], reference(*x, d ** -0.5, causal))
+
+
+def test_captured_calls():
+    """Under stream capture the parts' memory becomes nodes of the graph: replays give the bits of plain calls, on the inputs of the day."""
+    torch = pytest.importorskip("torch")
+    L = _lib.lib()
+    dev = torch.device("cuda", 0)
+    units, n, d, m, e = 4, 700, 64, 700, 1024
+    q, k, v, g = (torch.empty((units, n, d), device=dev) for _ in range(4))
+    x, w, b = torch.empty((m, e), device=dev), torch.empty((e, e), device=dev), torch.empty((e,), device=dev)
+    out = [torch.empty((units, n, d), device=dev) for _ in range(4)] + [torch.empty((units, n), device=dev), torch.empty((m, e), device=dev)]
+    ws = torch.empty(L.ember_attention_workspace_bytes(_lib.EMBER_OP_BWD, units, n, n, d, 0, 0), device=dev, dtype=torch.uint8)
+    s = torch.cuda.Stream(device=dev)
+
+    def calls():
+        sp = ctypes.c_void_p(s.cuda_stream)
+        o, dq, dk, dv, lse, y = (t.data_ptr() for t in out)
+        a = [t.data_ptr() for t in (q, k, v)]
+        _lib.check(L.ember_attention_fwd(*a, o, lse, units, n, n, d, 0.125, 1, 0, sp))
+        _lib.check(L.ember_attention_bwd(*a, o, lse, g.data_ptr(), dq, dk, dv, units, n, n, d, 0.125, 1, 0, ws.data_ptr(), ws.numel(), sp))
+        _lib.check(L.ember_linear_fwd(x.data_ptr(), w.data_ptr(), b.data_ptr(), y, m, e, e, 0, 0, 0, 0, 0, sp))
+
+    def fill(seed):
+        gen = torch.Generator(device=dev).manual_seed(seed)
+        for t in (q, k, v, g, x, w, b):
+            t.normal_(generator=gen)
+        torch.cuda.synchronize()
+
+    fill(1)
+    calls()
+    s.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=s):
+        calls()
+    for seed in (2, 3):
+        fill(seed)
+        for t in out:
+            t.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        got = [t.clone() for t in out]
+        calls()
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for a, b in zip(got, out))
 
 
 @pytest.mark.parametrize("d", [64, 96, 40])
@@ -92,11 +172,9 @@ def test_values_that_the_parts_cannot_hold(d, which, value):
     them, and the same numbers elsewhere."""
     x = inputs(2, 520, 600, d)
     x[which][1, 300, 5] = value
-    L = _lib.lib()
     got = run(*x, d ** -0.5, False)
-    L.ember_selftest_fail_scratch(2)
-    want = run(*x, d ** -0.5, False)
-    assert L.ember_selftest_fail_scratch(0) == 0  # both calls asked for that memory
+    want, asked = on_the_cuda_cores(*x, d ** -0.5, False)
+    assert asked == 2
     if value == 3e38:  # times score gradients that are nothing but the rounding of what cancels there: not dq and dk
         got, want = ([t[0], t[1], t[4]] for t in (got, want))
     for a, b in zip(got, want):
@@ -182,10 +260,8 @@ def test_zeros_stay_on_the_tensor_cores_and_give_means():
 
 def test_without_memory_for_the_parts():
     x = inputs(2, 600, 600, 64)
-    L = _lib.lib()
-    L.ember_selftest_fail_scratch(2)
-    got = run(*x, 0.125, True)
-    L.ember_selftest_fail_scratch(0)
+    got, asked = on_the_cuda_cores(*x, 0.125, True)
+    assert asked == 2
     close(got, reference(*x, 0.125, True))
 
 

@@ -39,10 +39,13 @@ def env():
 def _fwd(L, sp, q, k, v, causal, dtype):
     BH, Lq, D = q.shape[0] * q.shape[1], q.shape[2], q.shape[3]
     Lk = k.shape[2]
+    if dtype == _lib.EMBER_F32:
+        L.ember_selftest_fail_scratch(1)  # no memory for the tensor-core kernels' operands: the CUDA cores
     o = torch.empty_like(q)
     lse = torch.empty(q.shape[:3], device=q.device, dtype=torch.float32)
     _lib.check(L.ember_attention_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(), BH, Lq,
                                      Lk, D, 1.0 / math.sqrt(D), int(causal), dtype, sp))
+    assert L.ember_selftest_fail_scratch(0) == 0
     return o, lse
 
 
@@ -50,11 +53,14 @@ def _bwd(L, sp, q, k, v, o, lse, do, causal, dtype):
     BH, Lq, D = q.shape[0] * q.shape[1], q.shape[2], q.shape[3]
     Lk = k.shape[2]
     dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
+    if dtype == _lib.EMBER_F32:
+        L.ember_selftest_fail_scratch(1)
     n = L.ember_attention_workspace_bytes(_lib.EMBER_OP_BWD, BH, Lq, Lk, D, dtype, 0)
     ws = torch.empty(n, device=q.device, dtype=torch.uint8)
     _lib.check(L.ember_attention_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(),
                                      do.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), BH, Lq, Lk, D,
                                      1.0 / math.sqrt(D), int(causal), dtype, ws.data_ptr(), n, sp))
+    assert L.ember_selftest_fail_scratch(0) == 0
     return dq, dk, dv
 
 
@@ -65,7 +71,7 @@ def _no_fault(L, sp):
 
 def test_c2_causal_prefill_full_size(env):
     """B=4 H=32 L=4096 D=128 bf16 causal: tcgen05 kernel vs the float32-arithmetic kernel on the
-    same bf16 inputs (float32 storage routes to the CUDA-core kernel), plus one slice vs the oracle."""
+    same bf16 inputs (float32 storage, on the CUDA cores), plus one slice vs the oracle."""
     L, dev, sp = env
     B, H, S, D = 4, 32, 4096, 128
     q, k, v = (_rand((B, H, S, D), s, 0.5, dev) for s in (1, 2, 3))
