@@ -1,7 +1,7 @@
 // Float32 attention on the tensor cores: every operand is the sum of three bf16 parts (split_f32.cuh), a product of
 // two operands six tcgen05 products of their parts, small ones first, accumulated in float32 over at most 64 terms in
 // tensor memory and then added into float32 registers. Probabilities and score gradients are split the same way in
-// registers, so nothing is held or multiplied with less than 24 bits. Parts are of 2^20 times a value (a power of its own for score
+// registers, so nothing is held or multiplied with less than 24 bits. Parts are of 2^16 times a value (a power of its own for score
 // gradients), so that small ones keep all of theirs; where a result leaves the accumulators that is undone.
 //
 // The CUDA-core kernels (attn_simt.cu) do the same products at the FMA pipe's rate, 128 per clock and SM; six bf16 products for
@@ -105,7 +105,7 @@ struct Region {
     static __device__ __forceinline__ uint32_t part(uint32_t q) { return q == 2 ? LOW : q * 16; }
 };
 
-// 32 values of a row -> their parts in tensor memory, in a half of a region. UP: of 2^20 times the values.
+// 32 values of a row -> their parts in tensor memory, in a half of a region. UP: of 2^16 times the values.
 template <typename R, bool UP>
 __device__ __forceinline__ void split_to_tmem(const f32x2 *v, uint32_t taddr)
 {
@@ -1005,8 +1005,8 @@ int launch_bwd(const AttnArgs &a, const float *delta, const void *qp, const void
 // kernels, 2^12 keeps that below 5e-4.
 constexpr double kMostScore = 7.9e28, kMostScoreMixed = 4096;
 
-// Scales below 2^-60 times 2^-40 (the parts' factors) would end in float32's smallest exponents, those beyond 2^20 could take scores
-// of operands below 2^28 to the limit above.
+// Scales below 2^-60 times 2^-32 (the parts' factors) would end in float32's smallest exponents, those beyond 2^20 could take scores
+// of operands below 2^32 to the limit above.
 bool takes(const AttnArgs &a)
 {
     return a.dtype == EMBER_F32 && a.d <= 128 && fabsf(a.scale) <= 1048576.f && (a.scale == 0 || fabsf(a.scale) >= 8.7e-19f) && (long long)a.bh * 3 <= 0x7fffffffLL;

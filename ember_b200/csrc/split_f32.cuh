@@ -1,14 +1,14 @@
 // Float32 operands for the tensor cores. A float32 value is the exact sum of three bf16 values (24 significand
 // bits = 3 x 8): high, middle and low part, each the rounding of what the ones before left over. Of the nine products of
-// two such sums the six largest are formed, all in float32; what is left out is below 2^-26 of the product.
+// two such sums the six largest are formed, all in float32; what is left out is below 2^-24 of the product, 2^-27 as a rule.
 // The tensor core adds with truncation (a sum keeps 24 bits and loses the rest towards zero; within one MMA, terms are cut
 // at 2^-25 of the largest), so an accumulator that collects a whole contraction drifts: relative error of random sums of 64 /
 // 512 / 2048 terms 6.6e-8 / 4.7e-7 / 2.1e-6. The kernels therefore let it collect 64 terms at most, the
 // small products first, and add it into float32 registers with rounding.
-// Parts are made of the value times 2^20: bf16 ends at 2^-133, where the low part of a value below 2^-110 would lose its last bits
-// (a row of 1e-36 beside ordinary ones: 3e-5 of its results); 2^20 times the smallest float32 is held exactly. What is made of parts is
-// divided by the powers of two again where it leaves the accumulators.
-// Values that the parts cannot hold (infinities, NaN, 2^28 and above, whose sums of 2^31 products times 2^40 may pass float32) are
+// Parts are made of the value times 2^16: bf16 ends at 2^-133 (tcgen05 multiplies those small ones as they are), where the low part of a
+// value below 2^-110 would lose its last bits (a row of 1e-36 beside ordinary ones: 3e-5 of its results); 2^16 times the smallest float32 is
+// just held. What is made of parts is divided by the powers of two again where it leaves the accumulators.
+// Values that the parts cannot hold (infinities, NaN, 2^32 and above, whose sums of 2^31 products times 2^32 may pass float32) are
 // found while the parts are made: the tensor-core kernel then leaves the work to the CUDA-core kernel that is launched behind it and
 // otherwise returns at once.
 #pragma once
@@ -22,10 +22,10 @@ namespace ember {
 constexpr int kSplitMaxJobs = 4;
 constexpr int kSplitMaxBlocks = 592;               // 4 blocks of 256 threads per SM
 constexpr int kSplitMaxTensors = kSplitMaxJobs + 1;  // delta's largest magnitude is reported as well
-constexpr uint32_t kSplitHuge = 0x4D800000u;       // 2^28
+constexpr uint32_t kSplitHuge = 0x4F800000u;       // 2^32
 constexpr uint32_t kSplitHugeDelta = 0x67800000u;  // 2^80
-constexpr int kSplitShift = 20;
-constexpr float kSplitUp = 1048576.f, kSplitDown2 = 1.f / 1048576.f / 1048576.f;  // a part's factor, and what undoes it in a product of two
+constexpr int kSplitShift = 16;
+constexpr float kSplitUp = 65536.f, kSplitDown2 = 1.f / 65536.f / 65536.f;  // a part's factor, and what undoes it in a product of two
 
 // What a split launch leaves for the kernels behind it: the largest magnitude (as bits; a NaN is larger than all) that each of
 // its blocks saw, by tensor, and the word through which the tensor-core kernel tells the CUDA-core kernel to run.
@@ -102,8 +102,8 @@ __device__ __forceinline__ void split_pair(ptx::f32x2 v, uint32_t &hi, uint32_t 
 }
 #endif
 
-// One tensor to split: rows x cols float32, row-major -> three bf16 planes (of 2^20 times its values) of rows x cols rounded up to 8 (zeros there), one
-// after the other. dst null: only looked through for values out of range.
+// One tensor to split: rows x cols float32, row-major -> three bf16 planes (of 2^16 times its values) of rows x cols
+// rounded up to 8 (zeros there), one after the other. dst null: only looked through for values out of range.
 struct SplitJob {
     const float *src = nullptr;
     void *dst = nullptr;
