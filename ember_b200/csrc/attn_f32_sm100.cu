@@ -5,12 +5,13 @@
 // gradients), so that small ones keep all of theirs; where a result leaves the accumulators that is undone.
 //
 // The CUDA-core kernels (attn_simt.cu) do the same products at the FMA pipe's rate, 128 per clock and SM; six bf16 products for
-// each leave 683 per clock. Measured, 16 units x L1024, causal: d 64 forward 93 -> 29 us, backward 215 -> 61 us (and 6 us of
-// splitting each); d 128, 8 units: 105 -> 56 and 234 -> 103 us. What bounds them now: the compute warps (exponentials and the
-// splitting of 128 x 64 probabilities, 2500 clocks a tile) and the hand-overs between them and the products (1536 to 3456 clocks).
-// Errors against float64 (relative 2-norm, CUDA cores -> here): 16 units x L1024 d 64 causal: o 2.3e-7 -> 0.9e-7, dq 3.3e-7 ->
-// 2.6e-7, dk 7.7e-7 -> 2.9e-7, dv 7.8e-7 -> 2.2e-7, log-sum-exp 3.3e-8 both; 8 x 777 x 1301 d 80: o 6.5e-7 -> 1.3e-7, dq 7.1e-7 -> 3.3e-7, dk
-// 5.7e-7 -> 3.2e-7, dv 5.5e-7 -> 2.7e-7, log-sum-exp 2.9e-8 both.
+// each leave 683 per clock. Whole calls (split included), 16 units x L1024, causal: d 64 forward 93 -> 33 us, backward 215 -> 66; d 128, 8
+// units: 105 -> 55 and 234 -> 103. What bounds them now: the compute warps (exponentials, splitting of 128 x 64 probabilities) and the
+// hand-overs between them and the products. A tile takes, of its MMAs' clocks: forward 1930 of 1536 (d 64), 4160 of 3072 (d 128); backward, a
+// query block's 3940 of 2688 and 9300 of 5500 (one pair of tiles, loaded without overlap).
+// Errors against float64 (relative 2-norm, CUDA cores -> here): 16 units x L1024 d 64 causal: o 2.1e-7 -> 0.9e-7, dq 3.3e-7 ->
+// 2.6e-7, dk 7.8e-7 -> 2.9e-7, dv 7.7e-7 -> 2.2e-7, log-sum-exp 3.2e-8 both; 8 x 777 x 1301 d 80: o 6.5e-7 -> 1.3e-7, dq 7.1e-7 -> 3.2e-7, dk
+// 5.7e-7 -> 3.1e-7, dv 5.5e-7 -> 2.7e-7, log-sum-exp 2.9e-8 both.
 //
 // Common to the kernels: 128 rows of one operand belong to a CTA (a row per tensor-memory lane) and lie in tensor memory as
 // the A operand of the score product, tiles of 64 rows of the other operand's planes are streamed by TMA, eight compute

@@ -1,6 +1,6 @@
 // Float32 y = x w + b for at most 16 rows of x (a decode step's projections): CUDA cores, w streamed once.
 //
-// Bound: the bytes of w (up to 8 rows; 4.8 TB/s at 134 MB), from there on the shared-memory reads of x. The tiles of gemm_simt.cu load
+// Bound: the bytes of w (2048 x 16384, 134 MB: 4.8 TB/s with 1 row, 3.9 with 8), from there on the shared-memory reads of x. The tiles of gemm_simt.cu load
 // a slab of w and a slab of x, meet at a barrier and multiply, which left the memory idle for most of a round. Here a thread owns
 // 4 columns of all rows and reads its rows of w straight into registers, the next ones while it multiplies; x lies transposed in shared
 // memory, from where a step's rows are broadcast. 256 threads are 16 column groups x 16 contraction groups; a cluster of up to

@@ -13,9 +13,13 @@
  *     lse: (batch_heads, lq) float32, natural-log log-sum-exp of the scaled,
  *     masked scores of each query row.
  *   - dtype selects the storage type of q/k/v/out/dout/dq/dk/dv: EMBER_F32 or
- *     EMBER_BF16. Softmax and all accumulation are float32 in both modes. Float32 forwards and backwards
- *     of some size take temporary device memory (6 bytes per element of their inputs) from the stream's pool and
- *     free it in stream order (under stream capture: memory nodes); where there is none they run without.
+ *     EMBER_BF16. Softmax and all accumulation are float32 in both modes. Float32 calls of some size run on
+ *     the tensor cores with copies of k and v (backward: of q, k, v and dout; Linear: of the products'
+ *     operands) as three bf16 parts: temporary device memory of 6 bytes per element, rows rounded up to 8
+ *     elements, taken from the device's default pool (which keeps it for later calls, see below) and freed in
+ *     stream order. Where there is none they run on the CUDA cores. Under stream capture it becomes memory
+ *     nodes, and CUDA does not take a graph with memory nodes as a child graph or as the body of a conditional
+ *     node, nor two executable instances of it at a time.
  *   - causal != 0 masks key j for query i when j > i + (lk - lq) (lower
  *     triangle aligned to the bottom-right corner; requires lq <= lk). This is
  *     the additive {0,-inf} mask the reference would need a broadcast add for
@@ -251,9 +255,10 @@ EMBER_API int ember_gather_outputs(void *out_full, const void *out_slab, size_t 
  *
  * x is a logical (m, k) matrix, w is (k, n) row-major as the reference stores it (in_features,
  * out_features), bias has n elements (or NULL), y is (m, n). dtype selects storage as for attention
- * (EMBER_F32: float32 arithmetic on CUDA cores, or, by size, each operand as three bf16 parts on the tensor cores, which hold
- * a float32 exactly; bf16 tensor-core products with float32
- * accumulation for EMBER_BF16 when the shapes allow, else float32 arithmetic on bf16 storage).
+ * (EMBER_F32: float32 arithmetic on CUDA cores, or, by size, on the tensor cores with each operand as three
+ * bf16 parts, which hold every float32 below 2^32 exactly; calls with larger elements, infinities or NaN run on
+ * the CUDA cores. EMBER_BF16: tensor-core products with float32 accumulation when the shapes allow, else
+ * float32 arithmetic on bf16 storage).
  *
  * Head-major operands, so that no transpose runs between a projection and attention:
  *   x_heads > 0: x (and grad_x) lie as (batch, x_heads, seq, head_dim), the layout attention
@@ -266,8 +271,8 @@ EMBER_API int ember_gather_outputs(void *out_full, const void *out_slab, size_t 
  * bf16 products whose rows are no multiple of 16 bytes (or start off a 16-byte boundary) run on the
  * tensor cores with padded copies of those operands, where the product is large enough: temporary
  * memory of about the operands' size (rows padded to 8 elements) for the length of the call, taken
- * and freed in stream order; under stream capture it becomes memory nodes of the graph. Where there
- * is no memory for them the product runs on the CUDA cores, which need none.
+ * and freed in stream order; under stream capture it becomes memory nodes of the graph, as for float32 calls
+ * above. Where there is no memory for them the product runs on the CUDA cores, which need none.
  *
  * ember_linear_bwd: any of grad_x, grad_w, grad_b may be NULL and is then skipped. */
 EMBER_API int ember_linear_fwd(const void *x, const void *w, const void *bias, void *y, long long m, int n, int k,
