@@ -19,6 +19,8 @@
 #include <float.h>
 #include <math.h>
 
+#include <initializer_list>
+
 #include "common.cuh"
 #include "kernels.cuh"
 #include "ptx.cuh"
@@ -1003,7 +1005,8 @@ int launch_bwd(const AttnArgs &a, const float *delta, const void *qp, const void
 // 1e30 that stands for an infinite log-sum-exp. The backward's weights e^(score - log-sum-exp) carry the score's rounding error, unless
 // forward and backward form the same bits: both tensor-core kernels do, both CUDA-core kernels do, one of each does not (values'
 // gradients off by 1e-4 of their norm at scores of 1e4, 7e-3 at 1e6, NaN at 1e12). Where sizes send the two directions to different
-// kernels, 2^12 keeps that below 5e-4.
+// kernels, 2^12 keeps that below 5e-4. Units may be split over calls in one direction and not in the other (ember_attention_fwd_host
+// does), so sizes count as sending both here only if they do with one unit as well (from L 512 on, d 64 and 128).
 constexpr double kMostScore = 7.9e28, kMostScoreMixed = 4096;
 
 // Scales below 2^-60 times 2^-32 (the parts' factors) would end in float32's smallest exponents, those beyond 2^20 could take scores
@@ -1067,7 +1070,11 @@ namespace {
 // The guard's limit for the largest elements of q and k.
 float score_limit(const AttnArgs &a, int sms)
 {
-    const double most = sm100_f32_fwd_preferred(a, sms) && sm100_f32_bwd_preferred(a, sms) ? kMostScore : kMostScoreMixed;
+    AttnArgs one = a;
+    one.bh = 1;
+    bool both = true;
+    for (const AttnArgs *p : {(const AttnArgs *)&one, &a}) both = both && sm100_f32_fwd_preferred(*p, sms) && sm100_f32_bwd_preferred(*p, sms);
+    const double most = both ? kMostScore : kMostScoreMixed;
     const double limit = a.scale != 0 ? most / (a.d * fabs((double)a.scale)) : FLT_MAX;
     return limit < FLT_MAX ? (float)limit : FLT_MAX;
 }

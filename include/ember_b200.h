@@ -83,7 +83,8 @@ EMBER_API void sync_device(void);
  *      synchronised; otherwise the pool may hand the block to the next allocation while the kernel
  *      still runs. stream NULL = the library stream. ember_alloc_async returns NULL on failure
  *      (text in ember_last_error()). Freed blocks stay in the device's pool (release threshold
- *      unlimited) and are reused without a new driver allocation; ember_pool_stats reports what the
+ *      unlimited; cudaMemPoolTrimTo on the device's default pool gives them back) and are reused without a
+ *      new driver allocation; ember_pool_stats reports what the
  *      pool currently holds from the driver (reserved) and has handed out (used). ---- */
 EMBER_API void *ember_alloc_async(size_t bytes, void *stream);
 EMBER_API int ember_free_async(void *ptr, void *stream);

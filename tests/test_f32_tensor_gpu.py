@@ -193,17 +193,22 @@ def test_tensors_of_tiny_values_keep_their_precision(d):
     close(run(q, k, v, g, d ** -0.5, False), reference(q, k, v, g, d ** -0.5, False))
 
 
-@pytest.mark.parametrize("units,lq,lk,d", [(2, 520, 600, 64), (2, 520, 600, 128), (1, 600, 600, 40), (1, 200, 512, 64), (64, 128, 128, 64)])
-@pytest.mark.parametrize("size", [10.0, 30.0, 1e3, 1e5, 1e8, 4e14])
-def test_large_scores_leave_the_largest_a_weight_of_one(units, lq, lk, d, size):
-    """Elements of +-size: query i scores 10 times its other keys with key i + lk - lq, whose weight is 1 to the last bit wherever forward
-    and backward round scores alike. That key's value is the output, its gradient the upstream gradient. Scores' rounding errors may reach
-    the weight where the two run on different kernels, up to the 2^12 at which those calls stay on the CUDA cores: 2^-10 then (a few units
-    of 2^-23 of a score)."""
+def peaked(units, lq, lk, d, size):
+    """q and k of elements of +-size, query i along key i + lk - lq."""
     rng = np.random.default_rng(5)
     k = np.where(rng.standard_normal((units, lk, d)) < 0, -1, 1) * rng.uniform(0.75, 1.25, (units, lk, d)) * size
     k = k.astype(np.float32)
-    q = (k[:, lk - lq:] * np.float32(1.37)).astype(np.float32)
+    return (k[:, lk - lq:] * np.float32(1.37)).astype(np.float32), k
+
+
+@pytest.mark.parametrize("units,lq,lk,d", [(2, 520, 600, 64), (2, 520, 600, 128), (1, 600, 600, 40), (1, 200, 512, 64), (64, 128, 128, 64)])
+@pytest.mark.parametrize("size", [10.0, 30.0, 1e3, 1e5, 1e8, 4e14])
+def test_large_scores_leave_the_largest_a_weight_of_one(units, lq, lk, d, size):
+    """Elements of +-size: query i scores about twice what any other key gets with key i + lk - lq, whose weight is 1 to the last bit where forward
+    and backward round scores alike. That key's value is the output, its gradient the upstream gradient. Scores' rounding errors may reach
+    the weight where the two run on different kernels, up to the 2^12 at which those calls stay on the CUDA cores: 2^-10 then (a few units
+    of 2^-23 of a score)."""
+    q, k = peaked(units, lq, lk, d, size)
     v, g = seeded((units, lk, d), 2), seeded((units, lq, d), 3)
     scale = 0.25 if d == 40 else 0.125
     s = (q[0].astype(np.float64) @ k[0].T.astype(np.float64)) * scale
@@ -250,6 +255,21 @@ def test_scores_of_one_sign(d):
     want = reference(q, k, v, g, d ** -0.5, False)[1]
     score = np.einsum("uid,ud->ui", q.astype(np.float64), k.astype(np.float64).mean(1)) * d ** -0.5
     assert np.sqrt(((lse - want) ** 2).mean()) <= 2.5 * 2.0 ** -24 * np.sqrt((score ** 2).mean())
+
+
+@pytest.mark.parametrize("n", [256, 600])
+@pytest.mark.parametrize("size", [10.0, 30.0, 1e5])
+def test_large_scores_with_the_units_in_pieces(n, size):
+    """Forward one unit a call, backward all of them, which may go to different kernels: as above, 2^-10 of the scores' rounding errors up to
+    2^12, none beyond it nor where both directions take the same kernels whatever the number of units."""
+    units, d = 32, 64
+    q, k = peaked(units, n, n, d, size)
+    v, g = seeded((units, n, d), 2), seeded((units, n, d), 3)
+    pieces = [[t.to_np() for t in em.attention_forward(*(em.Tensor(x[None, u:u + 1]) for x in (q, k, v)), 0.125, False)] for u in range(units)]
+    o, lse = (em.Tensor(np.concatenate([p[i] for p in pieces], 1)) for i in range(2))
+    dv = em.attention_backward(*(em.Tensor(x[None]) for x in (q, k, v)), o, lse, em.Tensor(g[None]), 0.125, False)[2].to_np()[0]
+    assert np.abs(o.to_np()[0] - v).max() <= 2.0 ** -20 * np.abs(v).max()
+    assert np.abs(dv - g).max() <= (2.0 ** -10 if n == 256 and size == 10 else 2.0 ** -20) * np.abs(g).max()
 
 
 def test_zeros_stay_on_the_tensor_cores_and_give_means():
