@@ -36,6 +36,7 @@ constexpr int F32_THREADS = 384;       // warps 0-7 compute, 8 and 10 MMA issue,
 constexpr float LOG2E_T = 1.4426950408889634f;
 constexpr int SUB = 64 * 128;          // 64 rows x 128 bytes: one TMA box
 constexpr int TN = 64;                 // rows of a streamed tile
+constexpr int subs(int hd) { return (hd + 63) / 64; }  // 64-column sub-tiles
 
 enum { WF_Q = 301, WF_K, WF_V, WF_S, WF_P, WF_O, WF_OFREE, WF_KEMPTY, WF_VEMPTY, WB_A, WB_B0, WB_B1, WB_S, WB_P, WB_DP, WB_DS, WB_ACC, WB_FREE, WB_E0, WB_E1, WB_SMEM };
 
@@ -172,7 +173,7 @@ template <int HD, AKind KIND>
 __device__ __forceinline__ void mma_scores(uint32_t d, uint32_t a, uint32_t low_smem, uint32_t b_smem, int sub0, int sub1, int ksteps, uint32_t elected, bool mirrored)
 {
     constexpr uint32_t IDESC = idesc_bf16_f32(128, TN, 0, 0);
-    constexpr int PLANE = HD / 64 * SUB;
+    constexpr int PLANE = subs(HD) * SUB;
     const uint32_t b_lo = desc_lo(b_smem, 16), a_lo = KIND == A_SMEM ? desc_lo(a, 16) : a, low = desc_lo(low_smem, 16);
 #pragma unroll 1
     for (int i = 0; i < kSplitProducts; i++) {
@@ -190,7 +191,7 @@ __device__ __forceinline__ void mma_scores(uint32_t d, uint32_t a, uint32_t low_
 template <int HD, typename R>
 __device__ __forceinline__ void mma_results(uint32_t d, uint32_t region, uint32_t b_smem, uint32_t idesc, uint32_t elected)
 {
-    constexpr int PLANE = HD / 64 * SUB;
+    constexpr int PLANE = subs(HD) * SUB;
     const uint32_t b_lo = desc_lo(b_smem, SUB);
 #pragma unroll 1
     for (int i = 0; i < kSplitProducts; i++)
@@ -201,9 +202,9 @@ __device__ __forceinline__ void mma_results(uint32_t d, uint32_t region, uint32_
 template <int HD>
 __device__ __forceinline__ void load_planes(uint32_t dst, const CUtensorMap *map, uint32_t bar, int row, int unit, int units)
 {
-    mbar_arrive_expect_tx(bar, 3 * (HD / 64) * SUB);
+    mbar_arrive_expect_tx(bar, 3 * subs(HD) * SUB);
     for (int pl = 0; pl < 3; pl++)
-        for (int s = 0; s < HD / 64; s++) tma_load_3d(dst + (pl * (HD / 64) + s) * SUB, map, bar, s * 64, row, pl * units + unit);
+        for (int s = 0; s < subs(HD); s++) tma_load_3d(dst + (pl * subs(HD) + s) * SUB, map, bar, s * 64, row, pl * units + unit);
 }
 
 // Adds a partial result's first n columns (rounded up to 32) into registers: acc = acc * alpha + part.
@@ -257,18 +258,20 @@ __device__ __forceinline__ void store_cols(float *dst, const f32x2 (&v2)[N / 2],
 // the scheduler's own cache, an issuing warp needs 50 clocks for an MMA that takes 32 (alone 16), and one for both held a tile at 3570 clocks.
 template <int HD>
 struct F32FwdCfg {
-    static constexpr int TILE = 3 * (HD / 64) * SUB;  // 24 or 48 KB
+    static constexpr int TILE = 3 * subs(HD) * SUB;  // 24 or 48 KB
     static constexpr int KST = HD == 64 ? 3 : 2, VST = KST;
     static constexpr int OFF_K = 0, OFF_V = KST * TILE, OFF_BAR = OFF_V + VST * TILE;
     static constexpr int USED = OFF_BAR + 256, SMEM = USED + 1024;
-    // HD 64: one score buffer, read out at once, apart from the probabilities, and a partial output for each warpgroup, added up a
-    // turn later. HD 128: scores under the probabilities, formed and read in two halves of the contraction one after the other (side
-    // by side they fit only with the queries' low part in shared memory, and a product with that, between others, held a tile up for 800
-    // clocks: 1 x 32 x 2048, 87 us against 81), one partial output, added up before the next one's product.
-    static constexpr bool LATE = HD == 64;
+    // LATE, HD 64: one score buffer, read out at once, apart from the probabilities, and a partial output for each warpgroup, added up
+    // a turn later. Above: scores under the probabilities, one partial output, added up before the next one's product. HD 96: both accumulators
+    // of scores side by side. HALVES, HD 128: the two halves of the contraction formed and read one after the other (side by side they
+    // fit only with the queries' low part in shared memory, and a product with that, between others, held a tile up for 800 clocks:
+    // 1 x 32 x 2048, 87 us against 81; one after the other 8 x 842 d 96 takes 41.6 us, side by side 39.0).
+    static constexpr bool LATE = HD == 64, HALVES = HD == 128;
     using R = Region<false>;
-    static constexpr int T_Q = 0, T_S = 3 * HD / 2 + (LATE ? 0 : R::SCORES), T_P = 3 * HD / 2 + (LATE ? TN : 0), S_STEP = LATE ? 0 : R::COLS;
-    static constexpr int T_O = T_P + 2 * R::COLS, O_STEP = LATE ? HD : 0;
+    static constexpr int R_STEP = HD == 96 ? 128 : R::COLS, SCORES = HD == 96 ? 0 : R::SCORES;
+    static constexpr int T_Q = 0, T_P = 3 * HD / 2 + (LATE ? TN : 0), T_S = LATE ? 3 * HD / 2 : T_P + SCORES, S_STEP = LATE ? 0 : R_STEP;
+    static constexpr int T_O = T_P + 2 * R_STEP, O_STEP = LATE ? HD : 0;
     static_assert(T_O + HD + O_STEP <= 512, "");
     enum { B_Q, B_KFULL, B_KEMPTY = B_KFULL + KST, B_VFULL = B_KEMPTY + KST, B_VEMPTY = B_VFULL + VST, B_S = B_VEMPTY + VST, B_P = B_S + 2, B_O = B_P + 2, B_OFREE = B_O + 2, B_SREAD = B_OFREE + 2, NUM_BARS };
 };
@@ -367,12 +370,13 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
                 if (C::LATE && j > 0) ok = ok && mbar_wait(BAR(C::B_SREAD), (j - 1) & 1, abort_flag, p.status, WF_P);
                 if (!C::LATE && j > 1) ok = ok && mbar_wait(BAR(C::B_O + w), ((j - 2) >> 1) & 1, abort_flag, p.status, WF_P);
                 tc_fence_after();
-                for (int sub = 0; sub < HD / 64 && ok; sub++) {
-                    if (sub > 0) {
-                        ok = mbar_wait(BAR(C::B_SREAD), j & 1, abort_flag, p.status, WF_P);
-                        tc_fence_after();
-                    }
-                    mma_scores<HD, A_TMEM>(tmem + C::T_S + w * C::S_STEP, tmem + C::T_Q, 0, smem_base + C::OFF_K + (j % C::KST) * C::TILE, sub, sub + 1, ksteps, elected, false);
+                const uint32_t at = tmem + C::T_S + w * C::S_STEP, k_smem = smem_base + C::OFF_K + (j % C::KST) * C::TILE;
+                mma_scores<HD, A_TMEM>(at, tmem + C::T_Q, 0, k_smem, 0, C::HALVES ? 1 : subs(HD), ksteps, elected, false);
+                tc_commit_elect(BAR(C::B_S + w));
+                if (C::HALVES) {
+                    ok = ok && mbar_wait(BAR(C::B_SREAD), j & 1, abort_flag, p.status, WF_P);
+                    tc_fence_after();
+                    mma_scores<HD, A_TMEM>(at, tmem + C::T_Q, 0, k_smem, 1, 2, ksteps, elected, false);
                     tc_commit_elect(BAR(C::B_S + w));
                 }
                 tc_commit_elect(BAR(C::B_KEMPTY + j % C::KST));
@@ -389,7 +393,7 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
                 // the partial output has been added up (LATE: this warpgroup did so before it wrote its probabilities)
                 if (!C::LATE && j > 0) ok = ok && mbar_wait(BAR(C::B_OFREE + (w ^ 1)), ((j - 1) >> 1) & 1, abort_flag, p.status, WF_OFREE);
                 tc_fence_after();
-                mma_results<HD, typename C::R>(tmem + C::T_O + w * C::O_STEP, tmem + C::T_P + w * C::R::COLS, smem_base + C::OFF_V + (j % C::VST) * C::TILE, idesc_o, elected);
+                mma_results<HD, typename C::R>(tmem + C::T_O + w * C::O_STEP, tmem + C::T_P + w * C::R_STEP, smem_base + C::OFF_V + (j % C::VST) * C::TILE, idesc_o, elected);
                 tc_commit_elect(BAR(C::B_O + w));
                 tc_commit_elect(BAR(C::B_VEMPTY + j % C::VST));
             }
@@ -400,12 +404,12 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
         const int w = warp / 4, r = threadIdx.x % 128, row = q0 + r;
         const uint32_t lane_sel = (uint32_t)((warp % 4) * 32) << 16;
         const float *src = row < p.lq ? p.q + ((size_t)unit * p.lq + row) * p.d : nullptr;
-        row_to_tmem(src, p.d, p.vec_q, w * (HD / 2), HD / 64, tmem + lane_sel + C::T_Q, HD / 2, nullptr, r);
+        row_to_tmem(src, p.d, p.vec_q, HD == 64 ? w * 32 : w * 64, HD == 64 || (HD == 96 && w == 1) ? 1 : 2, tmem + lane_sel + C::T_Q, HD / 2, nullptr, r);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(BAR(C::B_Q));
 
-        const uint32_t scores = tmem + lane_sel + C::T_S + w * C::S_STEP, region = tmem + lane_sel + C::T_P + w * C::R::COLS, to = tmem + lane_sel + C::T_O + w * C::O_STEP;
+        const uint32_t scores = tmem + lane_sel + C::T_S + w * C::S_STEP, region = tmem + lane_sel + C::T_P + w * C::R_STEP, to = tmem + lane_sel + C::T_O + w * C::O_STEP;
         const int limit_row = p.causal ? min(p.lk - 1, row + off) : p.lk - 1;
         const int limit_tile = p.causal ? min(p.lk - 1, q0 + off) : p.lk - 1;
         const int cols = (p.d + 15) / 16 * 16;
@@ -418,19 +422,23 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
         bool ok = true;
         for (int j = w; j < n && ok; j += 2) {
             const int k0 = j * TN;
-            ok = ok && mbar_wait(BAR(C::B_S + w), C::LATE ? (j >> 1) & 1 : 0, abort_flag, p.status, WF_S);
+            ok = ok && mbar_wait(BAR(C::B_S + w), C::HALVES ? 0 : (j >> 1) & 1, abort_flag, p.status, WF_S);
             tc_fence_after();
             f32x2 s[32];
             load_scores<false>(scores, s);
             load_scores<false>(scores + 32, s + 16);
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(BAR(C::B_SREAD));
-            if (!C::LATE) {  // the other half of the contraction
+            if (C::LATE || C::HALVES) {
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(BAR(C::B_SREAD));
+            }
+            if (C::HALVES) {
                 ok = ok && mbar_wait(BAR(C::B_S + w), 1, abort_flag, p.status, WF_S);
                 tc_fence_after();
-                load_scores<true>(scores, s);
-                load_scores<true>(scores + 32, s + 16);
+            }
+            if (!C::LATE) {  // the other half of the contraction
+                load_scores<true>(scores + (C::HALVES ? 0 : 64), s);
+                load_scores<true>(scores + (C::HALVES ? 32 : 96), s + 16);
             }
 #pragma unroll
             for (int i = 0; i < 32; i++) s[i] = mul2(s[i], scale2);
@@ -499,7 +507,7 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
         }
         // ---- the two warpgroups' results: each finishes half of the columns, the other half goes to the other one through shared
         // memory (no copy is in flight any more, and after the barrier no product either)
-        constexpr int HALF = HD / 2, ROWB = HALF * 4;
+        constexpr int HALF = HD / 2, ROWB = HALF * 4, SWZ = HD == 96 ? 3 : 7;
         float2 *state = reinterpret_cast<float2 *>(smem_gen);                    // [2][128] maximum and sum
         uint8_t *xo = smem_gen + 2048;                                           // [2][128][HALF]: the half that warpgroup w finishes
         named_bar_sync(1, 256);
@@ -510,7 +518,7 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
             for (int c = 0; c < HALF / 4; c++) {
                 const int i = 2 * c;
                 const ulonglong2 v = w == 0 ? make_ulonglong2(o[HALF / 2 + i], o[HALF / 2 + i + 1]) : make_ulonglong2(o[i], o[i + 1]);
-                *reinterpret_cast<ulonglong2 *>(dst + (((c & ~7) | ((c ^ r) & 7)) << 4)) = v;
+                *reinterpret_cast<ulonglong2 *>(dst + (((c & ~SWZ) | ((c ^ r) & SWZ)) << 4)) = v;
             }
         }
         named_bar_sync(1, 256);
@@ -525,7 +533,7 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
             const f32x2 own2 = pack2(a_own, a_own), other2 = pack2(a_other, a_other);
 #pragma unroll
             for (int c = 0; c < HALF / 4; c++) {
-                const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(from + (((c & ~7) | ((c ^ r) & 7)) << 4));
+                const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(from + (((c & ~SWZ) | ((c ^ r) & SWZ)) << 4));
                 const int i = 2 * c;
                 res[i] = fma2(w == 0 ? o[i] : o[HALF / 2 + i], own2, mul2(v.x, other2));
                 res[i + 1] = fma2(w == 0 ? o[i + 1] : o[HALF / 2 + i + 1], own2, mul2(v.y, other2));
@@ -1092,7 +1100,9 @@ int sm100_f32_attention_fwd(const AttnArgs &a, DeviceState *st, cudaStream_t s)
     guard.pair[1] = 2;  // k or q, and the other one
     guard.pair_limit = score_limit(a, st->sm_count);
     if (rc == EMBER_OK)
-        rc = a.d <= 64 ? launch_fwd<64>(a, mem, mem + k_bytes, guard, st, s) : launch_fwd<128>(a, mem, mem + k_bytes, guard, st, s);
+        rc = a.d <= 64 ? launch_fwd<64>(a, mem, mem + k_bytes, guard, st, s)
+             : a.d <= 96 ? launch_fwd<96>(a, mem, mem + k_bytes, guard, st, s)
+                         : launch_fwd<128>(a, mem, mem + k_bytes, guard, st, s);
     if (rc == EMBER_OK) {
         AttnArgs t = a;
         t.only_if = guard.fallback;
