@@ -274,6 +274,7 @@ struct F32FwdCfg {
     static constexpr int T_O = T_P + 2 * R_STEP, O_STEP = LATE ? HD : 0;
     static_assert(T_O + HD + O_STEP <= 512, "");
     enum { B_Q, B_KFULL, B_KEMPTY = B_KFULL + KST, B_VFULL = B_KEMPTY + KST, B_VEMPTY = B_VFULL + VST, B_S = B_VEMPTY + VST, B_P = B_S + 2, B_O = B_P + 2, B_OFREE = B_O + 2, B_SREAD = B_OFREE + 2, NUM_BARS };
+    static_assert(8 * NUM_BARS + 8 + 4 * kSplitMaxTensors <= 256, "");
 };
 
 struct F32FwdParams {

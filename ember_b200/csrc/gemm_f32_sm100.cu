@@ -40,6 +40,7 @@ struct Cfg {
 };
 
 enum { B_FULL = 0, B_EMPTY = B_FULL + MAX_STAGES, B_ACCFULL = B_EMPTY + MAX_STAGES, B_ACCEMPTY = B_ACCFULL + 2, NUM_BARS = B_ACCEMPTY + 2 };
+static_assert(8 * NUM_BARS + 8 + 4 * kSplitMaxTensors <= 128, "");
 enum { WS_EMPTY = 401, WS_FULL, WS_ACCEMPTY, WS_ACCFULL, WS_SMEM };
 
 struct Params {

@@ -61,7 +61,7 @@ def close(got, want, rel=REL):
     (2, 640, 640, 64, True), (1, 1, 4097, 64, True), (2, 129, 577, 64, False), (1, 511, 513, 64, True), (3, 385, 1025, 64, True),
     (1, 1300, 1290 + 10, 40, False), (2, 200, 1152, 33, True), (1, 600, 1217, 61, False), (1, 1100, 1100, 8, True), (1, 1090, 1090, 3, False),
     (1, 512, 512, 128, True), (2, 127, 641, 128, False), (1, 65, 1023, 80, True), (2, 300, 700, 96, True), (1, 577, 577, 101, False), (1, 640, 576, 72, False),
-    (160, 256, 256, 64, True), (40, 256, 256, 128, False),
+    (160, 256, 256, 64, True), (40, 256, 256, 128, False), (1, 600, 641, 65, False), (2, 450, 520, 88, True), (1, 513, 600, 97, True),
 ])
 def test_edges_of_blocks_and_tiles(units, lq, lk, d, causal):
     x = inputs(units, lq, lk, d)
