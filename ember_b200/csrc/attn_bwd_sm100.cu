@@ -1020,16 +1020,20 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
             const uint32_t k_lo = desc_lo(ka, 16), v_lo = desc_lo(va, 16);
             auto q_addr = [&](int i) { return smem_base + C::OFF_A + (i % C::NA) * C::TILE_BYTES; };
             auto do_addr = [&](int i) { return smem_base + C::OFF_B + (i % C::NB) * C::TILE_BYTES; };
+            // Chains of four MMAs: with an elect.sync and descriptor words for each, 16 MMAs took 1260 to 1350 clocks to issue
+            // beside the compute warps, whatever their width; now 1000 (2 x 32 units x L4096, d 128 causal: 856 -> 745 us;
+            // 36 units x 777 x 1301, d 80: 71.6 -> 67.4 us; 128 units x L2048, d 64, compute-bound: 475 us both).
+            constexpr uint32_t SUB16 = C::SUB_BYTES >> 4;
+            const uint32_t elected = elect_one();
             bool ok = mbar_wait(BAR(C::B_RES), 0, abort_flag, p.status, WB_RES);
             if (warp == W_MMA_A) {
                 // score chain: S^T(0); then per tile dV(i) (reads P^T, dO) and S^T(i+1) (overwrites P^T)
                 auto issue_st = [&](int i) {  // S^T = K Q^T
                     const uint32_t q_lo = desc_lo(q_addr(i), 16);
 #pragma unroll
-                    for (int ks = 0; ks < HD / 16; ks++) {
-                        const uint32_t o16 = ((ks / 4) * C::SUB_BYTES + (ks % 4) * 32) >> 4;
-                        if (!PART || ks < ksteps) mma_ss_lo(tmem + C::T_S, k_lo + o16, q_lo + o16, IDESC_SS, ks > 0);
-                    }
+                    for (int sub = 0; sub < C::NSUB; sub++)
+                        if (!PART || sub * 4 < ksteps)
+                            mma_chain4_ss<2, 4, 6, 2, 4, 6>(tmem + C::T_S, k_lo + sub * SUB16, q_lo + sub * SUB16, IDESC_SS, elected, sub > 0, PART ? ksteps - sub * 4 : 4);
                     tc_commit_elect(BAR(C::B_S));
                 };
                 ok = ok && mbar_wait(BAR(C::B_FULLA + 0), 0, abort_flag, p.status, WB_FULL);
@@ -1042,9 +1046,8 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
                     tc_fence_after();
                     if (lane == 0) TR(8, i);
 #pragma unroll
-                    for (int ks = 0; ks < 8; ks++)  // dV += P^T dO
-                        mma_ts_lo(tmem + C::T_ACC0, tmem + C::T_S + ks * 8, domn_lo + ks * (2048 >> 4), IDESC_TS,
-                                  (i > 0 || ks > 0) ? 1u : 0u);
+                    for (int half = 0; half < 2; half++)  // dV += P^T dO
+                        mma_chain4_ts<8, 16, 24, 128, 256, 384>(tmem + C::T_ACC0, tmem + C::T_S + half * 32, domn_lo + half * 512, IDESC_TS, elected, i > 0 || half > 0);
                     tc_commit_elect(BAR(C::B_EMPTYB + i % C::NB));  // this chain's last read of dO(i)
                     if (i + 1 < n) {
                         ok = ok && mbar_wait(BAR(C::B_FULLA + (i + 1) % C::NA), ((i + 1) / C::NA) & 1, abort_flag,
@@ -1062,10 +1065,9 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
                 auto issue_dpt = [&](int i) {  // dP^T = V dO^T
                     const uint32_t do_lo = desc_lo(do_addr(i), 16);
 #pragma unroll
-                    for (int ks = 0; ks < HD / 16; ks++) {
-                        const uint32_t o16 = ((ks / 4) * C::SUB_BYTES + (ks % 4) * 32) >> 4;
-                        if (!PART || ks < ksteps) mma_ss_lo(tmem + C::T_DP, v_lo + o16, do_lo + o16, IDESC_SS, ks > 0);
-                    }
+                    for (int sub = 0; sub < C::NSUB; sub++)
+                        if (!PART || sub * 4 < ksteps)
+                            mma_chain4_ss<2, 4, 6, 2, 4, 6>(tmem + C::T_DP, v_lo + sub * SUB16, do_lo + sub * SUB16, IDESC_SS, elected, sub > 0, PART ? ksteps - sub * 4 : 4);
                     tc_commit_elect(BAR(C::B_DP));
                     tc_commit_elect(BAR(C::B_EMPTYB + i % C::NB));  // this chain's only read of dO(i)
                 };
@@ -1081,14 +1083,12 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
                     tc_fence_after();
                     if (lane == 0) TR(12, i);
 #pragma unroll
-                    for (int ks = 0; ks < 8; ks++)  // dQ(i) = dS K: 16 keys per step
-                        mma_ss_lo(tmem + C::T_DP, dsmn_lo + ks * (2048 >> 4), kmn_lo + ks * (2048 >> 4), IDESC_DQ, ks > 0);
+                    for (int half = 0; half < 2; half++)  // dQ(i) = dS K: 16 keys per step
+                        mma_chain4_ss<128, 256, 384, 128, 256, 384>(tmem + C::T_DP, dsmn_lo + half * 512, kmn_lo + half * 512, IDESC_DQ, elected, half > 0);
                     tc_commit_elect(BAR(C::B_DQ));  // the drain warps copy dQ(i) out while dK(i) is multiplied
 #pragma unroll
-                    for (int ks = 0; ks < 8; ks++) {  // dK += dS^T Q: 16 queries per step
-                        const uint32_t o16 = ((ks / 4) * C::SUB_BYTES + (ks % 4) * 32) >> 4;
-                        mma_ss_lo(tmem + C::T_ACC1, ds_lo + o16, qmn_lo + ks * (2048 >> 4), IDESC_TS, (i > 0 || ks > 0) ? 1u : 0u);
-                    }
+                    for (int half = 0; half < 2; half++)  // dK += dS^T Q: 16 queries per step
+                        mma_chain4_ss<2, 4, 6, 128, 256, 384>(tmem + C::T_ACC1, ds_lo + half * SUB16, qmn_lo + half * 512, IDESC_TS, elected, i > 0 || half > 0);
                     tc_commit_elect(BAR(C::B_DSFREE));
                     tc_commit_elect(BAR(C::B_EMPTYA + i % C::NA));  // this chain's last read of Q(i)
                     if (lane == 0) TR(13, i);

@@ -322,6 +322,39 @@ __device__ __forceinline__ void mma_ts_lo(uint32_t d_tmem, uint32_t a_tmem, uint
         : "memory");
 }
 
+// Four MMAs of 16 contraction steps each in one asm block, operands A1..A3 and B1..B3 further than the first (shared memory: units of
+// 16 bytes, tensor memory: columns). What an MMA costs to issue beside busy compute warps is the instructions it is made of (they leave
+// the scheduler's instruction cache), so `elected` (elect_one) is taken once per loop, not per MMA. left: MMAs from the left-th on are
+// predicated off (contractions that stop early); 4 or more: all four.
+#define EMBER_CHAIN4_HEAD "{\n.reg .pred p, q, e;\n.reg .b64 da, db;\n.reg .b32 t, u;\nsetp.ne.b32 e, %4, 0;\nsetp.ne.b32 p, %5, 0;\nsetp.gt.and.s32 q, %13, 0, e;\n"
+template <int A1, int A2, int A3, int B1, int B2, int B3>
+__device__ __forceinline__ void mma_chain4_ss(uint32_t d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t elected, uint32_t acc, int left = 4)
+{
+    asm volatile(EMBER_CHAIN4_HEAD
+                 "mov.b64 da, {%1, %6};\nmov.b64 db, {%2, %6};\n@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n"
+                 "setp.gt.and.s32 q, %13, 1, e;\nsetp.eq.u32 p, 0, 0;\n"
+                 "add.u32 u, %1, %7;\nmov.b64 da, {u, %6};\nadd.u32 t, %2, %10;\nmov.b64 db, {t, %6};\n@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n"
+                 "setp.gt.and.s32 q, %13, 2, e;\n"
+                 "add.u32 u, %1, %8;\nmov.b64 da, {u, %6};\nadd.u32 t, %2, %11;\nmov.b64 db, {t, %6};\n@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n"
+                 "setp.gt.and.s32 q, %13, 3, e;\n"
+                 "add.u32 u, %1, %9;\nmov.b64 da, {u, %6};\nadd.u32 t, %2, %12;\nmov.b64 db, {t, %6};\n@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n}\n"
+                 ::"r"(d), "r"(a), "r"(b), "r"(idesc), "r"(elected), "r"(acc), "r"(kDescHiSw128), "n"(A1), "n"(A2), "n"(A3), "n"(B1), "n"(B2), "n"(B3), "r"(left) : "memory");
+}
+template <int A1, int A2, int A3, int B1, int B2, int B3>
+__device__ __forceinline__ void mma_chain4_ts(uint32_t d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t elected, uint32_t acc, int left = 4)
+{
+    asm volatile(EMBER_CHAIN4_HEAD
+                 "mov.b64 db, {%2, %6};\n@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, p;\n"
+                 "setp.gt.and.s32 q, %13, 1, e;\nsetp.eq.u32 p, 0, 0;\n"
+                 "add.u32 u, %1, %7;\nadd.u32 t, %2, %10;\nmov.b64 db, {t, %6};\n@q tcgen05.mma.cta_group::1.kind::f16 [%0], [u], db, %3, p;\n"
+                 "setp.gt.and.s32 q, %13, 2, e;\n"
+                 "add.u32 u, %1, %8;\nadd.u32 t, %2, %11;\nmov.b64 db, {t, %6};\n@q tcgen05.mma.cta_group::1.kind::f16 [%0], [u], db, %3, p;\n"
+                 "setp.gt.and.s32 q, %13, 3, e;\n"
+                 "add.u32 u, %1, %9;\nadd.u32 t, %2, %12;\nmov.b64 db, {t, %6};\n@q tcgen05.mma.cta_group::1.kind::f16 [%0], [u], db, %3, p;\n}\n"
+                 ::"r"(d), "r"(a), "r"(b), "r"(idesc), "r"(elected), "r"(acc), "r"(kDescHiSw128), "n"(A1), "n"(A2), "n"(A3), "n"(B1), "n"(B2), "n"(B3), "r"(left) : "memory");
+}
+#undef EMBER_CHAIN4_HEAD
+
 // ---------------------------------------------------------------- CTA pairs (cta_group::2)
 // Two CTAs of a cluster (ranks 0 and 1, on the two SMs of one TPC) act as one 256-row MMA: rank 0
 // issues, each CTA supplies its own 128 rows of A and its own half of B's N columns from its own
