@@ -1,7 +1,8 @@
 // Prefill attention forward for sm_100a: bf16 in/out, float32 softmax and accumulation.
 //
 // One CTA owns 256 consecutive query rows of one (batch*head) as two 128-row tiles whose softmax
-// warpgroups run half a period apart, so that the tensor core always has the other tile's MMAs.
+// warpgroups run half a period apart, so that the tensor core always has the other tile's MMAs. (Small launches: 128 rows, one tile that both
+// warpgroups work on; see ONE and fwd_block_rows.)
 //
 //   warps 0-3   softmax + epilogue of tile 0 (one thread per query row, row state in registers)
 //   warps 4-7   softmax + epilogue of tile 1
@@ -97,7 +98,7 @@ struct FwdParams {
     int d;  // elements per row of q, k, v and out in memory (a multiple of 8, <= HD): the kernel works on
             // HD columns, the TMA copies read the columns past d as zero and the epilogue skips them
     int causal;
-    int block_rows;  // query rows per CTA: 256 (two tiles) or 128 (tile 0 alone; tile 1's warps idle)
+    int block_rows;  // query rows per CTA: 256 (two tiles) or 128 (ONE)
     float scale_log2;  // scale * log2(e)
     DeviceStatus *status;
     WorkOrder order;
@@ -112,11 +113,6 @@ struct FwdParams {
 // EMU: of every 4 pairs of exponentials, how many are evaluated as a polynomial on the FMA pipe
 // instead of the MUFU (0..4).
 // MMA, commit, allocation and arrival forms of a single CTA or of a CTA pair.
-template <bool PAIR>
-__device__ __forceinline__ void f_mma_ss(uint32_t d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t acc)
-{
-    if constexpr (PAIR) mma_ss_lo_pair(d, a, b, idesc, acc); else mma_ss_lo(d, a, b, idesc, acc);
-}
 __device__ __forceinline__ void mma_ts_lo_pair(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t idesc, uint32_t accumulate)
 {
     asm volatile(
@@ -130,11 +126,6 @@ __device__ __forceinline__ void mma_ts_lo_pair(uint32_t d_tmem, uint32_t a_tmem,
         "}\n"
         ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(kDescHiSw128)
         : "memory");
-}
-template <bool PAIR>
-__device__ __forceinline__ void f_mma_ts(uint32_t d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t acc)
-{
-    if constexpr (PAIR) mma_ts_lo_pair(d, a, b, idesc, acc); else mma_ts_lo(d, a, b, idesc, acc);
 }
 template <bool PAIR>
 __device__ __forceinline__ void f_commit(uint32_t bar)  // PAIR: the barrier of BOTH CTAs gets the arrival
@@ -156,16 +147,18 @@ __device__ __forceinline__ void f_tma_3d(uint32_t dst, const CUtensorMap *m, uin
     if constexpr (PAIR) tma_load_3d_pair(dst, m, bar, c0, c1, c2); else tma_load_3d(dst, m, bar, c0, c1, c2);
 }
 
+// ONE: one query tile per CTA. Both softmax warpgroups work on it, a row's keys [0, 64) and [64, 128) of every tile in a thread of each, which
+// agree on the row's maximum through shared memory.
 // PART: head dimensions below HD. The tiles in shared memory keep HD columns (zeros past d), but the score
 // products stop after the last 16 columns that hold anything and the PV products are that many columns wide.
-template <int HD, int EMU, bool PAIR, bool PART = false>
+template <int HD, int EMU, bool PAIR, bool PART = false, bool ONE = false>
 __global__ void __launch_bounds__(FWD_THREADS, 1)
     sm100_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                      const __grid_constant__ CUtensorMap tm_v, const FwdParams p)
 {
     using C = FwdCfg<HD, PAIR>;
     static_assert(!PAIR || HD == 128, "the pair form halves V along its 128 columns");
-    static_assert(!PAIR || !PART, "pairs take whole tiles");
+    static_assert(!PAIR || (!PART && !ONE), "pairs take whole tiles, two of them");
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t *smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -213,7 +206,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 1)
         // its last key tile fully masked), and a pair of tiles exists if its first tile does
         const int qs_first = PAIR ? qblock * 512 + t * 256 : q_base + t * 128;
         const int qs_last = PAIR ? qs_first + 128 : qs_first;
-        if (qs_first >= p.lq || (!PAIR && t == 1 && p.block_rows == 128)) {
+        if (qs_first >= p.lq || (ONE && t == 1)) {
             n_t[t] = 0;
         } else {
             const int visible = p.causal ? min(lk, qs_last + 128 + off) : lk;
@@ -235,7 +228,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 1)
         }
         for (int t = 0; t < 2; t++) {
             mbar_init(BAR(B_S + t), 1);
-            mbar_init(BAR(B_R + t), PAIR ? 8 : 4);          // one arrival per softmax warp (of both CTAs of a pair)
+            mbar_init(BAR(B_R + t), PAIR || ONE ? 8 : 4);   // one arrival per softmax warp (of both CTAs of a pair)
             mbar_init(BAR(B_P + 2 * t), PAIR ? 8 : 4);      // first 64 keys of P written (one arrival per warp)
             mbar_init(BAR(B_P + 2 * t + 1), PAIR ? 8 : 4);  // last 64 keys of P written
             mbar_init(BAR(B_O + t), 1);
@@ -267,7 +260,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 1)
     pdl_wait();
 
     if (warp >= 8) {
-        reg_dealloc_40();
+        if constexpr (ONE) asm volatile("setmaxnreg.dec.sync.aligned.u32 104;"); else reg_dealloc_40();
         if (warp == 10 && lane == 0) {
             // ------------------------------------------------------------ TMA producer
             // In a pair every CTA loads its own tiles; the bytes of both are counted by rank 0's
@@ -323,6 +316,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 1)
             const uint32_t IDESC_O = idesc_bf16_f32(PAIR ? 256 : 128, ksteps * 16, 0, 1);
             const int nt = n_t[t], no = n_t[1 - t];  // key tiles of this tile / of the other tile
             const uint32_t q_lo = desc_lo(smem_base + C::OFF_Q + t * C::TILE_BYTES, 16);
+            const uint32_t elected = elect_one();
             bool ok = mbar_wait(BAR(B_Q), 0, abort_flag, p.status, W_MMA_Q);
             // The score buffer is used in the order S0(0) S1(0) S0(1) S1(1) ...; each user waits until
             // the softmax warps of the previous user have copied their scores out.
@@ -340,24 +334,37 @@ __global__ void __launch_bounds__(FWD_THREADS, 1)
                 }
                 tc_fence_after();
                 const uint32_t k_lo = desc_lo(smem_base + C::OFF_K + (j % C::KSTAGES) * C::K_BYTES, 16);
+                if constexpr (PAIR) {
 #pragma unroll
-                for (int ks = 0; ks < HD / 16; ks++) {
-                    const uint32_t o16 = ((ks / 4) * C::SUB_BYTES + (ks % 4) * 32) >> 4;
-                    const uint32_t k16 = ((ks / 4) * C::K_SUB_BYTES + (ks % 4) * 32) >> 4;
-                    if (!PART || ks < ksteps) f_mma_ss<PAIR>(tmem + C::TMEM_S, q_lo + o16, k_lo + k16, IDESC_S, ks > 0);
+                    for (int ks = 0; ks < HD / 16; ks++) {
+                        const uint32_t o16 = ((ks / 4) * C::SUB_BYTES + (ks % 4) * 32) >> 4;
+                        const uint32_t k16 = ((ks / 4) * C::K_SUB_BYTES + (ks % 4) * 32) >> 4;
+                        mma_ss_lo_pair(tmem + C::TMEM_S, q_lo + o16, k_lo + k16, IDESC_S, ks > 0);
+                    }
+                } else {
+#pragma unroll
+                    for (int sub = 0; sub < C::NSUB; sub++)  // (a chain instead of single MMAs: 1 % at d 64 and long sequences, else the same)
+                        if (!PART || sub * 4 < ksteps)
+                            mma_chain4_ss<2, 4, 6, 2, 4, 6>(tmem + C::TMEM_S, q_lo + sub * (C::SUB_BYTES >> 4), k_lo + sub * (C::SUB_BYTES >> 4), IDESC_S, elected, sub > 0, PART ? ksteps - sub * 4 : 4);
                 }
                 f_commit<PAIR>(BAR(B_S + t));
             };
             // O_t += P_t(j) V_j for keys [64*half, 64*half + 64) of the tile
             auto issue_pv_half = [&](int j, int half) {
                 ok = ok && mbar_wait(BAR(B_P + 2 * t + half), j & 1, abort_flag, p.status, W_MMA_P);
+                if (ONE && half == 0) ok = ok && mbar_wait(BAR(B_P + 1), j & 1, abort_flag, p.status, W_MMA_P);  // each warpgroup rescales half of O's columns
                 tc_fence_after();
                 const uint32_t v_lo = desc_lo(smem_base + C::OFF_V + (j % C::VSTAGES) * C::V_BYTES, C::SUB_BYTES);
+                if constexpr (PAIR) {
 #pragma unroll
-                for (int k4 = 0; k4 < 4; k4++) {
-                    const int ks = half * 4 + k4;
-                    f_mma_ts<PAIR>(tmem + C::TMEM_O + t * HD, tmem + C::TMEM_P + t * 64 + ks * 8, v_lo + ks * (2048 >> 4),
-                                   IDESC_O, (j > 0 || ks > 0) ? 1u : 0u);
+                    for (int k4 = 0; k4 < 4; k4++) {
+                        const int ks = half * 4 + k4;
+                        mma_ts_lo_pair(tmem + C::TMEM_O + t * HD, tmem + C::TMEM_P + t * 64 + ks * 8, v_lo + ks * (2048 >> 4),
+                                       IDESC_O, (j > 0 || ks > 0) ? 1u : 0u);
+                    }
+                } else {
+                    mma_chain4_ts<8, 16, 24, 128, 256, 384>(tmem + C::TMEM_O + t * HD, tmem + C::TMEM_P + t * 64 + half * 32, v_lo + half * 512,
+                                                            IDESC_O, elected, j > 0 || half > 0);
                 }
                 if (half == 1) f_commit<PAIR>(BAR(B_O + t));
             };
@@ -400,6 +407,167 @@ __global__ void __launch_bounds__(FWD_THREADS, 1)
                 f_commit<PAIR>(BAR(B_VEMPTY + j % C::VSTAGES));  // our reads of V(j) are issued
             }
         }
+    } else if constexpr (ONE) {
+        // ---------------------------------------------------------------- softmax + epilogue, one tile
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 200;");  // 8 x 32 x 200 + 4 x 32 x 104 == 384 x 168 at launch
+        const int half = warp / 4;                // which 64 keys of a tile
+        const int r = threadIdx.x % 128;          // row inside the tile == TMEM lane
+        const int row = q_base + r;
+        const uint32_t lane_sel = (uint32_t)((warp % 4) * 32) << 16;
+        const uint32_t ts = tmem + lane_sel + C::TMEM_S + half * 64, tp = tmem + lane_sel + C::TMEM_P + half * 32, to = tmem + lane_sel + C::TMEM_O;
+        const int nk = n_t[0];
+        const float c = fabsf(p.scale_log2);      // a negative scale's sign goes to the scores
+        const int limit_row = p.causal ? min(lk - 1, row + off) : lk - 1;
+        const int limit_tile = p.causal ? min(lk - 1, q_base + off) : lk - 1;
+        // what the two threads of a row tell one another, in the place of the second query tile: maxima (two tiles' worth, so that
+        // one barrier of the two warps per tile is enough) and, at the end, sums
+        float *mine = reinterpret_cast<float *>(smem_gen + C::OFF_Q + C::TILE_BYTES) + half * 128 + r;
+        const float *other = reinterpret_cast<const float *>(smem_gen + C::OFF_Q + C::TILE_BYTES) + (half ^ 1) * 128 + r;
+
+        float m_ref = -INFINITY, l = 0.f;
+        bool ok = true;
+        for (int j = 0; j < nk; j++) {
+            ok = ok && mbar_wait(BAR(B_S), j & 1, abort_flag, p.status, W_SM_S);
+            tc_fence_after();
+            float s[64];
+#pragma unroll
+            for (int ch = 0; ch < 2; ch++) {
+                uint32_t u[32];
+                tmem_ld_32x32b_x32(ts + ch * 32, u);
+#pragma unroll
+                for (int i = 0; i < 32; i++) s[ch * 32 + i] = __uint_as_float(u[i]);
+            }
+            tmem_wait_ld();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(BAR(B_R));
+            if (p.scale_log2 < 0.f) {
+#pragma unroll
+                for (int i = 0; i < 64; i++) s[i] = -s[i];
+            }
+            if (j * 128 + 127 > limit_tile) {
+#pragma unroll
+                for (int i = 0; i < 64; i++)
+                    if (j * 128 + half * 64 + i > limit_row) s[i] = -INFINITY;
+            }
+            float mx8[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) mx8[i] = s[i];
+#pragma unroll
+            for (int i = 8; i + 16 <= 64; i += 16)
+#pragma unroll
+                for (int k8 = 0; k8 < 8; k8++) mx8[k8] = max3(mx8[k8], s[i + k8], s[i + 8 + k8]);
+#pragma unroll
+            for (int k8 = 0; k8 < 8; k8++) mx8[k8] = fmaxf(mx8[k8], s[56 + k8]);
+            float mx = max3(max3(mx8[0], mx8[1], mx8[2]), max3(mx8[3], mx8[4], mx8[5]), fmaxf(mx8[6], mx8[7]));
+            mine[(j & 1) * 256] = mx;
+            named_bar_sync(4 + warp % 4, 64);
+            mx = fmaxf(mx, other[(j & 1) * 256]);
+            const float m_new = fmaxf(m_ref, mx * c);
+            bool o_done = (j == 0);
+            if (j == 0) {
+                m_ref = m_new;  // finite: key 0 is visible to every row
+            } else {
+                const bool need = (m_new - m_ref) > RESCALE_THRESHOLD;
+                if (__any_sync(0xffffffffu, need)) {  // the same in both warps
+                    const float alpha = ex2(m_ref - m_new);
+                    m_ref = m_new;
+                    l *= alpha;
+                    ok = ok && mbar_wait(BAR(B_O), (j - 1) & 1, abort_flag, p.status, W_SM_O);
+                    o_done = true;
+                    tc_fence_after();
+#pragma unroll
+                    for (int ch = 0; ch < HD / 64; ch++) {
+                        uint32_t o[32];
+                        tmem_ld_32x32b_x32(to + half * (HD / 2) + ch * 32, o);
+                        tmem_wait_ld();
+#pragma unroll
+                        for (int i = 0; i < 32; i++) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+                        tmem_st_32x32b_x32(to + half * (HD / 2) + ch * 32, o);
+                    }
+                }
+            }
+            const f32x2 negm2 = pack2(-m_ref, -m_ref);
+            const f32x2 c2 = pack2(c, c);
+            f32x2 sum2[4] = {0, 0, 0, 0};  // bit pattern of (0.f, 0.f)
+            uint32_t pk[2][16];
+#pragma unroll
+            for (int ch = 0; ch < 2; ch++)
+#pragma unroll
+                for (int i = 0; i < 16; i++) {
+                    const f32x2 x2 = fma2(pack2(s[ch * 32 + 2 * i], s[ch * 32 + 2 * i + 1]), c2, negm2);
+                    float p0, p1;
+                    if (i % 4 < EMU) {  // polynomial on the FMA pipe
+                        exp2_poly2(x2, p0, p1);
+                    } else {            // MUFU
+                        float x0, x1;
+                        unpack2(x2, x0, x1);
+                        p0 = ex2(x0);
+                        p1 = ex2(x1);
+                    }
+                    sum2[i & 3] = add2(sum2[i & 3], pack2(p0, p1));
+                    pk[ch][i] = pack_bf16(p0, p1);
+                }
+            if (!o_done) {  // PV(j-1) must have read the old P
+                ok = ok && mbar_wait(BAR(B_O), (j - 1) & 1, abort_flag, p.status, W_SM_O);
+                tc_fence_after();
+            }
+            tmem_st_32x32b_x16(tp, pk[0]);
+            tmem_st_32x32b_x16(tp + 16, pk[1]);
+            tmem_wait_st();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(BAR(B_P + half));
+            float a0, a1;
+            unpack2(add2(add2(sum2[0], sum2[1]), add2(sum2[2], sum2[3])), a0, a1);
+            l += a0 + a1;
+        }
+
+        if (nk > 0) {
+            mine[512] = l;
+            named_bar_sync(4 + warp % 4, 64);
+            l = half == 0 ? l + other[512] : other[512] + l;
+            ok = ok && mbar_wait(BAR(B_O), (nk - 1) & 1, abort_flag, p.status, W_SM_OFINAL);
+            tc_fence_after();
+            const float inv = 1.f / l;
+            // as below, each warp half of its rows' columns
+            constexpr int ROWB = HD * 2, CHUNKS = ROWB / 32;  // 16-byte chunks of half a row
+            uint8_t *stage = smem_gen + C::OFF_Q;
+#pragma unroll
+            for (int ch = 0; ch < HD / 64; ch++) {
+                uint32_t o[32];
+                tmem_ld_32x32b_x32(to + half * (HD / 2) + ch * 32, o);
+                tmem_wait_ld();
+#pragma unroll
+                for (int q4 = 0; q4 < 4; q4++) {  // 8 columns = one 16-byte chunk
+                    uint4 wv;
+                    wv.x = pack_bf16(__uint_as_float(o[q4 * 8 + 0]) * inv, __uint_as_float(o[q4 * 8 + 1]) * inv);
+                    wv.y = pack_bf16(__uint_as_float(o[q4 * 8 + 2]) * inv, __uint_as_float(o[q4 * 8 + 3]) * inv);
+                    wv.z = pack_bf16(__uint_as_float(o[q4 * 8 + 4]) * inv, __uint_as_float(o[q4 * 8 + 5]) * inv);
+                    wv.w = pack_bf16(__uint_as_float(o[q4 * 8 + 6]) * inv, __uint_as_float(o[q4 * 8 + 7]) * inv);
+                    const int chunk = half * CHUNKS + ch * 4 + q4;
+                    const int sw = (chunk & ~7) | ((chunk ^ r) & 7);
+                    *reinterpret_cast<uint4 *>(stage + r * ROWB + sw * 16) = wv;
+                }
+            }
+            __syncwarp();
+            constexpr int ROWS_PER_ST = 32 / CHUNKS;
+            const int chunk = half * CHUNKS + lane % CHUNKS;
+#pragma unroll
+            for (int it = 0; it < 32 / ROWS_PER_ST; it++) {
+                const int rr = (warp % 4) * 32 + it * ROWS_PER_ST + lane / CHUNKS;
+                const int sw = (chunk & ~7) | ((chunk ^ rr) & 7);
+                const uint4 wv = *reinterpret_cast<const uint4 *>(stage + rr * ROWB + sw * 16);
+                const int grow = q_base + rr;
+                __nv_bfloat16 *dst = p.out + ((size_t)bh * p.lq + grow) * p.d + chunk * 8;
+                if (ok && grow < p.lq && chunk * 8 < p.d &&
+                    EMBER_STORE_OK(dst, p.out, (size_t)p.order.units * p.lq * p.d * 2, 16, p.status))
+                    *reinterpret_cast<uint4 *>(dst) = wv;
+            }
+            if (half == 0 && ok && row < p.lq && p.lse &&
+                EMBER_STORE_OK(p.lse + (size_t)bh * p.lq + row, p.lse, (size_t)p.order.units * p.lq * 4, 4, p.status))
+                p.lse[(size_t)bh * p.lq + row] = (m_ref + log2f(l)) * LN2_F;
+        }
     } else {
         // ---------------------------------------------------------------- softmax + epilogue
         reg_alloc_232();
@@ -421,7 +589,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 1)
             if constexpr (PAIR) mbar_arrive_cluster(bar); else mbar_arrive(bar);
         };
 
-        float m_ref = -INFINITY, l = 0.f;
+        float m_ref = -INFINITY, l0 = 0.f, l1 = 0.f;  // sums over keys [0, 64) and [64, 128) of the tiles, as the one-tile form has them
         bool ok = true;
         for (int j = 0; j < nk; j++) {
             ok = ok && mbar_wait(BAR(B_S + t), j & 1, abort_flag, p.status, W_SM_S);
@@ -476,7 +644,8 @@ __global__ void __launch_bounds__(FWD_THREADS, 1)
                 if (__any_sync(0xffffffffu, need)) {
                     const float alpha = ex2(m_ref - m_new);
                     m_ref = m_new;
-                    l *= alpha;
+                    l0 *= alpha;
+                    l1 *= alpha;
                     ok = ok && mbar_wait(BAR(B_O + t), (j - 1) & 1, abort_flag, p.status, W_SM_O);
                     o_done = true;
                     tc_fence_after();
@@ -493,9 +662,9 @@ __global__ void __launch_bounds__(FWD_THREADS, 1)
             }
             const f32x2 negm2 = pack2(-m_ref, -m_ref);
             const f32x2 c2 = pack2(c, c);
-            f32x2 sum2[4] = {0, 0, 0, 0};  // bit pattern of (0.f, 0.f)
 #pragma unroll
             for (int half = 0; half < 2; half++) {
+                f32x2 sum2[4] = {0, 0, 0, 0};  // bit pattern of (0.f, 0.f)
                 uint32_t pk[2][16];
 #pragma unroll
                 for (int c2i = 0; c2i < 2; c2i++) {
@@ -528,18 +697,16 @@ __global__ void __launch_bounds__(FWD_THREADS, 1)
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) arrive(bar_p + 8u * (uint32_t)half);
-            }
-            {
                 float a0, a1;
                 unpack2(add2(add2(sum2[0], sum2[1]), add2(sum2[2], sum2[3])), a0, a1);
-                l += a0 + a1;
+                (half == 0 ? l0 : l1) += a0 + a1;
             }
         }
 
         if (nk > 0) {
             ok = ok && mbar_wait(BAR(B_O + t), (nk - 1) & 1, abort_flag, p.status, W_SM_OFINAL);
             tc_fence_after();
-            const float inv = 1.f / l;
+            const float l = l0 + l1, inv = 1.f / l;
             const bool store = ok && row < p.lq;
             // O / l as bf16 goes through shared memory so that the global stores are coalesced (a
             // thread owns a whole row; storing rows directly makes every store instruction touch 32
@@ -642,13 +809,14 @@ int launch_pair(const AttnArgs &a, DeviceState *st, cudaStream_t s)
     return EMBER_OK;
 }
 
-// Query rows per CTA. Two tiles (256 rows) share the key/value stream and interleave their softmax
-// with each other's MMAs: 1.3x the throughput per SM of a CTA that works on tile 0 alone. One tile per
-// CTA (128 rows) makes twice as many CTAs of half the length, which wins while the SMs are not all
-// busy: measured at D = 128 on 148 SMs, a launch of up to one 128-row CTA per SM is 12-30 % faster that
-// way (8 units x L 2048: 32.8 -> 26.8 us causal, 39.6 -> 28.7 us without a mask), and under a causal
-// mask, whose last blocks are the longest, up to two per SM from L = 2048 (16 x 2048: 34.3 -> 30.8 us;
-// 8 x 4096: 59.5 -> 46.5 us); beyond that the two-tile form is faster (16 x 4096: 61.7 against 89.1 us).
+// Query rows per CTA. Two tiles (256 rows) share the key/value stream and interleave their softmax with each other's MMAs; one tile
+// (128 rows) has both softmax warpgroups to itself and is held by the exponentials of 128 x 128 scores (1024 clocks of every
+// scheduler's MUFU, which nothing else of the CTA overlaps: about 1860 a step), so that two of its steps take 1.3 times as long as one
+// step of two tiles. But it makes twice as many CTAs, of little more than half the length: which form ends first is
+// estimated from the lengths (in steps of one tile; a CTA's start and end are 3.7 of them), heaviest CTAs first.
+// Measured, us, two tiles / one: 8 units x L2048 37 / 24.6, causal 16 x 2048 32.1 / 25.8, 16 x 1024 21.5 / 14.8, 13 x 1536 24.6 / 17.7, 32 x 1024 19.8 / 18.4,
+// 8 x 4096 64 / 42, 4 x 100 rows x 4096 keys 42 / 38; the other way round 16 x 4096 64 / 82, 32 x 2048 42 / 53, 64 x 512 13.0 / 14.4, 36 x 777 x 1301
+// without a mask 24.6 / 32.5. (While the second warpgroup of a one-tile CTA was idle its step took 2000 to 2700 clocks: 8 x 2048 29.6.)
 // A row's arithmetic does not depend on the choice: both forms give the same bits.
 // ember_set_forward_block_rows (initially EMBER_FWD_ROWS=128|256) forces one form, for tests and tuning.
 static int g_fwd_rows = -1;  // -1: not read from the environment yet; 0: choose per call
@@ -667,15 +835,30 @@ static int fwd_block_rows(const AttnArgs &a, DeviceState *st)
 {
     const int forced = fwd_rows_setting();
     if (forced == 128 || forced == 256) return forced;
-    const long long ctas128 = (long long)a.bh * ((a.lq + 127) / 128);
+    if (a.lq <= 128) return 128;
     const int sms = st->sm_count > 0 ? st->sm_count : 148;
-    if (a.lq <= 128) return 256;  // a single tile either way
+    const long long ctas128 = (long long)a.bh * ((a.lq + 127) / 128);
     if (ctas128 <= sms) return 128;
-    if (a.causal && a.lq >= 2048 && ctas128 <= 2LL * sms) return 128;
-    return 256;
+    if (ctas128 > 4LL * sms) return 256;
+    auto end_of = [&](int rows, double step) {
+        const int blocks = (a.lq + rows - 1) / rows;
+        const long long ctas = (long long)a.bh * blocks;
+        auto length = [&](long long rank) {  // of the rank-th longest CTA
+            const int b = blocks - 1 - (int)(rank / a.bh);
+            const int visible = a.causal ? min(a.lk, (b + 1) * rows + a.lk - a.lq) : a.lk;
+            return 3.7 + step * ((visible + 127) / 128);
+        };
+        double total = 0;
+        for (int i = 0; i < blocks; i++) total += (double)a.bh * length((long long)i * a.bh);
+        double end = fmax(length(0), total / sms);
+        end = fmax(end, (double)((ctas + sms - 1) / sms) * length(ctas - 1));
+        if (ctas > sms) end = fmax(end, length(sms - 1) + length(sms));
+        return end;
+    };
+    return end_of(128, 1.0) < end_of(256, 1.55) ? 128 : 256;
 }
 
-template <int HD, int EMU, bool PART>
+template <int HD, int EMU, bool PART, bool ONE>
 int launch_form(const AttnArgs &a, DeviceState *st, cudaStream_t s)
 {
     using C = FwdCfg<HD>;
@@ -691,7 +874,7 @@ int launch_form(const AttnArgs &a, DeviceState *st, cudaStream_t s)
     p.lq = a.lq;
     p.lk = a.lk;
     p.d = a.d;
-    p.block_rows = fwd_block_rows(a, st);
+    p.block_rows = ONE ? 128 : 256;
     p.causal = a.causal;
     p.scale_log2 = a.scale * LOG2E_F;
     p.status = st->status;
@@ -699,7 +882,7 @@ int launch_form(const AttnArgs &a, DeviceState *st, cudaStream_t s)
     p.chunk = a.lk;
     p.lens_div = 1;
     p.seq_lens = nullptr;
-    auto kern = sm100_fwd_kernel<HD, EMU, false, PART>;
+    auto kern = sm100_fwd_kernel<HD, EMU, false, PART, ONE>;
     static SmemOptIn opt_in;
     EMBER_CUDA_TRY(opt_in(kern, C::SMEM_BYTES));
     p.order = make_work_order(a.bh, (a.lq + p.block_rows - 1) / p.block_rows, st->sm_count, ((size_t)a.lq + a.lk) * HD * 2 * 2,  // Q, O, K, V
@@ -718,7 +901,9 @@ int launch_form(const AttnArgs &a, DeviceState *st, cudaStream_t s)
 template <int HD, int EMU>
 int launch(const AttnArgs &a, DeviceState *st, cudaStream_t s)
 {
-    return a.d <= HD - 16 ? launch_form<HD, EMU, true>(a, st, s) : launch_form<HD, EMU, false>(a, st, s);
+    const bool one = fwd_block_rows(a, st) == 128;
+    if (a.d <= HD - 16) return one ? launch_form<HD, EMU, true, true>(a, st, s) : launch_form<HD, EMU, true, false>(a, st, s);
+    return one ? launch_form<HD, EMU, false, true>(a, st, s) : launch_form<HD, EMU, false, false>(a, st, s);
 }
 
 // Merges the normalised partial outputs of the splits of one (unit, query row):
