@@ -18,7 +18,7 @@ OBJ = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "libember_b200.so")
 
 SOURCES = ["core.cu", "tma_host.cu", "attn_simt.cu", "attn_decode.cu", "attn_fwd_sm100.cu",
-           "attn_bwd_sm100.cu", "split_f32.cu", "attn_f32_sm100.cu", "api.cu", "gemm_simt.cu", "gemm_sm100.cu", "gemm_f32_sm100.cu", "gemm_skinny_sm100.cu", "gemm_skinny_f32.cu", "linear_api.cu",
+           "attn_bwd_sm100.cu", "split_f32.cu", "attn_f32_sm100.cu", "api.cu", "gemm_simt.cu", "gemm_sm100.cu", "gemm_f32_sm100.cu", "gemm_skinny_sm100.cu", "gemm_skinny_f32.cu", "gemm_narrow_f32.cu", "linear_api.cu",
            "column_sums.cu",
            "softmax_ce.cu", "kv_cache.cu", "decode_sm100.cu", "comm.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-lineinfo",

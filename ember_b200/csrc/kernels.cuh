@@ -186,6 +186,10 @@ int make_tensor_map_bf16_view(CUtensorMap *map, const MatView &v, uint32_t box_c
 // Float32, at most 16 rows, y = x w + b (gemm_skinny_f32.cu): a decode step's projections on the CUDA cores.
 bool skinny_f32_supported(const GemmArgs &g);
 int skinny_f32_gemm(const GemmArgs &g, DeviceState *st, cudaStream_t s);
+
+// Float32, at most 12 columns, y = x w + b (gemm_narrow_f32.cu): a small classifier's logits on the CUDA cores.
+bool narrow_f32_supported(const GemmArgs &g);
+int narrow_f32_gemm(const GemmArgs &g, cudaStream_t s);
 // Float32 storage on the tensor cores, operands as three bf16 planes each (gemm_f32_sm100.cu, split_f32.cuh): a row-major view's rows
 // padded to 8 columns. _us: an estimate of the time, without the splitting.
 struct SplitGuard;

@@ -237,6 +237,7 @@ int run(GemmArgs g, DeviceState *st, cudaStream_t s, PackedOperands &packed)
     if (sm100_skinny_gemm_supported(g) && (!large || sm100_skinny_gemm_preferred(g))) return sm100_skinny_gemm(g, st, s);
     if (large) return sm100_gemm(g, st, s);
     if (skinny_f32_supported(g)) return skinny_f32_gemm(g, st, s);
+    if (narrow_f32_supported(g)) return narrow_f32_gemm(g, s);
     return simt_gemm(g, st, s);
 }
 
@@ -257,7 +258,7 @@ int ember_linear_fwd(const void *x, const void *w, const void *bias, void *y, lo
     g.bias = bias;
     PackedOperands packed(pick_stream(stream, st));
     F32Products f32;
-    if (dtype == EMBER_F32 && !skinny_f32_supported(g)) f32.add(g);
+    if (dtype == EMBER_F32 && !skinny_f32_supported(g) && !narrow_f32_supported(g)) f32.add(g);
     if (f32.preferred(st->sm_count) && (rc = f32.run(st, packed.stream)) != EMBER_ERR_NOMEM) return rc;
     return run(g, st, packed.stream, packed);
 }
@@ -306,7 +307,7 @@ const char *ember_linear_kernel_name(int product, long long m, int n, int k, int
         }
         F32Products f32;
         if (product == FORWARD) {
-            if (!skinny_f32_supported(g)) f32.add(g);
+            if (!skinny_f32_supported(g) && !narrow_f32_supported(g)) f32.add(g);
         } else {
             f32.add(product_of(GRAD_W, sh, at[0], at[1], at[2], at[3]));
             f32.add(product_of(GRAD_X, sh, at[0], at[1], at[2], at[3]));

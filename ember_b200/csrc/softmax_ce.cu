@@ -394,6 +394,65 @@ __global__ void __launch_bounds__(BLOCK) loss_finalize_kernel(const float *row_l
     if (threadIdx.x == 0) *loss = -red[0] / (float)rows;
 }
 
+// Cross-entropy of a small classifier: at most 32 classes and 256 rows, probabilities and the loss by one block, a row per thread (a
+// row's elements are few enough to be in flight at once, and nothing is exchanged until the losses are added, in a fixed order). One launch
+// and the way of the row losses through memory less than row_softmax_kernel and loss_finalize_kernel: 256 x 10 float32 3.6 + 2.8 -> 4.3 us.
+// A lane per class in its place took 6.3 us with one block (80 shuffles a warp on one SM) and 5.7 with a cluster of eight.
+constexpr int kSmallRows = 256, kSmallCols = 32;
+
+template <typename T>
+__global__ void __launch_bounds__(kSmallRows) ce_small_kernel(const T *__restrict__ x, const T *__restrict__ target, T *__restrict__ probs,
+                                                              float *__restrict__ loss, int rows, int cols)
+{
+    __shared__ float part[kSmallRows / 32];
+    ptx::pdl_launch_dependents();
+    ptx::pdl_wait();
+    const int row = threadIdx.x;
+    const size_t at = (size_t)row * cols;
+    constexpr float kLog2e = 1.4426950408889634f;
+    constexpr int G = 4;  // columns are taken four at a time, past the last of them with no weight
+    float v[kSmallCols], t[kSmallCols], m = -INFINITY, s = 0.f, sum = 0.f;
+    if (row < rows) {
+#pragma unroll
+        for (int j0 = 0; j0 < kSmallCols; j0 += G)
+            if (j0 < cols) {
+#pragma unroll
+                for (int j = j0; j < j0 + G; j++) {
+                    v[j] = j < cols ? ldf(x + at + j) : -INFINITY;
+                    t[j] = j < cols ? ldf(target + at + j) : 0.f;
+                }
+            }
+#pragma unroll
+        for (int j0 = 0; j0 < kSmallCols; j0 += G)
+            if (j0 < cols) m = fmaxf(m, fmaxf(fmaxf(v[j0], v[j0 + 1]), fmaxf(v[j0 + 2], v[j0 + 3])));
+        const float m2 = m * kLog2e;
+#pragma unroll
+        for (int j0 = 0; j0 < kSmallCols; j0 += G)
+            if (j0 < cols) {
+#pragma unroll
+                for (int j = j0; j < j0 + G; j++)
+                    if (j < cols) s += fast_exp2(fmaf(v[j], kLog2e, -m2));
+            }
+        const float lg = logf(s), mlg2 = (m + lg) * kLog2e;
+#pragma unroll
+        for (int j0 = 0; j0 < kSmallCols; j0 += G)
+            if (j0 < cols) {
+#pragma unroll
+                for (int j = j0; j < j0 + G; j++)
+                    if (j < cols) {
+                        sum = fmaf(t[j], (v[j] - m) - lg, sum);
+                        stf(probs + at + j, fast_exp2(fmaf(v[j], kLog2e, -mlg2)));
+                    }
+            }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (threadIdx.x % 32 == 0) part[threadIdx.x / 32] = sum;
+    __syncthreads();
+    if (threadIdx.x == 0)
+        *loss = -(((part[0] + part[1]) + (part[2] + part[3])) + ((part[4] + part[5]) + (part[6] + part[7]))) / (float)rows;
+}
+
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(BLOCK) ce_backward_kernel(const T *__restrict__ probs, const T *__restrict__ target,
                                                             T *__restrict__ grad, size_t total, float inv_n)
@@ -555,6 +614,14 @@ int ember_cross_entropy_fwd(const void *pred, const void *target, void *probs, f
     DeviceState *st = device_state();
     if (!st) return EMBER_ERR_CUDA;
     cudaStream_t s = pick_stream(stream, st);
+    if (rows <= kSmallRows && cols <= kSmallCols) {
+        if (dtype == EMBER_BF16)
+            EMBER_CUDA_TRY(launch_pdl(ce_small_kernel<__nv_bfloat16>, 1, kSmallRows, 0, s, (const __nv_bfloat16 *)pred, (const __nv_bfloat16 *)target,
+                                      (__nv_bfloat16 *)probs, loss, (int)rows, cols));
+        else
+            EMBER_CUDA_TRY(launch_pdl(ce_small_kernel<float>, 1, kSmallRows, 0, s, (const float *)pred, (const float *)target, (float *)probs, loss, (int)rows, cols));
+        return EMBER_OK;
+    }
     float *row_loss = (float *)workspace;
     if (dtype == EMBER_BF16)
         rc = launch_rows<__nv_bfloat16, MODE_CROSS_ENTROPY>((const __nv_bfloat16 *)pred, (const __nv_bfloat16 *)target,
