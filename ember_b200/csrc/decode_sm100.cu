@@ -244,6 +244,17 @@ __global__ void __launch_bounds__(THREADS, 1) decode_sm100_kernel(const __grid_c
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     pdl_launch_dependents();
+    if (warp == 5 && lane == 0 && !p.seq_lens) {  // the first tiles come into L2 while the kernel before this one ends
+        Slice ahead;
+        TileIter ti;
+        ahead.cut(p, blockIdx.x, gridDim.x, p.whole_units);
+        int n = 0;
+        for (bool more = ti.start(p, ahead); more && n < C::ST; more = ti.next(p), n++)
+            for (int sub = 0; sub < C::NSUB; sub++) {
+                tma_prefetch_3d(&tm_k, sub * 64, ti.kt * 128, ti.unit);
+                tma_prefetch_3d(&tm_v, sub * 64, ti.kt * 128, ti.unit);
+            }
+    }
     pdl_wait();  // the cache's new rows may come from the kernel before this one
 
     Slice slice;

@@ -103,6 +103,13 @@ __global__ void __launch_bounds__(THREADS) skinny_gemm_kernel(const __grid_const
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     pdl_launch_dependents();
+    // the first tiles of w come into L2 while the kernel before this one ends
+    if (warp == 5 && lane == 0)
+        for (int i = 0; i < min(nkb, C::STAGES); i++) {
+            const int kk = (kb0 + i) * KB;
+            tma_prefetch_5d(&tm_w, TRANS_W ? kk : n0, TRANS_W ? n0 : kk, 0, 0, 0);
+            if (!TRANS_W) tma_prefetch_5d(&tm_w, n0 + 64, kk, 0, 0, 0);
+        }
     pdl_wait();
 
     if (warp == 5) {

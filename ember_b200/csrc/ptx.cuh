@@ -112,6 +112,19 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst_smem, const CUtensorMap
         : "memory");
 }
 
+// The same boxes on their way into L2 only, for what a kernel will load once the kernels before it are done. (L2 is where all of them
+// write to and read from, so it does not matter if they still change the box.)
+__device__ __forceinline__ void tma_prefetch_3d(const CUtensorMap *m, int c0, int c1, int c2)
+{
+    asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global [%0, {%1, %2, %3}];" ::"l"(reinterpret_cast<uint64_t>(m)), "r"(c0), "r"(c1), "r"(c2) : "memory");
+}
+__device__ __forceinline__ void tma_prefetch_5d(const CUtensorMap *m, int c0, int c1, int c2, int c3, int c4)
+{
+    asm volatile("cp.async.bulk.prefetch.tensor.5d.L2.global [%0, {%1, %2, %3, %4, %5}];" ::"l"(reinterpret_cast<uint64_t>(m)), "r"(c0), "r"(c1),
+                 "r"(c2), "r"(c3), "r"(c4)
+                 : "memory");
+}
+
 // 5-D tile load (matrix views: column, row, head, batch, part).
 __device__ __forceinline__ void tma_load_5d(uint32_t dst_smem, const CUtensorMap *m, uint32_t bar, int c0, int c1,
                                             int c2, int c3, int c4)
