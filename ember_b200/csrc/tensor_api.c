@@ -608,6 +608,54 @@ static PyObject *_decode_cache(PyObject *module, PyObject *args)
     return Py_BuildValue("(NN)", out, lse);
 }
 
+/* _decode_step(x, w_qkv, b_qkv, w_o, b_o, k_cache, v_cache, B, H, D, capacity, pos, scale) -> y
+ * One position of a self-attention block over a cache, as MultiHeadAttention.decode_step chains it (_linear_fwd, _kv_append, _decode_cache,
+ * _linear_fwd), with what passes between the four in one temporary block. */
+static PyObject *_decode_step(PyObject *module, PyObject *args)
+{
+    _Tensor *x, *wq, *bq, *wo, *bo, *kc, *vc;
+    int B, H, D, cap, pos;
+    float scale;
+    if (!PyArg_ParseTuple(args, "O!O!O!O!O!O!O!iiiiif", &_TensorType, &x, &_TensorType, &wq, &_TensorType, &bq, &_TensorType, &wo,
+                          &_TensorType, &bo, &_TensorType, &kc, &_TensorType, &vc, &B, &H, &D, &cap, &pos, &scale))
+        return NULL;
+    const long long E = (long long)H * D, n = B * E, cache_n = n * cap;
+    if (B <= 0 || H <= 0 || D <= 0 || cap <= 0 || pos < 0 || pos >= cap || 3 * E > 2147483647LL || x->size64 != n || wq->size64 != 3 * E * E ||
+        bq->size64 != 3 * E || wo->size64 != E * E || bo->size64 != E || kc->size64 != cache_n || vc->size64 != cache_n) {
+        PyErr_SetString(PyExc_ValueError, "decode_step: size mismatch");
+        return NULL;
+    }
+    const int dt = x->dtype;
+    if (wq->dtype != dt || bq->dtype != dt || wo->dtype != dt || bo->dtype != dt || kc->dtype != dt || vc->dtype != dt) {
+        PyErr_SetString(PyExc_TypeError, "decode_step: all tensors must share a dtype");
+        return NULL;
+    }
+    const size_t row = ((size_t)n * elem_size(dt) + 255) / 256 * 256;
+    const size_t qkv_bytes = ((size_t)3 * n * elem_size(dt) + 255) / 256 * 256;
+    const size_t wsn = ember_attention_decode_cache_workspace_bytes(B, H, H, pos + 1, D, 0);
+    _Tensor *y = alloc_result(n, dt);
+    if (!y) return NULL;
+    char *tmp = alloc_memory(qkv_bytes + row + (wsn ? wsn : 256));
+    if (!tmp) {
+        Py_DECREF(y);
+        PyErr_Format(PyExc_MemoryError, "Failed to allocate device memory: %s", ember_last_error());
+        return NULL;
+    }
+    char *k = tmp + (size_t)n * elem_size(dt), *v = k + (size_t)n * elem_size(dt), *o = tmp + qkv_bytes;
+    int rc = ember_linear_fwd(x->d_ptr, wq->d_ptr, bq->d_ptr, tmp, B, (int)(3 * E), (int)E, dt, 0, H, 1, D, NULL);
+    if (!rc) rc = ember_kv_cache_append(kc->d_ptr, vc->d_ptr, k, v, B, H, cap, D, 1, pos, NULL, NULL, 0, 0, dt, NULL);
+    if (!rc)
+        rc = ember_attention_decode_cache(tmp, kc->d_ptr, vc->d_ptr, o, NULL, B, H, H, pos + 1, cap, D, scale, dt, NULL, NULL, 0, 0, 0,
+                                          o + row, wsn, NULL);
+    if (!rc) rc = ember_linear_fwd(o, wo->d_ptr, bo->d_ptr, y->d_ptr, B, (int)E, (int)E, dt, H, 0, 1, D, NULL);
+    free_memory(tmp); /* stream-ordered: released after the kernels that use it */
+    if (rc) {
+        Py_DECREF(y);
+        return raise_status(rc);
+    }
+    return (PyObject *)y;
+}
+
 static PyObject *_sync(PyObject *module, PyObject *noargs)
 {
     sync_device();
@@ -638,6 +686,7 @@ static PyMethodDef module_methods[] = {OP_METHOD(_from_numpy),
                                        OP_METHOD(_cross_entropy_bwd),
                                        OP_METHOD(_kv_append),
                                        OP_METHOD(_decode_cache),
+                                       OP_METHOD(_decode_step),
                                        {"_sync", (PyCFunction)_sync, METH_NOARGS, "Wait for the library stream"},
                                        {NULL, NULL, 0, NULL}};
 
