@@ -61,6 +61,7 @@ SIGNATURES = {
     "ember_linear_fwd": (_i, [_vp] * 4 + [ctypes.c_longlong] + [_i] * 7 + [_vp]),
     "ember_linear_bwd": (_i, [_vp] * 6 + [ctypes.c_longlong] + [_i] * 7 + [_vp]),
     "ember_linear_kernel_name": (ctypes.c_char_p, [_i, ctypes.c_longlong] + [_i] * 7),
+    "ember_linear_fwd_cached": (_i, [_vp] * 6 + [_i] * 6 + [_vp]),
     "ember_kv_cache_append": (_i, [_vp] * 4 + [_i] * 6 + [_vp, _vp, _i, _i, _i, _vp]),
     "ember_attention_decode_cache": (_i, [_vp] * 5 + [_i] * 6 + [ctypes.c_float, _i, _vp, _vp, _i, _i, _i, _vp, _sz, _vp]),
     "ember_attention_decode_cache_workspace_bytes": (_sz, [_i] * 6),

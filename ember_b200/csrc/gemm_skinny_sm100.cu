@@ -47,6 +47,7 @@ struct SkinnyParams {
     int m, n, k, splits;
     MatView y;
     const __nv_bfloat16 *bias;
+    CacheRows cache;  // k null: none
     DeviceStatus *status;
 };
 
@@ -175,6 +176,12 @@ __global__ void __launch_bounds__(THREADS) skinny_gemm_kernel(const __grid_const
         if (col < p.n && ok) {
             const float b = p.bias ? __bfloat162float(p.bias[col]) : 0.f;
             __nv_bfloat16 *y = (__nv_bfloat16 *)p.y.ptr + view_offset(p.y, 0, col);  // rows and columns of a view address independently
+            const bool cached = p.cache.k && col >= p.cache.from;
+            if (cached) {
+                const int c = col % p.cache.from;
+                y = (__nv_bfloat16 *)(col < 2 * p.cache.from ? p.cache.k : p.cache.v) + ((size_t)(c / p.cache.d) * p.cache.capacity + p.cache.pos) * p.cache.d + c % p.cache.d;
+            }
+            const size_t cache_step = (size_t)p.cache.heads * p.cache.capacity * p.cache.d;
             const uint32_t mine = smem_base + 4u * threadIdx.x;
             uint32_t peer[MAX_SPLIT];
 #pragma unroll
@@ -191,7 +198,7 @@ __global__ void __launch_bounds__(THREADS) skinny_gemm_kernel(const __grid_const
                 } else {
                     s = part[row * TILE_N + threadIdx.x];
                 }
-                y[view_offset(p.y, row, 0)] = __float2bfloat16_rn(s + b);
+                y[cached ? row * cache_step : view_offset(p.y, row, 0)] = __float2bfloat16_rn(s + b);
             }
         }
     }
@@ -213,8 +220,11 @@ int launch_mp(const GemmArgs &g, DeviceState *st, cudaStream_t s)
     const int sms = st->sm_count > 0 ? st->sm_count : 148;
     const int tiles = (g.n + TILE_N - 1) / TILE_N, kblocks = (g.k + KB - 1) / KB;
     int splits = 1;  // as many CTAs as two per SM hold, each with at least two contraction steps
-    while (splits < MAX_SPLIT && tiles * splits * 2 <= 2 * sms && kblocks >= splits * 4) splits *= 2;
-    SkinnyParams p = {(int)g.m, g.n, g.k, splits, g.c, (const __nv_bfloat16 *)g.bias, st->status};
+    // (a GPC's SMs do not divide into clusters of 8 without rest: 36 tiles in 8 parts 9.2 us, in 4 5.9, 8 x 1536 x 4608)
+    auto fit = [&](int parts) { return tiles * parts <= (parts == 8 ? 2 * sms * 7 / 8 : 2 * sms); };
+    while (splits < MAX_SPLIT && fit(splits * 2) && kblocks >= splits * 4) splits *= 2;
+    const CacheRows none = {};
+    SkinnyParams p = {(int)g.m, g.n, g.k, splits, g.c, (const __nv_bfloat16 *)g.bias, g.cache ? *g.cache : none, st->status};
     auto kern = skinny_gemm_kernel<MP, TRANS_W>;
     static SmemOptIn opt_in;
     EMBER_CUDA_TRY(opt_in(kern, C::SMEM_BYTES));

@@ -158,6 +158,13 @@ enum GemmMode {
     GEMM_NT = 1,  // A view (m x k), B view (n x k)
     GEMM_TN = 2   // A view (k x m), B view (k x n)
 };
+// Results of a few-row q/k/v projection that go straight into a key/value cache (batch, heads, capacity, d): columns
+// from `from` on are k, then v, `from` each; row b of the product is row `pos` of sequence b.
+struct CacheRows {
+    void *k, *v;
+    int from, heads, capacity, d, pos;
+};
+
 struct GemmArgs {
     int mode = GEMM_NN;
     MatView a, b, c;
@@ -165,6 +172,7 @@ struct GemmArgs {
     long long m = 0;
     int n = 0, k = 0;
     int dtype = EMBER_F32;
+    const CacheRows *cache = nullptr;  // gemm_skinny_sm100.cu
     const int *only_if = nullptr;  // CUDA-core kernel: return at once when this word of device memory is 0
 };
 

@@ -263,6 +263,31 @@ int ember_linear_fwd(const void *x, const void *w, const void *bias, void *y, lo
     return run(g, st, packed.stream, packed);
 }
 
+int ember_linear_fwd_cached(const void *x, const void *w, const void *bias, void *qkv, void *k_cache, void *v_cache, int batch, int heads, int d,
+                            int capacity, int pos, int dtype, void *stream)
+{
+    const LinearShape sh = {batch, 3 * heads * d, heads * d, dtype, 0, heads, 1, d};
+    int rc = check_linear("ember_linear_fwd_cached", sh);
+    if (rc) return rc;
+    EMBER_REQUIRE(x && w && qkv && k_cache && v_cache, "ember_linear_fwd_cached: NULL tensor pointer");
+    EMBER_REQUIRE(pos >= 0 && pos < capacity, "ember_linear_fwd_cached: row %d does not fit a cache of %d rows", pos, capacity);
+    DeviceState *st = device_state();
+    if (!st) return EMBER_ERR_CUDA;
+    GemmArgs g = product_of(FORWARD, sh, x, w, qkv, nullptr);
+    g.bias = bias;
+    // (caches that the copy of rows or the decode kernels refuse take the two calls, which say so)
+    if (d % 8 == 0 && (((uintptr_t)k_cache | (uintptr_t)v_cache) & 15) == 0 && sm100_skinny_gemm_supported(g) &&
+        (!sm100_gemm_supported(g) || sm100_skinny_gemm_preferred(g))) {
+        const CacheRows rows = {k_cache, v_cache, heads * d, heads, capacity, d, pos};
+        g.cache = &rows;
+        return sm100_skinny_gemm(g, st, pick_stream(stream, st));
+    }
+    if ((rc = ember_linear_fwd(x, w, bias, qkv, batch, sh.n, sh.k, dtype, 0, heads, 1, d, stream)) != EMBER_OK) return rc;
+    const size_t part = (size_t)batch * heads * d * dtype_size(dtype);
+    return ember_kv_cache_append(k_cache, v_cache, (const char *)qkv + part, (const char *)qkv + 2 * part, batch, heads, capacity, d, 1, pos, nullptr,
+                                 nullptr, 0, 0, dtype, stream);
+}
+
 int ember_linear_bwd(const void *x, const void *w, const void *dy, void *dx, void *dw, void *db, long long m, int n,
                      int k, int dtype, int x_heads, int y_heads, int seq, int head_dim, void *stream)
 {

@@ -609,7 +609,7 @@ static PyObject *_decode_cache(PyObject *module, PyObject *args)
 }
 
 /* _decode_step(x, w_qkv, b_qkv, w_o, b_o, k_cache, v_cache, B, H, D, capacity, pos, scale) -> y
- * One position of a self-attention block over a cache, as MultiHeadAttention.decode_step chains it (_linear_fwd, _kv_append, _decode_cache,
+ * One position of a self-attention block over a cache, as MultiHeadAttention.decode_step chains it (_linear_fwd and _kv_append, _decode_cache,
  * _linear_fwd), with what passes between the four in one temporary block. */
 static PyObject *_decode_step(PyObject *module, PyObject *args)
 {
@@ -641,9 +641,8 @@ static PyObject *_decode_step(PyObject *module, PyObject *args)
         PyErr_Format(PyExc_MemoryError, "Failed to allocate device memory: %s", ember_last_error());
         return NULL;
     }
-    char *k = tmp + (size_t)n * elem_size(dt), *v = k + (size_t)n * elem_size(dt), *o = tmp + qkv_bytes;
-    int rc = ember_linear_fwd(x->d_ptr, wq->d_ptr, bq->d_ptr, tmp, B, (int)(3 * E), (int)E, dt, 0, H, 1, D, NULL);
-    if (!rc) rc = ember_kv_cache_append(kc->d_ptr, vc->d_ptr, k, v, B, H, cap, D, 1, pos, NULL, NULL, 0, 0, dt, NULL);
+    char *o = tmp + qkv_bytes;
+    int rc = ember_linear_fwd_cached(x->d_ptr, wq->d_ptr, bq->d_ptr, tmp, kc->d_ptr, vc->d_ptr, B, H, D, cap, pos, dt, NULL);
     if (!rc)
         rc = ember_attention_decode_cache(tmp, kc->d_ptr, vc->d_ptr, o, NULL, B, H, H, pos + 1, cap, D, scale, dt, NULL, NULL, 0, 0, 0,
                                           o + row, wsn, NULL);

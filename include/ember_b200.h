@@ -342,6 +342,11 @@ EMBER_API int ember_cross_entropy_bwd(const void *probs, const void *target, voi
 EMBER_API int ember_kv_cache_append(void *k_cache, void *v_cache, const void *k_new, const void *v_new, int batch,
                                     int kv_heads, int capacity, int d, int n_new, int pos, const int *seq_lens,
                                     const int *block_table, int page_size, int max_blocks, int dtype, void *stream);
+/* The q/k/v projection of one position of `batch` sequences (x (batch, heads * d), w (heads * d, 3 * heads * d), bias or NULL) and
+ * ember_kv_cache_append of its keys and values at row `pos`: where a kernel for few rows takes the projection it writes them into the
+ * caches itself. qkv has room for (3, batch, heads, 1, d); its first part receives q, the other two may or may not be written. */
+EMBER_API int ember_linear_fwd_cached(const void *x, const void *w, const void *bias, void *qkv, void *k_cache, void *v_cache, int batch,
+                                      int heads, int d, int capacity, int pos, int dtype, void *stream);
 EMBER_API int ember_attention_decode_cache(const void *q, const void *k_cache, const void *v_cache, void *out, float *lse,
                                            int batch, int q_heads, int kv_heads, int lk, int capacity, int d, float scale,
                                            int dtype, const int *seq_lens, const int *block_table, int page_size,
