@@ -29,7 +29,7 @@ __device__ __forceinline__ float ld_peer_f32(uint32_t addr)
 
 // VEC: 16-byte pieces that are aligned and stay inside a row or head.
 template <typename T, bool VEC, int NTHR>
-__global__ void __launch_bounds__(NTHR) column_sum_kernel(const MatView a, T *__restrict__ out, int splits)
+__global__ void __launch_bounds__(NTHR) column_sum_kernel(const MatView a, T *__restrict__ out, int splits, bool late_wait)
 {
     constexpr int NV = VEC ? 16 / (int)sizeof(T) : 1;  // columns per load
     constexpr int TX = VEC ? 8 : 32, TY = NTHR / TX;   // threads along a strip's columns, rows per pass
@@ -37,7 +37,7 @@ __global__ void __launch_bounds__(NTHR) column_sum_kernel(const MatView a, T *__
     __shared__ float red[TY][COLS + 1];
     __shared__ float total[COLS];
     pdl_launch_dependents();
-    pdl_wait();
+    if (!late_wait) pdl_wait();
     const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;
     const int rank = splits > 1 ? (int)cluster_ctarank() : 0;
     const int col = ((int)blockIdx.x / splits) * COLS + tx * NV;
@@ -115,13 +115,14 @@ __global__ void __launch_bounds__(NTHR) column_sum_kernel(const MatView a, T *__
     if (rank == 0 && c < COLS && oc < a.cols) {
         if constexpr (sizeof(T) == 2) out[oc] = __float2bfloat16_rn(total[c]); else out[oc] = total[c];
     }
+    if (late_wait) pdl_wait();  // this kernel's end stands for the end of all before it
 }
 
 template <typename T, bool VEC>
 constexpr int strip_cols() { return VEC ? 128 / (int)sizeof(T) : 32; }
 
 template <typename T, bool VEC, int NTHR>
-int launch(const MatView &a, T *out, int sms, cudaStream_t s)
+int launch(const MatView &a, T *out, int sms, cudaStream_t s, bool beside)
 {
     constexpr int TY = NTHR / (VEC ? 8 : 32);
     const long long strips = (a.cols + strip_cols<T, VEC>() - 1) / strip_cols<T, VEC>();
@@ -135,34 +136,34 @@ int launch(const MatView &a, T *out, int sms, cudaStream_t s)
     cfg.stream = s;
     LaunchAttrs attrs;
     attrs.cluster((unsigned)splits).pdl().set(cfg);
-    EMBER_CUDA_TRY(cudaLaunchKernelEx(&cfg, column_sum_kernel<T, VEC, NTHR>, a, out, splits));
+    EMBER_CUDA_TRY(cudaLaunchKernelEx(&cfg, column_sum_kernel<T, VEC, NTHR>, a, out, splits, beside));
     return EMBER_OK;
 }
 
 // With up to 8 blocks for a strip, a tall matrix of few strips leaves most SMs idle and waits on what a block has in
 // flight: blocks of 1024 threads while those of 256 would not give every second SM one.
 template <typename T, bool VEC>
-int launch_size(const MatView &a, T *out, int sms, cudaStream_t s)
+int launch_size(const MatView &a, T *out, int sms, cudaStream_t s, bool beside)
 {
     const long long strips = (a.cols + strip_cols<T, VEC>() - 1) / strip_cols<T, VEC>();
-    if (a.rows >= 32768 && strips * 8 * 2 <= sms) return launch<T, VEC, 1024>(a, out, sms, s);
-    return launch<T, VEC, 256>(a, out, sms, s);
+    if (a.rows >= 32768 && strips * 8 * 2 <= sms) return launch<T, VEC, 1024>(a, out, sms, s, beside);
+    return launch<T, VEC, 256>(a, out, sms, s, beside);
 }
 
 template <typename T>
-int launch_any(const MatView &a, T *out, int sms, cudaStream_t s)
+int launch_any(const MatView &a, T *out, int sms, cudaStream_t s, bool beside)
 {
     constexpr int NV = 16 / (int)sizeof(T);
     const bool vec = ((uintptr_t)a.ptr & 15) == 0 && (a.heads ? a.dim % NV == 0 : a.cols % NV == 0);
-    return vec ? launch_size<T, true>(a, out, sms, s) : launch_size<T, false>(a, out, sms, s);
+    return vec ? launch_size<T, true>(a, out, sms, s, beside) : launch_size<T, false>(a, out, sms, s, beside);
 }
 
 }  // namespace
 
-int column_sums(const MatView &a, void *out, int dtype, DeviceState *st, cudaStream_t s)
+int column_sums(const MatView &a, void *out, int dtype, DeviceState *st, cudaStream_t s, bool beside)
 {
     const int sms = st->sm_count > 0 ? st->sm_count : 148;
-    return dtype == EMBER_BF16 ? launch_any(a, (__nv_bfloat16 *)out, sms, s) : launch_any(a, (float *)out, sms, s);
+    return dtype == EMBER_BF16 ? launch_any(a, (__nv_bfloat16 *)out, sms, s, beside) : launch_any(a, (float *)out, sms, s, beside);
 }
 
 }  // namespace ember

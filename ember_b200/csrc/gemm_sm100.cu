@@ -40,16 +40,19 @@ constexpr int A_BYTES = BM * BK * 2;
 constexpr int SUB_BYTES = 64 * 128;           // 64 rows x 128 bytes
 constexpr int GEMM_THREADS = 192;
 
-// BN: columns of a pair's tile, 256, or 128 for results of few tiles: see launch.
-template <int BN>
+// BN: columns of a pair's tile, 256, or 128 for results of few tiles: see launch. The epilogue stages OUT columns at a time: 128, or 64 in the
+// gradients' products, so that what is left of an SM's 228 KB of shared memory holds a block of column_sum_kernel. (64 in the
+// forward too: 8192 rows x 512 x 16384 137 -> 145 us, 2048 x 128 x 32768 64 -> 68.)
+template <int BN, int MODE>
 struct GemmCfg {
+    static constexpr int OUT = MODE == GEMM_NN ? 128 : 64;
     static constexpr int BNH = BN / 2;                     // B columns held by one CTA of a pair
     static constexpr int STAGE_BYTES = A_BYTES + BNH * BK * 2;
-    static constexpr int OFF_OUT = STAGES * STAGE_BYTES;   // 128 rows x 128 columns of bf16 for the epilogue
-    static constexpr int OFF_BIAS = OFF_OUT + BM * 128 * 2;  // BN floats
+    static constexpr int OFF_OUT = STAGES * STAGE_BYTES;   // 128 rows x OUT columns of bf16 for the epilogue
+    static constexpr int OFF_BIAS = OFF_OUT + BM * OUT * 2;  // BN floats
     static constexpr int OFF_BAR = OFF_BIAS + BN * 4;
     static constexpr int USED_BYTES = OFF_BAR + 128;
-    static constexpr int SMEM_BYTES = BN == 256 ? 232448 : USED_BYTES + 1024;  // 256: the whole opt-in limit; the base is checked in the kernel
+    static constexpr int SMEM_BYTES = USED_BYTES + 1024 < 232448 ? USED_BYTES + 1024 : 232448;  // at most the opt-in limit; the base is checked in the kernel
 };
 
 enum { B_FULL = 0, B_EMPTY = B_FULL + STAGES, B_ACCFULL = B_EMPTY + STAGES, B_ACCEMPTY = B_ACCFULL + 2, NUM_BARS = B_ACCEMPTY + 2 };
@@ -65,6 +68,9 @@ struct GemmParams {
     ViewGeom a, b;
     MatView c;
     int c_vec;  // rows of c are 16-byte aligned: 16-byte stores
+    // Beside the kernel before (GemmArgs::beside): the first `head_pairs` pairs, which find SMs at once, take `head_tiles` tiles each
+    // before the common order begins.
+    int late_wait, head_pairs, head_tiles;
     const __nv_bfloat16 *bias;
     DeviceStatus *status;
 };
@@ -74,7 +80,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     sm100_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
                       const GemmParams p)
 {
-    using C = GemmCfg<BN>;
+    using C = GemmCfg<BN, MODE>;
+    constexpr int OUT = C::OUT, CPR = OUT / 8;  // CPR: 16-byte chunks of a staged row
     constexpr int BNH = C::BNH, STAGE_BYTES = C::STAGE_BYTES, OFF_OUT = C::OFF_OUT, OFF_BIAS = C::OFF_BIAS, OFF_BAR = C::OFF_BAR,
                   USED_BYTES = C::USED_BYTES;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -129,15 +136,28 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     cluster_sync_all();  // both CTAs' barriers exist before either signals the other's
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    pdl_launch_dependents();
-    pdl_wait();
+    // What is launched behind this kernel may read what this one reads before it has waited itself (late_wait, column_sum_kernel), so it
+    // is let go only once the kernels before this one are done; a kernel with late_wait was let go that way and passes it on.
+    constexpr bool BESIDE = MODE != GEMM_NN;  // nothing runs beside a forward product
+    if (!BESIDE) pdl_launch_dependents();
+    if (!BESIDE || !p.late_wait) pdl_wait();
+    if (BESIDE) pdl_launch_dependents();
+    // the pair's i-th tile, num_tiles or more when there is none
+    auto tile_of = [&](int i) {
+        if (!BESIDE || p.head_pairs == 0) return i * npairs + pair;
+        if (pair < p.head_pairs) {
+            if (i < p.head_tiles) return i * p.head_pairs + pair;
+            i -= p.head_tiles;
+        }
+        return p.head_pairs * p.head_tiles + i * npairs + (npairs - 1 - pair);  // those with a head come last in a round
+    };
 
     if (warp == 5) {
         if (lane == 0) {
             // ------------------------------------------------------------ TMA producer (both CTAs)
             int it = 0;
             bool ok = true;
-            for (int tile = pair; tile < num_tiles && ok; tile += npairs) {
+            for (int i = 0, tile; (tile = tile_of(i)) < num_tiles && ok; i++) {
                 int tm, tn;
                 tile_coords(p.tiles_m, p.tiles_n, tile, tm, tn);
                 const int m0 = tm * 2 * BM + (int)rank * BM, n0 = tn * BN + (int)rank * BNH;  // this CTA's A rows and B columns
@@ -183,7 +203,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
             constexpr uint32_t B_LBO = MODE == GEMM_NT ? 16 : SUB_BYTES, B_STEP = (MODE == GEMM_NT ? 32 : 2048) >> 4;
             int it = 0, tcount = 0;
             bool ok = true;
-            for (int tile = pair; tile < num_tiles; tile += npairs, tcount++) {
+            for (; tile_of(tcount) < num_tiles; tcount++) {
                 const int buf = tcount & 1;
                 ok = ok && mbar_wait(BAR(B_ACCEMPTY + buf), ((tcount >> 1) & 1) ^ 1, abort_flag, p.status, WG_ACCEMPTY);
                 tc_fence_after();
@@ -210,7 +230,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
         const uint32_t accempty0 = map_to_cta(BAR(B_ACCEMPTY), 0);  // rank 0's barriers, as cluster addresses
         int tcount = 0;
         bool ok = true;
-        for (int tile = pair; tile < num_tiles; tile += npairs, tcount++) {
+        for (int tile; (tile = tile_of(tcount)) < num_tiles; tcount++) {
             int tm, tn;
             tile_coords(p.tiles_m, p.tiles_n, tile, tm, tn);
             const int buf = tcount & 1;
@@ -225,18 +245,18 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
             tc_fence_after();
             const uint32_t tacc = tmem + lane_sel + buf * BN;
 #pragma unroll 1
-            for (int half = 0; half < BN / 128; half++) {
+            for (int part = 0; part < BN / OUT; part++) {
 #pragma unroll
-                for (int ch = 0; ch < 4; ch++) {
+                for (int ch = 0; ch < OUT / 32; ch++) {
                     uint32_t u[32];
-                    tmem_ld_32x32b_x32(tacc + half * 128 + ch * 32, u);
+                    tmem_ld_32x32b_x32(tacc + part * OUT + ch * 32, u);
                     tmem_wait_ld();
-                    if (half == BN / 128 - 1 && ch == 3) {  // the accumulator is in registers: the next tile may use it
+                    if (part == BN / OUT - 1 && ch == OUT / 32 - 1) {  // the accumulator is in registers: the next tile may use it
                         tc_fence_before();
                         __syncwarp();
                         if (lane == 0) mbar_arrive_cluster(accempty0 + 8u * (uint32_t)buf);
                     }
-                    const float *bs = bias_s + half * 128 + ch * 32;
+                    const float *bs = bias_s + part * OUT + ch * 32;
 #pragma unroll
                     for (int q4 = 0; q4 < 4; q4++) {  // 8 columns = one 16-byte chunk
                         uint4 wv;
@@ -246,11 +266,11 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                         wv.w = pack_bf16(__uint_as_float(u[q4 * 8 + 6]) + bs[q4 * 8 + 6], __uint_as_float(u[q4 * 8 + 7]) + bs[q4 * 8 + 7]);
                         const int chunk = ch * 4 + q4;
                         const int sw = (chunk & ~7) | ((chunk ^ r) & 7);
-                        *reinterpret_cast<uint4 *>(stage + r * 256 + sw * 16) = wv;
+                        *reinterpret_cast<uint4 *>(stage + r * (OUT * 2) + sw * 16) = wv;
                     }
                 }
                 __syncwarp();
-                // Each warp copies its own 32 rows: two rows of 16 chunks per instruction. The destination
+                // Each warp copies its own 32 rows: two (four) rows of 16 (8) chunks per instruction. The destination
                 // of a chunk is found without divisions in the loop: this thread's column is fixed, and
                 // the 128 rows of a CTA's tile lie inside one batch entry and therefore at one distance
                 // from each other (row-major: `cols` apart; head-major: `dim`).
@@ -258,15 +278,15 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                     // Rows at any alignment (row-major, columns no multiple of 8): one element per lane,
                     // 64 contiguous bytes per store instruction.
                     if (rows_valid > 0) {
-                        __nv_bfloat16 *crow = cptr + ((size_t)l0 + warp * 32) * p.c.cols + n0 + half * 128;
-                        const int rows_here = min(32, rows_valid - warp * 32), cols_here = min(128, p.n - n0 - half * 128);
+                        __nv_bfloat16 *crow = cptr + ((size_t)l0 + warp * 32) * p.c.cols + n0 + part * OUT;
+                        const int rows_here = min(32, rows_valid - warp * 32), cols_here = min(OUT, p.n - n0 - part * OUT);
 #pragma unroll 4
                         for (int rr = 0; rr < rows_here; rr++) {
                             const int tr = warp * 32 + rr;
 #pragma unroll
-                            for (int i = 0; i < 4; i++) {
+                            for (int i = 0; i < OUT / 32; i++) {
                                 const int e = i * 32 + lane, chunk = e / 8, sw = (chunk & ~7) | ((chunk ^ tr) & 7);
-                                const __nv_bfloat16 v = *reinterpret_cast<const __nv_bfloat16 *>(stage + tr * 256 + sw * 16 + (e % 8) * 2);
+                                const __nv_bfloat16 v = *reinterpret_cast<const __nv_bfloat16 *>(stage + tr * (OUT * 2) + sw * 16 + (e % 8) * 2);
                                 if (ok && e < cols_here) crow[(size_t)rr * p.c.cols + e] = v;
                             }
                         }
@@ -274,15 +294,15 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                     __syncwarp();
                     continue;
                 }
-                const int chunk = lane % 16;
-                const int col = n0 + half * 128 + chunk * 8;
+                const int chunk = lane % CPR;
+                const int col = n0 + part * OUT + chunk * 8;
                 const size_t row_stride = p.c.heads == 0 ? (size_t)p.c.cols : (size_t)p.c.dim;
                 const size_t base = (rows_valid > 0 && col < p.n) ? view_offset(p.c, (long long)entry * p.seq + l0, col) : 0;
 #pragma unroll 4
-                for (int it2 = 0; it2 < 16; it2++) {
-                    const int rr = warp * 32 + it2 * 2 + lane / 16;
+                for (int it2 = 0; it2 < CPR; it2++) {
+                    const int rr = warp * 32 + it2 * (32 / CPR) + lane / CPR;
                     const int sw = (chunk & ~7) | ((chunk ^ rr) & 7);
-                    const uint4 wv = *reinterpret_cast<const uint4 *>(stage + rr * 256 + sw * 16);
+                    const uint4 wv = *reinterpret_cast<const uint4 *>(stage + rr * (OUT * 2) + sw * 16);
                     if (ok && rr < rows_valid && col < p.n) *reinterpret_cast<uint4 *>(cptr + base + (size_t)rr * row_stride) = wv;
                 }
                 __syncwarp();
@@ -294,6 +314,48 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     __syncthreads();
     cluster_sync_all();  // neither CTA leaves while the other may still signal its barriers or use the shared allocation
     if (warp == 4) tmem_dealloc_pair(tmem, 512);
+    if (BESIDE && p.late_wait) pdl_wait();  // this kernel's end stands for the end of all before it
+}
+
+// Tiles of 256 rows and 256 (or 128) columns, and the steps of the contraction.
+struct Tiling {
+    long long tiles_m, tiles_n;
+    int kblocks, bn;
+};
+
+Tiling tiling(const GemmArgs &g, int sms)
+{
+    const RowPlan rows = row_plan(g);
+    Tiling t;
+    t.tiles_m = ((g.mode == GEMM_TN ? g.m : (long long)rows.batch * rows.seq_pad) + 2 * BM - 1) / (2 * BM);
+    t.kblocks = g.mode == GEMM_TN && rows.by_entry ? rows.batch * (rows.seq_pad / BK) : (g.k + BK - 1) / BK;
+    t.bn = t.tiles_m * ((g.n + 255) / 256) * 2 <= sms / 2 ? 128 : 256;
+    t.tiles_n = (g.n + t.bn - 1) / t.bn;
+    return t;
+}
+
+// A product beside the one before it finds the SMs at once that the other's last round leaves idle. The first `pairs` CTA pairs get
+// there first; they take `tiles` tiles each ahead of the rest, as many as make the end come soonest. false: no end comes sooner for it.
+bool head_of(const Tiling &before, const Tiling &t, int npairs, int &pairs, int &tiles)  // npairs: what the SMs hold
+{
+    pairs = tiles = 0;
+    const long long all = t.tiles_m * t.tiles_n, idle = npairs - before.tiles_m * before.tiles_n % npairs;
+    if (idle >= npairs) return false;
+    if (all <= npairs) return true;  // at most a tile each, on whatever SMs are free
+    const double late = (double)before.kblocks * before.bn / ((double)t.kblocks * t.bn);  // the others' start, in tiles
+    const double alone = late + (all + npairs - 1) / npairs;
+    double best = alone;
+    for (int x = 0; x <= late + 1 && x * idle <= all; x++) {
+        const long long rest = all - x * idle, full = rest / npairs, rem = rest % npairs;
+        const double end = fmax(late + full + (rem > 0), x + full + (rem > npairs - idle));
+        if (end < best - 1e-9) {
+            best = end;
+            pairs = (int)idle;
+            tiles = x;
+        }
+    }
+    if (tiles == 0) pairs = 0;
+    return best < alone - 1e-9;
 }
 
 bool c_rows_aligned(const GemmArgs &g) { return g.n % 8 == 0 && ((uintptr_t)g.c.ptr & 15) == 0; }
@@ -301,7 +363,7 @@ bool c_rows_aligned(const GemmArgs &g) { return g.n % 8 == 0 && ((uintptr_t)g.c.
 template <int MODE, int BN>
 int launch_tile(const GemmArgs &g, DeviceState *st, cudaStream_t s)
 {
-    using C = GemmCfg<BN>;
+    using C = GemmCfg<BN, MODE>;
     constexpr int BNH = C::BNH, SMEM_BYTES = C::SMEM_BYTES;
     const RowPlan rows = row_plan(g);
     MatView va = g.a, vb = g.b;
@@ -346,6 +408,9 @@ int launch_tile(const GemmArgs &g, DeviceState *st, cudaStream_t s)
     const long long tiles = (long long)p.tiles_m * p.tiles_n;
     const int sms = st->sm_count > 0 ? st->sm_count : 148;
     const int pairs = (int)(tiles < sms / 2 ? tiles : sms / 2);
+    p.late_wait = g.beside != nullptr;
+    p.head_pairs = p.head_tiles = 0;
+    if (g.beside) head_of(tiling(*g.beside, sms), tiling(g, sms), sms / 2, p.head_pairs, p.head_tiles);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * pairs);
     cfg.blockDim = dim3(GEMM_THREADS);
@@ -365,11 +430,8 @@ int launch_tile(const GemmArgs &g, DeviceState *st, cudaStream_t s)
 template <int MODE>
 int launch(const GemmArgs &g, DeviceState *st, cudaStream_t s)
 {
-    const RowPlan rows = row_plan(g);
-    const long long m = MODE == GEMM_TN ? g.m : (long long)rows.batch * rows.seq_pad;
-    const long long tiles = (m + 2 * BM - 1) / (2 * BM) * ((g.n + 255) / 256);
     const int sms = st->sm_count > 0 ? st->sm_count : 148;
-    return tiles * 2 <= (sms / 2) ? launch_tile<MODE, 128>(g, st, s) : launch_tile<MODE, 256>(g, st, s);
+    return tiling(g, sms).bn == 128 ? launch_tile<MODE, 128>(g, st, s) : launch_tile<MODE, 256>(g, st, s);
 }
 
 }  // namespace
@@ -449,6 +511,13 @@ int pack_rows(const MatView &v, void *dst, cudaStream_t s)
     attrs.pdl().set(cfg);
     EMBER_CUDA_TRY(cudaLaunchKernelEx(&cfg, pack_rows_kernel, (const unsigned short *)v.ptr, (uint4 *)dst, v.rows, v.cols, chunks));
     return EMBER_OK;
+}
+
+bool sm100_gemm_gains_beside(const GemmArgs &before, const GemmArgs &g, DeviceState *st)
+{
+    const int sms = st->sm_count > 0 ? st->sm_count : 148;
+    int pairs, head;
+    return head_of(tiling(before, sms), tiling(g, sms), sms / 2, pairs, head);
 }
 
 int sm100_gemm(const GemmArgs &g, DeviceState *st, cudaStream_t s)

@@ -18,7 +18,11 @@ namespace ember {
 //     all before it (the single-pass backward reads q, k, v and dO earlier: the delta kernel before it passes
 //     pdl_wait() first and lets it start afterwards);
 //   - a kernel that allocates tensor memory passes pdl_launch_dependents() after the allocation: a later kernel's
-//     block can then never hold the columns that an earlier one's, which it waits for, still needs.
+//     block can then never hold the columns that an earlier one's, which it waits for, still needs;
+//   - sm100_gemm_kernel passes pdl_wait() before pdl_launch_dependents(). What is launched behind it finds every kernel before it done, and
+//     may begin without pdl_wait() if it neither reads nor overwrites anything of the product itself: the products and the bias gradient of one
+//     backward call ("beside"). Such a kernel passes pdl_wait() last, so that its end, too, implies the end of all before it, and
+//     pdl_launch_dependents() first, for another of its kind.
 bool pdl_enabled();
 
 struct LaunchAttrs {
@@ -173,16 +177,21 @@ struct GemmArgs {
     int n = 0, k = 0;
     int dtype = EMBER_F32;
     const CacheRows *cache = nullptr;  // gemm_skinny_sm100.cu
+    // gemm_sm100.cu: the product launched just before this one, which neither reads this one's results nor writes what this one reads:
+    // the two run side by side where SMs are free (rules beside pdl_enabled).
+    const GemmArgs *beside = nullptr;
     const int *only_if = nullptr;  // CUDA-core kernel: return at once when this word of device memory is 0
 };
 
 // CUDA-core kernels (gemm_simt.cu): float32 math, any shape and view.
 int simt_gemm(const GemmArgs &g, DeviceState *st, cudaStream_t s);
 // column_sums.cu: out[j] = sum over rows of a(:, j), any shape and view
-int column_sums(const MatView &a, void *out, int dtype, DeviceState *st, cudaStream_t s);
+// beside: the kernel launched just before neither writes a nor touches out and runs beside this one (rules beside pdl_enabled)
+int column_sums(const MatView &a, void *out, int dtype, DeviceState *st, cudaStream_t s, bool beside = false);
 // tcgen05 kernel (gemm_sm100.cu): bf16 storage; see sm100_gemm_supported for the shapes it takes.
 bool sm100_gemm_supported(const GemmArgs &g);
 int sm100_gemm(const GemmArgs &g, DeviceState *st, cudaStream_t s);
+bool sm100_gemm_gains_beside(const GemmArgs &before, const GemmArgs &g, DeviceState *st);  // whether GemmArgs::beside makes g end sooner
 // dst (bf16, 16-byte aligned, rows of v.cols rounded up to 8) = v (row-major, any alignment), zeros past v.cols
 int pack_rows(const MatView &v, void *dst, cudaStream_t s);
 // tcgen05 kernel for at most 128 rows (gemm_skinny_sm100.cu): a decode step's projections.

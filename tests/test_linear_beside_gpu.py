@@ -1,0 +1,57 @@
+"""Both gradients and the bias gradient of one call run side by side on the GPU: the bits of three calls, call after call, with results that
+lie over one another's operands kept in order, and with what follows on the stream waiting for all of them."""
+import numpy as np
+import pytest
+
+import ember_b200 as em
+from conftest import bf16_round, seeded
+from ember_b200 import _lib
+
+pytestmark = pytest.mark.gpu
+
+BF16 = 1
+
+
+def bwd(x, w, g, dx, dw, db, m, n, k, heads=(0, 0, 0, 0)):
+    at = lambda t: t.ptr if t is not None else None  # noqa: E731
+    _lib.check(_lib.lib().ember_linear_bwd(at(x), at(w), at(g), at(dx), at(dw), at(db), m, n, k, BF16, *heads, None))
+
+
+# rows x inputs x outputs: one tile, several per pair, more pairs than tiles, both last rounds ragged, odd rows of results
+@pytest.mark.parametrize("m,k,n", [(256, 256, 256), (300, 264, 520), (8192, 256, 768), (2048, 2048, 2048), (4104, 1544, 4616), (1000, 512, 1536), (2048, 128, 8192)])
+def test_side_by_side_is_one_after_the_other(m, k, n):
+    x, w, g = (em.Tensor(bf16_round(seeded(s, i)), "bfloat16") for i, s in enumerate([(m, k), (k, n), (m, n)]))
+    new = lambda: [em.Tensor.empty(s, "bfloat16") for s in [(m, k), (k, n), (n,)]]  # noqa: E731
+    dx, dw, db = new()
+    bwd(x, w, g, dx, None, None, m, n, k)
+    bwd(x, w, g, None, dw, None, m, n, k)
+    bwd(x, w, g, None, None, db, m, n, k)
+    want = [t.to_np() for t in (dx, dw, db)]
+    for _ in range(3):
+        outs = new()
+        bwd(x, w, g, *outs, m, n, k)
+        for a, b in zip(outs, want):
+            assert np.array_equal(a.to_np(), b)
+    # a chain in which every call reads what the one before it wrote, nothing waited for in between
+    ys = [x]
+    for _ in range(4):
+        outs = new()
+        bwd(ys[-1], w, g, *outs, m, n, k)
+        ys.append(outs[0])
+        last = outs
+    assert np.array_equal(last[0].to_np(), want[0]) and np.array_equal(last[2].to_np(), want[2])
+    ref = new()
+    bwd(dx, w, g, None, ref[1], None, m, n, k)
+    assert np.array_equal(last[1].to_np(), ref[1].to_np())
+
+
+def test_results_over_operands():
+    m, k, n = 1024, 512, 768
+    x, w, g = (bf16_round(seeded(s, i)) for i, s in enumerate([(m, k), (k, n), (m, n)]))
+    T = lambda a: em.Tensor(a, "bfloat16")  # noqa: E731
+    dx, dw, db = (em.Tensor.empty(s, "bfloat16") for s in [(m, k), (k, n), (n,)])
+    bwd(T(x), T(w), T(g), dx, dw, db, m, n, k)
+    over, dw2, db2 = T(x), em.Tensor.empty((k, n), "bfloat16"), em.Tensor.empty((n,), "bfloat16")
+    bwd(over, T(w), T(g), over, dw2, db2, m, n, k)  # grad_x in the place of x, which grad_w still reads
+    for a, b in ((over, dx), (dw2, dw), (db2, db)):
+        assert np.array_equal(a.to_np(), b.to_np())
