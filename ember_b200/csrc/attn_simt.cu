@@ -225,6 +225,31 @@ __device__ __forceinline__ void store_row(T *dst, const f32x2 (&v)[Cols<DPAD>::N
     }
 }
 
+// Behind a tensor-core kernel these kernels are launched programmatically, to leave at once if it did the work (*only_if is 0).
+__device__ __forceinline__ bool not_needed(const int *only_if)
+{
+    if (!only_if) return false;
+    ptx::pdl_launch_dependents();
+    ptx::pdl_wait();
+    return *only_if == 0;
+}
+
+// Plain order otherwise: with blocks that wait on every SM 16 units x L1024 took 385 us instead of 305, forward and backward.
+template <typename P>
+int launch_simt(void (*kern)(P), long long grid, size_t smem, cudaStream_t s, const P &p)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3(NT);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    LaunchAttrs attrs;
+    if (p.only_if) attrs.pdl();
+    attrs.set(cfg);
+    EMBER_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, p));
+    return EMBER_OK;
+}
+
 struct SimtFwd {
     const void *q, *k, *v;
     void *out;
@@ -237,7 +262,7 @@ struct SimtFwd {
 template <typename T, bool FAST, int DPAD, int R>
 __global__ void __launch_bounds__(NT) simt_fwd_kernel(const SimtFwd p)
 {
-    if (p.only_if && *p.only_if == 0) return;  // the tensor-core kernel before this one did the work
+    if (not_needed(p.only_if)) return;
     constexpr int BM = 8 * R, NP = Cols<DPAD>::NP;
     extern __shared__ __align__(1024) char smem[];
     char *Qs = smem, *Ks = Qs + BM * DPAD * 4, *Vs = Ks + TN * DPAD * 4, *Ps = Vs + TN * DPAD * 4;
@@ -347,7 +372,7 @@ struct SimtBwd {
 template <typename T, bool FAST, int DPAD, int R>
 __global__ void __launch_bounds__(NT) simt_bwd_kernel(const SimtBwd p)
 {
-    if (p.only_if && *p.only_if == 0) return;  // the tensor-core kernel before this one did the work
+    if (not_needed(p.only_if)) return;
     constexpr int BM = 8 * R, NP = Cols<DPAD>::NP;
     extern __shared__ __align__(1024) char smem[];
     // A0, A1: this block's rows (K and V, or Q and dO); B0, B1: the streamed 64-row tiles (Q and dO, or K and V)
@@ -485,9 +510,7 @@ int launch_fwd(const AttnArgs &a, cudaStream_t s)
     SimtFwd p = {a.q, a.k, a.v, a.out, a.lse, a.bh, a.lq, a.lk, a.d, a.causal, (a.lq + BM - 1) / BM, a.scale, a.only_if};
     const long long grid = (long long)p.bh * p.blocks;
     if (grid > 0x7fffffffLL) return too_many_blocks();
-    kern<<<(unsigned)grid, NT, smem, s>>>(p);
-    EMBER_CUDA_TRY(cudaGetLastError());
-    return EMBER_OK;
+    return launch_simt(kern, grid, smem, s, p);
 }
 
 template <typename T, bool FAST, int DPAD, int R>
@@ -502,9 +525,7 @@ int launch_bwd(const AttnArgs &a, const float *delta, cudaStream_t s)
                  (a.lk + BM - 1) / BM, (a.lq + BM - 1) / BM, a.scale, a.only_if};
     const long long grid = (long long)p.bh * ((long long)p.kblocks + p.qblocks);
     if (grid > 0x7fffffffLL) return too_many_blocks();
-    kern<<<(unsigned)grid, NT, smem, s>>>(p);
-    EMBER_CUDA_TRY(cudaGetLastError());
-    return EMBER_OK;
+    return launch_simt(kern, grid, smem, s, p);
 }
 
 bool fast_rows(const AttnArgs &a)
