@@ -267,11 +267,10 @@ __device__ __forceinline__ void store_staged(const uint8_t *stage, __nv_bfloat16
 #ifndef BWD_EMU_PAIRS_OF_4
 #define BWD_EMU_PAIRS_OF_4 2  // pairs per group of 4 whose exponentials avoid the MUFU (128 columns)
 #endif
-// At 64 columns every exponential of the two-kernel form goes through the MUFU: a tile pair has half the tensor and
+// At 64 columns every exponential goes through the MUFU: a tile pair has half the tensor and
 // shared-memory work there, the compute warps' instruction issue is the limit, and the polynomial costs
 // more instructions than it frees MUFU slots (measured at 128 units x L4096: 1.57 against 1.70 ms without
-// a mask, 0.906 against 0.913 ms causal). The single-pass kernel, whose threads fetch a quarter of the row-vector elements, takes half of them
-// off it there too: 128 units x L2048 467 -> 452 us.
+// a mask, 0.906 against 0.913 ms causal).
 template <int HD>
 struct BwdEmu {
     static constexpr int PAIRS_OF_4 = HD >= 128 ? BWD_EMU_PAIRS_OF_4 : 0;
@@ -304,38 +303,6 @@ __device__ __forceinline__ void warp_arrive(uint32_t bar, int lane)
     tc_fence_before();
     __syncwarp();
     if (lane == 0) mbar_arrive(bar);
-}
-
-// two floats of shared memory
-__device__ __forceinline__ f32x2 lds_2(uint32_t addr)
-{
-    f32x2 v;
-    asm volatile("ld.shared.b64 %0, [%1];" : "=l"(v) : "r"(addr));
-    return v;
-}
-
-// Fragments of 16 lanes: registers 4 j .. 4 j + 3 of a thread are columns 8 j + 2 (lane % 4) + {0, 1} of tensor-memory lane lane / 4, then
-// of lane lane / 4 + 8 (the accumulator layout of mma.m16n8). 16x128b: register 2 j + b is 32-bit column 4 j + lane % 4 of lane lane / 4 + 8 b.
-__device__ __forceinline__ void tmem_ld_16x256b_x8(uint32_t taddr, uint32_t (&r)[32])
-{
-    asm volatile("tcgen05.ld.sync.aligned.16x256b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-                 : "r"(taddr));
-}
-__device__ __forceinline__ void tmem_ld_16x256b_x4(uint32_t taddr, uint32_t (&r)[16])
-{
-    asm volatile("tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-                 : "r"(taddr));
-}
-__device__ __forceinline__ void tmem_st_16x128b_x8(uint32_t taddr, const uint32_t (&r)[16])
-{
-    asm volatile("tcgen05.st.sync.aligned.16x128b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
-}
-// Four 8 x 8 matrices of 16-bit values, a register each (row lane / 4, columns 2 (lane % 4) + {0, 1}); lane l gives the address of row l % 8 of matrix l / 8.
-__device__ __forceinline__ void stmatrix_x4(uint32_t addr, const uint32_t (&r)[4])
-{
-    asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]) : "memory");
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -806,14 +773,14 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
 //   * the dP^T columns of tensor memory are dead once the compute warps have read them, so dQ(i)
 //     is accumulated there (tensor memory is full otherwise at HD = 128); four drain warps copy a
 //     whole row of it into registers at once while dK(i) is multiplied (dP^T(i+1) waits for that),
-//     then pass it through shared staging buffers to cp.reduce.async.bulk add.f32. Adding straight
-//     from registers with red.global.add.v4 is slower, for one chunk of four already (64 units x L4096: 745 -> 823 us, for all
-//     830 to 880): the additions back up in the load/store path that everything else of the SM uses.
+//     then pass it through shared staging buffers to cp.reduce.async.bulk add.f32. (Adding straight
+//     from registers with red.global measured slower: the additions back up in the load/store path
+//     that the compute warps' shared-memory and barrier traffic also uses.)
 //   * with all operands of S^T, dP^T, dK and dQ read from shared memory (128 bytes per clock, which
 //     one 128x128x16 product per 64 clocks uses up by itself), the kernel is bound by shared-memory
-//     bandwidth at 128 columns: about 544 KB per tile pair (288 KB of operands, 96 KB written by TMA and the dS^T
-//     stores, 128 KB through the staging buffers, 32 KB of row vectors) = 4250 clocks, and 4100 to 4300 are measured. At 64 columns
-//     the compute warps are the limit: 2900 clocks, 1480 to the stored P^T and 800 from dP^T to the stored dS^T.
+//     bandwidth: about 512 KB per tile pair (288 KB of operands, 96 KB written by TMA and the dS^T
+//     stores, 128 KB through the staging buffers) = 4000 clocks, against 3750 for the two kernels
+//     above together, which in practice take 5800.
 //   * the accumulator's layout is private to the two kernels: per (unit, query tile, lane quarter,
 //     32-column chunk) one contiguous 4 KB block holding [4-column group][row][4 floats], which makes
 //     the staging writes conflict-free and every bulk operation one contiguous block.
@@ -821,7 +788,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
 // to rounding (dK and dV stay bit-reproducible); the two-kernel form remains available for callers
 // who need run-to-run identical bits.
 //
-//   warps 0-7   compute                        warp 8       MMA issue: one order for all, so that dV(i+1) does not hold up dP^T(i+1)
+//   warps 0-7   compute (as above)            warp 8 / 9   MMA issue: score chain / gradient chain
 //   warp 10     TMA producer                   warp 11      tensor-memory allocation
 //   warps 12-15 drain dQ(i) from tensor memory into the global accumulator
 constexpr int SP_THREADS = (NCW + 8) * 32;
@@ -933,11 +900,11 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
         mbar_init(BAR(C::B_RES), 1);
         for (int s = 0; s < C::NA; s++) {
             mbar_init(BAR(C::B_FULLA + s), 1);
-            mbar_init(BAR(C::B_EMPTYA + s), 1);
+            mbar_init(BAR(C::B_EMPTYA + s), 2);  // released by both MMA warps
         }
         for (int s = 0; s < C::NB; s++) {
             mbar_init(BAR(C::B_FULLB + s), 1);
-            mbar_init(BAR(C::B_EMPTYB + s), 1);
+            mbar_init(BAR(C::B_EMPTYB + s), 2);  // dO is read by both chains (dP^T and dV)
         }
         mbar_init(BAR(C::B_S), 1);
         mbar_init(BAR(C::B_DP), 1);
@@ -946,7 +913,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
         mbar_init(BAR(C::B_DSFREE), 1);
         mbar_init(BAR(C::B_DQ), 1);
         mbar_init(BAR(C::B_DQFREE), 4);
-        mbar_init(BAR(C::B_ACC), 1);
+        mbar_init(BAR(C::B_ACC), 2);
         fence_mbar_init();
     }
     if (warp == W_ALLOC) {
@@ -967,7 +934,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
     pdl_launch_dependents();  // the dQ finish kernel may be placed on SMs as they fall idle; it waits for this grid's end
     if (warp >= W_DRAIN0) {
         // -------------------------------------------------------------------- drain dQ(i)
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 152;");  // holds a row of dQ(i)
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");  // holds half a row (64 columns) of dQ(i) at a time
         pdl_wait();  // the accumulator is cleared by the delta launch before this one
         const int w = warp - W_DRAIN0;  // == warp % 4: the tensor-memory lane quarter this warp may read
         const uint32_t t_dq = tmem + ((uint32_t)(w * 32) << 16) + C::T_DP;
@@ -981,31 +948,38 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
             tc_fence_after();
             if (w == 0 && lane == 0) TR(16, i);
             float *gdst = p.dq_acc + ((((size_t)bh * nqt + (i_begin + i)) * 4 + w) * chunks) * 1024;
-            // The whole row leaves tensor memory at once: dP^T(i+1) may overwrite it as soon as it is in registers, and the way
-            // through the staging buffers is slow while dK(i) reads its operands from shared memory at full rate.
-            uint32_t u[HD / 32][32];
+            // The row leaves tensor memory in two halves of 64 columns (the registers of these warps are
+            // what the compute warps do not get); dP^T(i+1) may overwrite it once the second half is read.
 #pragma unroll
-            for (int c = 0; c < HD / 32; c++) tmem_ld_32x32b_x32(t_dq + c * 32, u[c]);
-            tmem_wait_ld();
-            warp_arrive(BAR(C::B_DQFREE), lane);
-            if (w == 0 && lane == 0) TR(17, i);
-#pragma unroll
-            for (int c = 0; c < HD / 32; c++) {
-                if (PART && c >= chunks) break;
-                // the bulk operation that read this buffer two chunks ago must be done with it
-                if (lane == 0) bulk_wait_read_1();
-                __syncwarp();
-                uint8_t *buf = stage + (cnt & 1) * 4096;
-#pragma unroll
-                for (int cg = 0; cg < 8; cg++)
-                    *reinterpret_cast<uint4 *>(buf + (cg * 32 + lane) * 16) = make_uint4(u[c][4 * cg], u[c][4 * cg + 1], u[c][4 * cg + 2], u[c][4 * cg + 3]);
-                fence_proxy_async();
-                __syncwarp();
-                if (lane == 0) {
-                    if (ok) bulk_reduce_add_f32(gdst + c * 1024, stage_u32 + (cnt & 1) * 4096, 4096);
-                    bulk_commit();
+            for (int hf = 0; hf < HD / 64; hf++) {
+                uint32_t u[2][32];
+                tmem_ld_32x32b_x32(t_dq + hf * 64, u[0]);
+                tmem_ld_32x32b_x32(t_dq + hf * 64 + 32, u[1]);
+                tmem_wait_ld();
+                if (hf == HD / 64 - 1) {
+                    warp_arrive(BAR(C::B_DQFREE), lane);
+                    if (w == 0 && lane == 0) TR(17, i);
                 }
-                cnt++;
+#pragma unroll
+                for (int c2 = 0; c2 < 2; c2++) {
+                    const int c = hf * 2 + c2;
+                    if (PART && c >= chunks) break;
+                    // the bulk operation that read this buffer two chunks ago must be done with it
+                    if (lane == 0) bulk_wait_read_1();
+                    __syncwarp();
+                    uint8_t *buf = stage + (cnt & 1) * 4096;
+#pragma unroll
+                    for (int cg = 0; cg < 8; cg++)
+                        *reinterpret_cast<uint4 *>(buf + (cg * 32 + lane) * 16) =
+                            make_uint4(u[c2][4 * cg], u[c2][4 * cg + 1], u[c2][4 * cg + 2], u[c2][4 * cg + 3]);
+                    fence_proxy_async();
+                    __syncwarp();
+                    if (lane == 0) {
+                        if (ok) bulk_reduce_add_f32(gdst + c * 1024, stage_u32 + (cnt & 1) * 4096, 4096);
+                        bulk_commit();
+                    }
+                    cnt++;
+                }
             }
         }
         if (lane == 0) bulk_wait_all();
@@ -1036,7 +1010,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
                 issued_b = i + 1;
             }
             drain_copies<C>(bar0, issued_a, issued_b);
-        } else if (warp == W_MMA_A) {  // all 32 lanes, converged; one elected lane issues
+        } else if (warp == W_MMA_A || warp == W_MMA_B) {  // all 32 lanes, converged; one elected lane issues
             // ---------------------------------------------------------------- MMA issue
             constexpr uint32_t IDESC_SS = idesc_bf16_f32(128, 128, 0, 0);
             const int ksteps = PART ? (p.d + 15) / 16 : HD / 16;
@@ -1052,83 +1026,99 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
             constexpr uint32_t SUB16 = C::SUB_BYTES >> 4;
             const uint32_t elected = elect_one();
             bool ok = mbar_wait(BAR(C::B_RES), 0, abort_flag, p.status, WB_RES);
-            auto issue_scores = [&](uint32_t d, uint32_t a_lo, uint32_t b_lo) {
+            if (warp == W_MMA_A) {
+                // score chain: S^T(0); then per tile dV(i) (reads P^T, dO) and S^T(i+1) (overwrites P^T)
+                auto issue_st = [&](int i) {  // S^T = K Q^T
+                    const uint32_t q_lo = desc_lo(q_addr(i), 16);
 #pragma unroll
-                for (int sub = 0; sub < C::NSUB; sub++)
-                    if (!PART || sub * 4 < ksteps)
-                        mma_chain4_ss<2, 4, 6, 2, 4, 6>(tmem + d, a_lo + sub * SUB16, b_lo + sub * SUB16, IDESC_SS, elected, sub > 0, PART ? ksteps - sub * 4 : 4);
-            };
-            auto issue_st = [&](int i) {  // S^T = K Q^T
-                ok = ok && mbar_wait(BAR(C::B_FULLA + i % C::NA), (i / C::NA) & 1, abort_flag, p.status, WB_FULL);
+                    for (int sub = 0; sub < C::NSUB; sub++)
+                        if (!PART || sub * 4 < ksteps)
+                            mma_chain4_ss<2, 4, 6, 2, 4, 6>(tmem + C::T_S, k_lo + sub * SUB16, q_lo + sub * SUB16, IDESC_SS, elected, sub > 0, PART ? ksteps - sub * 4 : 4);
+                    tc_commit_elect(BAR(C::B_S));
+                };
+                ok = ok && mbar_wait(BAR(C::B_FULLA + 0), 0, abort_flag, p.status, WB_FULL);
                 tc_fence_after();
-                issue_scores(C::T_S, k_lo, desc_lo(q_addr(i), 16));
-                tc_commit_elect(BAR(C::B_S));
-            };
-            auto issue_dpt = [&](int i) {  // dP^T = V dO^T
-                ok = ok && mbar_wait(BAR(C::B_FULLB + i % C::NB), (i / C::NB) & 1, abort_flag, p.status, WB_FULL);
-                tc_fence_after();
-                issue_scores(C::T_DP, v_lo, desc_lo(do_addr(i), 16));
-                tc_commit_elect(BAR(C::B_DP));
-            };
-            const uint32_t ds_lo = desc_lo(dsa, 16), dsmn_lo = desc_lo(dsa, C::SUB_BYTES);
-            const uint32_t kmn_lo = desc_lo(ka, C::SUB_BYTES);
-            issue_st(0);
-            issue_dpt(0);
-            for (int i = 0; i < n && ok; i++) {
-                // dV(i) (reads P^T, dO), then S^T(i+1), which overwrites P^T(i): ordered by issue
-                const uint32_t domn_lo = desc_lo(do_addr(i), C::SUB_BYTES), qmn_lo = desc_lo(q_addr(i), C::SUB_BYTES);
-                ok = ok && mbar_wait(BAR(C::B_P), i & 1, abort_flag, p.status, WB_P);
-                tc_fence_after();
-                if (lane == 0) TR(8, i);
+                issue_st(0);
+                for (int i = 0; i < n && ok; i++) {
+                    const uint32_t domn_lo = desc_lo(do_addr(i), C::SUB_BYTES);
+                    ok = ok && mbar_wait(BAR(C::B_FULLB + i % C::NB), (i / C::NB) & 1, abort_flag, p.status, WB_FULL);
+                    ok = ok && mbar_wait(BAR(C::B_P), i & 1, abort_flag, p.status, WB_P);
+                    tc_fence_after();
+                    if (lane == 0) TR(8, i);
 #pragma unroll
-                for (int half = 0; half < 2; half++)  // dV += P^T dO
-                    mma_chain4_ts<8, 16, 24, 128, 256, 384>(tmem + C::T_ACC0, tmem + C::T_S + half * 64, domn_lo + half * 512, IDESC_TS, elected, i > 0 || half > 0);
-                tc_commit_elect(BAR(C::B_EMPTYB + i % C::NB));  // the last read of dO(i)
-                if (i + 1 < n) issue_st(i + 1);
-                if (lane == 0) TR(9, i);
-                // dQ(i), dK(i) (both read dS^T from shared memory), then dP^T(i+1), which overwrites dQ(i) and therefore waits for the drain warps
-                ok = ok && mbar_wait(BAR(C::B_DS), i & 1, abort_flag, p.status, WB_DS);
-                tc_fence_after();
-                if (lane == 0) TR(12, i);
-#pragma unroll
-                for (int half = 0; half < 2; half++)  // dQ(i) = dS K: 16 keys per step
-                    mma_chain4_ss<128, 256, 384, 128, 256, 384>(tmem + C::T_DP, dsmn_lo + half * 512, kmn_lo + half * 512, IDESC_DQ, elected, half > 0);
-                tc_commit_elect(BAR(C::B_DQ));  // the drain warps copy dQ(i) out while dK(i) is multiplied
-#pragma unroll
-                for (int half = 0; half < 2; half++)  // dK += dS^T Q: 16 queries per step
-                    mma_chain4_ss<2, 4, 6, 128, 256, 384>(tmem + C::T_ACC1, ds_lo + half * SUB16, qmn_lo + half * 512, IDESC_TS, elected, i > 0 || half > 0);
-                tc_commit_elect(BAR(C::B_DSFREE));
-                tc_commit_elect(BAR(C::B_EMPTYA + i % C::NA));  // the last read of Q(i)
-                if (lane == 0) TR(13, i);
-                if (i + 1 < n) {
-                    ok = ok && mbar_wait(BAR(C::B_DQFREE), i & 1, abort_flag, p.status, WB_ACC);
-                    if (lane == 0) TR(14, i);
-                    issue_dpt(i + 1);
-                    if (lane == 0) TR(15, i);
+                    for (int half = 0; half < 2; half++)  // dV += P^T dO
+                        mma_chain4_ts<8, 16, 24, 128, 256, 384>(tmem + C::T_ACC0, tmem + C::T_S + half * 32, domn_lo + half * 512, IDESC_TS, elected, i > 0 || half > 0);
+                    tc_commit_elect(BAR(C::B_EMPTYB + i % C::NB));  // this chain's last read of dO(i)
+                    if (i + 1 < n) {
+                        ok = ok && mbar_wait(BAR(C::B_FULLA + (i + 1) % C::NA), ((i + 1) / C::NA) & 1, abort_flag,
+                                             p.status, WB_FULL);
+                        tc_fence_after();
+                        issue_st(i + 1);  // overwrites P^T(i): ordered after dV(i) by issue order
+                    }
+                    if (lane == 0) TR(9, i);
+                    tc_commit_elect(BAR(C::B_EMPTYA + i % C::NA));  // this chain's last read of Q(i) was S^T(i)
                 }
+                tc_commit_elect(BAR(C::B_ACC));
+            } else {
+                // gradient chain: dP^T(0); then per tile dQ(i), dK(i) (both read dS^T from shared memory)
+                // and dP^T(i+1), which overwrites dQ(i) and therefore waits for the drain warps
+                auto issue_dpt = [&](int i) {  // dP^T = V dO^T
+                    const uint32_t do_lo = desc_lo(do_addr(i), 16);
+#pragma unroll
+                    for (int sub = 0; sub < C::NSUB; sub++)
+                        if (!PART || sub * 4 < ksteps)
+                            mma_chain4_ss<2, 4, 6, 2, 4, 6>(tmem + C::T_DP, v_lo + sub * SUB16, do_lo + sub * SUB16, IDESC_SS, elected, sub > 0, PART ? ksteps - sub * 4 : 4);
+                    tc_commit_elect(BAR(C::B_DP));
+                    tc_commit_elect(BAR(C::B_EMPTYB + i % C::NB));  // this chain's only read of dO(i)
+                };
+                const uint32_t ds_lo = desc_lo(dsa, 16), dsmn_lo = desc_lo(dsa, C::SUB_BYTES);
+                const uint32_t kmn_lo = desc_lo(ka, C::SUB_BYTES);
+                ok = ok && mbar_wait(BAR(C::B_FULLB + 0), 0, abort_flag, p.status, WB_FULL);
+                tc_fence_after();
+                issue_dpt(0);
+                for (int i = 0; i < n && ok; i++) {
+                    const uint32_t qmn_lo = desc_lo(q_addr(i), C::SUB_BYTES);
+                    ok = ok && mbar_wait(BAR(C::B_FULLA + i % C::NA), (i / C::NA) & 1, abort_flag, p.status, WB_FULL);
+                    ok = ok && mbar_wait(BAR(C::B_DS), i & 1, abort_flag, p.status, WB_DS);
+                    tc_fence_after();
+                    if (lane == 0) TR(12, i);
+#pragma unroll
+                    for (int half = 0; half < 2; half++)  // dQ(i) = dS K: 16 keys per step
+                        mma_chain4_ss<128, 256, 384, 128, 256, 384>(tmem + C::T_DP, dsmn_lo + half * 512, kmn_lo + half * 512, IDESC_DQ, elected, half > 0);
+                    tc_commit_elect(BAR(C::B_DQ));  // the drain warps copy dQ(i) out while dK(i) is multiplied
+#pragma unroll
+                    for (int half = 0; half < 2; half++)  // dK += dS^T Q: 16 queries per step
+                        mma_chain4_ss<2, 4, 6, 128, 256, 384>(tmem + C::T_ACC1, ds_lo + half * SUB16, qmn_lo + half * 512, IDESC_TS, elected, i > 0 || half > 0);
+                    tc_commit_elect(BAR(C::B_DSFREE));
+                    tc_commit_elect(BAR(C::B_EMPTYA + i % C::NA));  // this chain's last read of Q(i)
+                    if (lane == 0) TR(13, i);
+                    if (i + 1 < n) {
+                        ok = ok && mbar_wait(BAR(C::B_DQFREE), i & 1, abort_flag, p.status, WB_ACC);
+                        if (lane == 0) TR(14, i);
+                        ok = ok && mbar_wait(BAR(C::B_FULLB + (i + 1) % C::NB), ((i + 1) / C::NB) & 1, abort_flag,
+                                             p.status, WB_FULL);
+                        tc_fence_after();
+                        issue_dpt(i + 1);
+                        if (lane == 0) TR(15, i);
+                    }
+                }
+                tc_commit_elect(BAR(C::B_ACC));
             }
-            tc_commit_elect(BAR(C::B_ACC));
         }
     } else {
         // -------------------------------------------------------------------- compute
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 160;");  // 8 x 32 x 160 + 4 x 32 x 40 + 4 x 32 x 152 == 65536 == 512 x 128 at launch
-        // A thread owns 4 keys x 16 queries of its warp's 32 keys x 64 queries (the 16x256b fragments of tensor memory): keys
-        // lane / 4 + 8 b + 16 g, queries 8 j + 2 (lane % 4) + {0, 1}. With one key and 64 queries the queries' lse and delta came
-        // out of shared memory once for every thread, 128 KB a tile pair through the 128 bytes per clock that the MMAs' operands need
-        // too; so it is 32 KB. With the drain below, 128 units x L2048 d 64 475 -> 440 us, 36 units x 777 x 1301 d 80 67.2 -> 64.5.
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 192;");  // 8 x 32 x 192 + 4 x 32 x 40 + 4 x 32 x 88 == 65536
         const int h = warp / 4;                // which 64-column half of the 128 score columns (queries)
         const int r = threadIdx.x % 128;       // TMEM lane == key row inside the tile
-        const int key = k0 + (warp % 4) * 32 + lane / 4;
-        const int qcol = h * 64 + (lane % 4) * 2;
+        const int key = k0 + r;
         const uint32_t lane_sel = (uint32_t)((warp % 4) * 32) << 16;
         const uint32_t t_s = tmem + lane_sel + C::T_S, t_dp = tmem + lane_sel + C::T_DP;
-        constexpr uint32_t LANES16 = 16u << 16;
         const float c = p.scale_log2;
         const float *lse_g = p.lse + (size_t)bh * p.lq;
         const float *delta_g = p.delta + (size_t)bh * p.lq;
-        // row r of dS^T's sub-tile of these 64 queries: 16-byte chunk j of the row lies at chunk position j ^ (r % 8) (the 128-byte
-        // swizzle of the MMA descriptors)
-        const uint32_t ds_row = smem_base + C::OFF_DS + h * C::SUB_BYTES + r * 128;
+        // this thread's 128 bytes of dS^T: row r of the sub-tile of its 64 queries; 16-byte chunk j of
+        // the row lies at chunk position j ^ (r % 8) (the 128-byte swizzle of the MMA descriptors)
+        uint8_t *ds_row = smem_gen + C::OFF_DS + h * C::SUB_BYTES + r * 128;
         bool ok = true;
         const float *rowvec_src = (threadIdx.x < 128 ? lse_g : delta_g);
         auto fetch_raw = [&](int i) -> float {
@@ -1137,68 +1127,52 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
             if (i < n && qrow < p.lq) asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(rowvec_src + qrow));
             return v;
         };
-        // -lse * log2(e) and delta of tile i are in half (i & 1) of the row vectors, written by the first and the last 128 threads a
-        // tile ahead. One barrier a tile, between the two phases: lse(i+1) is written before it (lse(i-1) was last read before the
-        // barrier of tile i-1), delta(i+1) after it (delta(i-1) was last read before the barrier of tile i), so that either phase can
-        // fetch its 64 values ahead of the wait for its product.
-        auto put = [&](int i, float raw) {
-            const bool in_range = (i_begin + i) * 128 + (int)(threadIdx.x & 127) < p.lq;
-            rowvec[(i & 1) * 256 + threadIdx.x] = threadIdx.x < 128 ? (in_range ? -raw * LOG2E_B : -INFINITY) : (in_range ? raw : 0.f);
-        };
-        const uint32_t rv_u32 = smem_base + C::OFF_ROWVEC + qcol * 4;
         // Everything up to here (and the producer's copies and the first two products) needs nothing
         // from the delta launch before this one; the delta vector does.
         pdl_wait();
-        put(0, fetch_raw(0));
-        float raw_next = fetch_raw(1);
-        named_bar_sync(1, NCT);
+        float raw_next = fetch_raw(0);
         for (int i = 0; i < n; i++) {
             const int q0 = (i_begin + i) * 128;
-            const uint32_t rv = rv_u32 + (i & 1) * 1024;
+            float *rv = rowvec + (i & 1) * 256;
+            {
+                const bool in_range = q0 + (threadIdx.x & 127) < p.lq;
+                rv[threadIdx.x] = threadIdx.x < 128 ? (in_range ? -raw_next * LOG2E_B : -INFINITY) : (in_range ? raw_next : 0.f);
+            }
+            raw_next = fetch_raw(i + 1);
             // ---- phase 1: P^T = exp2(S^T * c - lse2), bf16 into tensor memory for dV += P^T dO
-            f32x2 lse2[8], delta2[8];
-#pragma unroll
-            for (int j = 0; j < 8; j++) lse2[j] = lds_2(rv + j * 32);
             ok = ok && mbar_wait(BAR(C::B_S), i & 1, abort_flag, p.status, WB_S);
             tc_fence_after();
             if (threadIdx.x == 0) TR(0, i);
-            uint32_t pv[2][32];  // [g][4 j + 2 b + e]
-            tmem_ld_16x256b_x8(t_s + h * 64, pv[0]);
-            tmem_ld_16x256b_x8(t_s + LANES16 + h * 64, pv[1]);
-            tmem_wait_ld();
+            float pv[64];
+            tmem_ld_cols<64>(t_s + h * 64, pv);
+            // every thread has read its scores (the bf16 P^T overwrites columns another thread of the
+            // same lane still needs) and the lse/delta vectors are visible
+            named_bar_sync(1, NCT);
             if (threadIdx.x == 0) TR(1, i);
             if (p.causal && (k0 + 127 > q0 + off)) {  // tile crossed by the diagonal: mask before the exp
-                const uint32_t masked = __float_as_uint(c > 0.f ? -INFINITY : INFINITY);
-                const int ahead = key - (q0 + qcol + off);  // of the thread's first query
+                const float masked = c > 0.f ? -INFINITY : INFINITY;
 #pragma unroll
-                for (int g = 0; g < 2; g++)
-#pragma unroll
-                    for (int x = 0; x < 32; x++)
-                        if (ahead + 16 * g + 8 * (x / 2 % 2) > 8 * (x / 4) + x % 2) pv[g][x] = masked;
+                for (int cc = 0; cc < 64; cc++)
+                    if (key > q0 + h * 64 + cc + off) pv[cc] = masked;
             }
             const f32x2 c2 = pack2(c, c);
 #pragma unroll
-            for (int g = 0; g < 2; g++) {
-                uint32_t pk[16];
+            for (int ch = 0; ch < 4; ch++) {
+                uint32_t pk[8];
 #pragma unroll
-                for (int x = 0; x < 16; x++) {
-                    const f32x2 x2 = fma2(pack2(__uint_as_float(pv[g][2 * x]), __uint_as_float(pv[g][2 * x + 1])), c2, lse2[x / 2]);
+                for (int x = 0; x < 8; x++) {
+                    const int cc = ch * 16 + 2 * x;
+                    const f32x2 x2 = fma2(pack2(pv[cc], pv[cc + 1]), c2, *reinterpret_cast<const f32x2 *>(&rv[h * 64 + cc]));
                     float p0, p1;
-                    exp2_pair<BWD_EMU_PAIRS_OF_4>(x2, x, p0, p1);
-                    pv[g][2 * x] = __float_as_uint(p0);
-                    pv[g][2 * x + 1] = __float_as_uint(p1);
+                    exp2_pair<BwdEmu<HD>::PAIRS_OF_4>(x2, x, p0, p1);
+                    pv[cc] = p0;
+                    pv[cc + 1] = p1;
                     pk[x] = pack_bf16(p0, p1);
                 }
-                tmem_st_16x128b_x8(t_s + g * LANES16 + h * 64, pk);  // 64 score columns -> 32 packed columns, among this warp's own
+                tmem_st_x8(t_s + h * 32 + ch * 8, pk);  // 16 score columns -> 8 packed columns
             }
-            if (threadIdx.x < 128) put(i + 1, raw_next);
             tmem_wait_st();
             warp_arrive(BAR(C::B_P), lane);
-            named_bar_sync(1, NCT);
-            if (threadIdx.x >= 128) put(i + 1, raw_next);
-            raw_next = fetch_raw(i + 2);
-#pragma unroll
-            for (int j = 0; j < 8; j++) delta2[j] = lds_2(rv + 512 + j * 32);
             if (threadIdx.x == 0) TR(2, i);
 
             // ---- phase 2: dS^T = P^T * (dP^T - delta), bf16 into shared memory for dQ = dS K and dK += dS^T Q
@@ -1207,25 +1181,23 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
             tc_fence_after();
             if (threadIdx.x == 0) TR(3, i);
 #pragma unroll
-            for (int half = 0; half < 2; half++) {  // 32 queries
-                uint32_t dp[2][16];
-                tmem_ld_16x256b_x4(t_dp + h * 64 + half * 32, dp[0]);
-                tmem_ld_16x256b_x4(t_dp + LANES16 + h * 64 + half * 32, dp[1]);
-                tmem_wait_ld();
+            for (int half = 0; half < 2; half++) {
+                float dp[32];
+                tmem_ld_cols<32>(t_dp + h * 64 + half * 32, dp);
 #pragma unroll
-                for (int jj = 0; jj < 4; jj++) {  // 8 queries of the warp's 32 keys: a 16-byte chunk of each row, four 8 x 8 matrices
-                    const int j = half * 4 + jj;
+                for (int q4 = 0; q4 < 4; q4++) {  // 8 queries = one 16-byte chunk
                     uint32_t w4[4];
 #pragma unroll
                     for (int x = 0; x < 4; x++) {
-                        const int g = x / 2, at = 4 * j + 2 * (x % 2), ad = 4 * jj + 2 * (x % 2);
-                        const f32x2 ds2 = mul2(pack2(__uint_as_float(pv[g][at]), __uint_as_float(pv[g][at + 1])),
-                                               sub2(pack2(__uint_as_float(dp[g][ad]), __uint_as_float(dp[g][ad + 1])), delta2[j]));
+                        const int cd = q4 * 8 + 2 * x, cc = half * 32 + cd;
+                        const f32x2 ds2 = mul2(pack2(pv[cc], pv[cc + 1]),
+                                               sub2(pack2(dp[cd], dp[cd + 1]), *reinterpret_cast<const f32x2 *>(&rv[128 + h * 64 + cc])));
                         float d0, d1;
                         unpack2(ds2, d0, d1);
                         w4[x] = pack_bf16(d0, d1);
                     }
-                    stmatrix_x4(ds_row + ((j ^ (r & 7)) << 4), w4);
+                    const int chunk = half * 4 + q4;
+                    *reinterpret_cast<uint4 *>(ds_row + ((chunk ^ (r & 7)) << 4)) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
                 }
             }
             fence_proxy_async();  // the MMAs read dS^T through the async proxy
