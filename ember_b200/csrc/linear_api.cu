@@ -328,9 +328,10 @@ int ember_linear_bwd(const void *x, const void *w, const void *dy, void *dx, voi
     // 4096 x 1536 x 4608 116 -> 92, 1000 x 512 x 1536 26.5 -> 18, 2048 x 128 x 32768 202 -> 177, 8192 x 2048 x 32768, which is bound by power,
     // 1612 -> 1593 (1633 with the bias gradient beside the input gradient).
     const size_t xs = (size_t)m * k * 2, ws = (size_t)k * n * 2, ys = (size_t)m * n * 2, bs = (size_t)n * 2;
-    if (!done && dw && dx && on_tile_kernel(gw) && on_tile_kernel(gx) && apart(dx, xs, x, xs) && apart(dx, xs, dw, ws) && apart(dw, ws, w, ws) &&
-        apart(dw, ws, dy, ys) && (!db || (apart(db, bs, x, xs) && apart(db, bs, w, ws) && apart(db, bs, dy, ys) && apart(db, bs, dw, ws) &&
-                                          apart(db, bs, dx, xs) && apart(dx, xs, dy, ys)))) {
+    // Each result has to lie apart from what the other two read: dx from x and dy, dw from w and dy, db from all; and from one another.
+    if (!done && dw && dx && on_tile_kernel(gw) && on_tile_kernel(gx) && apart(dx, xs, x, xs) && apart(dx, xs, dy, ys) && apart(dx, xs, dw, ws) &&
+        apart(dw, ws, w, ws) && apart(dw, ws, dy, ys) &&
+        (!db || (apart(db, bs, x, xs) && apart(db, bs, w, ws) && apart(db, bs, dy, ys) && apart(db, bs, dw, ws) && apart(db, bs, dx, xs)))) {
         if ((rc = sm100_gemm(gw, st, s)) != EMBER_OK) return rc;
         const bool gains = sm100_gemm_gains_beside(gw, gx, st);
         if (!gains && db && (rc = column_sums(gw.b, db, dtype, st, s, true)) != EMBER_OK) return rc;

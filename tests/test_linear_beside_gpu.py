@@ -57,6 +57,25 @@ def test_results_over_operands():
         assert np.array_equal(a.to_np(), b.to_np())
 
 
+@pytest.mark.parametrize("bias", [False, True])
+@pytest.mark.parametrize("m", [300, 8192])
+def test_grad_x_in_the_place_of_grad_y(m, bias):
+    """One tile of columns: a tile's rows of grad_y are all read before its grad_x is stored, so that the input gradient alone may take their
+    place; the weight and bias gradients, which read grad_y too, then have to be done before it."""
+    n = k = 128
+    x, w, g = (em.Tensor(bf16_round(seeded(s, i)), "bfloat16") for i, s in enumerate([(m, k), (k, n), (m, n)]))
+    new = lambda: [em.Tensor.empty(s, "bfloat16") for s in [(m, k), (k, n), (n,)]]  # noqa: E731
+    dx, dw, db = new()
+    bwd(x, w, g, dx, None, None, m, n, k)
+    bwd(x, w, g, None, dw, db, m, n, k)
+    want = [t.to_np() for t in (dx, dw, db)][:3 if bias else 2]
+    for _ in range(5):
+        over, dw2, db2 = em.Tensor(g.to_np(), "bfloat16"), *new()[1:]
+        bwd(x, w, over, over, dw2, db2 if bias else None, m, n, k)
+        for a, b in zip((over, dw2, db2), want):
+            assert np.array_equal(a.to_np(), b)
+
+
 @pytest.mark.parametrize("m,k,n", [(4104, 1544, 4616), (1000, 512, 1536), (1024, 512, 32768)])
 def test_captured_and_on_another_stream(m, k, n):
     """In a graph, whose first and last kernels write what is read and read what is written: each replay sees its own inputs through."""
