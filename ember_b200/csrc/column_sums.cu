@@ -28,8 +28,11 @@ __device__ __forceinline__ float ld_peer_f32(uint32_t addr)
 }
 
 // VEC: 16-byte pieces that are aligned and stay inside a row or head.
-template <typename T, bool VEC, int NTHR>
-__global__ void __launch_bounds__(NTHR) column_sum_kernel(const MatView a, T *__restrict__ out, int splits, bool late_wait)
+// BESIDE: beside the kernel before it (rules beside pdl_enabled), it reads before it waits. The kernels that wrote `a` are done by then and their
+// writes in L2; the fence drops what this SM's L1 may still hold from before them, and nothing writes `a` while this kernel runs. (Loads past
+// L1, or relaxed ones, in its place: 1946 x 512 x 1536 backward 18.5 -> 24.5 us, 2468 x 1024 x 3072 45 -> 50; with the fence as without it.)
+template <typename T, bool VEC, int NTHR, bool BESIDE>
+__global__ void __launch_bounds__(NTHR) column_sum_kernel(const MatView a, T *__restrict__ out, int splits)
 {
     constexpr int NV = VEC ? 16 / (int)sizeof(T) : 1;  // columns per load
     constexpr int TX = VEC ? 8 : 32, TY = NTHR / TX;   // threads along a strip's columns, rows per pass
@@ -37,7 +40,7 @@ __global__ void __launch_bounds__(NTHR) column_sum_kernel(const MatView a, T *__
     __shared__ float red[TY][COLS + 1];
     __shared__ float total[COLS];
     pdl_launch_dependents();
-    if (!late_wait) pdl_wait();
+    if constexpr (BESIDE) __threadfence(); else pdl_wait();
     const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;
     const int rank = splits > 1 ? (int)cluster_ctarank() : 0;
     const int col = ((int)blockIdx.x / splits) * COLS + tx * NV;
@@ -115,7 +118,7 @@ __global__ void __launch_bounds__(NTHR) column_sum_kernel(const MatView a, T *__
     if (rank == 0 && c < COLS && oc < a.cols) {
         if constexpr (sizeof(T) == 2) out[oc] = __float2bfloat16_rn(total[c]); else out[oc] = total[c];
     }
-    if (late_wait) pdl_wait();  // this kernel's end stands for the end of all before it
+    if constexpr (BESIDE) pdl_wait();  // this kernel's end stands for the end of all before it
 }
 
 template <typename T, bool VEC>
@@ -136,7 +139,7 @@ int launch(const MatView &a, T *out, int sms, cudaStream_t s, bool beside)
     cfg.stream = s;
     LaunchAttrs attrs;
     attrs.cluster((unsigned)splits).pdl().set(cfg);
-    EMBER_CUDA_TRY(cudaLaunchKernelEx(&cfg, column_sum_kernel<T, VEC, NTHR>, a, out, splits, beside));
+    EMBER_CUDA_TRY(cudaLaunchKernelEx(&cfg, beside ? column_sum_kernel<T, VEC, NTHR, true> : column_sum_kernel<T, VEC, NTHR, false>, a, out, splits));
     return EMBER_OK;
 }
 

@@ -22,7 +22,9 @@ namespace ember {
 //   - sm100_gemm_kernel passes pdl_wait() before pdl_launch_dependents(). What is launched behind it finds every kernel before it done, and
 //     may begin without pdl_wait() if it neither reads nor overwrites anything of the product itself: the products and the bias gradient of one
 //     backward call ("beside"). Such a kernel passes pdl_wait() last, so that its end, too, implies the end of all before it, and
-//     pdl_launch_dependents() first, for another of its kind.
+//     pdl_launch_dependents() first, for another of its kind;
+//   - what is read before pdl_wait() comes from L2: by TMA, or behind a fence that empties the SM's L1. Being let go early makes the writes of the
+//     kernels before visible nowhere else, and L1 may hold older lines of recycled memory.
 bool pdl_enabled();
 
 struct LaunchAttrs {
