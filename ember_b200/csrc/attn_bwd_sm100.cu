@@ -879,7 +879,10 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t *smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
-    if (!smem_layout_fits<C>(smem_u32(smem_raw), smem_base, p.status)) return;
+    if (!smem_layout_fits<C>(smem_u32(smem_raw), smem_base, p.status)) {
+        pdl_wait();  // also a kernel that does nothing ends after all before it
+        return;
+    }
     const uint32_t bar0 = smem_base + C::OFF_BAR;
     auto BAR = [&](int i) { return bar0 + 8u * (uint32_t)i; };
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem_gen + C::OFF_BAR + 8 * C::NUM_BARS);

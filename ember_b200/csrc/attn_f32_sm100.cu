@@ -637,6 +637,7 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
                 p.status->block = blockIdx.x;
                 p.status->extra = (int)(smem_base - smem_u32(smem_raw));
             }
+            pdl_wait();  // also a kernel that does nothing ends after all before it
             return;
         }
     }

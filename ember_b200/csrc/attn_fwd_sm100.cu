@@ -188,7 +188,8 @@ __global__ void __launch_bounds__(FWD_THREADS, 1)
     if (!PAIR && lk <= 0) {
         // An empty split (a sequence shorter than the others): its partial is "no weight". Every
         // thread leaves here, before any barrier or tensor-memory allocation exists. Without splits
-        // the (empty) sequence's result is defined as zeros with lse = -inf.
+        // the (empty) sequence's result is defined as zeros with lse = -inf. (With lengths or splits: launched in plain order.)
+        pdl_wait();
         if (p.lse && (int)threadIdx.x < p.block_rows && q_base + (int)threadIdx.x < p.lq)
             p.lse[(size_t)bh * p.lq + q_base + threadIdx.x] = -INFINITY;
         if (p.splits == 1)

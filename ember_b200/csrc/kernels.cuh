@@ -16,7 +16,7 @@ namespace ember {
 //   - every thread passes pdl_wait() before it reads or writes global memory (prefetching a tensor map and
 //     setting up barriers and tensor memory may come before), so that a kernel's end implies the end of
 //     all before it (the single-pass backward reads q, k, v and dO earlier: the delta kernel before it passes
-//     pdl_wait() first and lets it start afterwards);
+//     pdl_wait() first and lets it start afterwards); that goes for blocks that leave early, too;
 //   - a kernel that allocates tensor memory passes pdl_launch_dependents() after the allocation: a later kernel's
 //     block can then never hold the columns that an earlier one's, which it waits for, still needs;
 //   - sm100_gemm_kernel passes pdl_wait() before pdl_launch_dependents(). What is launched behind it finds every kernel before it done, and
