@@ -205,6 +205,12 @@ class MultiHeadAttention(Layer):
         return grad_x
 
     # ---- generation: the same block over a key/value cache -----------------------------------
+    def _weights_as_made(self) -> bool:
+        """Whether the weights are as reset() makes them. Others (no bias, an output of another width) are for linear_forward to take or refuse."""
+        e, w, o = self.embed_dim, self.w_qkv, self.w_o
+        return isinstance(w, Tensor) and w.shape == (e, 3 * e) and isinstance(o, Tensor) and o.shape == (e, e) and \
+            isinstance(self.b_qkv, Tensor) and isinstance(self.b_o, Tensor)
+
     def prefill(self, x: Tensor, cache) -> Tensor:
         """forward(x) under the causal mask that also stores the keys and values of x's positions in
         ``cache`` (a ``KVCache`` with kv_heads == num_heads), ready for ``decode_step``."""
@@ -221,7 +227,8 @@ class MultiHeadAttention(Layer):
         if len(x_t.shape) != 3 or x_t.shape[1] != 1 or x_t.shape[2] != self.embed_dim:
             raise ValueError(f"decode_step expects (B, 1, {self.embed_dim}), got {x_t.shape}")
         B, H, D = x_t.shape[0], self.num_heads, self.embed_dim // self.num_heads
-        if type(cache) is KVCache and isinstance(x_t, Tensor) and (cache.batch, cache.kv_heads, cache.head_dim) == (B, H, D) and cache.length < cache.capacity:
+        if type(cache) is KVCache and isinstance(x_t, Tensor) and (cache.batch, cache.kv_heads, cache.head_dim) == (B, H, D) and \
+                cache.length < cache.capacity and self._weights_as_made():
             # the same four calls made natively: from Python they take the host 22 us, as long as the GPU
             y = _core._decode_step(x_t._core, self.w_qkv._core, self.b_qkv._core, self.w_o._core, self.b_o._core, cache.k._core, cache.v._core,
                                    B, H, D, cache.capacity, cache.length, 1.0 / math.sqrt(D))

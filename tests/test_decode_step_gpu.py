@@ -31,3 +31,30 @@ def test_native_step_is_the_four_calls(batch, heads, dim, fill, dtype):
         assert np.array_equal(a, b)
     with pytest.raises((TypeError, ValueError)):
         layer.decode_step(em.Tensor(seeded((batch, 1, heads * dim), 9), "float32" if dtype == "bfloat16" else "bfloat16"), em.KVCache(batch, heads, 4, dim, dtype))
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_other_weights_than_the_layer_made(dtype):
+    """Set by the caller: no biases and an output of another width are taken, weights of the right size and a wrong shape are refused."""
+    batch, heads, dim, fill = 3, 4, 64, 5
+    e = heads * dim
+    rows = [em.Tensor(seeded((batch, heads, fill, dim), s, 0.5), dtype) for s in (2, 3)]
+    x = em.Tensor(seeded((batch, 1, e), 4), dtype)
+    got = []
+    for kind in (em.KVCache, PlainCache):
+        layer = em.nn.MultiHeadAttention(e, heads, causal=True, dtype=dtype, seed=1)
+        layer.b_qkv = layer.b_o = None
+        layer.w_o = em.Tensor(seeded((e, 2 * e), 5, 0.1), dtype)
+        cache = kind(batch, heads, fill + 1, dim, dtype)
+        cache.append(*rows)
+        y = layer.decode_step(x, cache)
+        assert y.shape == (batch, 1, 2 * e) and cache.length == fill + 1
+        got.append([t.to_np() for t in (y, cache.k, cache.v)])
+    for a, b in zip(*got):
+        assert np.array_equal(a, b)
+    for name, shape in (("w_qkv", (3 * e, e)), ("w_o", (2 * e, e // 2))):
+        layer, cache = em.nn.MultiHeadAttention(e, heads, causal=True, dtype=dtype, seed=1), em.KVCache(batch, heads, fill + 1, dim, dtype)
+        cache.append(*rows)
+        setattr(layer, name, em.Tensor(seeded(shape, 6, 0.1), dtype))
+        with pytest.raises(ValueError):
+            layer.decode_step(x, cache)
