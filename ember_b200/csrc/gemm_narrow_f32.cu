@@ -105,9 +105,27 @@ bool narrow_f32_supported(const GemmArgs &g)
 {
     if (g.dtype != EMBER_F32 || g.mode != GEMM_NN || g.m <= 0 || g.n <= 0 || g.n > 12 || g.k <= 0 || g.k % 4 != 0) return false;
     if (g.a.heads != 0 || g.b.heads != 0 || g.c.heads != 0 || (((uintptr_t)g.a.ptr | (uintptr_t)g.b.ptr) & 15) != 0) return false;
-    // Short contractions leave most of a block's threads without work: with many rows the tiles are quicker (8192 rows, 64 x 9: 10.3 us there, 15.5
-    // here; 128 x 9: 15.9 and 16.4; 256 x 10: 27 and 14). From 13 columns on the registers hold fewer blocks (4096 x 784 x 16: 15.8 and 21.3).
-    return g.m <= 0x7ffffff0LL && (g.k >= 256 || g.m <= 2048);
+    if (g.m > 0x7ffffff0LL || g.k > 0x7fffffff - 1024) return false;  // the kernel counts in ints, 1024 at a time
+    // us, the kernels that took these calls before (gemm_simt.cu, from some sizes on gemm_f32_sm100.cu) / here, calls back to back in a graph.
+    // Few rows and long contractions stay here, although a block's contraction is a chain and there are only m / 4 blocks: 17 x 4096 x 10
+    // 19.4 / 6.4, 17 x 65536 x 10 232 / 56, 1 x 65536 x 12 91 / 87, 1 x 262144 x 12 350 / 340, 256 x 65536 x 4 155 / 84.
+    // Short contractions leave most of a block's threads without work: with more rows than two blocks an SM take at once the tiles are quicker
+    // (2048 x 16 x 7 3.6 / 3.9, x 9 3.7 / 4.4, x 64 x 12 3.7 / 4.3; 1536 x 16 x 7 3.5 / 2.8, 2048 x 64 x 10 4.8 / 3.6; 8192 x 64 x 10 10.2 / 9.9, 65536 x 64 x 9 27 / 88).
+    const bool slow = g.n == 8 || g.n == 9 || g.n == 12;  // tiles move 8 and 12 columns in pieces of 16 bytes; the sums of 9 divide unevenly among lanes
+    if (g.m <= 1184) return true;
+    if (g.m <= 2048) return g.k >= (g.n == 12 ? 96 : slow || g.n == 11 || (g.n >= 6 && g.n != 10 && g.m > 1536) ? 64 : 0);
+    if (g.k < 256) return false;
+    // 8 and 12 columns while the tiles that gemm_simt.cu takes by then fill the SMs: 6000 rows x 256 9.9 / 10.3 and 9.9 / 11, x 372 x 12 12.1 / 12.9, 16384 x 256 19 / 24 both, x 384
+    // 26.6 / 27.5; on either side 3072 x 256 7.8 / 6.5, 8192 x 256 18 / 13, 12000 x 320 23 / 19.5, 18900 x 256 31 / 27, 32768 x 256 55 / 45.
+    if (g.n == 8 || g.n == 12) {
+        if (g.m >= 4096 && g.m <= 7040) return g.k >= 384;
+        if (g.m > 13500 && g.m <= 147 * 128) return g.k >= (g.m > 15500 ? 512 : 320);
+    }
+    // Very tall: 61000 x 256 x 8 and 12 1.22, x 448 1.1 times as long here, 262144 x 660 x 8 1.17 (65536 x 768 x 8 197 / 172); other
+    // widths 383000 x 256 x 4 1.22, x 6 1.37, x 10 1.2, x 11 1.46, x 320 1.02 to 1.24, from 384 on level or quicker here (65536 x 256 x 4 69 / 43, x 10 86 / 72).
+    if (slow && g.m > 55000) return g.k >= 768;
+    if (g.n >= 4 && g.m > 84000) return g.k >= 384;
+    return true;  // from 13 columns on the registers hold fewer blocks (4096 x 784 x 16: 15.8 / 21.3)
 }
 
 int narrow_f32_gemm(const GemmArgs &g, cudaStream_t s) { return launch<1>(g, s); }

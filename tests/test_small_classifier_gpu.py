@@ -40,3 +40,18 @@ def test_small_cross_entropy(rows, cols, dtype):
     assert (np.abs(loss.probs.to_np() - np.exp(lp)) <= rel * np.exp(lp) + 1e-30).all()
     ref = -(y * lp).sum() / rows
     assert abs(value - ref) <= 4e-6 * max(1.0, abs(ref))
+
+
+@pytest.mark.parametrize("k", [2**31 - 1024 - 4, 2**31 - 1024])
+def test_narrow_projection_of_a_longest_contraction(k):
+    """On either side of the last contraction that the kernel takes, whose counter stays below 2^31 past the end."""
+    torch = pytest.importorskip("torch")
+    from ember_b200 import _lib
+
+    x, w, y = (torch.zeros(n, device="cuda") for n in (k, k, 1))
+    at = torch.tensor([0, 3, 1024, 2**30 + 5, k - 1029, k - 1], device="cuda")
+    x[at], w[at] = torch.arange(1.0, 7.0, device="cuda"), 0.5
+    torch.cuda.synchronize()
+    _lib.check(_lib.lib().ember_linear_fwd(x.data_ptr(), w.data_ptr(), None, y.data_ptr(), 1, 1, k, 0, 0, 0, 0, 0, None))
+    em._core._sync()
+    assert y.item() == 10.5
