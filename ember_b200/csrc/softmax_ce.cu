@@ -394,11 +394,21 @@ __global__ void __launch_bounds__(BLOCK) loss_finalize_kernel(const float *row_l
     if (threadIdx.x == 0) *loss = -red[0] / (float)rows;
 }
 
-// Cross-entropy of a small classifier: at most 32 classes and 256 rows, probabilities and the loss by one block, a row per thread (a
+// Cross-entropy of a small classifier: few classes and at most 256 rows, probabilities and the loss by one block, a row per thread (a
 // row's elements are few enough to be in flight at once, and nothing is exchanged until the losses are added, in a fixed order). One launch
-// and the way of the row losses through memory less than row_softmax_kernel and loss_finalize_kernel: 256 x 10 float32 3.6 + 2.8 -> 4.3 us.
+// and the way of the row losses through memory less than row_softmax_kernel and loss_finalize_kernel.
+// A warp's load touches as many lines as a row has elements, so the time grows with rows x columns^2, where the other two kernels take 3.1 to 3.5 us
+// whatever the size. us, those two / this one, calls back to back in a graph: float32 256 x 10 3.5 / 3.2, 256 x 12 3.2 / 3.7, 192 x 12 3.1 / 2.9,
+// 128 x 12 3.1 / 2.5, 128 x 16 3.1 / 3.7, 64 x 20 3.1 / 2.6, 64 x 24 3.1 / 3.2, 32 x 28 3.1 / 2.6, 256 x 32 3.2 / 14; bfloat16, element loads of half the
+// bytes, 256 x 10 3.4 / 3.0, 128 x 16 3.2 / 3.6, 96 x 16 3.2 / 3.1, 64 x 20 3.4 / 3.1, 8 x 24 3.2 / 3.1, 8 x 28 3.3 / 3.5, 256 x 32 3.2 / 11.8. (The second launch
+// costs the host about 2 us more, which is what a caller of few rows waits for.)
 // A lane per class in its place took 6.3 us with one block (80 shuffles a warp on one SM) and 5.7 with a cluster of eight.
 constexpr int kSmallRows = 256, kSmallCols = 32;
+
+bool ce_small(long long rows, int cols, int dtype)
+{
+    return rows <= kSmallRows && cols <= (dtype == EMBER_BF16 ? 24 : kSmallCols) && rows * cols * cols <= kSmallRows * 110;
+}
 
 template <typename T>
 __global__ void __launch_bounds__(kSmallRows) ce_small_kernel(const T *__restrict__ x, const T *__restrict__ target, T *__restrict__ probs,
@@ -614,7 +624,7 @@ int ember_cross_entropy_fwd(const void *pred, const void *target, void *probs, f
     DeviceState *st = device_state();
     if (!st) return EMBER_ERR_CUDA;
     cudaStream_t s = pick_stream(stream, st);
-    if (rows <= kSmallRows && cols <= kSmallCols) {
+    if (ce_small(rows, cols, dtype)) {
         if (dtype == EMBER_BF16)
             EMBER_CUDA_TRY(launch_pdl(ce_small_kernel<__nv_bfloat16>, 1, kSmallRows, 0, s, (const __nv_bfloat16 *)pred, (const __nv_bfloat16 *)target,
                                       (__nv_bfloat16 *)probs, loss, (int)rows, cols));

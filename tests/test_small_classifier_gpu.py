@@ -1,4 +1,4 @@
-"""The kernels of a small classifier step: float32 projections to at most 12 columns, and cross-entropy of at most 32 classes and few rows,
+"""The kernels of a small classifier step: float32 projections to at most 12 columns, and cross-entropy of few classes and rows,
 at the edges of what sends a call to them, against float64."""
 import numpy as np
 import pytest
@@ -24,8 +24,8 @@ def test_narrow_projection(m, k, n, bias):
 
 
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
-@pytest.mark.parametrize("rows", [1, 31, 32, 33, 100, 255, 256, 257, 1000])
-@pytest.mark.parametrize("cols", [1, 2, 10, 31, 32, 33])
+@pytest.mark.parametrize("rows", [1, 31, 32, 33, 100, 195, 196, 255, 256, 257, 1000])  # 195 x 12: the last of that width in one block
+@pytest.mark.parametrize("cols", [1, 2, 10, 12, 24, 25, 31, 32, 33])
 def test_small_cross_entropy(rows, cols, dtype):
     x = seeded((rows, cols), 4, 3.0)
     x = bf16_round(x) if dtype == "bfloat16" else x
