@@ -40,12 +40,11 @@ constexpr int A_BYTES = BM * BK * 2;
 constexpr int SUB_BYTES = 64 * 128;           // 64 rows x 128 bytes
 constexpr int GEMM_THREADS = 192;
 
-// BN: columns of a pair's tile, 256, or 128 for results of few tiles: see launch. The epilogue stages OUT columns at a time: 128, or 64 in the
-// gradients' products, so that what is left of an SM's 228 KB of shared memory holds a block of column_sum_kernel. (64 in the
-// forward too: 8192 rows x 512 x 16384 137 -> 145 us, 2048 x 128 x 32768 64 -> 68.)
-template <int BN, int MODE>
+// BN: columns of a pair's tile, 256, or 128 for results of few tiles: see launch. The epilogue stages OUT columns at a time: 128, or 64 where
+// column sums run beside the product, so that what is left of an SM's 228 KB of shared memory holds a block of column_sum_kernel. (64 where
+// nothing does: forward of 8192 rows x 512 x 16384 137 -> 145 us, 2048 x 128 x 32768 64 -> 68.)
+template <int BN, int OUT>
 struct GemmCfg {
-    static constexpr int OUT = MODE == GEMM_NN ? 128 : 64;
     static constexpr int BNH = BN / 2;                     // B columns held by one CTA of a pair
     static constexpr int STAGE_BYTES = A_BYTES + BNH * BK * 2;
     static constexpr int OFF_OUT = STAGES * STAGE_BYTES;   // 128 rows x OUT columns of bf16 for the epilogue
@@ -75,13 +74,14 @@ struct GemmParams {
     DeviceStatus *status;
 };
 
-template <int MODE, int BN>
+// SIDE: one of a backward call's products that run side by side, or with column sums beside it.
+template <int MODE, int BN, int OUT, bool SIDE>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
     sm100_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
                       const GemmParams p)
 {
-    using C = GemmCfg<BN, MODE>;
-    constexpr int OUT = C::OUT, CPR = OUT / 8;  // CPR: 16-byte chunks of a staged row
+    using C = GemmCfg<BN, OUT>;
+    constexpr int CPR = OUT / 8;  // CPR: 16-byte chunks of a staged row
     constexpr int BNH = C::BNH, STAGE_BYTES = C::STAGE_BYTES, OFF_OUT = C::OFF_OUT, OFF_BIAS = C::OFF_BIAS, OFF_BAR = C::OFF_BAR,
                   USED_BYTES = C::USED_BYTES;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -137,15 +137,14 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     cluster_sync_all();  // both CTAs' barriers exist before either signals the other's
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    // What is launched behind this kernel may read what this one reads before it has waited itself (late_wait, column_sum_kernel), so it
+    // What is launched behind a SIDE kernel may read what this one reads before it has waited itself (late_wait, column_sum_kernel), so it
     // is let go only once the kernels before this one are done; a kernel with late_wait was let go that way and passes it on.
-    constexpr bool BESIDE = MODE != GEMM_NN;  // nothing runs beside a forward product
-    if (!BESIDE) pdl_launch_dependents();
-    if (!BESIDE || !p.late_wait) pdl_wait();
-    if (BESIDE) pdl_launch_dependents();
+    if (!SIDE) pdl_launch_dependents();
+    if (!SIDE || !p.late_wait) pdl_wait();
+    if (SIDE) pdl_launch_dependents();
     // the pair's i-th tile, num_tiles or more when there is none
     auto tile_of = [&](int i) {
-        if (!BESIDE || p.head_pairs == 0) return i * npairs + pair;
+        if (!SIDE || p.head_pairs == 0) return i * npairs + pair;
         if (pair < p.head_pairs) {
             if (i < p.head_tiles) return i * p.head_pairs + pair;
             i -= p.head_tiles;
@@ -315,7 +314,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     __syncthreads();
     cluster_sync_all();  // neither CTA leaves while the other may still signal its barriers or use the shared allocation
     if (warp == 4) tmem_dealloc_pair(tmem, 512);
-    if (BESIDE && p.late_wait) pdl_wait();  // this kernel's end stands for the end of all before it
+    if (SIDE && p.late_wait) pdl_wait();  // this kernel's end stands for the end of all before it
 }
 
 // Tiles of 256 rows and 256 (or 128) columns, and the steps of the contraction.
@@ -337,12 +336,15 @@ Tiling tiling(const GemmArgs &g, int sms)
 
 // A product beside the one before it finds the SMs at once that the other's last round leaves idle. The first `pairs` CTA pairs get
 // there first; they take `tiles` tiles each ahead of the rest, as many as make the end come soonest. false: no end comes sooner for it.
-bool head_of(const Tiling &before, const Tiling &t, int npairs, int &pairs, int &tiles)  // npairs: what the SMs hold
+// sums: the bias gradient runs behind both, beside this product, and so begins the sooner.
+bool head_of(const Tiling &before, const Tiling &t, int npairs, bool sums, int &pairs, int &tiles)  // npairs: what the SMs hold
 {
     pairs = tiles = 0;
     const long long all = t.tiles_m * t.tiles_n, idle = npairs - before.tiles_m * before.tiles_n % npairs;
     if (idle >= npairs) return false;
-    if (all <= npairs) return true;  // at most a tile each, on whatever SMs are free
+    // At most a tile each. With SMs free at once for all of them; for the bias gradient's sake also else (both gradients and bias of 1542 x 2048 x 6144
+    // 79 -> 71 us; without bias 2208 x 1024 x 1024 in 32 sequences 37 -> 39, 264 x 1024 x 1024 in 11 18.8 -> 19.8).
+    if (all <= (sums ? npairs : idle)) return true;
     const double late = (double)before.kblocks * before.bn / ((double)t.kblocks * t.bn);  // the others' start, in tiles
     const double alone = late + (all + npairs - 1) / npairs;
     double best = alone;
@@ -361,10 +363,10 @@ bool head_of(const Tiling &before, const Tiling &t, int npairs, int &pairs, int 
 
 bool c_rows_aligned(const GemmArgs &g) { return g.n % 8 == 0 && ((uintptr_t)g.c.ptr & 15) == 0; }
 
-template <int MODE, int BN>
+template <int MODE, int BN, int OUT, bool SIDE>
 int launch_tile(const GemmArgs &g, DeviceState *st, cudaStream_t s)
 {
-    using C = GemmCfg<BN, MODE>;
+    using C = GemmCfg<BN, OUT>;
     constexpr int BNH = C::BNH, SMEM_BYTES = C::SMEM_BYTES;
     const RowPlan rows = row_plan(g);
     MatView va = g.a, vb = g.b;
@@ -403,7 +405,7 @@ int launch_tile(const GemmArgs &g, DeviceState *st, cudaStream_t s)
     p.c_vec = c_rows_aligned(g);
     p.bias = (const __nv_bfloat16 *)g.bias;
     p.status = st->status;
-    auto kern = sm100_gemm_kernel<MODE, BN>;
+    auto kern = sm100_gemm_kernel<MODE, BN, OUT, SIDE>;
     static SmemOptIn opt_in;
     EMBER_CUDA_TRY(opt_in(kern, SMEM_BYTES));
     const long long tiles = (long long)p.tiles_m * p.tiles_n;
@@ -411,7 +413,7 @@ int launch_tile(const GemmArgs &g, DeviceState *st, cudaStream_t s)
     const int pairs = (int)(tiles < sms / 2 ? tiles : sms / 2);
     p.late_wait = g.beside != nullptr;
     p.head_pairs = p.head_tiles = 0;
-    if (g.beside) head_of(tiling(*g.beside, sms), tiling(g, sms), sms / 2, p.head_pairs, p.head_tiles);
+    if (g.beside) head_of(tiling(*g.beside, sms), tiling(g, sms), sms / 2, g.leaves_room, p.head_pairs, p.head_tiles);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * pairs);
     cfg.blockDim = dim3(GEMM_THREADS);
@@ -432,7 +434,12 @@ template <int MODE>
 int launch(const GemmArgs &g, DeviceState *st, cudaStream_t s)
 {
     const int sms = st->sm_count > 0 ? st->sm_count : 148;
-    return tiling(g, sms).bn == 128 ? launch_tile<MODE, 128>(g, st, s) : launch_tile<MODE, 256>(g, st, s);
+    const bool narrow = tiling(g, sms).bn == 128;
+    if constexpr (MODE != GEMM_NN) {  // nothing runs beside a forward product
+        if (g.leaves_room) return narrow ? launch_tile<MODE, 128, 64, true>(g, st, s) : launch_tile<MODE, 256, 64, true>(g, st, s);
+        if (g.held || g.beside) return narrow ? launch_tile<MODE, 128, 128, true>(g, st, s) : launch_tile<MODE, 256, 128, true>(g, st, s);
+    }
+    return narrow ? launch_tile<MODE, 128, 128, false>(g, st, s) : launch_tile<MODE, 256, 128, false>(g, st, s);
 }
 
 }  // namespace
@@ -518,7 +525,7 @@ bool sm100_gemm_gains_beside(const GemmArgs &before, const GemmArgs &g, DeviceSt
 {
     const int sms = st->sm_count > 0 ? st->sm_count : 148;
     int pairs, head;
-    return head_of(tiling(before, sms), tiling(g, sms), sms / 2, pairs, head);
+    return head_of(tiling(before, sms), tiling(g, sms), sms / 2, g.leaves_room, pairs, head);
 }
 
 int sm100_gemm(const GemmArgs &g, DeviceState *st, cudaStream_t s)

@@ -19,8 +19,8 @@ namespace ember {
 //     pdl_wait() first and lets it start afterwards); that goes for blocks that leave early, too;
 //   - a kernel that allocates tensor memory passes pdl_launch_dependents() after the allocation: a later kernel's
 //     block can then never hold the columns that an earlier one's, which it waits for, still needs;
-//   - sm100_gemm_kernel passes pdl_wait() before pdl_launch_dependents(). What is launched behind it finds every kernel before it done, and
-//     may begin without pdl_wait() if it neither reads nor overwrites anything of the product itself: the products and the bias gradient of one
+//   - sm100_gemm_kernel, where a call asks for it (GemmArgs::held, beside), passes pdl_wait() before pdl_launch_dependents(). What is launched behind it finds every
+//     kernel before it done, and may begin without pdl_wait() if it neither reads nor overwrites anything of the product itself: the products and the bias gradient of one
 //     backward call ("beside"). Such a kernel passes pdl_wait() last, so that its end, too, implies the end of all before it, and
 //     pdl_launch_dependents() first, for another of its kind;
 //   - what is read before pdl_wait() comes from L2: by TMA, or behind a fence that empties the SM's L1. Being let go early makes the writes of the
@@ -182,6 +182,8 @@ struct GemmArgs {
     // gemm_sm100.cu: the product launched just before this one, which neither reads this one's results nor writes what this one reads:
     // the two run side by side where SMs are free (rules beside pdl_enabled).
     const GemmArgs *beside = nullptr;
+    bool held = false;         // gemm_sm100.cu: what is launched next runs beside this product
+    bool leaves_room = false;  // the same, with room for blocks of column_sum_kernel on this product's SMs
     const int *only_if = nullptr;  // CUDA-core kernel: return at once when this word of device memory is 0
 };
 

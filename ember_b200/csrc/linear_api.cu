@@ -312,7 +312,7 @@ int ember_linear_bwd(const void *x, const void *w, const void *dy, void *dx, voi
     if (!st) return EMBER_ERR_CUDA;
     cudaStream_t s = pick_stream(stream, st);
     PackedOperands packed(s);
-    const GemmArgs gw = product_of(GRAD_W, sh, x, w, dy, dw), gx = product_of(GRAD_X, sh, x, w, dy, dx);
+    GemmArgs gw = product_of(GRAD_W, sh, x, w, dy, dw), gx = product_of(GRAD_X, sh, x, w, dy, dx);
     F32Products f32;
     if (dtype == EMBER_F32 && dw) f32.add(gw);
     if (dtype == EMBER_F32 && dx) f32.add(gx);
@@ -321,7 +321,7 @@ int ember_linear_bwd(const void *x, const void *w, const void *dy, void *dx, voi
         if ((rc = f32.run(st, s)) != EMBER_OK && rc != EMBER_ERR_NOMEM) return rc;
         done = rc == EMBER_OK;
     }
-    // Both products on the tile kernel: they and the bias gradient run side by side. The input gradient starts on the SMs that the weight
+    // The products on the tile kernel: they and the bias gradient run side by side. The input gradient starts on the SMs that the weight
     // gradient's last round leaves idle, where that makes it end sooner, and the bias gradient's blocks fit beside a product's on its SM, whose
     // memory bandwidth the product leaves alone: beside the input gradient, or beside the weight gradient where the input gradient waits for
     // both. us, one after the other -> side by side (rows x inputs x outputs): 8192 x 2048 x 6144 323 -> 304, 8192 x 2048 x 2048 116 -> 102,
@@ -329,15 +329,15 @@ int ember_linear_bwd(const void *x, const void *w, const void *dy, void *dx, voi
     // 1612 -> 1593 (1633 with the bias gradient beside the input gradient).
     const size_t xs = (size_t)m * k * 2, ws = (size_t)k * n * 2, ys = (size_t)m * n * 2, bs = (size_t)n * 2;
     // Each result has to lie apart from what the other two read: dx from x and dy, dw from w and dy, db from all; and from one another.
-    if (!done && dw && dx && on_tile_kernel(gw) && on_tile_kernel(gx) && apart(dx, xs, x, xs) && apart(dx, xs, dy, ys) && apart(dx, xs, dw, ws) &&
-        apart(dw, ws, w, ws) && apart(dw, ws, dy, ys) &&
-        (!db || (apart(db, bs, x, xs) && apart(db, bs, w, ws) && apart(db, bs, dy, ys) && apart(db, bs, dw, ws) && apart(db, bs, dx, xs)))) {
+    if (!done && dw && (dx || db) && on_tile_kernel(gw) && apart(dw, ws, dy, ys) &&
+        (!dx || (on_tile_kernel(gx) && apart(dx, xs, x, xs) && apart(dx, xs, dy, ys) && apart(dx, xs, dw, ws) && apart(dw, ws, w, ws))) &&
+        (!db || (apart(db, bs, x, xs) && apart(db, bs, w, ws) && apart(db, bs, dy, ys) && apart(db, bs, dw, ws) && (!dx || apart(db, bs, dx, xs))))) {
+        gw.leaves_room = gx.leaves_room = db != nullptr;
+        const bool gains = gw.held = dx && sm100_gemm_gains_beside(gw, gx, st);
+        if (gains) gx.beside = &gw; else gx.leaves_room = false;
         if ((rc = sm100_gemm(gw, st, s)) != EMBER_OK) return rc;
-        const bool gains = sm100_gemm_gains_beside(gw, gx, st);
         if (!gains && db && (rc = column_sums(gw.b, db, dtype, st, s, true)) != EMBER_OK) return rc;
-        GemmArgs g = gx;
-        if (gains) g.beside = &gw;
-        if ((rc = sm100_gemm(g, st, s)) != EMBER_OK) return rc;
+        if (dx && (rc = sm100_gemm(gx, st, s)) != EMBER_OK) return rc;
         return gains && db ? column_sums(gw.b, db, dtype, st, s, true) : EMBER_OK;
     }
     if (!done && dw && (rc = run(gw, st, s, packed)) != EMBER_OK) return rc;
