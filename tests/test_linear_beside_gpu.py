@@ -17,31 +17,35 @@ def bwd(x, w, g, dx, dw, db, m, n, k, heads=(0, 0, 0, 0)):
     _lib.check(_lib.lib().ember_linear_bwd(at(x), at(w), at(g), at(dx), at(dw), at(db), m, n, k, BF16, *heads, None))
 
 
-# rows x inputs x outputs: one tile, several per pair, more pairs than tiles, both last rounds ragged, odd rows of results
-@pytest.mark.parametrize("m,k,n", [(256, 256, 256), (300, 264, 520), (8192, 256, 768), (2048, 2048, 2048), (4104, 1544, 4616), (1000, 512, 1536), (2048, 128, 8192)])
-def test_side_by_side_is_one_after_the_other(m, k, n):
+# rows x inputs x outputs: one tile, several per pair, more pairs than tiles, both last rounds ragged, odd rows of results; then
+# (x_heads, y_heads, sequence, head dimension) as a block's projections have them, sequences of whole tiles and of others
+@pytest.mark.parametrize("m,k,n,heads", [
+    *((m, k, n, (0, 0, 0, 0)) for m, k, n in [(256, 256, 256), (300, 264, 520), (8192, 256, 768), (2048, 2048, 2048), (4104, 1544, 4616), (1000, 512, 1536), (2048, 128, 8192)]),
+    (1024, 512, 1536, (0, 4, 256, 128)), (1542, 2048, 6144, (0, 16, 1542, 128)), (2208, 1024, 3072, (0, 16, 69, 64)), (6000, 1024, 3072, (0, 16, 375, 64)),
+    (1024, 512, 512, (4, 0, 512, 128)), (264, 1024, 1024, (8, 0, 24, 128)), (2208, 1024, 1024, (8, 0, 69, 128)), (4224, 512, 512, (8, 0, 1408, 64))])
+def test_side_by_side_is_one_after_the_other(m, k, n, heads):
     x, w, g = (em.Tensor(bf16_round(seeded(s, i)), "bfloat16") for i, s in enumerate([(m, k), (k, n), (m, n)]))
     new = lambda: [em.Tensor.empty(s, "bfloat16") for s in [(m, k), (k, n), (n,)]]  # noqa: E731
     dx, dw, db = new()
-    bwd(x, w, g, dx, None, None, m, n, k)
-    bwd(x, w, g, None, dw, None, m, n, k)
-    bwd(x, w, g, None, None, db, m, n, k)
+    bwd(x, w, g, dx, None, None, m, n, k, heads)
+    bwd(x, w, g, None, dw, None, m, n, k, heads)
+    bwd(x, w, g, None, None, db, m, n, k, heads)
     want = [t.to_np() for t in (dx, dw, db)]
     for asked in ((1, 1, 1), (1, 1, 0), (0, 1, 1)) * 2:
         outs = [t if a else None for t, a in zip(new(), asked)]
-        bwd(x, w, g, *outs, m, n, k)
+        bwd(x, w, g, *outs, m, n, k, heads)
         for a, b in zip(outs, want):
             assert a is None or np.array_equal(a.to_np(), b)
     # a chain in which every call reads what the one before it wrote, nothing waited for in between
     ys = [x]
     for _ in range(4):
         outs = new()
-        bwd(ys[-1], w, g, *outs, m, n, k)
+        bwd(ys[-1], w, g, *outs, m, n, k, heads)
         ys.append(outs[0])
         last = outs
     assert np.array_equal(last[0].to_np(), want[0]) and np.array_equal(last[2].to_np(), want[2])
     ref = new()
-    bwd(dx, w, g, None, ref[1], None, m, n, k)
+    bwd(dx, w, g, None, ref[1], None, m, n, k, heads)
     assert np.array_equal(last[1].to_np(), ref[1].to_np())
 
 
@@ -80,6 +84,25 @@ def test_results_over_operands():
     bwd(over, T(w), T(g), over, dw2, db2, m, n, k)  # grad_x in the place of x, which grad_w still reads
     for a, b in ((over, dx), (dw2, dw), (db2, db)):
         assert np.array_equal(a.to_np(), b.to_np())
+
+
+@pytest.mark.parametrize("over", ["dx x", "dw w", "db x", "db w", "db dy", "db dw", "db dx", "dw dx"])
+def test_results_over_operands_and_one_another(over):
+    """A result that starts where an operand or another result does, where the products one after the other make that well defined: what
+    three calls in the order weight, bias, input gradient leave behind."""
+    result, place = over.split()
+    sizes = {"x": (1024, 512), "w": (512, 768), "dy": (1024, 768), "dx": (1024, 512), "dw": (512, 768), "db": (768,)}
+    (m, k), n = sizes["x"], 768
+    values = {name: bf16_round(seeded(sizes[name], i)) for i, name in enumerate(("x", "w", "dy"))}
+    got = []
+    for together in (True, False):
+        T = {name: em.Tensor(values[name], "bfloat16") if name in values else em.Tensor.empty(shape, "bfloat16") for name, shape in sizes.items()}
+        T[result] = T[place].view(0, sizes[result])
+        for wanted in [("dx", "dw", "db")] if together else [("dw",), ("db",), ("dx",)]:
+            bwd(T["x"], T["w"], T["dy"], *(T[r] if r in wanted else None for r in ("dx", "dw", "db")), m, n, k)
+        got.append({name: t.to_np() for name, t in T.items()})
+    for name in sizes:
+        assert np.array_equal(got[0][name], got[1][name]), name
 
 
 @pytest.mark.parametrize("bias", [False, True])
