@@ -772,15 +772,15 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
 //     row, keys = K across rows); K itself, resident in shared memory, is the MN-major B operand.
 //   * the dP^T columns of tensor memory are dead once the compute warps have read them, so dQ(i)
 //     is accumulated there (tensor memory is full otherwise at HD = 128); four drain warps copy a
-//     whole row of it into registers at once while dK(i) is multiplied (dP^T(i+1) waits for that),
-//     then pass it through shared staging buffers to cp.reduce.async.bulk add.f32. (Adding straight
+//     row of it into registers in halves of 64 columns while dK(i) is multiplied (dP^T(i+1) waits for that),
+//     and pass it through shared staging buffers to cp.reduce.async.bulk add.f32. (Adding straight
 //     from registers with red.global measured slower: the additions back up in the load/store path
 //     that the compute warps' shared-memory and barrier traffic also uses.)
 //   * with all operands of S^T, dP^T, dK and dQ read from shared memory (128 bytes per clock, which
-//     one 128x128x16 product per 64 clocks uses up by itself), the kernel is bound by shared-memory
-//     bandwidth: about 512 KB per tile pair (288 KB of operands, 96 KB written by TMA and the dS^T
-//     stores, 128 KB through the staging buffers) and the row vectors, which every compute thread reads for its
-//     64 queries; 4000 to 4200 clocks are measured, against 5800 of the two kernels above together.
+//     one 128x128x16 product per 64 clocks uses up by itself), shared-memory bandwidth is the likely bound:
+//     an estimate of 512 KB per tile pair (288 KB of operands, 96 KB written by TMA and the dS^T
+//     stores, 128 KB through the staging buffers), 4096 clocks; 4000 to 4200 are measured, against 5800 of the two
+//     kernels above together. (The row vectors, broadcast to a warp's lanes, do not show: with a quarter of their reads the period was the same.)
 //   * the accumulator's layout is private to the two kernels: per (unit, query tile, lane quarter,
 //     32-column chunk) one contiguous 4 KB block holding [4-column group][row][4 floats], which makes
 //     the staging writes conflict-free and every bulk operation one contiguous block.

@@ -326,7 +326,8 @@ int ember_linear_bwd(const void *x, const void *w, const void *dy, void *dx, voi
     // memory bandwidth the product leaves alone: beside the input gradient, or beside the weight gradient where the input gradient waits for
     // both. us, one after the other -> side by side (rows x inputs x outputs): 8192 x 2048 x 6144 323 -> 304, 8192 x 2048 x 2048 116 -> 102,
     // 4096 x 1536 x 4608 116 -> 92, 1000 x 512 x 1536 26.5 -> 18, 2048 x 128 x 32768 202 -> 177, 8192 x 2048 x 32768, which is bound by power,
-    // 1612 -> 1593 (1633 with the bias gradient beside the input gradient).
+    // 1612 -> 1593 (1633 with the bias gradient beside the input gradient). Weight and bias gradient alone: 42 x 2048 x 6144 21.8 -> 17.9, 8712 x 1024 x 1024
+    // 54 -> 48.5, over 90 shapes 0.87.
     const size_t xs = (size_t)m * k * 2, ws = (size_t)k * n * 2, ys = (size_t)m * n * 2, bs = (size_t)n * 2;
     // Each result has to lie apart from what the other two read: dx from x and dy, dw from w and dy, db from all; and from one another.
     if (!done && dw && (dx || db) && on_tile_kernel(gw) && apart(dw, ws, dy, ys) &&
