@@ -6,12 +6,13 @@
 //
 //   warps 0-3   softmax + epilogue of tile 0 (one thread per query row, row state in registers)
 //   warps 4-7   softmax + epilogue of tile 1
-//   warp  8/9   MMA issue for tile 0 / tile 1 (warp-collective, one elected lane each): S = Q K^T and
-//               O += P V with tcgen05.mma, accumulators in TMEM. One issuing warp per tile, on
-//               different schedulers: an issuing warp shares its scheduler with two busy softmax
-//               warps and a single one could not keep up with both tiles.
+//   warp  8/9   MMA issue of O += P V for tile 0 / tile 1 (warp-collective, one elected lane each)
 //   warp 10     TMA producer (one lane): Q once, then K (2-stage ring) and V (3-stage ring)
-//   warp 11     TMEM allocation / release
+//   warp 11     MMA issue of S = Q K^T for both tiles; TMEM allocation / release
+// The scores have an issuing warp of their own: a tcgen05.commit holds its warp until the MMAs before it have left the queue (430 to 570
+// clocks behind the eight of a score product), and each barrier wait beside busy softmax warps takes 130 to 200 more even if the phase is
+// over, so that one warp per tile issued P V only when its next scores had long been finished and the tensor core idled 900 clocks of a
+// step (2690 to 2730 clocks a step with the exponentials left out, 2310 now; with them 3050 -> 2900: now the softmax warps are the limit).
 //
 // Tensor memory (512 columns x 128 lanes of 32 bit):
 //   P0 [0,64)  P1 [64,128)  S [128,256)  O0 [256,256+HD)  O1 [256+HD,256+2HD)
@@ -221,11 +222,11 @@ __global__ void __launch_bounds__(FWD_THREADS, 1)
         mbar_init(BAR(B_Q), 1);
         for (int s = 0; s < C::KSTAGES; s++) {
             mbar_init(BAR(B_KFULL + s), 1);
-            mbar_init(BAR(B_KEMPTY + s), 2);  // one commit from each MMA warp
+            mbar_init(BAR(B_KEMPTY + s), 1);
         }
         for (int s = 0; s < C::VSTAGES; s++) {
             mbar_init(BAR(B_VFULL + s), 1);
-            mbar_init(BAR(B_VEMPTY + s), 2);
+            mbar_init(BAR(B_VEMPTY + s), 2);  // one commit from the issuing warp of each tile
         }
         for (int t = 0; t < 2; t++) {
             mbar_init(BAR(B_S + t), 1);
@@ -309,83 +310,54 @@ __global__ void __launch_bounds__(FWD_THREADS, 1)
                            clock64() - t0 < kWaitLimitCycles) {}
                 while (!mbar_try_wait(BAR(B_Q), 0) && clock64() - t0 < kWaitLimitCycles) {}
             }
-        } else if ((warp == 8 || warp == 9) && crank == 0) {  // all 32 lanes, converged; one elected lane issues
-            // ------------------------------------------------------------ MMA issue for tile t (of both CTAs of a pair)
-            const int t = warp - 8;
+        } else if (warp == 11 && crank == 0) {  // all 32 lanes, converged; one elected lane issues
+            // ------------------------------------------------------------ MMA issue: scores of both tiles (of both CTAs of a pair)
             constexpr uint32_t IDESC_S = idesc_bf16_f32(PAIR ? 256 : 128, 128, 0, 0);
             const int ksteps = PART ? (p.d + 15) / 16 : HD / 16;
-            const uint32_t IDESC_O = idesc_bf16_f32(PAIR ? 256 : 128, ksteps * 16, 0, 1);
-            const int nt = n_t[t], no = n_t[1 - t];  // key tiles of this tile / of the other tile
-            const uint32_t q_lo = desc_lo(smem_base + C::OFF_Q + t * C::TILE_BYTES, 16);
             const uint32_t elected = elect_one();
             bool ok = mbar_wait(BAR(B_Q), 0, abort_flag, p.status, W_MMA_Q);
-            // The score buffer is used in the order S0(0) S1(0) S0(1) S1(1) ...; each user waits until
-            // the softmax warps of the previous user have copied their scores out.
-            auto issue_s = [&](int j) {
-                if (t == 0) {
-                    if (j >= 1) {  // previous user: S1(j-1) if the other tile has it, else our own S0(j-1)
-                        const int pt = (j - 1 < no) ? 1 : 0;
-                        ok = ok && mbar_wait(BAR(B_R + pt), (j - 1) & 1, abort_flag, p.status, W_MMA_R);
-                    }
-                } else {           // previous user: S0(j) if the other tile has it, else our own S1(j-1)
-                    if (j < no)
-                        ok = ok && mbar_wait(BAR(B_R + 0), j & 1, abort_flag, p.status, W_MMA_R);
-                    else if (j >= 1)
-                        ok = ok && mbar_wait(BAR(B_R + 1), (j - 1) & 1, abort_flag, p.status, W_MMA_R);
-                }
-                tc_fence_after();
-                const uint32_t k_lo = desc_lo(smem_base + C::OFF_K + (j % C::KSTAGES) * C::K_BYTES, 16);
-                if constexpr (PAIR) {
-#pragma unroll
-                    for (int ks = 0; ks < HD / 16; ks++) {
-                        const uint32_t o16 = ((ks / 4) * C::SUB_BYTES + (ks % 4) * 32) >> 4;
-                        const uint32_t k16 = ((ks / 4) * C::K_SUB_BYTES + (ks % 4) * 32) >> 4;
-                        mma_ss_lo_pair(tmem + C::TMEM_S, q_lo + o16, k_lo + k16, IDESC_S, ks > 0);
-                    }
-                } else {
-#pragma unroll
-                    for (int sub = 0; sub < C::NSUB; sub++)  // (a chain instead of single MMAs: 1 % at d 64 and long sequences, else the same)
-                        if (!PART || sub * 4 < ksteps)
-                            mma_chain4_ss<2, 4, 6, 2, 4, 6>(tmem + C::TMEM_S, q_lo + sub * (C::SUB_BYTES >> 4), k_lo + sub * (C::SUB_BYTES >> 4), IDESC_S, elected, sub > 0, PART ? ksteps - sub * 4 : 4);
-                }
-                f_commit<PAIR>(BAR(B_S + t));
-            };
-            // O_t += P_t(j) V_j for keys [64*half, 64*half + 64) of the tile
-            auto issue_pv_half = [&](int j, int half) {
-                ok = ok && mbar_wait(BAR(B_P + 2 * t + half), j & 1, abort_flag, p.status, W_MMA_P);
-                if (ONE && half == 0) ok = ok && mbar_wait(BAR(B_P + 1), j & 1, abort_flag, p.status, W_MMA_P);  // each warpgroup rescales half of O's columns
-                tc_fence_after();
-                const uint32_t v_lo = desc_lo(smem_base + C::OFF_V + (j % C::VSTAGES) * C::V_BYTES, C::SUB_BYTES);
-                if constexpr (PAIR) {
-#pragma unroll
-                    for (int k4 = 0; k4 < 4; k4++) {
-                        const int ks = half * 4 + k4;
-                        mma_ts_lo_pair(tmem + C::TMEM_O + t * HD, tmem + C::TMEM_P + t * 64 + ks * 8, v_lo + ks * (2048 >> 4),
-                                       IDESC_O, (j > 0 || ks > 0) ? 1u : 0u);
-                    }
-                } else {
-                    mma_chain4_ts<8, 16, 24, 128, 256, 384>(tmem + C::TMEM_O + t * HD, tmem + C::TMEM_P + t * 64 + half * 32, v_lo + half * 512,
-                                                            IDESC_O, elected, j > 0 || half > 0);
-                }
-                if (half == 1) f_commit<PAIR>(BAR(B_O + t));
-            };
-            // Both MMA warps release every K and V stage (the "empty" barriers count two commits), also
-            // for key tiles this query tile does not visit; a warp waits for the stage to be full
-            // before it commits, so that its arrival can never land in an earlier phase of the barrier.
-            ok = ok && mbar_wait(BAR(B_KFULL + 0), 0, abort_flag, p.status, W_MMA_K);
-            if (nt > 0) issue_s(0);
-            f_commit<PAIR>(BAR(B_KEMPTY + 0));
-            // Step j of this tile: S_t(j+1), then the two halves of PV_t(j). The score MMA comes
-            // first: its buffer is free (the other tile copied out) about half a period before this
-            // tile's probabilities are ready.
             for (int j = 0; j < n && ok; j++) {
-                if (j + 1 < n) {
-                    ok = ok && mbar_wait(BAR(B_KFULL + (j + 1) % C::KSTAGES), ((j + 1) / C::KSTAGES) & 1, abort_flag,
-                                         p.status, W_MMA_K);
-                    if (j + 1 < nt) issue_s(j + 1);
-                    f_commit<PAIR>(BAR(B_KEMPTY + (j + 1) % C::KSTAGES));  // our reads of K(j+1) are issued
+                ok = ok && mbar_wait(BAR(B_KFULL + j % C::KSTAGES), (j / C::KSTAGES) & 1, abort_flag, p.status, W_MMA_K);
+                const uint32_t k_lo = desc_lo(smem_base + C::OFF_K + (j % C::KSTAGES) * C::K_BYTES, 16);
+#pragma unroll 1
+                for (int t = 0; t < 2; t++) {
+                    if (j >= n_t[t]) continue;
+                    // The score buffer is used in the order S0(0) S1(0) S0(1) S1(1) ...; each user waits until the softmax warps of the
+                    // previous user have copied their scores out: the other tile's before this one if it has them, else this tile's last.
+                    const int pj = t == 0 || j >= n_t[0] ? j - 1 : j, pt = t == 0 ? (pj < n_t[1] ? 1 : 0) : (pj == j ? 0 : 1);
+                    if (pj >= 0) ok = ok && mbar_wait(BAR(B_R + pt), pj & 1, abort_flag, p.status, W_MMA_R);
+                    tc_fence_after();
+                    const uint32_t q_lo = desc_lo(smem_base + C::OFF_Q + t * C::TILE_BYTES, 16);
+                    if constexpr (PAIR) {
+#pragma unroll
+                        for (int ks = 0; ks < HD / 16; ks++) {
+                            const uint32_t o16 = ((ks / 4) * C::SUB_BYTES + (ks % 4) * 32) >> 4;
+                            const uint32_t k16 = ((ks / 4) * C::K_SUB_BYTES + (ks % 4) * 32) >> 4;
+                            mma_ss_lo_pair(tmem + C::TMEM_S, q_lo + o16, k_lo + k16, IDESC_S, ks > 0);
+                        }
+                    } else {
+#pragma unroll
+                        for (int sub = 0; sub < C::NSUB; sub++)  // (a chain instead of single MMAs: 1 % at d 64 and long sequences, else the same)
+                            if (!PART || sub * 4 < ksteps)
+                                mma_chain4_ss<2, 4, 6, 2, 4, 6>(tmem + C::TMEM_S, q_lo + sub * (C::SUB_BYTES >> 4), k_lo + sub * (C::SUB_BYTES >> 4), IDESC_S, elected, sub > 0, PART ? ksteps - sub * 4 : 4);
+                    }
+                    f_commit<PAIR>(BAR(B_S + t));
                 }
+                f_commit<PAIR>(BAR(B_KEMPTY + j % C::KSTAGES));  // all reads of K(j) are issued
+            }
+        } else if ((warp == 8 || warp == 9) && crank == 0) {
+            // ------------------------------------------------------------ MMA issue: O of tile t (of both CTAs of a pair)
+            const int t = warp - 8;
+            const int ksteps = PART ? (p.d + 15) / 16 : HD / 16;
+            const uint32_t IDESC_O = idesc_bf16_f32(PAIR ? 256 : 128, ksteps * 16, 0, 1);
+            const int nt = n_t[t];  // key tiles of this tile
+            const uint32_t elected = elect_one();
+            bool ok = true;
+            // Both warps release every V stage (the "empty" barrier counts two commits), also for key tiles this query tile does not
+            // visit; a warp waits for the stage to be full before it commits, so that its arrival can never land in an earlier phase.
+            for (int j = 0; j < n && ok; j++) {
                 ok = ok && mbar_wait(BAR(B_VFULL + j % C::VSTAGES), (j / C::VSTAGES) & 1, abort_flag, p.status, W_MMA_V);
+                const uint32_t v_lo = desc_lo(smem_base + C::OFF_V + (j % C::VSTAGES) * C::V_BYTES, C::SUB_BYTES);
                 if (!PAIR && p.seq_lens && j < nt && j * 128 + 128 > lk) {
                     // Cache decode with a per-sequence length below the tensor map's extent: TMA only
                     // zero-fills rows past the MAP's end, so V rows [lk, ...) of this tile hold whatever
@@ -402,8 +374,24 @@ __global__ void __launch_bounds__(FWD_THREADS, 1)
                     __syncwarp();
                 }
                 if (j < nt) {
-                    issue_pv_half(j, 0);
-                    issue_pv_half(j, 1);
+#pragma unroll
+                    for (int half = 0; half < 2; half++) {  // O_t += P_t(j) V_j for keys [64*half, 64*half + 64) of the tile
+                        ok = ok && mbar_wait(BAR(B_P + 2 * t + half), j & 1, abort_flag, p.status, W_MMA_P);
+                        if (ONE && half == 0) ok = ok && mbar_wait(BAR(B_P + 1), j & 1, abort_flag, p.status, W_MMA_P);  // each warpgroup rescales half of O's columns
+                        tc_fence_after();
+                        if constexpr (PAIR) {
+#pragma unroll
+                            for (int k4 = 0; k4 < 4; k4++) {
+                                const int ks = half * 4 + k4;
+                                mma_ts_lo_pair(tmem + C::TMEM_O + t * HD, tmem + C::TMEM_P + t * 64 + ks * 8, v_lo + ks * (2048 >> 4),
+                                               IDESC_O, (j > 0 || ks > 0) ? 1u : 0u);
+                            }
+                        } else {
+                            mma_chain4_ts<8, 16, 24, 128, 256, 384>(tmem + C::TMEM_O + t * HD, tmem + C::TMEM_P + t * 64 + half * 32, v_lo + half * 512,
+                                                                    IDESC_O, elected, j > 0 || half > 0);
+                        }
+                    }
+                    f_commit<PAIR>(BAR(B_O + t));
                 }
                 f_commit<PAIR>(BAR(B_VEMPTY + j % C::VSTAGES));  // our reads of V(j) are issued
             }
@@ -508,6 +496,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 1)
                     }
                     sum2[i & 3] = add2(sum2[i & 3], pack2(p0, p1));
                     pk[ch][i] = pack_bf16(p0, p1);
+                    if (ch == 1 && i == 7 && !o_done) o_done = mbar_try_wait(BAR(B_O), (j - 1) & 1);  // asked here, needed eight pairs later
                 }
             if (!o_done) {  // PV(j-1) must have read the old P
                 ok = ok && mbar_wait(BAR(B_O), (j - 1) & 1, abort_flag, p.status, W_SM_O);
@@ -663,45 +652,57 @@ __global__ void __launch_bounds__(FWD_THREADS, 1)
             }
             const f32x2 negm2 = pack2(-m_ref, -m_ref);
             const f32x2 c2 = pack2(c, c);
+            // weights of pairs [from, from + 8) of the scores at x: exponentials, their sum and bf16 pairs
+            auto weights = [&](const float *x, int from, f32x2 (&sum2)[4], uint32_t *pk) {
 #pragma unroll
-            for (int half = 0; half < 2; half++) {
-                f32x2 sum2[4] = {0, 0, 0, 0};  // bit pattern of (0.f, 0.f)
-                uint32_t pk[2][16];
-#pragma unroll
-                for (int c2i = 0; c2i < 2; c2i++) {
-                    const int ch = 2 * half + c2i;
-#pragma unroll
-                    for (int i = 0; i < 16; i++) {
-                        const f32x2 x2 = fma2(pack2(s[ch * 32 + 2 * i], s[ch * 32 + 2 * i + 1]), c2, negm2);
-                        float p0, p1;
-                        if (i % 4 < EMU) {  // polynomial on the FMA pipe
-                            exp2_poly2(x2, p0, p1);
-                        } else {            // MUFU
-                            float x0, x1;
-                            unpack2(x2, x0, x1);
-                            p0 = ex2(x0);
-                            p1 = ex2(x1);
-                        }
-                        sum2[i & 3] = add2(sum2[i & 3], pack2(p0, p1));
-                        pk[c2i][i] = pack_bf16(p0, p1);
+                for (int i = from; i < from + 8; i++) {
+                    const f32x2 x2 = fma2(pack2(x[2 * i], x[2 * i + 1]), c2, negm2);
+                    float p0, p1;
+                    if (i % 4 < EMU) {  // polynomial on the FMA pipe
+                        exp2_poly2(x2, p0, p1);
+                    } else {            // MUFU
+                        float x0, x1;
+                        unpack2(x2, x0, x1);
+                        p0 = ex2(x0);
+                        p1 = ex2(x1);
                     }
+                    sum2[i & 3] = add2(sum2[i & 3], pack2(p0, p1));
+                    pk[i] = pack_bf16(p0, p1);
                 }
-                if (!o_done) {  // before the first store: PV(j-1) must have read the old P (waited for as
-                                // late as possible: the 64 probabilities of this half are already computed)
-                    ok = ok && mbar_wait(BAR(B_O + t), (j - 1) & 1, abort_flag, p.status, W_SM_O);
-                    tc_fence_after();
-                    o_done = true;
-                }
-                tmem_st_32x32b_x16(tp + (2 * half) * 16, pk[0]);
-                tmem_st_32x32b_x16(tp + (2 * half + 1) * 16, pk[1]);
+            };
+            auto total = [](const f32x2 (&sum2)[4]) {
+                float a0, a1;
+                unpack2(add2(add2(sum2[0], sum2[1]), add2(sum2[2], sum2[3])), a0, a1);
+                return a0 + a1;
+            };
+            auto written = [&](int half) {
                 tmem_wait_st();
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) arrive(bar_p + 8u * (uint32_t)half);
-                float a0, a1;
-                unpack2(add2(add2(sum2[0], sum2[1]), add2(sum2[2], sum2[3])), a0, a1);
-                (half == 0 ? l0 : l1) += a0 + a1;
-            }
+            };
+            uint32_t pk[32];
+            f32x2 sum_a[4] = {0, 0, 0, 0}, sum_b[4] = {0, 0, 0, 0};  // bit pattern of (0.f, 0.f)
+            weights(s, 0, sum_a, pk);
+            weights(s, 8, sum_a, pk);
+            weights(s, 16, sum_a, pk);
+            if (!o_done) o_done = mbar_try_wait(BAR(B_O + t), (j - 1) & 1);  // asked here, needed eight pairs later
+            weights(s, 24, sum_a, pk);
+            if (!o_done)  // before the first store: PV(j-1) must have read the old P
+                ok = ok && mbar_wait(BAR(B_O + t), (j - 1) & 1, abort_flag, p.status, W_SM_O);
+            tc_fence_after();
+            tmem_st_32x32b_x16(tp, pk);
+            tmem_st_32x32b_x16(tp + 16, pk + 16);
+            written(0);
+            l0 += total(sum_a);
+            weights(s + 64, 0, sum_b, pk);
+            weights(s + 64, 8, sum_b, pk);
+            weights(s + 64, 16, sum_b, pk);
+            weights(s + 64, 24, sum_b, pk);
+            tmem_st_32x32b_x16(tp + 32, pk);
+            tmem_st_32x32b_x16(tp + 48, pk + 16);
+            written(1);
+            l1 += total(sum_b);
         }
 
         if (nk > 0) {
