@@ -772,15 +772,16 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
 //     row, keys = K across rows); K itself, resident in shared memory, is the MN-major B operand.
 //   * the dP^T columns of tensor memory are dead once the compute warps have read them, so dQ(i)
 //     is accumulated there (tensor memory is full otherwise at HD = 128); four drain warps copy a
-//     row of it into registers in halves of 64 columns while dK(i) is multiplied (dP^T(i+1) waits for that),
+//     row of it into registers while dK(i) is multiplied (dP^T(i+1) waits for that),
 //     and pass it through shared staging buffers to cp.reduce.async.bulk add.f32. (Adding straight
 //     from registers with red.global measured slower: the additions back up in the load/store path
 //     that the compute warps' shared-memory and barrier traffic also uses.)
 //   * with all operands of S^T, dP^T, dK and dQ read from shared memory (128 bytes per clock, which
-//     one 128x128x16 product per 64 clocks uses up by itself), shared-memory bandwidth is the likely bound:
-//     an estimate of 512 KB per tile pair (288 KB of operands, 96 KB written by TMA and the dS^T
-//     stores, 128 KB through the staging buffers), 4096 clocks; 4000 to 4200 are measured, against 5800 of the two
-//     kernels above together. (The row vectors, broadcast to a warp's lanes, do not show: with a quarter of their reads the period was the same.)
+//     one 128x128x16 product per 64 clocks uses up by itself), shared-memory bandwidth is the bound at 128 columns:
+//     512 KB per tile pair (288 KB of operands, 96 KB written by TMA and the dS^T
+//     stores, 128 KB through the staging buffers) are 4096 clocks, and 4110 are measured (with the way through the staging
+//     buffers left out 3170 for 3072, with its stores alone 3660 for 3584), against 5800 of the two kernels above together.
+//     The row vectors, broadcast to a warp's lanes, do not show there; at 64 columns they do (102 us; 97 with a constant in their place).
 //   * the accumulator's layout is private to the two kernels: per (unit, query tile, lane quarter,
 //     32-column chunk) one contiguous 4 KB block holding [4-column group][row][4 floats], which makes
 //     the staging writes conflict-free and every bulk operation one contiguous block.
@@ -788,13 +789,21 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
 // to rounding (dK and dV stay bit-reproducible); the two-kernel form remains available for callers
 // who need run-to-run identical bits.
 //
-//   warps 0-7   compute (as above)            warp 8 / 9   MMA issue: score chain / gradient chain
-//   warp 10     TMA producer                   warp 11      tensor-memory allocation
-//   warps 12-15 drain dQ(i) from tensor memory into the global accumulator
+//   warps 0-7   compute (as above)             warp 8       MMA issue: dV(i), S^T(i+1)
+//   warp  9     MMA issue: dQ(i), dK(i)         warp 11      MMA issue: dP^T(i+1); tensor-memory allocation
+//   warp 10     TMA producer                    warps 12-15  drain dQ(i) from tensor memory into the global accumulator
+// (A tcgen05.commit holds its warp until the MMAs before it have left the queue, and a wait beside busy compute warps takes 130 to 200 clocks:
+// dP^T(i+1), which the compute warps wait for, is issued by a warp that does nothing else. With the drain of whole rows 64 query tiles x 16
+// key tiles of d 128 152.5 -> 143.8 us, d 80 140 -> 132, 2 x 32 x 8192 d 128 causal 2980 -> 2920, 36 x 777 x 1301 d 80 67 -> 64.8.)
+// BESIDE (64 columns): tensor memory has room for dQ beside dP^T, so that dP^T(i+1) waits for no drain, and dS^T goes to tensor memory too,
+// over the dP^T columns that its thread has read: dK takes it from there and reads 16 KB of shared memory a tile instead of 48. The compute
+// warps are the limit (1310 clocks to P^T, 820 to dS^T of 2770): 128 x 4096 d 64 causal 1040 -> 1015 us, 64 x 2048 without a mask
+// 258 -> 246. Not below 49 columns (128 x 1024 d 40 103 -> 104); with 65 to 80, where dQ would fit as well, the one buffer of dO and the
+// shared memory hold it (132 -> 141).
 constexpr int SP_THREADS = (NCW + 8) * 32;
 constexpr int W_DRAIN0 = NCW + 4;
 
-template <int HD>
+template <int HD, bool BESIDE>
 struct SpCfg {
     static constexpr int NSUB = HD / 64;
     static constexpr int SUB_BYTES = 128 * 128;
@@ -814,14 +823,15 @@ struct SpCfg {
     static constexpr int OFF_ROWVEC = OFF_BAR + 192;
     static constexpr int USED_BYTES = OFF_ROWVEC + 2048;
     static constexpr int SMEM_BYTES = HD == 128 ? 232448 : USED_BYTES + 1024;
-    static constexpr int T_S = 0, T_DP = 128, T_ACC0 = 256, T_ACC1 = 256 + HD;
+    static constexpr int T_S = 0, T_DP = 128, T_ACC0 = 256, T_ACC1 = 256 + HD, T_DQ = BESIDE ? 256 + 2 * HD : T_DP;
+    static_assert(T_DQ + HD <= 512, "tensor memory");
     static constexpr int B_RES = 0, B_FULLA = 1, B_EMPTYA = B_FULLA + NA, B_FULLB = B_EMPTYA + NA,
                          B_EMPTYB = B_FULLB + NB,
                          B_S = B_EMPTYB + NB,   // S^T of the current tile is in tensor memory
                          B_DP = B_S + 1,        // dP^T is in tensor memory
                          B_P = B_DP + 1,        // P^T written (one arrival per compute warp)
                          B_DS = B_P + 1,        // dS^T written to shared memory (one arrival per compute warp)
-                         B_DSFREE = B_DS + 1,   // dQ(i) and dK(i) have read dS^T(i)
+                         B_DSFREE = B_DS + 1,   // the products that read dS^T(i) from shared memory are done
                          B_DQ = B_DSFREE + 1,   // dQ(i) is in tensor memory
                          B_DQFREE = B_DQ + 1,   // the drain warps have copied dQ(i) out (4 arrivals)
                          B_ACC = B_DQFREE + 1, NUM_BARS = B_ACC + 1;
@@ -857,7 +867,7 @@ __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wa
 __device__ long long g_bwd_trace[64 * 32];
 #define TR(slot, it)                                                                          \
     do {                                                                                      \
-        if (blockIdx.x == gridDim.x / 2 && (it) < 64) g_bwd_trace[(it) * 32 + (slot)] = clock64(); \
+        if (blockIdx.x == gridDim.x / 2 && (unsigned)(it) < 64u) g_bwd_trace[(it) * 32 + (slot)] = clock64(); \
     } while (0)
 #else
 #define TR(slot, it) \
@@ -869,13 +879,13 @@ __device__ long long g_bwd_trace[64 * 32];
 // 16 columns that hold anything, dQ, dK and dV are that many columns wide, and only the 32-column chunks of
 // dQ that hold one of the d columns are added into the accumulator. At d = 80 that is 396 KB of shared-memory
 // traffic per tile pair instead of 512 KB; forward and backward of 36 units x 777 x 1301 at d = 80 went 105.6 -> 100.5 us.
-template <int HD, bool PART>
+template <int HD, bool PART, bool BESIDE>
 __global__ void __launch_bounds__(SP_THREADS, 1)
     sm100_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                            const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
                            const SpParams p)
 {
-    using C = SpCfg<HD>;
+    using C = SpCfg<HD, BESIDE>;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t *smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -916,7 +926,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
         mbar_init(BAR(C::B_DSFREE), 1);
         mbar_init(BAR(C::B_DQ), 1);
         mbar_init(BAR(C::B_DQFREE), 4);
-        mbar_init(BAR(C::B_ACC), 2);
+        mbar_init(BAR(C::B_ACC), 3);  // one commit from each issuing warp
         fence_mbar_init();
     }
     if (warp == W_ALLOC) {
@@ -937,10 +947,13 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
     pdl_launch_dependents();  // the dQ finish kernel may be placed on SMs as they fall idle; it waits for this grid's end
     if (warp >= W_DRAIN0) {
         // -------------------------------------------------------------------- drain dQ(i)
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");  // holds half a row (64 columns) of dQ(i) at a time
+        if constexpr (HD == 64)  // a row of dQ(i) is held in registers
+            asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
+        else
+            asm volatile("setmaxnreg.inc.sync.aligned.u32 152;");
         pdl_wait();  // the accumulator is cleared by the delta launch before this one
         const int w = warp - W_DRAIN0;  // == warp % 4: the tensor-memory lane quarter this warp may read
-        const uint32_t t_dq = tmem + ((uint32_t)(w * 32) << 16) + C::T_DP;
+        const uint32_t t_dq = tmem + ((uint32_t)(w * 32) << 16) + C::T_DQ;
         uint8_t *stage = smem_gen + C::OFF_STAGE + w * C::STAGE_WARP_BYTES;
         const uint32_t stage_u32 = smem_base + C::OFF_STAGE + w * C::STAGE_WARP_BYTES;
         bool ok = true;
@@ -951,21 +964,17 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
             tc_fence_after();
             if (w == 0 && lane == 0) TR(16, i);
             float *gdst = p.dq_acc + ((((size_t)bh * nqt + (i_begin + i)) * 4 + w) * chunks) * 1024;
-            // The row leaves tensor memory in two halves of 64 columns (the registers of these warps are
-            // what the compute warps do not get); dP^T(i+1) may overwrite it once the second half is read.
+            // The whole row leaves tensor memory at once: with 64 columns at a time its second half waited for the first one's way through
+            // the staging buffers, 1090 clocks at 128 columns while dK(i) reads its operands, and dP^T(i+1) with it (now 200).
+            uint32_t u[HD / 32][32];
 #pragma unroll
-            for (int hf = 0; hf < HD / 64; hf++) {
-                uint32_t u[2][32];
-                tmem_ld_32x32b_x32(t_dq + hf * 64, u[0]);
-                tmem_ld_32x32b_x32(t_dq + hf * 64 + 32, u[1]);
-                tmem_wait_ld();
-                if (hf == HD / 64 - 1) {
-                    warp_arrive(BAR(C::B_DQFREE), lane);
-                    if (w == 0 && lane == 0) TR(17, i);
-                }
+            for (int c = 0; c < HD / 32; c++) tmem_ld_32x32b_x32(t_dq + c * 32, u[c]);
+            tmem_wait_ld();
+            warp_arrive(BAR(C::B_DQFREE), lane);
+            if (w == 0 && lane == 0) TR(17, i);
+            {
 #pragma unroll
-                for (int c2 = 0; c2 < 2; c2++) {
-                    const int c = hf * 2 + c2;
+                for (int c = 0; c < HD / 32; c++) {
                     if (PART && c >= chunks) break;
                     // the bulk operation that read this buffer two chunks ago must be done with it
                     if (lane == 0) bulk_wait_read_1();
@@ -974,7 +983,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
 #pragma unroll
                     for (int cg = 0; cg < 8; cg++)
                         *reinterpret_cast<uint4 *>(buf + (cg * 32 + lane) * 16) =
-                            make_uint4(u[c2][4 * cg], u[c2][4 * cg + 1], u[c2][4 * cg + 2], u[c2][4 * cg + 3]);
+                            make_uint4(u[c][4 * cg], u[c][4 * cg + 1], u[c][4 * cg + 2], u[c][4 * cg + 3]);
                     fence_proxy_async();
                     __syncwarp();
                     if (lane == 0) {
@@ -1013,7 +1022,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
                 issued_b = i + 1;
             }
             drain_copies<C>(bar0, issued_a, issued_b);
-        } else if (warp == W_MMA_A || warp == W_MMA_B) {  // all 32 lanes, converged; one elected lane issues
+        } else if (warp == W_MMA_A || warp == W_MMA_B || warp == W_ALLOC) {  // all 32 lanes, converged; one elected lane issues
             // ---------------------------------------------------------------- MMA issue
             constexpr uint32_t IDESC_SS = idesc_bf16_f32(128, 128, 0, 0);
             const int ksteps = PART ? (p.d + 15) / 16 : HD / 16;
@@ -1063,9 +1072,9 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
                 }
                 tc_commit_elect(BAR(C::B_ACC));
             } else {
-                // gradient chain: dP^T(0); then per tile dQ(i), dK(i) (both read dS^T from shared memory)
-                // and dP^T(i+1), which overwrites dQ(i) and therefore waits for the drain warps
                 auto issue_dpt = [&](int i) {  // dP^T = V dO^T
+                    ok = ok && mbar_wait(BAR(C::B_FULLB + i % C::NB), (i / C::NB) & 1, abort_flag, p.status, WB_FULL);
+                    tc_fence_after();
                     const uint32_t do_lo = desc_lo(do_addr(i), 16);
 #pragma unroll
                     for (int sub = 0; sub < C::NSUB; sub++)
@@ -1073,36 +1082,52 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
                             mma_chain4_ss<2, 4, 6, 2, 4, 6>(tmem + C::T_DP, v_lo + sub * SUB16, do_lo + sub * SUB16, IDESC_SS, elected, sub > 0, PART ? ksteps - sub * 4 : 4);
                     tc_commit_elect(BAR(C::B_DP));
                     tc_commit_elect(BAR(C::B_EMPTYB + i % C::NB));  // this chain's only read of dO(i)
+                    if (lane == 0) TR(15, i - 1);
                 };
                 const uint32_t ds_lo = desc_lo(dsa, 16), dsmn_lo = desc_lo(dsa, C::SUB_BYTES);
                 const uint32_t kmn_lo = desc_lo(ka, C::SUB_BYTES);
-                ok = ok && mbar_wait(BAR(C::B_FULLB + 0), 0, abort_flag, p.status, WB_FULL);
-                tc_fence_after();
-                issue_dpt(0);
-                for (int i = 0; i < n && ok; i++) {
+                auto issue_dq = [&]() {  // dQ(i) = dS K: 16 keys per step
+#pragma unroll
+                    for (int half = 0; half < 2; half++)
+                        mma_chain4_ss<128, 256, 384, 128, 256, 384>(tmem + C::T_DQ, dsmn_lo + half * 512, kmn_lo + half * 512, IDESC_DQ, elected, half > 0);
+                    tc_commit_elect(BAR(C::B_DQ));
+                };
+                auto issue_dk = [&](int i) {  // dK += dS^T Q: 16 queries per step
                     const uint32_t qmn_lo = desc_lo(q_addr(i), C::SUB_BYTES);
-                    ok = ok && mbar_wait(BAR(C::B_FULLA + i % C::NA), (i / C::NA) & 1, abort_flag, p.status, WB_FULL);
-                    ok = ok && mbar_wait(BAR(C::B_DS), i & 1, abort_flag, p.status, WB_DS);
-                    tc_fence_after();
-                    if (lane == 0) TR(12, i);
 #pragma unroll
-                    for (int half = 0; half < 2; half++)  // dQ(i) = dS K: 16 keys per step
-                        mma_chain4_ss<128, 256, 384, 128, 256, 384>(tmem + C::T_DP, dsmn_lo + half * 512, kmn_lo + half * 512, IDESC_DQ, elected, half > 0);
-                    tc_commit_elect(BAR(C::B_DQ));  // the drain warps copy dQ(i) out while dK(i) is multiplied
-#pragma unroll
-                    for (int half = 0; half < 2; half++)  // dK += dS^T Q: 16 queries per step
-                        mma_chain4_ss<2, 4, 6, 128, 256, 384>(tmem + C::T_ACC1, ds_lo + half * SUB16, qmn_lo + half * 512, IDESC_TS, elected, i > 0 || half > 0);
-                    tc_commit_elect(BAR(C::B_DSFREE));
-                    tc_commit_elect(BAR(C::B_EMPTYA + i % C::NA));  // this chain's last read of Q(i)
-                    if (lane == 0) TR(13, i);
-                    if (i + 1 < n) {
+                    for (int half = 0; half < 2; half++) {
+                        if constexpr (BESIDE)
+                            mma_chain4_ts<8, 16, 24, 128, 256, 384>(tmem + C::T_ACC1, tmem + C::T_DP + half * 64, qmn_lo + half * 512, IDESC_TS, elected, i > 0 || half > 0);
+                        else
+                            mma_chain4_ss<2, 4, 6, 128, 256, 384>(tmem + C::T_ACC1, ds_lo + half * SUB16, qmn_lo + half * 512, IDESC_TS, elected, i > 0 || half > 0);
+                    }
+                };
+                // Both warps follow dS^T. BESIDE: the first one issues dK(i), then dP^T(i+1) over what dK(i) has read (ordered by issue), the
+                // other one dQ(i) once the drain warps have copied dQ(i-1) out. Otherwise the first one issues dQ(i) and dK(i), the other
+                // one dP^T(i+1) once the drain warps have copied dQ(i) out of its columns.
+                const bool first = warp == W_MMA_B;
+                if (BESIDE == first) issue_dpt(0);
+                for (int i = 0; i < n && ok; i++) {
+                    if (BESIDE || first) {
+                        ok = ok && mbar_wait(BAR(C::B_DS), i & 1, abort_flag, p.status, WB_DS);
+                        if (BESIDE && !first && i > 0) ok = ok && mbar_wait(BAR(C::B_DQFREE), (i - 1) & 1, abort_flag, p.status, WB_ACC);
+                        tc_fence_after();
+                        if (lane == 0) TR(12, i);
+                        if (BESIDE != first) {
+                            issue_dq();
+                            if (BESIDE) tc_commit_elect(BAR(C::B_DSFREE));
+                        }
+                        if (first) {
+                            issue_dk(i);
+                            if (!BESIDE) tc_commit_elect(BAR(C::B_DSFREE));
+                            if (BESIDE && i + 1 < n) issue_dpt(i + 1);
+                            tc_commit_elect(BAR(C::B_EMPTYA + i % C::NA));  // this chain's last read of Q(i)
+                            if (lane == 0) TR(13, i);
+                        }
+                    } else if (i + 1 < n) {
                         ok = ok && mbar_wait(BAR(C::B_DQFREE), i & 1, abort_flag, p.status, WB_ACC);
                         if (lane == 0) TR(14, i);
-                        ok = ok && mbar_wait(BAR(C::B_FULLB + (i + 1) % C::NB), ((i + 1) / C::NB) & 1, abort_flag,
-                                             p.status, WB_FULL);
-                        tc_fence_after();
                         issue_dpt(i + 1);
-                        if (lane == 0) TR(15, i);
                     }
                 }
                 tc_commit_elect(BAR(C::B_ACC));
@@ -1110,7 +1135,10 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
         }
     } else {
         // -------------------------------------------------------------------- compute
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 192;");  // 8 x 32 x 192 + 4 x 32 x 40 + 4 x 32 x 88 == 65536
+        if constexpr (HD == 64)
+            asm volatile("setmaxnreg.inc.sync.aligned.u32 192;");  // 8 x 32 x 192 + 4 x 32 x 40 + 4 x 32 x 88 == 512 x 128 at launch
+        else
+            asm volatile("setmaxnreg.inc.sync.aligned.u32 160;");  // 8 x 32 x 160 + 4 x 32 x 40 + 4 x 32 x 152
         const int h = warp / 4;                // which 64-column half of the 128 score columns (queries)
         const int r = threadIdx.x % 128;       // TMEM lane == key row inside the tile
         const int key = k0 + r;
@@ -1186,6 +1214,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
 #pragma unroll
             for (int half = 0; half < 2; half++) {
                 float dp[32];
+                uint32_t dsp[16];
                 tmem_ld_cols<32>(t_dp + h * 64 + half * 32, dp);
 #pragma unroll
                 for (int q4 = 0; q4 < 4; q4++) {  // 8 queries = one 16-byte chunk
@@ -1198,11 +1227,15 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
                         float d0, d1;
                         unpack2(ds2, d0, d1);
                         w4[x] = pack_bf16(d0, d1);
+                        if constexpr (BESIDE) dsp[q4 * 4 + x] = w4[x];
                     }
                     const int chunk = half * 4 + q4;
                     *reinterpret_cast<uint4 *>(ds_row + ((chunk ^ (r & 7)) << 4)) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
                 }
+                // BESIDE: the A operand of dK, over the first half of this thread's own dP^T columns, which it has read
+                if constexpr (BESIDE) tmem_st_32x32b_x16(t_dp + h * 64 + half * 16, dsp);
             }
+            if constexpr (BESIDE) tmem_wait_st();
             fence_proxy_async();  // the MMAs read dS^T through the async proxy
             warp_arrive(BAR(C::B_DS), lane);
             if (threadIdx.x == 0) TR(4, i);
@@ -1359,10 +1392,10 @@ int launch_delta_bf16(const AttnArgs &a, float *delta, cudaStream_t s, void *zer
     return EMBER_OK;
 }
 
-template <int HD, bool PART>
+template <int HD, bool PART, bool BESIDE>
 int launch_fused_form(const AttnArgs &a, float *delta, float *dq_acc, DeviceState *st, cudaStream_t s)
 {
-    using C = SpCfg<HD>;
+    using C = SpCfg<HD, BESIDE>;
     static_assert(NCW == 8, "the single-pass kernel is written for eight compute warps");
     const int nqt = (a.lq + 127) / 128;
     // delta, and the accumulator cleared by the same launch
@@ -1388,7 +1421,7 @@ int launch_fused_form(const AttnArgs &a, float *delta, float *dq_acc, DeviceStat
     p.scale = a.scale;
     p.scale_log2 = a.scale * LOG2E_B;
     p.status = st->status;
-    auto k1 = sm100_bwd_fused_kernel<HD, PART>;
+    auto k1 = sm100_bwd_fused_kernel<HD, PART, BESIDE>;
     static SmemOptIn opt_in1;
     EMBER_CUDA_TRY(opt_in1(k1, C::SMEM_BYTES));
     const size_t touched = ((size_t)a.lq + a.lk) * HD * 2 * 4 + (size_t)a.lq * HD * 4;  // + the float32 dQ accumulator
@@ -1414,7 +1447,9 @@ int launch_fused_form(const AttnArgs &a, float *delta, float *dq_acc, DeviceStat
 template <int HD>
 int launch_fused(const AttnArgs &a, float *delta, float *dq_acc, DeviceState *st, cudaStream_t s)
 {
-    return a.d <= HD - 16 ? launch_fused_form<HD, true>(a, delta, dq_acc, st, s) : launch_fused_form<HD, false>(a, delta, dq_acc, st, s);
+    if constexpr (HD == 64)
+        return a.d <= 48 ? launch_fused_form<64, true, false>(a, delta, dq_acc, st, s) : launch_fused_form<64, false, true>(a, delta, dq_acc, st, s);
+    return a.d <= 112 ? launch_fused_form<128, true, false>(a, delta, dq_acc, st, s) : launch_fused_form<128, false, false>(a, delta, dq_acc, st, s);
 }
 
 template <int HD>
