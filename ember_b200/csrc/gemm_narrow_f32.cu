@@ -99,7 +99,228 @@ int launch(const GemmArgs &g, cudaStream_t s)
     }
 }
 
+// The backward of such a layer in one launch: grad_w = x^T grad_y and, with it, grad_b in the first `sum_blocks` blocks, grad_x = grad_y w^T in the others.
+//
+// Bound: latency again at a few hundred rows (three launches, of which the weight gradient's contraction over the rows was a chain of tiles on
+// 25 blocks: 13 us for 784 x 256 x 10), the bytes of x and grad_x at thousands. A lane has four columns of x or grad_x, a warp 128 of them, so
+// that every access of a row is 512 bytes in one piece; the N values of grad_y that go with a row are the same for the whole warp. The rows
+// of a weight gradient are shared by a cluster of up to eight blocks of eight warps, whose sums are added in a fixed order: no atomics.
+template <int N>
+__device__ __forceinline__ void load_row(const float *p, float (&v)[N])
+{
+    if constexpr (N % 4 == 0) {
+#pragma unroll
+        for (int i = 0; i < N / 4; i++) {
+            const float4 f = reinterpret_cast<const float4 *>(p)[i];
+            v[4 * i] = f.x; v[4 * i + 1] = f.y; v[4 * i + 2] = f.z; v[4 * i + 3] = f.w;
+        }
+    } else if constexpr (N % 2 == 0) {
+#pragma unroll
+        for (int i = 0; i < N / 2; i++) {
+            const float2 f = reinterpret_cast<const float2 *>(p)[i];
+            v[2 * i] = f.x; v[2 * i + 1] = f.y;
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < N; i++) v[i] = p[i];
+    }
+}
+
+struct NarrowBwd {
+    const float *x, *w, *dy;
+    float *dx, *dw, *db;  // dx, db: may be NULL
+    int m, k, tiles;      // tiles of 128 columns
+    int cluster;          // blocks that share the rows of a tile
+    int sum_blocks, chunk_rows;
+};
+
+// what lies at `mine` in the shared memory of another block of the cluster
+__device__ __forceinline__ float ld_cluster(const float *mine, int rank)
+{
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(map_to_cta(smem_u32(mine), rank)) : "memory");
+    return v;
+}
+__device__ __forceinline__ double ld_cluster(const double *mine, int rank)
+{
+    double v;
+    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(map_to_cta(smem_u32(mine), rank)) : "memory");
+    return v;
+}
+
+template <int N>
+__global__ void __launch_bounds__(256) narrow_f32_bwd_kernel(const NarrowBwd p)
+{
+    extern __shared__ float red[];     // [8][N][128]: the warps' sums
+    __shared__ float total[N * 128];   // the block's: [N][128]
+    __shared__ double total_b[N], red_b[8][N];  // grad_b: a few sums of m values, in 64 bits for what that costs
+    constexpr int U = 4;               // rows of a warp in flight
+    pdl_launch_dependents();
+    pdl_wait();
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    if ((int)blockIdx.x >= p.sum_blocks) {
+        // ---------------------------------------------------------------- grad_x
+        const int b = blockIdx.x - p.sum_blocks, tile = b % p.tiles, col = tile * 128 + lane * 4;
+        const int r0 = b / p.tiles * p.chunk_rows, r1 = min(p.m, r0 + p.chunk_rows);
+        if (r0 < p.m && col < p.k) {
+            float wv[4 * N];
+#pragma unroll
+            for (int i = 0; i < N; i++) {
+                const float4 f = reinterpret_cast<const float4 *>(p.w + (size_t)col * N)[i];
+                wv[4 * i] = f.x; wv[4 * i + 1] = f.y; wv[4 * i + 2] = f.z; wv[4 * i + 3] = f.w;
+            }
+            for (int r = r0 + warp * U; r < r1; r += 8 * U) {
+                float g[U][N];
+#pragma unroll
+                for (int u = 0; u < U; u++) load_row<N>(p.dy + (size_t)min(r + u, p.m - 1) * N, g[u]);
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    float o[4];
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {
+                        o[j] = g[u][0] * wv[j * N];
+#pragma unroll
+                        for (int c = 1; c < N; c++) o[j] = fmaf(g[u][c], wv[j * N + c], o[j]);
+                    }
+                    if (r + u < r1) *reinterpret_cast<float4 *>(p.dx + (size_t)(r + u) * p.k + col) = make_float4(o[0], o[1], o[2], o[3]);
+                }
+            }
+        }
+        return;  // (its cluster, if any, is of such blocks alone)
+    }
+    // -------------------------------------------------------------------- grad_w, grad_b
+    const int rank = p.cluster > 1 ? (int)cluster_ctarank() : 0, tile = blockIdx.x / p.cluster, col = tile * 128 + lane * 4;
+    const int r0 = (int)((long long)p.m * rank / p.cluster), r1 = (int)((long long)p.m * (rank + 1) / p.cluster);
+    const bool sum_b = p.db && tile == 0;
+    float acc[N][4] = {};
+    double acc_b = 0.;
+    for (int r = r0 + warp * U; r < r1; r += 8 * U) {
+        float4 xv[U];
+        float g[U][N];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            xv[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (r + u < r1 && col < p.k) xv[u] = *reinterpret_cast<const float4 *>(p.x + (size_t)(r + u) * p.k + col);
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) load_row<N>(p.dy + (size_t)min(r + u, r1 - 1) * N, g[u]);
+        float gb[U] = {};
+        if (sum_b && lane < N) {
+#pragma unroll
+            for (int u = 0; u < U; u++)
+                if (r + u < r1) gb[u] = p.dy[(size_t)(r + u) * N + lane];
+        }
+        if (sum_b) acc_b += ((double)gb[0] + gb[1]) + ((double)gb[2] + gb[3]);
+#pragma unroll
+        for (int u = 1; u < U; u++)
+            if (r + u >= r1) {  // another row's values, which could be infinite
+#pragma unroll
+                for (int c = 0; c < N; c++) g[u][c] = 0.f;
+            }
+        // four products are added up before they meet the sums: a chain of m / 256 additions instead of m / 64
+        // (8192 x 784 x 10: grad_w 1.3e-7 of its norm off; row by row 2.2e-7, gemm_simt.cu 1.7e-7)
+#pragma unroll
+        for (int c = 0; c < N; c++) {
+            acc[c][0] += fmaf(xv[3].x, g[3][c], fmaf(xv[2].x, g[2][c], fmaf(xv[1].x, g[1][c], xv[0].x * g[0][c])));
+            acc[c][1] += fmaf(xv[3].y, g[3][c], fmaf(xv[2].y, g[2][c], fmaf(xv[1].y, g[1][c], xv[0].y * g[0][c])));
+            acc[c][2] += fmaf(xv[3].z, g[3][c], fmaf(xv[2].z, g[2][c], fmaf(xv[1].z, g[1][c], xv[0].z * g[0][c])));
+            acc[c][3] += fmaf(xv[3].w, g[3][c], fmaf(xv[2].w, g[2][c], fmaf(xv[1].w, g[1][c], xv[0].w * g[0][c])));
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < N; c++) *reinterpret_cast<float4 *>(red + (warp * N + c) * 128 + lane * 4) = make_float4(acc[c][0], acc[c][1], acc[c][2], acc[c][3]);
+    if (sum_b && lane < N) red_b[warp][lane] = acc_b;
+    __syncthreads();
+    for (int e = threadIdx.x; e < N * 128; e += 256) {
+        const float *a = red + e;
+        constexpr int W = N * 128;
+        total[e] = ((a[0] + a[W]) + (a[2 * W] + a[3 * W])) + ((a[4 * W] + a[5 * W]) + (a[6 * W] + a[7 * W]));
+    }
+    if (sum_b && threadIdx.x < N) {
+        const int e = threadIdx.x;
+        total_b[e] = ((red_b[0][e] + red_b[1][e]) + (red_b[2][e] + red_b[3][e])) + ((red_b[4][e] + red_b[5][e]) + (red_b[6][e] + red_b[7][e]));
+    }
+    if (p.cluster > 1) cluster_sync_all(); else __syncthreads();
+    // element e of the tile's 128 x N results, as they lie in memory; a block of the cluster has every cluster-th run of 256
+    for (int e = rank * 256 + threadIdx.x; e < 128 * N; e += p.cluster * 256) {
+        const int j = e / N, c = e - j * N;
+        if (tile * 128 + j >= p.k) break;
+        float v = 0.f;
+        for (int q = 0; q < p.cluster; q++) v += p.cluster > 1 ? ld_cluster(total + c * 128 + j, q) : total[c * 128 + j];
+        p.dw[(size_t)tile * 128 * N + e] = v;
+    }
+    if (sum_b && rank == 0 && threadIdx.x < N) {
+        double v = 0.;
+        for (int q = 0; q < p.cluster; q++) v += p.cluster > 1 ? ld_cluster(total_b + threadIdx.x, q) : total_b[threadIdx.x];
+        p.db[threadIdx.x] = (float)v;
+    }
+    if (p.cluster > 1) cluster_sync_all();  // no block leaves while another may read its sums
+}
+
+template <int N>
+int launch_bwd(NarrowBwd p, int n, DeviceState *st, cudaStream_t s)
+{
+    if constexpr (N > 12) {
+        return EMBER_ERR_UNSUPPORTED;
+    } else {
+        if (n != N) return launch_bwd<N + 1>(p, n, st, s);
+        p.tiles = (p.k + 127) / 128;
+        p.cluster = 1;
+        while (p.cluster < 8 && p.m >= p.cluster * 64) p.cluster *= 2;  // at least 32 rows each, four for a warp
+        p.sum_blocks = p.tiles * p.cluster;
+        long long blocks = p.sum_blocks;
+        if (p.dx) {
+            const int chunks = max(1, min((p.m + 31) / 32, 4 * st->sm_count / p.tiles));
+            p.chunk_rows = ((p.m + chunks - 1) / chunks + 31) / 32 * 32;
+            blocks += (long long)p.tiles * ((p.m + p.chunk_rows - 1) / p.chunk_rows);
+        }
+        blocks = (blocks + p.cluster - 1) / p.cluster * p.cluster;
+        const int smem = 8 * N * 128 * (int)sizeof(float);
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)blocks);
+        cfg.blockDim = dim3(256);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = s;
+        auto kern = narrow_f32_bwd_kernel<N>;
+        static SmemOptIn opt_in;
+        EMBER_CUDA_TRY(opt_in(kern, smem));
+        LaunchAttrs attrs;
+        attrs.cluster(p.cluster);
+        if (cfg.gridDim.x <= (unsigned)kPdlMaxGrid) attrs.pdl();
+        attrs.set(cfg);
+        EMBER_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, p));
+        return EMBER_OK;
+    }
+}
+
 }  // namespace
+
+bool narrow_f32_bwd_supported(const void *x, const void *w, const void *dy, const void *dx, const void *db, long long m, int n, int k)
+{
+    if (n > 12 || k % 4 != 0 || k > 0x7fffffff - 1024 || (((uintptr_t)x | (uintptr_t)w | (uintptr_t)dy | (uintptr_t)dx) & 15) != 0) return false;
+    // us, the kernels that took these calls before (gemm_simt.cu, from some sizes on gemm_f32_sm100.cu, column_sums.cu) / here, calls back to back in
+    // a graph, grad_x, grad_w and grad_b: 256 x 784 x 10 14.8 / 5.7, 32 x 64 x 10 8.3 / 3.7, 1000 x 512 x 12 15.4 / 10, 8192 x 784 x 10 68 / 32,
+    // 8192 x 2048 x 10 138 / 45; over 500 sizes (1 to 16384 rows, contractions of 4 to 2048) 0.44 of the time.
+    // At most eight blocks share the rows of 128 columns, which is too few for tall matrices: 32768 x 784 x 10 231 / 213, 68047 x 536 x 11 420 / 444,
+    // 122465 x 308 x 8 395 / 949; with 8 and 12 columns, which tiles move in pieces of 16 bytes, from 4097 rows on if they are also narrow (9277 x 8 x 12
+    // 28 / 34, 14721 x 200 x 8 36 / 37.5). A weight gradient of 12 columns alone is quicker as tiles (95 x 220 4.1 / 5.2, 1576 x 156 7.7 / 9.3).
+    if (m > 16384 || ((n == 8 || n == 12) && m > 4096 && k < 512)) return false;
+    return n != 12 || dx || db;
+}
+
+int narrow_f32_backward(const void *x, const void *w, const void *dy, void *dx, void *dw, void *db, long long m, int n, int k, DeviceState *st, cudaStream_t s)
+{
+    NarrowBwd p = {};
+    p.x = (const float *)x;
+    p.w = (const float *)w;
+    p.dy = (const float *)dy;
+    p.dx = (float *)dx;
+    p.dw = (float *)dw;
+    p.db = (float *)db;
+    p.m = (int)m;
+    p.k = k;
+    return launch_bwd<1>(p, n, st, s);
+}
 
 bool narrow_f32_supported(const GemmArgs &g)
 {

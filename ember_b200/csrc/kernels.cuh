@@ -211,6 +211,9 @@ int skinny_f32_gemm(const GemmArgs &g, DeviceState *st, cudaStream_t s);
 // Float32, at most 12 columns, y = x w + b (gemm_narrow_f32.cu): a small classifier's logits on the CUDA cores.
 bool narrow_f32_supported(const GemmArgs &g);
 int narrow_f32_gemm(const GemmArgs &g, cudaStream_t s);
+// All gradients of such a layer (dx, db may be NULL) in one launch, where they lie apart from the operands and from one another.
+bool narrow_f32_bwd_supported(const void *x, const void *w, const void *dy, const void *dx, const void *db, long long m, int n, int k);
+int narrow_f32_backward(const void *x, const void *w, const void *dy, void *dx, void *dw, void *db, long long m, int n, int k, DeviceState *st, cudaStream_t s);
 // Float32 storage on the tensor cores, operands as three bf16 planes each (gemm_f32_sm100.cu, split_f32.cuh): a row-major view's rows
 // padded to 8 columns. _us: an estimate of the time, without the splitting.
 struct SplitGuard;

@@ -311,6 +311,13 @@ int ember_linear_bwd(const void *x, const void *w, const void *dy, void *dx, voi
     DeviceState *st = device_state();
     if (!st) return EMBER_ERR_CUDA;
     cudaStream_t s = pick_stream(stream, st);
+    if (dtype == EMBER_F32 && dw && !x_heads && !y_heads && narrow_f32_bwd_supported(x, w, dy, dx, db, m, n, k)) {
+        const size_t xs = (size_t)m * k * 4, ws = (size_t)k * n * 4, ys = (size_t)m * n * 4, bs = (size_t)n * 4;
+        if (apart(dw, ws, x, xs) && apart(dw, ws, w, ws) && apart(dw, ws, dy, ys) &&
+            (!dx || (apart(dx, xs, x, xs) && apart(dx, xs, w, ws) && apart(dx, xs, dy, ys) && apart(dx, xs, dw, ws))) &&
+            (!db || (apart(db, bs, x, xs) && apart(db, bs, w, ws) && apart(db, bs, dy, ys) && apart(db, bs, dw, ws) && (!dx || apart(db, bs, dx, xs)))))
+            return narrow_f32_backward(x, w, dy, dx, dw, db, m, n, k, st, s);
+    }
     PackedOperands packed(s);
     GemmArgs gw = product_of(GRAD_W, sh, x, w, dy, dw), gx = product_of(GRAD_X, sh, x, w, dy, dx);
     F32Products f32;
