@@ -694,6 +694,10 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
     if (!leave) pdl_launch_dependents();  // as in the forward
 
     const uint32_t t_s = tmem + C::T_S, t_p = tmem + C::T_P, t_d = tmem + C::T_D, t_r = tmem + C::T_R;
+    // At 64 columns the queries' role, which multiplies no P, has dP in P's columns: the next tile's may be formed as soon as this one's has been read
+    // (B_DS), and not only when the product with the dS that would lie over it is done.
+    const bool dp_apart = HD == 64 && is_q;
+    const uint32_t t_dp = dp_apart ? t_p : t_d + C::R::SCORES;
     if (leave) {
         // the kernel behind this one does the work
     } else if (warp >= 8) {
@@ -763,9 +767,9 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
                     continue;
                 }
                 wait(C::B_FULL1 + s, j / stages, WB_B1);
-                if (j > 0) wait(role == R_DKDV ? C::B_R1 : C::B_R0, j - 1, WB_ACC);  // over dS
+                if (j > 0) wait(dp_apart ? C::B_DS : role == R_DKDV ? C::B_R1 : C::B_R0, j - 1, WB_ACC);  // over dS, or over the last dP
                 tc_fence_after();
-                mma_scores<HD, A_SMEM>(t_d + C::R::SCORES, smem_base + C::OFF_A1, 0, b0 + C::TILE, 0, HD / 64, ksteps, elected, false);
+                mma_scores<HD, A_SMEM>(t_dp, smem_base + C::OFF_A1, 0, b0 + C::TILE, 0, HD / 64, ksteps, elected, false);
                 tc_commit_elect(BAR(C::B_DP));
                 tc_commit_elect(BAR(C::B_EMPTY1 + s));
             }
@@ -905,7 +909,7 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
                 ok = ok && mbar_wait(BAR(C::B_DP), j & 1, abort_flag, p.status, WB_DP);
                 tc_fence_after();
                 f32x2 dp[16];
-                load_scores<false>(t_d + lane_sel + C::R::SCORES + w * 32, dp);
+                load_scores<false>(t_dp + lane_sel + w * 32, dp);
                 if (HD == 128) load_scores<true>(t_d + lane_sel + 64 + w * 32, dp);
 #pragma unroll
                 for (int i = 0; i < 16; i += 2) {
