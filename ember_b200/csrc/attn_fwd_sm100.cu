@@ -855,6 +855,8 @@ static int fwd_block_rows(const AttnArgs &a, DeviceState *st)
         double end = fmax(length(0), total / sms);
         end = fmax(end, (double)((ctas + sms - 1) / sms) * length(ctas - 1));
         if (ctas > sms) end = fmax(end, length(sms - 1) + length(sms));
+        // with three CTAs and more on an SM the last ones do not fill the SMs evenly (20 units x L2048 causal 32.5 with one tile, 30.5 with two; 12 x L4096 60.9 / 55.7)
+        if (ctas > 2 * sms) end = fmax(end, total / sms + 0.3 * total / ctas);
         return end;
     };
     return end_of(128, 1.0) < end_of(256, 1.55) ? 128 : 256;
