@@ -995,7 +995,7 @@ bool sm100_fwd_supported(const AttnArgs &a)
 }
 
 // EMBER_FWD_EMU=0..2 sets the share of polynomial exponentials (read once). Default at 128 columns 0:
-// the MUFU needs 2048 of a step's 2850 clocks and alone does not bound it; every exponential there measured 1.3 % faster at
+// the MUFU needs 2048 of a step's 2900 clocks and alone does not bound it (a quarter on the FMA pipe is level at full clock); every exponential there measured 1.3 % faster at
 // B4 H32 L4096 than a quarter of them on the FMA pipe (0.487 against 0.494 ms), and half of them 5 %
 // slower. Default at 64 columns 1: a key tile then needs half the tensor time for the same 16384
 // exponentials, the MUFU is the limit, and a quarter on the FMA pipe measured 2.7 % faster (0.421 against
