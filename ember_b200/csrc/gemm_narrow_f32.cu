@@ -148,8 +148,9 @@ __device__ __forceinline__ double ld_cluster(const double *mine, int rank)
     return v;
 }
 
+// Two blocks an SM: 12 columns would take 167 registers and leave one (8055 x 2056 x 12 82 -> 50 us, 200 x 116552 x 12 193 -> 123).
 template <int N>
-__global__ void __launch_bounds__(256) narrow_f32_bwd_kernel(const NarrowBwd p)
+__global__ void __launch_bounds__(256, 2) narrow_f32_bwd_kernel(const NarrowBwd p)
 {
     extern __shared__ float red[];     // [8][N][128]: the warps' sums
     __shared__ float total[N * 128];   // the block's: [N][128]
@@ -266,7 +267,9 @@ int launch_bwd(NarrowBwd p, int n, DeviceState *st, cudaStream_t s)
         if (n != N) return launch_bwd<N + 1>(p, n, st, s);
         p.tiles = (p.k + 127) / 128;
         p.cluster = 1;
-        while (p.cluster < 8 && p.m >= p.cluster * 64) p.cluster *= 2;  // at least 32 rows each, four for a warp
+        // At least 32 rows each, four for a warp, and only until there are two blocks an SM: with few rows a block's end (its warps' sums added up, two
+        // waits for the cluster) is most of its time (always up to eight / this: 362 x 12152 x 8 26.9 / 19.5 us, 282 x 29424 x 10 40.7 / 17.0, 800 x 149512 x 4 256 / 185).
+        while (p.cluster < 8 && p.m >= p.cluster * 64 && p.tiles * p.cluster < 2 * st->sm_count) p.cluster *= 2;
         p.sum_blocks = p.tiles * p.cluster;
         long long blocks = p.sum_blocks;
         if (p.dx) {
@@ -300,11 +303,14 @@ bool narrow_f32_bwd_supported(const void *x, const void *w, const void *dy, cons
     if (n > 12 || k % 4 != 0 || k > 0x7fffffff - 1024 || (((uintptr_t)x | (uintptr_t)w | (uintptr_t)dy | (uintptr_t)dx) & 15) != 0) return false;
     // us, the kernels that took these calls before (gemm_simt.cu, from some sizes on gemm_f32_sm100.cu, column_sums.cu) / here, calls back to back in
     // a graph, grad_x, grad_w and grad_b: 256 x 784 x 10 14.8 / 5.7, 32 x 64 x 10 8.3 / 3.7, 1000 x 512 x 12 15.4 / 10, 8192 x 784 x 10 68 / 32,
-    // 8192 x 2048 x 10 138 / 45; over 500 sizes (1 to 16384 rows, contractions of 4 to 2048) 0.44 of the time.
+    // 8192 x 2048 x 10 138 / 45; over 500 sizes (1 to 16384 rows, contractions of 4 to 2048) 0.44 of the time,
+    // over 200 with contractions to 262144 (up to 2^27 elements of x) 0.43.
     // At most eight blocks share the rows of 128 columns, which is too few for tall matrices: 32768 x 784 x 10 231 / 213, 68047 x 536 x 11 420 / 444,
     // 122465 x 308 x 8 395 / 949; with 8 and 12 columns, which tiles move in pieces of 16 bytes, from 4097 rows on if they are also narrow (9277 x 8 x 12
     // 28 / 34, 14721 x 200 x 8 36 / 37.5). A weight gradient of 12 columns alone is quicker as tiles (95 x 220 4.1 / 5.2, 1576 x 156 7.7 / 9.3).
-    if (m > 16384 || ((n == 8 || n == 12) && m > 4096 && k < 512)) return false;
+    // Few rows and a wide weight gradient without grad_x, with the same columns: a block then has little but its end to do (6 x 145280 x 8 8.2 / 10.1,
+    // 12 x 167224 x 12 14.3 / 15.8).
+    if (m > 16384 || ((n == 8 || n == 12) && (m > 4096 && k < 512 || m <= 16 && k > 32768 && !dx))) return false;
     return n != 12 || dx || db;
 }
 

@@ -371,7 +371,7 @@ const char *ember_linear_kernel_name(int product, long long m, int n, int k, int
         F32Products f32;
         if (product == FORWARD) {
             if (!skinny_f32_supported(g) && !narrow_f32_supported(g)) f32.add(g);
-        } else {
+        } else if (x_heads || y_heads || !narrow_f32_bwd_supported(at[0], at[1], at[2], at[3], nullptr, m, n, k)) {
             f32.add(product_of(GRAD_W, sh, at[0], at[1], at[2], at[3]));
             f32.add(product_of(GRAD_X, sh, at[0], at[1], at[2], at[3]));
         }
