@@ -227,8 +227,8 @@ __device__ __forceinline__ void flush(f32x2 (&acc)[N32 * 16], uint32_t taddr, in
     }
 }
 
-template <int N>
-__device__ __forceinline__ void store_cols(float *dst, const f32x2 (&v2)[N / 2], float down, float scale, int col0, int d, bool vec, const void *base, size_t bytes,
+template <int N, int M>
+__device__ __forceinline__ void store_cols(float *dst, const f32x2 (&v2)[M], float down, float scale, int col0, int d, bool vec, const void *base, size_t bytes,
                                            DeviceStatus *status)
 {
     (void)base; (void)bytes; (void)status;
@@ -286,9 +286,12 @@ struct F32FwdParams {
     SplitGuard guard;
     DeviceStatus *status;
     WorkOrder order;
+    int paired;  // items that two CTAs share
 };
 
-template <int HD>
+// PAIR: where query blocks would leave SMs without one, two CTAs share a block's keys and put their results together through one another's shared
+// memory (no memory of the call's, no second launch; about 1.7 us).
+template <int HD, bool PAIR>
 __global__ void __launch_bounds__(F32_THREADS, 1)
     sm100_f32_fwd_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v, const F32FwdParams p)
 {
@@ -303,9 +306,19 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
 
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     int unit, rank;
-    work_item(p.order, blockIdx.x, unit, rank);
+    // PAIR: the first p.paired items have a cluster each, whose two CTAs share the queries: the first takes the earlier half of their tiles, the
+    // second the rest (of one tile: none). Behind them a cluster holds two items that know nothing of each other.
+    const bool pair = PAIR && blockIdx.x < 2u * p.paired;
+    const unsigned item = !PAIR ? blockIdx.x : pair ? blockIdx.x / 2 : blockIdx.x - p.paired;
+    if (PAIR && item >= (unsigned)p.order.units * p.order.blocks) {  // there is an odd number of items
+        pdl_wait();
+        return;
+    }
+    work_item(p.order, (int)item, unit, rank);
     const int q0 = (p.order.blocks - 1 - rank) * 128, off = p.lk - p.lq;  // heaviest (latest) causal rows first
-    const int n = ((p.causal ? min(p.lk, q0 + 128 + off) : p.lk) + TN - 1) / TN;
+    const int tiles = ((p.causal ? min(p.lk, q0 + 128 + off) : p.lk) + TN - 1) / TN;
+    const int half = pair ? (int)cluster_ctarank() : 0, first = half * ((tiles + 1) / 2);
+    const int n = !pair ? tiles : half ? tiles - first : (tiles + 1) / 2;
 
     if (threadIdx.x == 0) {
         *abort_flag = 0;
@@ -349,10 +362,10 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
             for (int j = 0; j < n; j++) {
                 const int ks = j % C::KST, vs = j % C::VST;
                 if (!mbar_wait(BAR(C::B_KEMPTY + ks), ((j / C::KST) & 1) ^ 1, abort_flag, p.status, WF_KEMPTY)) break;
-                load_planes<HD>(smem_base + C::OFF_K + ks * C::TILE, &tm_k, BAR(C::B_KFULL + ks), j * TN, unit, p.order.units);
+                load_planes<HD>(smem_base + C::OFF_K + ks * C::TILE, &tm_k, BAR(C::B_KFULL + ks), (first + j) * TN, unit, p.order.units);
                 k_issued = j + 1;
                 if (!mbar_wait(BAR(C::B_VEMPTY + vs), ((j / C::VST) & 1) ^ 1, abort_flag, p.status, WF_VEMPTY)) break;
-                load_planes<HD>(smem_base + C::OFF_V + vs * C::TILE, &tm_v, BAR(C::B_VFULL + vs), j * TN, unit, p.order.units);
+                load_planes<HD>(smem_base + C::OFF_V + vs * C::TILE, &tm_v, BAR(C::B_VFULL + vs), (first + j) * TN, unit, p.order.units);
                 v_issued = j + 1;
             }
             // do not leave while a copy is still landing in shared memory
@@ -424,7 +437,7 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
         const f32x2 scale2 = pack2(p.scale * kSplitDown2, p.scale * kSplitDown2), l2e = pack2(LOG2E_T, LOG2E_T);
         bool ok = true;
         for (int j = w; j < n && ok; j += 2) {
-            const int k0 = j * TN;
+            const int k0 = (first + j) * TN;
             ok = ok && mbar_wait(BAR(C::B_S + w), C::HALVES ? 0 : (j >> 1) & 1, abort_flag, p.status, WF_S);
             tc_fence_after();
             f32x2 s[32];
@@ -526,10 +539,10 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
         }
         named_bar_sync(1, 256);
         const float2 other = state[(w ^ 1) * 128 + r];
-        const float mm = fmaxf(m, other.x);
-        const float a_own = exp_nat(m - mm), a_other = exp_nat(other.x - mm);
-        const float ll = w == 0 ? l * a_own + other.y * a_other : other.y * a_other + l * a_own;
-        const float inv = 1.f / ll;
+        float mm = fmaxf(m, other.x);
+        const float ref = pair && mm == -INFINITY ? 0.f : mm;  // the other CTA's keys may be the only ones that a row sees
+        const float a_own = exp_nat(m - ref), a_other = exp_nat(other.x - ref);
+        float ll = w == 0 ? l * a_own + other.y * a_other : other.y * a_other + l * a_own;
         f32x2 res[HALF / 2];
         {
             const uint8_t *from = xo + (w * 128 + r) * ROWB;
@@ -542,11 +555,50 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
                 res[i + 1] = fma2(w == 0 ? o[i + 1] : o[HALF / 2 + i + 1], own2, mul2(v.y, other2));
             }
         }
-        if (ok && row < p.lq) {
-            const size_t at = (size_t)unit * p.lq + row;
-            store_cols<HALF>(p.out + at * p.d, res, kSplitDown2, inv, w * HALF, p.d, p.vec_o, p.out, (size_t)p.order.units * p.lq * p.d * 4, p.status);
-            if (p.lse && w == 0 && EMBER_STORE_OK(p.lse + at, p.lse, (size_t)p.order.units * p.lq * 4, 4, p.status)) p.lse[at] = mm + logf(ll);
+        const bool stores = ok && row < p.lq;
+        const size_t at = (size_t)unit * p.lq + row, o_bytes = (size_t)p.order.units * p.lq * p.d * 4;
+        if (PAIR && pair) {
+            // ---- each CTA of the pair finishes half of every thread's columns; what the other one needs, it reads from here
+            constexpr int PART = HALF / 2;
+            uint8_t *state2 = xo + 2 * 128 * ROWB, *xo2 = state2 + 1024;         // [128] maximum and sum, [PART / 4][256] 16 bytes
+            if (w == 0) reinterpret_cast<float2 *>(state2)[r] = make_float2(mm, ll);
+#pragma unroll
+            for (int c = 0; c < PART / 4; c++) {
+                const int i = 2 * c;
+                reinterpret_cast<ulonglong2 *>(xo2)[c * 256 + threadIdx.x] = half == 0 ? make_ulonglong2(res[PART / 2 + i], res[PART / 2 + i + 1]) : make_ulonglong2(res[i], res[i + 1]);
+            }
+            cluster_arrive();
+            cluster_wait();
+            const uint32_t there = map_to_cta(smem_u32(state2), half ^ 1);
+            const float4 st2 = ld_cluster4(there + r / 2 * 16);
+            float4 v[PART / 4];
+#pragma unroll
+            for (int c = 0; c < PART / 4; c++) v[c] = ld_cluster4(there + 1024 + (c * 256 + threadIdx.x) * 16);
+            const float m2 = r % 2 ? st2.z : st2.x, l2 = r % 2 ? st2.w : st2.y, top = fmaxf(mm, m2);
+            const float a_here = exp_nat(mm - top), a_there = exp_nat(m2 - top);
+            ll = half == 0 ? ll * a_here + l2 * a_there : l2 * a_there + ll * a_here;
+            mm = top;
+            const f32x2 here2 = pack2(a_here, a_here), there2 = pack2(a_there, a_there);
+#pragma unroll
+            for (int c = 0; c < PART / 4; c++) {
+                const int i = 2 * c;
+                res[i] = fma2(half == 0 ? res[i] : res[PART / 2 + i], here2, mul2(pack2(v[c].x, v[c].y), there2));
+                res[i + 1] = fma2(half == 0 ? res[i + 1] : res[PART / 2 + i + 1], here2, mul2(pack2(v[c].z, v[c].w), there2));
+            }
+            if (stores) store_cols<PART>(p.out + at * p.d, res, kSplitDown2, 1.f / ll, w * HALF + half * PART, p.d, p.vec_o, p.out, o_bytes, p.status);
+        } else if (stores) {
+            store_cols<HALF>(p.out + at * p.d, res, kSplitDown2, 1.f / ll, w * HALF, p.d, p.vec_o, p.out, o_bytes, p.status);
         }
+        if (stores && p.lse && w == 0 && half == 0 && EMBER_STORE_OK(p.lse + at, p.lse, (size_t)p.order.units * p.lq * 4, 4, p.status)) p.lse[at] = mm + logf(ll);
+    }
+    if (PAIR && pair && !leave) {
+        __syncwarp();
+        if (warp >= 8) {  // the compute warps' first meeting
+            cluster_arrive();
+            cluster_wait();
+        }
+        cluster_arrive();
+        cluster_wait();   // the other CTA has read what it needs
     }
     tc_fence_before();
     __syncthreads();
@@ -956,10 +1008,44 @@ cudaError_t launch_cfg(cudaLaunchConfig_t &cfg, LaunchAttrs &attrs, long long gr
     return cudaSuccess;
 }
 
+// How many query blocks, from the longest on, two CTAs share: all, where that still is one wave, or as many as there are SMs left, where the mask
+// makes blocks of different lengths and the longest that stays whole is then enough shorter. us, calls back to back, whole / shared:
+//   all    d 64   1 x 512 17.4 / 15.0   8 x 1024 causal 33 / 24.5   4 x 2048 causal 47.3 / 32.9   22 x 5 x 2171 50.1 / 35.4   1 x 23 x 5882 101 / 60
+//          d 128  1 x 512 30 / 23   8 x 1024 causal 50.2 / 35.4   28 x 21 x 4542 209 / 139
+//   some   d 64   16 x 1024 31.5 / 30.2   8 x 2048 48.2 / 45.8   6 x 1686 41.0 / 30.3   12 x 1095 31.3 / 27.3   d 128  16 x 1024 53.4 / 50.1   3 x 4594 170 / 117
+// Up to four tiles (64 columns) or two, what the two spend on each other is what they save (36 x 221, d 48, 14.8 / 15.1). So it is where one tile
+// fewer is left (22 x 544 21.6 / 22.5) or little of many (45 x 215 x 3049 86 / 91). In two waves a start and an end more cost as much as the better
+// balance gives: 92 blocks x 4711 keys 94.5 / 106, 364 x 775 58 / 77, all of 16 x 1024 causal 31.3 / 33.4 (160 x 5010, d 128, 373 / 304, is the exception).
+int fwd_paired(const AttnArgs &a, const WorkOrder &order, int sms)
+{
+    const long long items = (long long)order.units * order.blocks;
+    if (a.lk <= (a.d <= 64 ? 4 : 2) * TN) return 0;
+    if (2 * items <= sms) return (int)items;
+    if (!a.causal || order.ngroups != 1 || items + order.units > sms) return 0;
+    const int left = (int)(sms - items), whole = order.blocks - 1 - left / order.units;  // the last block that stays whole
+    const auto tiles = [&](int block) { return (min((long long)a.lk, (block + 1) * 128LL + a.lk - a.lq) + TN - 1) / TN; };
+    const long long most = tiles(order.blocks - 1), saved = most - tiles(whole);
+    return saved >= 2 && 12 * saved >= most ? left : 0;
+}
+
+template <int HD, bool PAIR>
+int launch_fwd_form(const CUtensorMap &tk, const CUtensorMap &tv, const F32FwdParams &p, cudaStream_t s)
+{
+    auto kern = sm100_f32_fwd_kernel<HD, PAIR>;
+    static SmemOptIn opt_in;
+    EMBER_CUDA_TRY(opt_in(kern, F32FwdCfg<HD>::SMEM));
+    cudaLaunchConfig_t cfg = {};
+    LaunchAttrs attrs;
+    attrs.cluster(PAIR ? 2 : 1);
+    const long long ctas = (long long)p.order.units * p.order.blocks + p.paired;
+    launch_cfg(cfg, attrs, PAIR ? (ctas + 1) / 2 * 2 : ctas, F32FwdCfg<HD>::SMEM, s);
+    EMBER_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, tk, tv, p));
+    return EMBER_OK;
+}
+
 template <int HD>
 int launch_fwd(const AttnArgs &a, const void *kp, const void *vp, const SplitGuard &guard, DeviceState *st, cudaStream_t s)
 {
-    using C = F32FwdCfg<HD>;
     CUtensorMap tk, tv;
     int rc;
     if ((rc = plane_map(&tk, kp, a.d, a.lk, a.bh)) != EMBER_OK || (rc = plane_map(&tv, vp, a.d, a.lk, a.bh)) != EMBER_OK) return rc;
@@ -974,14 +1060,8 @@ int launch_fwd(const AttnArgs &a, const void *kp, const void *vp, const SplitGua
     p.guard = guard;
     p.status = st->status;
     p.order = make_work_order(a.bh, (a.lq + 127) / 128, st->sm_count, (size_t)a.lk * a.d * 12 + (size_t)a.lq * a.d * 8, a.causal != 0);
-    auto kern = sm100_f32_fwd_kernel<HD>;
-    static SmemOptIn opt_in;
-    EMBER_CUDA_TRY(opt_in(kern, C::SMEM));
-    cudaLaunchConfig_t cfg = {};
-    LaunchAttrs attrs;
-    launch_cfg(cfg, attrs, (long long)p.order.units * p.order.blocks, C::SMEM, s);
-    EMBER_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, tk, tv, p));
-    return EMBER_OK;
+    p.paired = fwd_paired(a, p.order, st->sm_count);
+    return p.paired > 0 ? launch_fwd_form<HD, true>(tk, tv, p, s) : launch_fwd_form<HD, false>(tk, tv, p, s);
 }
 
 template <int HD>
