@@ -648,14 +648,15 @@ struct F32BwdParams {
     SplitGuard guard;
     DeviceStatus *status;
     WorkOrder order;
+    int paired;  // items that two CTAs share
 };
 
 // Which role and block the rank-th heaviest item of a unit is.
 template <int HD>
-__device__ __forceinline__ void bwd_item(int rank, int kb, int qb, int &role, int &blk)
+EMBER_HD void bwd_item(int rank, int kb, int qb, int &role, int &blk)
 {
     constexpr int NR = HD == 64 ? 2 : 3;
-    const int m = min(kb, qb);
+    const int m = kb < qb ? kb : qb;
     if (rank < NR * m) {
         const int i = rank % NR;
         blk = rank / NR;
@@ -673,7 +674,8 @@ __device__ __forceinline__ void bwd_item(int rank, int kb, int qb, int &role, in
     }
 }
 
-template <int HD>
+// PAIR: as in the forward, two CTAs share the tiles that an item's 128 rows meet, and add up their results.
+template <int HD, bool PAIR>
 __global__ void __launch_bounds__(F32_THREADS, 1)
     sm100_f32_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                          const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do, const F32BwdParams p)
@@ -702,16 +704,23 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
 
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     int unit, rank, role, blk;
-    work_item(p.order, blockIdx.x, unit, rank);
+    const bool pair = PAIR && blockIdx.x < 2u * p.paired;  // the items as in the forward
+    const unsigned item = !PAIR ? blockIdx.x : pair ? blockIdx.x / 2 : blockIdx.x - p.paired;
+    if (PAIR && item >= (unsigned)p.order.units * p.order.blocks) {
+        pdl_wait();
+        return;
+    }
+    work_item(p.order, (int)item, unit, rank);
     bwd_item<HD>(rank, p.kblocks, p.qblocks, role, blk);
     const bool is_q = role == R_DQ;
     const bool has_p = role == R_DKDV || role == R_DV, has_ds = role != R_DV;  // which results
     const int off = p.lk - p.lq;
     const int row0 = (is_q ? p.qblocks - 1 - blk : blk) * 128;  // heaviest first: the last queries, the first keys
     // the streamed tiles: rows [first, ...) of the other side
-    const int first = is_q || !p.causal ? 0 : max(0, (row0 - off) / TN) * TN;
+    const int start = is_q || !p.causal ? 0 : max(0, (row0 - off) / TN) * TN;
     const int end = is_q ? (p.causal ? min(p.lk, row0 + 128 + off) : p.lk) : p.lq;
-    const int n = (end - first + TN - 1) / TN;
+    const int tiles = (end - start + TN - 1) / TN, half = pair ? (int)cluster_ctarank() : 0, first = start + half * ((tiles + 1) / 2) * TN;
+    const int n = !pair ? tiles : half ? tiles - (tiles + 1) / 2 : (tiles + 1) / 2;
     const int stages = role == R_DV ? 2 : C::STAGES;
 
     if (threadIdx.x == 0) {
@@ -976,12 +985,41 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
                 if (lane == 0) mbar_arrive(BAR(C::B_DS));
             }
         }
-        if (ok) add_result(n - 1);
-        if (ok && row < rows && acc_cols > 0) {
-            float *dst = is_q ? p.dq : role == R_DKDV ? (w == 0 ? p.dv : p.dk) : role == R_DK ? p.dk : p.dv;
-            const bool is_dv = role == R_DV || (role == R_DKDV && w == 0);
-            store_cols<64>(dst + row_at, acc, is_dv ? kSplitDown2 : ds_down, is_dv ? 1.f : p.scale, acc_col0, role == R_DKDV ? p.d : min(p.d, acc_col0 + HD / 2), p.vec_out, dst, (size_t)p.units * rows * p.d * 4, p.status);
+        if (ok && n > 0) add_result(n - 1);
+        float *dst = is_q ? p.dq : role == R_DKDV ? (w == 0 ? p.dv : p.dk) : role == R_DK ? p.dk : p.dv;
+        const bool is_dv = role == R_DV || (role == R_DKDV && w == 0), stores = ok && row < rows && acc_cols > 0;
+        const float down = is_dv ? kSplitDown2 : ds_down, scale = is_dv ? 1.f : p.scale;
+        const int limit = role == R_DKDV ? p.d : min(p.d, acc_col0 + HD / 2);
+        const size_t bytes = (size_t)p.units * rows * p.d * 4;
+        if (PAIR && pair) {
+            // ---- each CTA of the pair finishes half of every thread's columns. The tiles have been multiplied, by both warpgroups' last results
+            ulonglong2 *mine = reinterpret_cast<ulonglong2 *>(smem_gen + C::OFF_B);  // [8][256] 16 bytes
+            named_bar_sync(1, 256);
+#pragma unroll
+            for (int c = 0; c < 8; c++) mine[c * 256 + threadIdx.x] = half == 0 ? make_ulonglong2(acc[16 + 2 * c], acc[17 + 2 * c]) : make_ulonglong2(acc[2 * c], acc[2 * c + 1]);
+            cluster_arrive();
+            cluster_wait();
+            const uint32_t there = map_to_cta(smem_u32(mine), half ^ 1);
+            f32x2 res[16];
+#pragma unroll
+            for (int c = 0; c < 8; c++) {
+                const float4 v = ld_cluster4(there + (c * 256 + threadIdx.x) * 16);
+                res[2 * c] = add2(half == 0 ? acc[2 * c] : acc[16 + 2 * c], pack2(v.x, v.y));
+                res[2 * c + 1] = add2(half == 0 ? acc[2 * c + 1] : acc[17 + 2 * c], pack2(v.z, v.w));
+            }
+            if (stores) store_cols<32>(dst + row_at, res, down, scale, acc_col0 + half * 32, limit, p.vec_out, dst, bytes, p.status);
+        } else if (stores) {
+            store_cols<64>(dst + row_at, acc, down, scale, acc_col0, limit, p.vec_out, dst, bytes, p.status);
         }
+    }
+    if (PAIR && pair && !leave) {
+        __syncwarp();
+        if (warp >= 8) {  // the compute warps' first meeting
+            cluster_arrive();
+            cluster_wait();
+        }
+        cluster_arrive();
+        cluster_wait();   // the other CTA has read what it needs
     }
     tc_fence_before();
     __syncthreads();
@@ -1064,6 +1102,50 @@ int launch_fwd(const AttnArgs &a, const void *kp, const void *vp, const SplitGua
     return p.paired > 0 ? launch_fwd_form<HD, true>(tk, tv, p, s) : launch_fwd_form<HD, false>(tk, tv, p, s);
 }
 
+// How many items, from the longest on, two CTAs share: the forward's rule over both kinds of rows. us, calls back to back, whole / shared:
+//   all    d 64   1 x 512 causal 28.7 / 21.4   4 x 1024 causal 49.6 / 33.7   1 x 2048 causal 81.6 / 48.1   17 x 203, d 48, 20.7 / 18.0
+//          d 128  1 x 442 46.9 / 33.3   2 x 1024 causal 93.0 / 54.8   1 x 1533 x 3558, d 72, 263 / 140
+//   some   d 64   6 x 1024 51.3 / 34.6   3 x 2414 100.5 / 73.1   14 x 346 28.5 / 23.0   d 128  1 x 3278 269 / 144   4 x 438 x 1647, d 96, 127 / 115.5
+// Over 87 sizes with more than two tiles, 0.54 to 0.91 of the time.
+template <int HD>
+int bwd_paired(const F32BwdParams &p, int sms)
+{
+    const long long items = (long long)p.order.units * p.order.blocks;
+    if ((p.lk > p.lq ? p.lk : p.lq) <= 2 * TN) return 0;
+    if (2 * items <= sms) return (int)items;
+    if (!p.causal || p.order.ngroups != 1 || items + p.order.units > sms) return 0;
+    const auto tiles = [&](int rank) {
+        int role, blk;
+        bwd_item<HD>(rank, p.kblocks, p.qblocks, role, blk);
+        const long long off = p.lk - p.lq, row0 = 128LL * (role == R_DQ ? p.qblocks - 1 - blk : blk);
+        const long long begin = role == R_DQ || row0 < off ? 0 : (row0 - off) / TN * TN, end = role != R_DQ ? p.lq : row0 + 128 + off < p.lk ? row0 + 128 + off : p.lk;
+        return (end - begin + TN - 1) / TN;
+    };
+    const int left = (int)(sms - items), whole = left / p.order.units;  // rank of the first item that stays whole
+    long long most = 0, rest = 0;
+    for (int r = 0; r < p.order.blocks; r++) {
+        const long long t = tiles(r);
+        most = most > t ? most : t;
+        if (r >= whole) rest = rest > t ? rest : t;
+    }
+    return most - rest >= 2 && 12 * (most - rest) >= most ? left : 0;
+}
+
+template <int HD, bool PAIR>
+int launch_bwd_form(const CUtensorMap &tq, const CUtensorMap &tk, const CUtensorMap &tv, const CUtensorMap &tg, const F32BwdParams &p, cudaStream_t s)
+{
+    auto kern = sm100_f32_bwd_kernel<HD, PAIR>;
+    static SmemOptIn opt_in;
+    EMBER_CUDA_TRY(opt_in(kern, F32BwdCfg<HD>::SMEM));
+    cudaLaunchConfig_t cfg = {};
+    LaunchAttrs attrs;
+    attrs.cluster(PAIR ? 2 : 1);
+    const long long ctas = (long long)p.order.units * p.order.blocks + p.paired;
+    launch_cfg(cfg, attrs, PAIR ? (ctas + 1) / 2 * 2 : ctas, F32BwdCfg<HD>::SMEM, s);
+    EMBER_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, tq, tk, tv, tg, p));
+    return EMBER_OK;
+}
+
 template <int HD>
 int launch_bwd(const AttnArgs &a, const float *delta, const void *qp, const void *kp, const void *vp, const void *gp, const SplitGuard &guard,
                DeviceState *st, cudaStream_t s)
@@ -1087,14 +1169,8 @@ int launch_bwd(const AttnArgs &a, const float *delta, const void *qp, const void
     p.guard = guard;
     p.status = st->status;
     p.order = make_work_order(a.bh, (HD == 64 ? 1 : 2) * p.kblocks + p.qblocks, st->sm_count, ((size_t)a.lk + a.lq) * a.d * 24, a.causal != 0);
-    auto kern = sm100_f32_bwd_kernel<HD>;
-    static SmemOptIn opt_in;
-    EMBER_CUDA_TRY(opt_in(kern, C::SMEM));
-    cudaLaunchConfig_t cfg = {};
-    LaunchAttrs attrs;
-    launch_cfg(cfg, attrs, (long long)p.order.units * p.order.blocks, C::SMEM, s);
-    EMBER_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, tq, tk, tv, tg, p));
-    return EMBER_OK;
+    p.paired = bwd_paired<HD>(p, st->sm_count);
+    return p.paired > 0 ? launch_bwd_form<HD, true>(tq, tk, tv, tg, p, s) : launch_bwd_form<HD, false>(tq, tk, tv, tg, p, s);
 }
 
 // What scores may reach (columns x the largest elements of q and k x scale) before the CUDA cores take over. 2^96 keeps them below the
