@@ -1198,7 +1198,8 @@ bool takes(const AttnArgs &a)
 //           1 x 512 F 25 / 23 B 43 / 33    8 x 1024 F 74 / 34 B 206 / 56  4 x 2048 F 141 / 52 B 393 / 92  512 x 128 F 56 / 66 B 172 / 145
 //   d 128   8 x 256 F 23 / 27 B 52 / 39    1 x 512 F 39 / 34 B 68 / 57    8 x 1024 F 105 / 56 B 234 / 103 4 x 2048 F 197 / 89 B 444 / 182
 //   rows against keys, d 64   512 x 32 x 2048 F 293 / 411 B 1668 / 1165   128 x 32 x 2048 F 121 / 106 B 483 / 318   512 x 64 x 64 F 26 / 44 B 67 / 87
-// The estimates are within a quarter of these.
+// The estimates are within a quarter of these. They know nothing of blocks that two CTAs share, which are up to 1.9 times as fast: what goes to the tensor
+// cores is better there than they say.
 namespace {
 struct Shape {
     double units, lq, lk, d, visible;  // visible: the share of (query, key) pairs under the mask
