@@ -496,12 +496,14 @@ __global__ void __launch_bounds__(FWD_THREADS, 1)
                     }
                     sum2[i & 3] = add2(sum2[i & 3], pack2(p0, p1));
                     pk[ch][i] = pack_bf16(p0, p1);
-                    if (ch == 1 && i == 7 && !o_done) o_done = mbar_try_wait(BAR(B_O), (j - 1) & 1);  // asked here, needed eight pairs later
+                    // Asked here, needed eight pairs later. With a try_wait, which may hold the warp until the phase is over, the exponentials behind it
+                    // wait too (8 x 2048 d 128 24.1 us against 21.0; not asked at all 21.0, but 16 x 2048 d 64 causal 21.2 against 20.8).
+                    if (ch == 1 && i == 7 && !o_done) o_done = mbar_test_wait(BAR(B_O), (j - 1) & 1);
                 }
-            if (!o_done) {  // PV(j-1) must have read the old P
+            if (!o_done)  // PV(j-1) must have read the old P
                 ok = ok && mbar_wait(BAR(B_O), (j - 1) & 1, abort_flag, p.status, W_SM_O);
-                tc_fence_after();
-            }
+            __syncwarp();      // lanes may have had different answers
+            tc_fence_after();  // orders the stores behind PV(j-1) whichever way its end was seen
             tmem_st_32x32b_x16(tp, pk[0]);
             tmem_st_32x32b_x16(tp + 16, pk[1]);
             tmem_wait_st();
@@ -690,6 +692,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 1)
             weights(s, 24, sum_a, pk);
             if (!o_done)  // before the first store: PV(j-1) must have read the old P
                 ok = ok && mbar_wait(BAR(B_O + t), (j - 1) & 1, abort_flag, p.status, W_SM_O);
+            __syncwarp();  // lanes may have had different answers
             tc_fence_after();
             tmem_st_32x32b_x16(tp, pk);
             tmem_st_32x32b_x16(tp + 16, pk + 16);

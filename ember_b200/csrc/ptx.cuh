@@ -68,6 +68,22 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity)
     return ok != 0;
 }
 
+// Whether the phase with the given parity is over, answered at once (a try_wait may hold the warp for a while before it says no).
+__device__ __forceinline__ bool mbar_test_wait(uint32_t bar, uint32_t parity)
+{
+    uint32_t ok;
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        "selp.u32 %0, 1, 0, p;\n"
+        "}\n"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+
 // Upper bound of one wait, in SM clock cycles (about a quarter of a second). A healthy kernel
 // never comes near it: the longest legitimate wait is one CTA's whole work, a few milliseconds.
 constexpr long long kWaitLimitCycles = 400LL * 1000 * 1000;
