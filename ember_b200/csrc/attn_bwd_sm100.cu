@@ -880,7 +880,7 @@ __device__ long long g_bwd_trace[64 * 32];
 // 16 columns that hold anything, dQ, dK and dV are that many columns wide, and only the 32-column chunks of
 // dQ that hold one of the d columns are added into the accumulator. At d = 80 that is 396 KB of shared-memory
 // traffic per tile pair instead of 512 KB; forward and backward of 36 units x 777 x 1301 at d = 80 went 105.6 -> 100.5 us.
-template <int HD, bool PART, bool BESIDE>
+template <int HD, bool PART, bool BESIDE, bool SHORT>
 __global__ void __launch_bounds__(SP_THREADS, 1)
     sm100_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                            const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
@@ -967,17 +967,22 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
             if (w == 0 && lane == 0) TR(16, i);
             float *gdst = p.dq_acc + ((((size_t)bh * nqt + (i_begin + i)) * 4 + w) * chunks) * 1024;
             // The whole row leaves tensor memory at once: with 64 columns at a time its second half waited for the first one's way through
-            // the staging buffers, 1090 clocks at 128 columns while dK(i) reads its operands, and dP^T(i+1) with it (now 200).
-            uint32_t u[HD / 32][32];
+            // the staging buffers, 1090 clocks at 128 columns while dK(i) reads its operands, and dP^T(i+1) with it (now 200). SHORT: in halves, of
+            // which the first is on its way sooner, where hardly a tile waits for the row (see launch_fused).
+            constexpr int AT_ONCE = SHORT ? 2 : HD / 32;
 #pragma unroll
-            for (int c = 0; c < HD / 32; c++) tmem_ld_32x32b_x32(t_dq + c * 32, u[c]);
-            tmem_wait_ld();
-            warp_arrive(BAR(C::B_DQFREE), lane);
-            if (w == 0 && lane == 0) TR(17, i);
-            {
+            for (int c0 = 0; c0 < HD / 32; c0 += AT_ONCE) {
+                uint32_t u[AT_ONCE][32];
 #pragma unroll
-                for (int c = 0; c < HD / 32; c++) {
-                    if (PART && c >= chunks) break;
+                for (int c = 0; c < AT_ONCE; c++) tmem_ld_32x32b_x32(t_dq + (c0 + c) * 32, u[c]);
+                tmem_wait_ld();
+                if (c0 + AT_ONCE == HD / 32) {
+                    warp_arrive(BAR(C::B_DQFREE), lane);
+                    if (w == 0 && lane == 0) TR(17, i);
+                }
+#pragma unroll
+                for (int c = 0; c < AT_ONCE; c++) {
+                    if (PART && c0 + c >= chunks) break;
                     // the bulk operation that read this buffer two chunks ago must be done with it
                     if (lane == 0) bulk_wait_read_1();
                     __syncwarp();
@@ -989,7 +994,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
                     fence_proxy_async();
                     __syncwarp();
                     if (lane == 0) {
-                        if (ok) bulk_reduce_add_f32(gdst + c * 1024, stage_u32 + (cnt & 1) * 4096, 4096);
+                        if (ok) bulk_reduce_add_f32(gdst + (c0 + c) * 1024, stage_u32 + (cnt & 1) * 4096, 4096);
                         bulk_commit();
                     }
                     cnt++;
@@ -1395,7 +1400,7 @@ int launch_delta_bf16(const AttnArgs &a, float *delta, cudaStream_t s, void *zer
     return EMBER_OK;
 }
 
-template <int HD, bool PART, bool BESIDE>
+template <int HD, bool PART, bool BESIDE, bool SHORT = false>
 int launch_fused_form(const AttnArgs &a, float *delta, float *dq_acc, DeviceState *st, cudaStream_t s)
 {
     using C = SpCfg<HD, BESIDE>;
@@ -1424,7 +1429,7 @@ int launch_fused_form(const AttnArgs &a, float *delta, float *dq_acc, DeviceStat
     p.scale = a.scale;
     p.scale_log2 = a.scale * LOG2E_B;
     p.status = st->status;
-    auto k1 = sm100_bwd_fused_kernel<HD, PART, BESIDE>;
+    auto k1 = sm100_bwd_fused_kernel<HD, PART, BESIDE, SHORT>;
     static SmemOptIn opt_in1;
     EMBER_CUDA_TRY(opt_in1(k1, C::SMEM_BYTES));
     const size_t touched = ((size_t)a.lq + a.lk) * HD * 2 * 4 + (size_t)a.lq * HD * 4;  // + the float32 dQ accumulator
@@ -1456,6 +1461,10 @@ int launch_fused(const AttnArgs &a, float *delta, float *dq_acc, DeviceState *st
         return a.d <= 48 ? launch_fused_form<64, true, false>(a, delta, dq_acc, st, s)
                : a.lq <= 1024 ? launch_fused_form<64, false, false>(a, delta, dq_acc, st, s)
                               : launch_fused_form<64, false, true>(a, delta, dq_acc, st, s);
+    // SHORT up to two query tiles: us, whole rows / halves, 42 units x 56 d 128 10.13 / 9.78, 21 x 135 12.57 / 12.32, 367 x 37 x 54 33.8 / 33.2, 16 x 256 causal
+    // 12.22 / 12.06; three tiles and four are level (16 x 384 causal 14.95 / 14.93), 16 x 2048 causal is 56.4 / 60.0.
+    if (a.lq <= 256)
+        return a.d <= 112 ? launch_fused_form<128, true, false, true>(a, delta, dq_acc, st, s) : launch_fused_form<128, false, false, true>(a, delta, dq_acc, st, s);
     return a.d <= 112 ? launch_fused_form<128, true, false>(a, delta, dq_acc, st, s) : launch_fused_form<128, false, false>(a, delta, dq_acc, st, s);
 }
 
