@@ -179,9 +179,13 @@ __global__ void __launch_bounds__(256, 2) narrow_f32_bwd_kernel(const NarrowBwd 
                     float o[4];
 #pragma unroll
                     for (int j = 0; j < 4; j++) {
-                        o[j] = g[u][0] * wv[j * N];
+                        // Above four columns in two sums, of every other column: one chain is off by more than the tiles' sums were
+                        // (256 x 784 x 10 5.5e-8 of the norm as tiles, 6.0e-8 in one chain, 5.2e-8 in two; 64 x 784 x 12 5.8, 6.4, 5.5).
+                        constexpr int CHAINS = N > 4 ? 2 : 1;
+                        float s[CHAINS];
 #pragma unroll
-                        for (int c = 1; c < N; c++) o[j] = fmaf(g[u][c], wv[j * N + c], o[j]);
+                        for (int c = 0; c < N; c++) s[c % CHAINS] = c < CHAINS ? g[u][c] * wv[j * N + c] : fmaf(g[u][c], wv[j * N + c], s[c % CHAINS]);
+                        o[j] = CHAINS == 2 ? s[0] + s[CHAINS - 1] : s[0];
                     }
                     if (r + u < r1) *reinterpret_cast<float4 *>(p.dx + (size_t)(r + u) * p.k + col) = make_float4(o[0], o[1], o[2], o[3]);
                 }
