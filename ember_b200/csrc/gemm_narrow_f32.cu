@@ -222,8 +222,9 @@ __global__ void __launch_bounds__(256, 2) narrow_f32_bwd_kernel(const NarrowBwd 
 #pragma unroll
                 for (int c = 0; c < N; c++) g[u][c] = 0.f;
             }
-        // four products are added up before they meet the sums: a chain of m / 256 additions instead of m / 64
-        // (8192 x 784 x 10: grad_w 1.3e-7 of its norm off; row by row 2.2e-7, gemm_simt.cu 1.7e-7)
+        // Four products are added up before they meet the sums: a chain of m / (32 cluster) additions instead of m / (8 cluster)
+        // (8192 x 784 x 10, eight blocks: grad_w 1.3e-7 of its norm off; row by row 2.2e-7, gemm_simt.cu 1.7e-7). Wide layers, whose blocks have all
+        // rows, have the longest: 16384 x 40000 x 8, 512 additions, 4.1e-7, gemm_simt.cu 2.3e-6; 1024 x 200000 x 10 1.2e-7 and 5.8e-7.
 #pragma unroll
         for (int c = 0; c < N; c++) {
             acc[c][0] += fmaf(xv[3].x, g[3][c], fmaf(xv[2].x, g[2][c], fmaf(xv[1].x, g[1][c], xv[0].x * g[0][c])));
@@ -306,8 +307,8 @@ bool narrow_f32_bwd_supported(const void *x, const void *w, const void *dy, cons
 {
     if (n > 12 || k % 4 != 0 || k > 0x7fffffff - 1024 || (((uintptr_t)x | (uintptr_t)w | (uintptr_t)dy | (uintptr_t)dx) & 15) != 0) return false;
     // us, the kernels that took these calls before (gemm_simt.cu, from some sizes on gemm_f32_sm100.cu, column_sums.cu) / here, calls back to back in
-    // a graph, grad_x, grad_w and grad_b: 256 x 784 x 10 14.8 / 5.7, 32 x 64 x 10 8.3 / 3.7, 1000 x 512 x 12 15.4 / 10, 8192 x 784 x 10 68 / 32,
-    // 8192 x 2048 x 10 138 / 45; over 500 sizes (1 to 16384 rows, contractions of 4 to 2048) 0.44 of the time,
+    // a graph, grad_x, grad_w and grad_b: 256 x 784 x 10 14.8 / 5.7, 32 x 64 x 10 8.3 / 3.7, 1000 x 512 x 12 15.4 / 10, 8192 x 784 x 10 68 / 33,
+    // 8192 x 2048 x 10 136 / 46; over 500 sizes (1 to 16384 rows, contractions of 4 to 2048) 0.44 of the time,
     // over 200 with contractions to 262144 (up to 2^27 elements of x) 0.43.
     // At most eight blocks share the rows of 128 columns, which is too few for tall matrices: 32768 x 784 x 10 231 / 213, 68047 x 536 x 11 420 / 444,
     // 122465 x 308 x 8 395 / 949; with 8 and 12 columns, which tiles move in pieces of 16 bytes, from 4097 rows on if they are also narrow (9277 x 8 x 12
