@@ -5,8 +5,8 @@
 // gradients), so that small ones keep all of theirs; where a result leaves the accumulators that is undone.
 //
 // The CUDA-core kernels (attn_simt.cu) do the same products at the FMA pipe's rate, 128 per clock and SM; six bf16 products for
-// each leave 683 per clock. Whole calls (split included), 16 units x L1024, causal: d 64 forward 93 -> 33 us, backward 215 -> 66; d 128, 8
-// units: 105 -> 55 and 234 -> 103. What bounds them now: the compute warps (exponentials, splitting of 128 x 64 probabilities) and the
+// each leave 683 per clock. Whole calls (split included), 16 units x L1024, causal: d 64 forward 93 -> 32 us, backward 215 -> 64; d 128, 8
+// units: 105 -> 36 and 234 -> 100. What bounds them now: the compute warps (exponentials, splitting of 128 x 64 probabilities) and the
 // hand-overs between them and the products. A tile takes, of its MMAs' clocks: forward 1930 of 1536 (d 64), 4160 of 3072 (d 128); backward, a
 // query block's 3940 of 2688 and 9300 of 5500 (one pair of tiles, loaded without overlap).
 // Errors against float64 (relative 2-norm, CUDA cores -> here): 16 units x L1024 d 64 causal: o 2.1e-7 -> 0.9e-7, dq 3.3e-7 ->
@@ -1106,7 +1106,7 @@ int launch_fwd(const AttnArgs &a, const void *kp, const void *vp, const SplitGua
 //   all    d 64   1 x 512 causal 28.7 / 21.4   4 x 1024 causal 49.6 / 33.7   1 x 2048 causal 81.6 / 48.1   17 x 203, d 48, 20.7 / 18.0
 //          d 128  1 x 442 46.9 / 33.3   2 x 1024 causal 93.0 / 54.8   1 x 1533 x 3558, d 72, 263 / 140
 //   some   d 64   6 x 1024 51.3 / 34.6   3 x 2414 100.5 / 73.1   14 x 346 28.5 / 23.0   d 128  1 x 3278 269 / 144   4 x 438 x 1647, d 96, 127 / 115.5
-// Over 87 sizes with more than two tiles, 0.54 to 0.91 of the time.
+// Over 87 sizes with more than two tiles, 0.53 to 0.91 of the time.
 template <int HD>
 int bwd_paired(const F32BwdParams &p, int sms)
 {
@@ -1199,7 +1199,8 @@ bool takes(const AttnArgs &a)
 //   d 128   8 x 256 F 23 / 27 B 52 / 39    1 x 512 F 39 / 34 B 68 / 57    8 x 1024 F 105 / 56 B 234 / 103 4 x 2048 F 197 / 89 B 444 / 182
 //   rows against keys, d 64   512 x 32 x 2048 F 293 / 411 B 1668 / 1165   128 x 32 x 2048 F 121 / 106 B 483 / 318   512 x 64 x 64 F 26 / 44 B 67 / 87
 // The estimates are within a quarter of these. They know nothing of blocks that two CTAs share, which are up to 1.9 times as fast: what goes to the tensor
-// cores is better there than they say.
+// cores is better there than they say (back to back, causal, d 64: 1 x 512 F 22 / 15 B 40 / 21, 8 x 256 B 28 / 18.5), and some forwards of few blocks stay on the
+// CUDA cores that would be quicker on the others (1 x 384 without a mask 17.4; 2 x 384, which go, 17.4 / 14.1).
 namespace {
 struct Shape {
     double units, lq, lk, d, visible;  // visible: the share of (query, key) pairs under the mask

@@ -816,12 +816,13 @@ int launch_pair(const AttnArgs &a, DeviceState *st, cudaStream_t s)
 
 // Query rows per CTA. Two tiles (256 rows) share the key/value stream and interleave their softmax with each other's MMAs; one tile
 // (128 rows) has both softmax warpgroups to itself and is held by the exponentials of 128 x 128 scores (1024 clocks of every
-// scheduler's MUFU, which nothing else of the CTA overlaps: about 1860 a step), so that two of its steps take 1.3 times as long as one
-// step of two tiles. But it makes twice as many CTAs, of little more than half the length: which form ends first is
+// scheduler's MUFU, which nothing else of the CTA overlaps: 1990 a step at 128 columns, 1780 at 64, against 2930 and 2680 of two tiles), so that two
+// of its steps take 1.35 times as long as one step of two tiles. But it makes twice as many CTAs, of little more than half the length: which form ends first is
 // estimated from the lengths (in steps of one tile; a CTA's start and end are 3.7 of them), heaviest CTAs first.
-// Measured, us, two tiles / one: 8 units x L2048 37 / 24.6, causal 16 x 2048 32.1 / 25.8, 16 x 1024 21.5 / 14.8, 13 x 1536 24.6 / 17.7, 32 x 1024 19.8 / 18.4,
-// 8 x 4096 64 / 42, 4 x 100 rows x 4096 keys 42 / 38; the other way round 16 x 4096 64 / 82, 32 x 2048 42 / 53, 64 x 512 13.0 / 14.4, 36 x 777 x 1301
-// without a mask 24.6 / 32.5. (While the second warpgroup of a one-tile CTA was idle its step took 2000 to 2700 clocks: 8 x 2048 29.6.)
+// Measured, us, calls back to back, two tiles / one: 8 units x L2048 29.5 / 21.0, causal 16 x 2048 30.5 / 24.1, 16 x 1024 17.0 / 12.7, 13 x 1536 23.5 / 16.8,
+// 32 x 1024 18.2 / 17.1, 8 x 4096 55.6 / 38.2, 4 x 100 rows x 4096 keys 38.5 / 35.8; the other way round 16 x 4096 57 / 75, 32 x 2048 37.7 / 50.7, 64 x 512 12.1 / 14.0,
+// 36 x 777 x 1301 d 80 without a mask 23.4 / 30.7. Over 106 drawn shapes of 60 to 900 CTAs the choice is the better form but for five, which are 1 to 12 % longer
+// (40 x 554 causal 11.5 / 12.8 and 28 x 1526 x 6803 causal 163 / 173, both taken by one tile).
 // A row's arithmetic does not depend on the choice: both forms give the same bits.
 // ember_set_forward_block_rows (initially EMBER_FWD_ROWS=128|256) forces one form, for tests and tuning.
 static int g_fwd_rows = -1;  // -1: not read from the environment yet; 0: choose per call
@@ -858,7 +859,7 @@ static int fwd_block_rows(const AttnArgs &a, DeviceState *st)
         double end = fmax(length(0), total / sms);
         end = fmax(end, (double)((ctas + sms - 1) / sms) * length(ctas - 1));
         if (ctas > sms) end = fmax(end, length(sms - 1) + length(sms));
-        // with three CTAs and more on an SM the last ones do not fill the SMs evenly (20 units x L2048 causal 32.5 with one tile, 30.5 with two; 12 x L4096 60.9 / 55.7)
+        // with three CTAs and more on an SM the last ones do not fill the SMs evenly (20 units x L2048 causal 32.6 with one tile, 30.6 with two; 12 x L4096 61.0 / 54.7)
         if (ctas > 2 * sms) end = fmax(end, total / sms + 0.3 * total / ctas);
         return end;
     };

@@ -121,7 +121,11 @@ EMBER_API int ember_selftest_fail_scratch(int count);
  *      multiply src/tensor/operators.def:54, softmax ember/tensor/tensor.py:430-437
  *      (max_axis src/tensor/operators_gpu.cu:198-219, sum_axis :175-196).
  *      k is taken in its natural (batch_heads, lk, d) layout; no host transpose.
- *      lse may be NULL when the caller does not need it. ---- */
+ *      lse may be NULL when the caller does not need it.
+ *      Float32, here and in the backward: which kernel takes a call, and whether two CTAs share a block of rows, depends on
+ *      batch_heads, so a unit's results may be rounded differently in calls of different batch_heads (a slab of a sharded
+ *      batch, a chunk of ember_attention_fwd_host). The same call gives the same bits. The bf16
+ *      tensor-core kernels give a unit the same bits in any batch (dQ: see ember_set_deterministic). ---- */
 EMBER_API int ember_attention_fwd(const void *q, const void *k, const void *v, void *out, float *lse,
                         int batch_heads, int lq, int lk, int d, float scale, int causal, int dtype,
                         void *stream);
